@@ -56,6 +56,10 @@ SIGNATURES = {
                                             C.c_int, _vp]),
     "cerium_resolve2": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _sz, C.c_uint32, C.c_uint32, C.c_int, _vp]),
     "cerium_mod2": (C.c_int, [_vp, _vp, _sz, _vp, _vp, _u32p, C.c_int, _vp]),
+    "cerium_residues": (C.c_int, [_vp, _vp, _sz, _vp, _vp, _u32p, C.c_int, _vp]),
+    "cerium_compose_create": (C.c_int, [_vp, C.POINTER(_vp), _u32p, C.c_int]),
+    "cerium_compose_destroy": (C.c_int, [_vp]),
+    "cerium_compose_apply": (C.c_int, [_vp, _vp, _vp, _sz, _vp]),
     "cerium_bconv_create": (C.c_int, [_vp, C.POINTER(_vp), C.c_int, _u32p, C.c_int, _u32p, C.c_int]),
     "cerium_bconv_destroy": (C.c_int, [_vp]),
     "cerium_bconv_apply": (C.c_int, [_vp, _vp, _sz, _vp, _sz, _vp]),
@@ -252,6 +256,11 @@ class Context:
         n = self.n
         self.lib.check(self.lib.dll.cerium_automorph(self.h, out, n, inp, n, galois_elt, count, stream))
 
+    def residues(self, out: int, values: int, prime_idx: Sequence[int], small: int = 0, stream: int = 0):
+        """Residues of N integer-valued doubles (plus N small integers): coefficient-form limbs."""
+        self.lib.check(self.lib.dll.cerium_residues(self.h, out, self.n, values, small or None, _u32(prime_idx),
+                                                    len(prime_idx), stream))
+
     def resolve2(self, lo: int, hi: int, x0: int, x1: int, prime0: int, prime1: int, count: int = 1, stream: int = 0):
         self.lib.check(self.lib.dll.cerium_resolve2(self.h, lo, hi, x0, x1, self.n, prime0, prime1, count, stream))
 
@@ -447,6 +456,30 @@ class Program:
     def close(self):
         if getattr(self, "h", None) and self.ctx.h:
             self.ctx.lib.dll.cerium_program_destroy(self.h)
+        self.h = None
+
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
+
+
+class Composer:
+    """Exact CRT composition of coefficient-form limbs to centred doubles (handle of ``cerium_compose``)."""
+
+    def __init__(self, ctx: Context, prime_idx: Sequence[int]):
+        self.ctx = ctx
+        h = _vp()
+        ctx.lib.check(ctx.lib.dll.cerium_compose_create(ctx.h, C.byref(h), _u32(prime_idx), len(prime_idx)))
+        self.h = h
+
+    def apply(self, out: int, inp: int, stream: int = 0):
+        self.ctx.lib.check(self.ctx.lib.dll.cerium_compose_apply(self.h, out, inp, self.ctx.n, stream))
+
+    def close(self):
+        if getattr(self, "h", None) and self.ctx.h:
+            self.ctx.lib.dll.cerium_compose_destroy(self.h)
         self.h = None
 
     def __del__(self):

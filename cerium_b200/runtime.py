@@ -24,6 +24,7 @@ equivalent, not byte-identical.  One process drives one GPU; a function compiled
 from __future__ import annotations
 
 import os
+import threading
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -63,6 +64,7 @@ class Context:
             self.device = torch.device("cpu")
         self.handle = _capi.Context(self.lib, self.moduli, 32, device=device, logn=self.logn)
         self._q = torch.tensor(self.moduli, dtype=torch.int64, device=self.device)
+        self._composers: Dict[Tuple[int, ...], _capi.Composer] = {}
 
     @property
     def coeff_count(self) -> int:
@@ -98,20 +100,25 @@ class Context:
         t = self.torch.from_numpy(np.asarray(v, dtype=np.int64)).to(self.device)
         return t.view(1, -1) % self.q(idx)
 
-    def float_to_rns(self, c: np.ndarray, idx: Sequence[int]):
-        """Integer-valued doubles of any magnitude -> exact residues: c = M * 2^E with a 53-bit M."""
-        m, e = np.frexp(np.abs(c))
-        big = (m * 2.0 ** 53).astype(np.int64)
-        e = e.astype(np.int64) - 53
-        small = np.where(e < 0, big >> np.minimum(-e, 63), big)         # c is an integer: the shifted-out bits are zero
-        up = np.maximum(e, 0)
-        out = np.empty((len(idx), c.size), dtype=np.int64)
-        for k, p in enumerate(idx):
-            q = self.moduli[p]
-            pow2 = np.array([pow(2, int(s), q) for s in range(int(up.max()) + 1)], dtype=np.int64)
-            r = (small % q) * pow2[up] % q
-            out[k] = np.where(c < 0, (q - r) % q, r)
-        return self.torch.from_numpy(out).to(self.device)
+    def composer(self, idx: Sequence[int]) -> "_capi.Composer":
+        """CRT composition over these primes; the last few prime lists are kept."""
+        key = tuple(idx)
+        c = self._composers.pop(key, None) or _capi.Composer(self.handle, key)
+        self._composers[key] = c
+        while len(self._composers) > 8:
+            self._composers.pop(next(iter(self._composers)))
+        return c
+
+    def words_ntt(self, idx: Sequence[int], values=None, small=None):
+        """NTT form of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
+        on the device."""
+        t = self.torch
+        v = t.from_numpy(values).to(self.device) if values is not None else t.zeros(self.n, dtype=t.float64, device=self.device)
+        e = t.from_numpy(small).to(self.device) if small is not None else None
+        w = t.empty((len(idx), self.n), dtype=t.int32, device=self.device)
+        self.handle.residues(w.data_ptr(), v.data_ptr(), idx, small=e.data_ptr() if e is not None else 0, stream=self.stream())
+        self.handle.ntt_forward(w.data_ptr(), w.data_ptr(), idx, stream=self.stream())
+        return w
 
 
 class Ciphertext:
@@ -186,6 +193,7 @@ class CKKSEncryptorContext:
         self.secret_key_rns = context.ntt(context.signed_to_rns(sk, all_idx), all_idx)
         self.ephemeral_key_rns = context.ntt(context.signed_to_rns(ek, all_idx), all_idx)
         self.secret_key_squared_rns = self.secret_key_rns * self.secret_key_rns % context.q(all_idx)
+        self.secret_key_words = self.secret_key_rns.to(context.torch.int32)     # the form the kernels multiply with
 
 
 def _rng(seed):
@@ -202,64 +210,114 @@ class CKKSEncryptor:
         self.context = encryptor_context.context
         self.rng = _rng(prng_seed if prng_seed is not None else encryptor_context.seed)
         self.encoder = _Encoder(self.context.n)
+        self._stage: Dict[str, object] = {}
+
+    # -- staging ----------------------------------------------------------------------------------------
+    def _staging(self, name: str, rows: int):
+        """Page-locked host words [rows][n] (a plain array where the library computes in host memory), kept and grown
+        with this encryptor: copies to and from the device then run at the link's rate and beside the host's work."""
+        t = self._stage.get(name)
+        if t is None or t.shape[0] < rows:
+            torch = self.context.torch
+            t = torch.empty((rows, self.context.n), dtype=torch.int32, pin_memory=self.context.device.type == "cuda")
+            self._stage[name] = t
+        return t[:rows]
 
     # -- sampling ---------------------------------------------------------------------------------------
-    def _noise(self, idx):
-        """Centred binomial error, 21 coin pairs per coefficient (standard deviation 3.24), in NTT form."""
-        n = self.context.n
-        bits = self.rng.integers(0, 1 << 21, size=(2, n), dtype=np.int64)
-        pop = np.zeros((2, n), dtype=np.int64)
-        for b in range(21):
-            pop += (bits >> b) & 1
-        return self.context.ntt(self.context.signed_to_rns(pop[0] - pop[1], idx), idx)
+    def _noise(self) -> np.ndarray:
+        """Centred binomial error, 21 coin pairs per coefficient (standard deviation 3.24)."""
+        bits = self.rng.integers(0, 1 << 21, size=(2, self.context.n), dtype=np.uint32)
+        pop = np.bitwise_count(bits).astype(np.int32)
+        return pop[0] - pop[1]
 
     def _uniform(self, idx):
+        """Uniform residues, (host, device) words: the draws of one limb go up while the next limb's are made."""
         ctx = self.context
-        rows = [self.rng.integers(0, ctx.moduli[p], size=ctx.n, dtype=np.int64) for p in idx]
-        return ctx.torch.from_numpy(np.stack(rows)).to(ctx.device)
+        stage = self._staging("uniform", len(idx))
+        host = np.empty((len(idx), ctx.n), dtype=np.uint32)
+        dev = ctx.torch.empty((len(idx), ctx.n), dtype=ctx.torch.int32, device=ctx.device)
+        for k, p in enumerate(idx):
+            host[k] = self.rng.integers(0, ctx.moduli[p], size=ctx.n, dtype=np.uint32)
+            stage[k].numpy().view(np.uint32)[:] = host[k]
+            dev[k].copy_(stage[k], non_blocking=True)
+        return host, dev
+
+    def _encrypt(self, key_words, idx, message=None):
+        """(c0, c1) = (-(a s) + e + m, a) over the primes `idx`: device words of c0, host and device words of c1.
+        `key_words`: NTT form of the key on these primes, words; `message`: () -> integer-valued coefficients, or None."""
+        ctx = self.context
+        values = []
+        worker = None
+        if message is not None:                 # the encoder's FFT and the draws are independent host work
+            def work():
+                try:
+                    values.append(message())
+                except Exception:           # met again, and raised, by the caller below
+                    pass
+            worker = threading.Thread(target=work)
+            worker.start()
+        host1, dev1 = self._uniform(idx)
+        noise = self._noise()
+        if worker is not None:
+            worker.join()
+            if not values:
+                values.append(message())
+        c0 = ctx.words_ntt(idx, values[0] if values else None, noise)
+        prod = ctx.torch.empty_like(c0)
+        ew = ctx.handle.ewise
+        ew(_capi.EW_MUL, prod.data_ptr(), dev1.data_ptr(), idx, b=key_words.data_ptr(), stream=ctx.stream())
+        ew(_capi.EW_SUB, c0.data_ptr(), c0.data_ptr(), idx, b=prod.data_ptr(), stream=ctx.stream())
+        return c0, host1, dev1
 
     def encrypt_zero(self, key_rns, idx):
         """(c0, c1) = (-(a s) + e, a) over the primes `idx` under the key whose chain-wide NTT form is `key_rns`."""
         ctx = self.context
-        q = ctx.q(idx)
         sel = ctx.torch.tensor(list(idx), dtype=ctx.torch.int64, device=ctx.device)
-        c1 = self._uniform(idx)
-        c0 = (q - c1 * key_rns[sel] % q + self._noise(idx)) % q
-        return c0, c1
+        c0, _, c1 = self._encrypt(key_rns[sel].to(ctx.torch.int32), list(idx))
+        ctx._sync()                             # the staging rows are free for the next draws
+        return c0.to(ctx.torch.int64), c1.to(ctx.torch.int64)
 
     # -- messages ---------------------------------------------------------------------------------------
     def encode(self, message, scale: float, rns_base_ids: Sequence[int]):
         """Plaintext polynomial in NTT form on the given primes ([k][n] int64 tensor of residues)."""
-        ctx = self.context
-        return ctx.ntt(ctx.float_to_rns(self.encoder.encode(message, scale), rns_base_ids), rns_base_ids)
+        return self.context.words_ntt(list(rns_base_ids), self.encoder.encode(message, scale)).to(self.context.torch.int64)
+
+    def _key_rows(self, idx):
+        """Rows of the secret key for these primes: a view where they are consecutive."""
+        w = self.ectx.secret_key_words
+        if list(idx) == list(range(idx[0], idx[0] + len(idx))):
+            return w[idx[0]:idx[0] + len(idx)]
+        return w[self.context.torch.tensor(list(idx), dtype=self.context.torch.int64, device=self.context.device)]
 
     def encode_and_encrypt(self, message, scale: float, rns_base_ids: Sequence[int]) -> Ciphertext:
-        ctx = self.context
         idx = list(rns_base_ids)
-        c0, c1 = self.encrypt_zero(self.ectx.secret_key_rns, idx)
-        c0 = (c0 + self.encode(message, scale, idx)) % ctx.q(idx)
-        return Ciphertext(_words(c0), _words(c1), idx)
+        c0, host1, _ = self._encrypt(self._key_rows(idx), idx, lambda: self.encoder.encode(message, scale))
+        stage = self._staging("result", len(idx))
+        stage.copy_(c0, non_blocking=True)
+        self.context._sync()
+        return Ciphertext(stage.numpy().view(np.uint32).copy(), host1, idx)
 
     def decrypt_and_decode(self, ciphertext: Ciphertext, scale: float) -> np.ndarray:
         """Complex slot values of c0 + c1 s, composed over every limb of the ciphertext."""
-        ctx = self.context
+        ctx, t = self.context, self.context.torch
         idx = ciphertext.rns_base_ids
-        q = ctx.q(idx)
-        sel = ctx.torch.tensor(idx, dtype=ctx.torch.int64, device=ctx.device)
-        c0 = ctx.torch.from_numpy(ciphertext.c0.astype(np.int64)).to(ctx.device) % q
-        c1 = ctx.torch.from_numpy(ciphertext.c1.astype(np.int64)).to(ctx.device) % q
-        m = ctx.ntt((c0 + c1 * self.ectx.secret_key_rns[sel]) % q, idx, inverse=True).cpu().numpy()
-        mods = [ctx.moduli[p] for p in idx]
-        big_q = 1
-        for p in mods:
-            big_q *= p
-        vals = np.zeros(ctx.n, dtype=object)
-        for i, p in enumerate(mods):
-            qi = big_q // p
-            vals = vals + m[i].astype(object) * (qi * pow(qi, -1, p) % big_q)
-        vals = vals % big_q
-        centred = np.where(vals > big_q // 2, vals - big_q, vals)
-        return self.encoder.decode(centred.astype(np.float64), scale)
+        stage = self._staging("input", 2 * len(idx))
+        w = t.empty((2 * len(idx), ctx.n), dtype=t.int32, device=ctx.device)
+        for k, c in ((1, ciphertext.c1), (0, ciphertext.c0)):
+            half = slice(k * len(idx), (k + 1) * len(idx))
+            stage[half].numpy().view(np.uint32)[:] = c
+            w[half].copy_(stage[half], non_blocking=True)
+        m, a = w[:len(idx)], w[len(idx):]
+        ew, st = ctx.handle.ewise, ctx.stream()
+        ew(_capi.EW_REDUCE, w.data_ptr(), w.data_ptr(), idx + idx, stream=st)     # a program's outputs may exceed q
+        ew(_capi.EW_MAD, m.data_ptr(), a.data_ptr(), idx, b=self._key_rows(idx).data_ptr(), c=m.data_ptr(), stream=st)
+        ctx.handle.ntt_inverse(m.data_ptr(), m.data_ptr(), idx, stream=st)
+        centred = t.empty(ctx.n, dtype=t.float64, device=ctx.device)
+        ctx.composer(idx).apply(centred.data_ptr(), m.data_ptr(), st)
+        coeff = centred.cpu().numpy()
+        if np.isinf(coeff).any():
+            raise OverflowError("a composed coefficient passes the range of a double")
+        return self.encoder.decode(coeff, scale)
 
     # -- evaluation keys --------------------------------------------------------------------------------
     def key_rns_base_ids(self, level: int, extension_size: int) -> List[int]:
@@ -443,7 +501,7 @@ class _PlainEncoder:
             raise ValueError("values_size must be equal to context slots or elt_size")
         if z.size == ctx.slots and elt < ctx.slots:
             z = z[:elt]
-        full = ctx.ntt(ctx.float_to_rns(self.encoder.encode(z, scale), rns_base_ids), rns_base_ids)
+        full = ctx.words_ntt(list(rns_base_ids), self.encoder.encode(z, scale)).to(ctx.torch.int64)
         return full[:, ::ctx.slots // elt].contiguous()
 
 

@@ -64,6 +64,7 @@ extern "C" {
 
 typedef struct cerium_context cerium_context;
 typedef struct cerium_bconv cerium_bconv;
+typedef struct cerium_compose cerium_compose;
 typedef struct cerium_keyswitch cerium_keyswitch;
 typedef struct cerium_comm cerium_comm;
 typedef struct cerium_program cerium_program;
@@ -217,6 +218,23 @@ CERIUM_API int cerium_resolve2(cerium_context *ctx, void *lo, void *hi, const vo
                     size_t stride, uint32_t prime0, uint32_t prime1, int count, void *stream);
 CERIUM_API int cerium_mod2(cerium_context *ctx, void *out, size_t out_stride, const void *lo, const void *hi,
                 const uint32_t *prime_idx, int count, void *stream);
+
+/*
+ * Residues of integer-valued doubles: out[l] = (values + small) mod q_{prime_idx[l]}, coefficient form,
+ * canonical.  values is a DEVICE array of N integer-valued doubles of any magnitude, small (may be NULL) a
+ * DEVICE array of N integers added to them (encryption noise): the step of the reference's encoder from
+ * rounded coefficients to RNS limbs (cerium/runtime/io/ckks-encoder.h:205-372).
+ *
+ * cerium_compose_*: the decoder's way back (cerium/runtime/io/ckks-encoder.h:170-204).  For `count` (1..255)
+ * coefficient-form limbs, out[i] is the integer in (-Q/2, Q/2) with these residues, composed exactly and
+ * rounded once to the nearest double (infinite past the range of a double).  32-bit contexts; out is a
+ * DEVICE array of N doubles.  The handle holds the CRT tables of one prime list.
+ */
+CERIUM_API int cerium_residues(cerium_context *ctx, void *out, size_t out_stride, const double *values,
+                               const int32_t *small, const uint32_t *prime_idx, int count, void *stream);
+CERIUM_API int cerium_compose_create(cerium_context *ctx, cerium_compose **out, const uint32_t *prime_idx, int count);
+CERIUM_API int cerium_compose_destroy(cerium_compose *c);
+CERIUM_API int cerium_compose_apply(cerium_compose *c, double *out, const void *in, size_t in_stride, void *stream);
 
 /*
  * Base converter from the primes in_primes[0..n_in) to out_primes[0..n_out).
