@@ -3,6 +3,7 @@
 // arithmetic lives in the *_kernels.cuh headers.  Mirrors the role of
 // cerium/runtime/execution/evaluator.cpp (Evaluator::fn_*) and device_utils.cu (execute_*).
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -98,7 +99,7 @@ int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t strea
 }
 
 int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale, const void* scale_shoup,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, const void* add) {
   if (c.count == 0) return CERIUM_OK;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
@@ -119,6 +120,7 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale,
         sc.scale = static_cast<const W*>(scale) + first;
         sc.scale_shoup = static_cast<const W*>(scale_shoup) + first;
       }
+      if (add != nullptr) sc.add = static_cast<const W*>(add) + first;
       if (c.src_pos != nullptr) {
         // entry b reads limb src_pos[b] of `in` and writes limb pos[b] of `out`
         GatherBatch<W> gb{};
@@ -210,6 +212,8 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
           auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, ReduceLoader<W>>;
           CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, ld, tw, pcs);
         }
+      } else if (c.lazy_src) {
+        { auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, LazyLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, LazyLoader<W>{}, tw, pcs); }
       } else {
         { auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, PlainLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, PlainLoader<W>{}, tw, pcs); }
       }
@@ -318,85 +322,62 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
     }
     for (int j = 0; j < n_out; j++) out_sub[j] = half_mod(m[out_primes[j]]);
   }
-  // 64-bit words, at most 8 inputs: outputs may take their quotient from the FP64 pipe.  The estimate
-  // c ~ sum_i y_i f_i / p_j (f_i centred) is off by at most e = (I + 2) 2^-53 sum_i q_i |f_i| / p_j + 1/2
-  // (rounding of RN(f_i / p_j), of y_i as a double, of every partial sum; then rounding to an integer),
-  // so |sum - c p_j| <= e p_j: class 1 when that is below 3 p_j, class 2 when it is below 2^62.
-  bc->fp_in = bits == 64 && n_in <= kBconvRegInputs && ctx->allow_fp;
-  std::vector<uint8_t> fp_class(n_out, 0);
-  if (bc->fp_in) {
-    bool any = false;
-    for (int j = 0; j < n_out; j++) {
-      const uint64_t pj = m[out_primes[j]];
-      long double b = 0.0L;
-      for (int i = 0; i < n_in; i++) {
-        const uint64_t f = factors[(size_t)j * n_in + i];
-        const uint64_t mag = f > pj / 2 ? pj - f : f;
-        b += (long double)m[in_primes[i]] * (long double)mag / (long double)pj;
-      }
-      const long double e = (long double)(n_in + 2) * b * 0x1p-53L + 0.5L;
-      if (e < 2.9L) fp_class[j] = 1;
-      else if ((e + 1.0L) * (long double)pj < 0x1p62L) fp_class[j] = 2;
-      any = any || fp_class[j] != 0;
-    }
-    bc->fp_in = any;
-  }
+  bc->in_add_host = in_add;
   const bool use_inv = mode == CERIUM_BCONV_EXACT && !opt.prescaled && n_in > 1;
   Blob blob;
-  size_t o_fac = 0, o_inv = 0, o_invs = 0, o_add = 0, o_sub = 0;
+  size_t o_inv = 0, o_invs = 0;
   dispatch_word(bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    o_fac = blob.append_words<W>(factors);
     o_inv = blob.append_words<W>(inv);
     o_invs = blob.append_words<W>(inv_shoup);
-    o_add = blob.append_words<W>(in_add);
-    o_sub = blob.append_words<W>(out_sub);
     return 0;
   });
-  size_t o_outc = 0, o_split = 0, o_fpfac = 0;
-  const bool split = bits == 64 && n_in <= kBconvRegInputs;
+  size_t o_outc = 0, o_table = 0;
   dispatch_word(bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    std::vector<BconvOut<W>> outc(n_out);
+    // table entry of (output j, byte plane m, input i, byte k): byte m of factor[j][i] * 2^(8k) mod p_j, laid out as
+    // the fragments of an m16n8k32 product (bconv_mma.cuh)
+    bc->steps = (n_in * (int)sizeof(W) + 31) / 32;
+    if (sizeof(W) == 4 && bc->steps == 3) bc->steps = 4;  // kernels with fragments in registers come for 1, 2 and 4 steps
+    std::vector<uint4> table(bconv_mma_table_entries<W>(n_out, bc->steps), make_uint4(0, 0, 0, 0));
+    unsigned char* bytes = reinterpret_cast<unsigned char*>(table.data());
+    std::vector<BconvMmaOut<W>> outc(n_out);
     for (int j = 0; j < n_out; j++) {
-      const uint32_t pj = out_primes[j];
-      BconvOut<W>& o = outc[j];
+      const uint64_t q = m[out_primes[j]];
+      for (int i = 0; i < n_in; i++)
+        for (int k = 0; k < (int)sizeof(W); k++) {
+          const uint64_t g = host::mulmod(factors[(size_t)j * n_in + i], ((uint64_t)1 << (8 * k)) % q, q);
+          const int group = j / kMmaRows<W>, in_group = j % kMmaRows<W>, col = i * (int)sizeof(W) + k;
+          const bool pair = sizeof(W) == 8 || n_out - group * kMmaRows<W> <= 8;
+          for (int b = 0; b < (int)sizeof(W); b++) {
+            const int frag = pair ? b / 2 : b, row = pair ? in_group + 8 * (b & 1) : in_group;
+            const int step = col / 32, lane = (row % 8) * 4 + col % 16 / 4, reg = row / 8 + 2 * (col % 32 / 16);
+            const size_t entry = bconv_mma_entry<W>(group, bc->steps) + ((size_t)frag * bc->steps + step) * 32 + lane;
+            bytes[entry * 16 + reg * 4 + col % 4] = (unsigned char)(g >> (8 * b));
+          }
+        }
+      BconvMmaOut<W>& o = outc[j];
       std::memset(&o, 0, sizeof(o));
-      o.q = (W)m[pj];
-      o.q2 = (W)(2 * m[pj]);
-      o.mu_hi = (W)ctx->mu_hi[pj];
-      o.mu_lo = (W)ctx->mu_lo[pj];
-      o.sub = out_sub.empty() ? (W)0 : (W)out_sub[j];
+      o.nq = (W)0 - (W)q;
+      o.add = out_sub.empty() ? (W)0 : (W)(q - out_sub[j]);
       o.pos = opt.out_pos.empty() ? (uint32_t)j : opt.out_pos[j];
-      o.has_sub = out_sub.empty() ? 0 : 1;
-      o.strict = (ctx->lazy_ok[pj] && !ctx->fp_ok[pj]) ? 0 : 1;
-      o.fp = (split && bc->fp_in) ? fp_class[j] : 0;
-      const double qinv = 1.0 / (double)m[pj];
-      uint64_t qinv_bits;
-      std::memcpy(&qinv_bits, &qinv, 8);
-      o.fp_qinv = (W)qinv_bits;
+      o.cls = sizeof(W) == 4 || q >= ((uint64_t)1 << 48) ? kMmaWide : q >= ((uint64_t)1 << 40) ? kMmaNarrow : kMmaTiny;
+      bc->all_wide = bc->all_wide && o.cls == kMmaWide;
+      if (o.cls == kMmaTiny) {
+        o.mu = (W)host::shoup(1, q, 64);
+      } else if (o.cls == kMmaNarrow) {
+        uint64_t mu = 0;
+        while ((mu = (uint64_t)(((unsigned __int128)1 << (64 + o.shift)) / q)) < ((uint64_t)1 << 31)) o.shift++;
+        o.mu = (W)mu;
+      } else {
+        o.mu = (W)(((unsigned __int128)1 << (sizeof(W) == 8 ? 80 : 48)) / q);
+      }
     }
-    o_outc = blob.append(outc.data(), outc.size() * sizeof(BconvOut<W>));
+    o_outc = blob.append(outc.data(), outc.size() * sizeof(BconvMmaOut<W>));
+    o_table = blob.append(table.data(), table.size() * sizeof(uint4));
     return 0;
   });
-  if (split) {
-    std::vector<uint2> sf(factors.size());
-    std::vector<double2> ff(factors.size());
-    for (size_t k = 0; k < factors.size(); k++) {
-      const uint64_t f = factors[k], q = m[out_primes[k / n_in]];
-      sf[k] = make_uint2((uint32_t)f & 0x3fffffffu, (uint32_t)(f >> 30));
-      // centred factor (as the bit pattern of an int64) and its quotient by q rounded to a double
-      const long long fc = f > q / 2 ? -(long long)(q - f) : (long long)f;
-      double fbits;
-      std::memcpy(&fbits, &fc, 8);
-      ff[k] = make_double2(fbits, (double)((long double)fc / (long double)q));
-    }
-    o_split = blob.append(sf.data(), sf.size() * sizeof(uint2));
-    o_fpfac = blob.append(ff.data(), ff.size() * sizeof(double2));
-  }
   const size_t o_ip = blob.append(bc->in_primes.data(), bc->in_primes.size() * 4);
-  const size_t o_op = blob.append(bc->out_primes.data(), bc->out_primes.size() * 4);
-  const size_t o_pos = blob.append(opt.out_pos.data(), opt.out_pos.size() * 4);
   const size_t o_ipos = blob.append(opt.in_pos.data(), opt.in_pos.size() * 4);
   if (cudaMalloc(&bc->d_block, blob.bytes.size() + 16) != cudaSuccess) {
     delete bc;
@@ -408,96 +389,105 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
     return fail(CERIUM_ERR_CUDA, "bconv_create: upload failed");
   }
   char* base = static_cast<char*>(bc->d_block);
-  bc->d_factors = base + o_fac;
   bc->d_outc = base + o_outc;
-  bc->d_split_fac = split ? base + o_split : nullptr;
-  bc->d_fp_fac = (split && bc->fp_in) ? base + o_fpfac : nullptr;
+  bc->d_table = base + o_table;
   bc->d_inv = use_inv ? base + o_inv : nullptr;
   bc->d_inv_shoup = use_inv ? base + o_invs : nullptr;
-  bc->d_in_add = in_add.empty() ? nullptr : base + o_add;
-  bc->d_out_sub = out_sub.empty() ? nullptr : base + o_sub;
   bc->d_in_prime = reinterpret_cast<uint32_t*>(base + o_ip);
-  bc->d_out_prime = reinterpret_cast<uint32_t*>(base + o_op);
-  bc->d_out_pos = opt.out_pos.empty() ? nullptr : reinterpret_cast<uint32_t*>(base + o_pos);
   bc->d_in_pos = opt.in_pos.empty() ? nullptr : reinterpret_cast<uint32_t*>(base + o_ipos);
   *out = bc;
   return CERIUM_OK;
 }
 
-int launch_bconv(cerium_context* ctx, const BconvCall* calls, int count, cudaStream_t stream) {
-  if (count == 0) return CERIUM_OK;
-  return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
-    using W = decltype(tag);
-    static bool smem_opt_in[kMaxDevices][2] = {};  // the attribute is per device
-    for (int first = 0; first < count; first += kBconvMaxBatch) {
-      const int cnt = std::min(kBconvMaxBatch, count - first);
-      BconvBatch<W> batch{};
-      size_t smem = 0;
-      int max_o = 1;
-      bool pair = sizeof(W) == 4;  // two coefficients per thread (see bconv_body_pair32)
-      for (int k = 0; k < cnt; k++) {
-        const BconvCall& c = calls[first + k];
-        const cerium_bconv* bc = c.bc;
-        BconvDesc<W>& d = batch.d[k];
-        d.in = static_cast<const W*>(c.in);
-        d.out = static_cast<W*>(c.out);
-        d.in_stride = c.in_stride;
-        d.out_stride = c.out_stride;
-        d.factors = static_cast<const W*>(bc->d_factors);
-        d.inv = static_cast<const W*>(bc->d_inv);
-        d.inv_shoup = static_cast<const W*>(bc->d_inv_shoup);
-        d.in_add = static_cast<const W*>(bc->d_in_add);
-        d.out_sub = static_cast<const W*>(bc->d_out_sub);
-        d.in_prime = bc->d_in_prime;
-        d.out_prime = bc->d_out_prime;
-        d.out_pos = bc->d_out_pos;
-        d.in_pos = bc->d_in_pos;
-        d.outc = static_cast<const BconvOut<W>*>(bc->d_outc);
-        d.split_fac = static_cast<const uint2*>(bc->d_split_fac);
-        d.fp_fac = static_cast<const double2*>(bc->d_fp_fac);
-        d.lazy_out = bc->lazy_out ? 1 : 0;
-        d.fp_in = bc->fp_in ? 1 : 0;
-        d.I = bc->I;
-        d.O = bc->O;
-        smem = std::max(smem, bconv_smem_bytes<W>(bc->I, bc->O));
-        max_o = std::max(max_o, bc->O);
-        pair = pair && bc->I <= kBconvRegInputs && ((uintptr_t)c.in | (uintptr_t)c.out) % 8 == 0 &&
-               (c.in_stride * sizeof(W)) % 8 == 0 && (c.out_stride * sizeof(W)) % 8 == 0;
-      }
-      if (smem > 48 * 1024) {
-        if (smem > 200 * 1024) return fail(CERIUM_ERR_UNSUPPORTED, "bconv: conversion needs more than 200 KiB of shared memory");
-        const int slot = sizeof(W) == 4 ? 0 : 1;
-        const int dev = ctx->device;
-        if (dev < 0 || dev >= kMaxDevices || !smem_opt_in[dev][slot]) {
-          CERIUM_CUDA(cudaFuncSetAttribute(bconv_kernel<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-          CERIUM_CUDA(cudaFuncSetAttribute(bconv_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-          if (dev >= 0 && dev < kMaxDevices) smem_opt_in[dev][slot] = true;
-        }
-      }
-      {
-        // grid.z splits the outputs of a conversion over nz CTAs (each reloads the inputs and restages its
-        // tables): take the nz in 1..4 with the best waves x per-CTA-work estimate on this GPU
-        auto kfn = pair ? bconv_kernel<W, true> : bconv_kernel<W, false>;
-        const int blocks = pair ? (kBconvBlocks + 1) / 2 : kBconvBlocks;
-        const int slots = 5 * ctx->sm_count;
-        int nz = 1;
-        double best = 1e30;
-        for (int cand = 1; cand <= std::min(4, (max_o + 3) / 4); cand++) {
-          const int ctas = blocks * cnt * cand;
-          const double cost = (double)((ctas + slots - 1) / slots) * (1.0 / cand + 0.15);
-          if (cost < best - 1e-9) {
-            best = cost;
-            nz = cand;
-          }
-        }
-        const int out_chunk = (max_o + nz - 1) / nz;
-        CERIUM_LAUNCH(kfn, dim3(blocks, cnt, (max_o + out_chunk - 1) / out_chunk), kBconvThreads, smem, stream,
-                      batch, out_chunk, static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+// Kernel of a batch: fragments in registers up to the number of steps they fit for, then the way outputs are finished.
+template <typename W, bool kPrepare>
+static auto bconv_mma_pick(int steps, int finish) -> decltype(&bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>) {
+  if constexpr (sizeof(W) == 8) {
+    if (finish == kMmaBig) return bconv_mma_kernel<W, 0, kMmaBig, kPrepare>;
+    if (finish <= kMmaLazyAdd && !kPrepare) {
+      const bool add = finish == kMmaLazyAdd;
+      if (steps == 1) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false> : bconv_mma_kernel<W, 1, kMmaLazy, false>;
+      if (steps == 2) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false> : bconv_mma_kernel<W, 2, kMmaLazy, false>;
+    }
+    if (steps == 1) return bconv_mma_kernel<W, 1, kMmaGeneral, kPrepare>;
+    if (steps == 2) return bconv_mma_kernel<W, 2, kMmaGeneral, kPrepare>;
+  } else {
+    if (finish <= kMmaLazyAdd && !kPrepare) {
+      const bool add = finish == kMmaLazyAdd;
+      if (steps == 1) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false> : bconv_mma_kernel<W, 1, kMmaLazy, false>;
+      if (steps == 2) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false> : bconv_mma_kernel<W, 2, kMmaLazy, false>;
+      if (steps == 4) return add ? bconv_mma_kernel<W, 4, kMmaLazyAdd, false> : bconv_mma_kernel<W, 4, kMmaLazy, false>;
+    }
+    if (steps == 1) return bconv_mma_kernel<W, 1, kMmaGeneral, kPrepare>;
+    if (steps == 2) return bconv_mma_kernel<W, 2, kMmaGeneral, kPrepare>;
+    if (steps == 4) return bconv_mma_kernel<W, 4, kMmaGeneral, kPrepare>;
+  }
+  return bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>;
+}
+
+template <typename W>
+static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int count, cudaStream_t stream) {
+  for (int first = 0; first < count;) {
+    // conversions of one launch share the number of steps (which is how they come: the digits of a key switch)
+    BconvMmaBatch<W> batch{};
+    const int steps = calls[first].bc->steps;
+    bool lazy = true, prepare = false, add = false;
+    int cnt = 0, max_groups = 1, max_i = 1;
+    for (; cnt < kMmaMaxBatch && first + cnt < count && calls[first + cnt].bc->steps == steps; cnt++) {
+      const BconvCall& c = calls[first + cnt];
+      const cerium_bconv* bc = c.bc;
+      BconvMmaDesc<W>& d = batch.d[cnt];
+      d.in = static_cast<const W*>(c.in);
+      d.out = static_cast<W*>(c.out);
+      d.in_stride = c.in_stride;
+      d.out_stride = c.out_stride;
+      d.inv = static_cast<const W*>(bc->d_inv);
+      d.inv_shoup = static_cast<const W*>(bc->d_inv_shoup);
+      d.in_prime = bc->d_in_prime;
+      d.in_pos = bc->d_in_pos;
+      d.table = static_cast<const uint4*>(bc->d_table);
+      d.outc = static_cast<const BconvMmaOut<W>*>(bc->d_outc);
+      d.I = bc->I;
+      d.O = bc->O;
+      d.steps = steps;
+      lazy = lazy && bc->lazy_out && bc->all_wide;
+      prepare = prepare || bc->d_inv != nullptr;
+      add = add || !bc->in_add_host.empty();
+      max_i = std::max(max_i, bc->I);
+      max_groups = std::max(max_groups, bconv_mma_groups<W>(bc->O));
+    }
+    const int finish = sizeof(W) == 8 && max_i > kMmaPairInputs ? kMmaBig : !lazy ? kMmaGeneral : add ? kMmaLazyAdd : kMmaLazy;
+    auto kfn = prepare ? bconv_mma_pick<W, true>(steps, finish) : bconv_mma_pick<W, false>(steps, finish);
+    // A warp per group of outputs, at most 8 to a CTA.  Stages of a CTA: a long walk spreads what a CTA does first
+    // (fragments, constants, filling the buffers: worth about two stages), whole rounds of CTAs keep the SMs
+    // busy to the end; an SM holds 24 warps of 80 registers a thread, 16 of the kernels that take 128.
+    const int slices = (max_groups + kMmaMaxWarps - 1) / kMmaMaxWarps, warps = (max_groups + slices - 1) / slices;
+    const size_t smem = bconv_mma_smem_bytes<W>(max_i);
+    const bool wide_regs = prepare || (sizeof(W) == 4 && steps == 4);
+    const int resident = std::max(1, std::min((wide_regs ? 16 : 25) / warps, (int)(220 * 1024 / (smem + 1024))));
+    constexpr int kStages = kN / kMmaStage;
+    int stages = 1;
+    double best = 1e30;
+    for (int t = 1; t <= 32; t++) {
+      const double ctas = (double)((kStages + t - 1) / t) * slices * cnt;
+      const double cost = std::ceil(ctas / ((double)resident * ctx->sm_count)) * (t + 2);
+      if (cost < best) {
+        best = cost;
+        stages = t;
       }
     }
-    CERIUM_LAUNCH_CHECK("bconv");
-    return CERIUM_OK;
-  });
+    if (smem > 48 * 1024) CERIUM_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CERIUM_LAUNCH(kfn, dim3((kStages + stages - 1) / stages, cnt, slices), 32 * warps, smem, stream, batch, stages,
+                  static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+    first += cnt;
+  }
+  CERIUM_LAUNCH_CHECK("bconv");
+  return CERIUM_OK;
+}
+
+int launch_bconv(cerium_context* ctx, const BconvCall* calls, int count, cudaStream_t stream) {
+  if (count == 0) return CERIUM_OK;
+  return dispatch_word(ctx->word_bits, [&](auto tag) -> int { return launch_bconv_words<decltype(tag)>(ctx, calls, count, stream); });
 }
 
 }  // namespace cerium
@@ -792,10 +782,8 @@ int cerium_bconv_ptrs(cerium_context* ctx, void* const* outs, const size_t* n_ou
     using W = decltype(tag);
     static bool smem_opt_in[kMaxDevices][2] = {};  // the attribute is per device
     // the shapes live on the device: size the shared memory for the caller's bounds (inputs staged per
-    // thread when there are more than kBconvRegInputs of them); smaller shapes inside the bounds may need
-    // more than the bound shape itself (the double-precision factor pairs of up to 8 inputs)
-    size_t smem = bconv_smem_bytes<W>((int)max_in, (int)max_out);
-    smem = std::max(smem, bconv_smem_bytes<W>((int)std::min<size_t>(max_in, kBconvRegInputs), (int)max_out));
+    // thread when there are more than kBconvRegInputs of them)
+    const size_t smem = bconv_smem_bytes<W>((int)max_in, (int)max_out);
     if (smem > 200 * 1024) return fail(CERIUM_ERR_UNSUPPORTED, "bconv_ptrs: conversion needs more than 200 KiB of shared memory");
     if (smem > 48 * 1024) {
       const int slot = sizeof(W) == 4 ? 0 : 1;

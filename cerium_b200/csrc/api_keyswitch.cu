@@ -49,8 +49,10 @@ struct cerium_keyswitch {
     cerium_bconv* down = nullptr;
     std::vector<uint64_t> pinv;              // [L - r]
     std::vector<uint32_t> ext_pos, ext_prime;  // both accumulators: slots [L - r, LK) of each
+    void* d_block = nullptr;                 // what the next three point into
     void* d_scale = nullptr;                 // exact mode: per entry of ext_pos, then the Shoup companions
     void* d_scale_shoup = nullptr;
+    void* d_add = nullptr;                   // rounding term of the same entries, or null
   };
   std::vector<FusedDown> fused;
   // transform batches
@@ -69,6 +71,7 @@ struct cerium_keyswitch {
   void* d_scale_q_shoup = nullptr;
   void* d_scale_p = nullptr;
   void* d_scale_p_shoup = nullptr;
+  void* d_add_p = nullptr;  // [2K] rounding term of the ModDown, added by the inverse transform, or null
   // workspace
   void* ws = nullptr;
   size_t ws_bytes = 0;
@@ -291,7 +294,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       // 5. iNTT of the extension limbs and the dropped Q limbs of both accumulators, in place
       {
         NttCall c{acc, acc, n, n, fd.ext_pos.data(), fd.ext_prime.data(), (int)fd.ext_pos.size()};
-        if (int rc = launch_ntt_inverse(ctx, c, fd.d_scale, fd.d_scale_shoup, stream)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, fd.d_scale, fd.d_scale_shoup, stream, fd.d_add)) return rc;
       }
       // 6. base conversion (dropped Q limbs, P) -> remaining Q limbs
       {
@@ -312,6 +315,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
         SudCall s{};
         s.src = conv + (size_t)p * Lr * n;
         s.src_stride = n;
+        s.lazy_src = true;
         s.work = conv + (size_t)p * Lr * n;
         s.work_stride = n;
         s.dst = p == 0 ? out0 : out1;
@@ -336,7 +340,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       if (!ks->ext_split) {
         // 5. iNTT of the extension limbs of both accumulators, in place
         NttCall c{acc, acc, n, n, ks->ext_pos.data(), ks->ext_prime.data(), 2 * K};
-        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream, ks->d_add_p)) return rc;
       } else {
         // 5. iNTT of the LOCAL extension limbs into this rank's block of the gather buffer
         //    ([world][2][pgather_limbs]), then the all-gather: every rank needs all K limbs to convert
@@ -345,7 +349,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
         W* mine = pg + (size_t)ks->rank * block;
         NttCall c{acc, mine, n, n, ks->ext_dst.data(), ks->ext_prime.data(), 2 * K};
         c.src_pos = ks->ext_pos.data();
-        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream, ks->d_add_p)) return rc;
         if (int rc = comm_allgather(comm, pg, mine, block * sizeof(W), stream)) return rc;
         p0 = pg;
         p1 = pg + (size_t)ks->pgather_limbs * n;
@@ -369,6 +373,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       SudCall s{};
       s.src = conv;
       s.src_stride = n;
+      s.lazy_src = true;
       s.work = conv;
       s.work_stride = n;
       s.dst = out0;
@@ -392,6 +397,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
         SudCall s{};
         s.src = conv + (size_t)p * L * n;
         s.src_stride = n;
+        s.lazy_src = true;
         s.work = conv + (size_t)p * L * n;
         s.work_stride = n;
         s.dst = p == 0 ? out0 : out1;
@@ -576,6 +582,7 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
     BconvOptions opt;
     opt.prescaled = exact;
     opt.round_half = round_mode == CERIUM_ROUND_HALF;
+    opt.lazy_out = true;  // the SuD's transform takes values below 4q
     if (ks->ext_split) {
       std::vector<int> seen(world, 0);
       for (int k = 0; k < Kg; k++) {
@@ -594,6 +601,16 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
       for (int i = 0; i < Kg; i++)
         if (i != k) prod = host::mulmod(prod, ctx->moduli[p_idx[i]] % pk, pk);
       scale_p[j] = scale_p[Kl + j] = Kg > 1 ? host::invmod(prod, pk) : 1;
+    }
+  }
+  // rounding term of the ModDown on this rank's extension limbs: floor(P / 2) modulo p_k, scaled as the limb is
+  std::vector<uint64_t> add_p(std::max(Kl, 1), 0);
+  if (rc == CERIUM_OK && round_mode == CERIUM_ROUND_HALF) {
+    const std::vector<uint32_t> p_all(p_idx, p_idx + Kg);
+    for (int j = 0; j < Kl; j++) {
+      const uint64_t pk = ctx->moduli[ks->p_idx[j]];
+      const uint64_t pm1 = (host::product_mod(ctx->moduli, p_all, pk) + pk - 1) % pk;
+      add_p[j] = host::mulmod(host::mulmod(pm1, host::invmod(2, pk), pk), exact ? scale_p[j] : 1, pk);
     }
   }
   if (rc != CERIUM_OK) {
@@ -621,6 +638,15 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
   }
   const size_t wb = ctx->word_bytes();
   const size_t n = kN;
+  auto upload = [&](const std::vector<uint64_t>& v, void** dst) {
+    std::vector<char> bytes(v.size() * wb);
+    for (size_t i = 0; i < v.size(); i++) {
+      if (bits == 32) reinterpret_cast<uint32_t*>(bytes.data())[i] = (uint32_t)v[i];
+      else reinterpret_cast<uint64_t*>(bytes.data())[i] = v[i];
+    }
+    return cudaMalloc(dst, bytes.size()) == cudaSuccess &&
+           cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+  };
   // ModDown with rescale levels folded in (one-GPU plans only)
   for (int r = 1; r <= 2 && world == 1 && !lifted && L - r >= 1; r++) {
     cerium_keyswitch::FusedDown fd;
@@ -631,6 +657,7 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
     BconvOptions opt;
     opt.prescaled = exact;
     opt.round_half = round_mode == CERIUM_ROUND_HALF;
+    opt.lazy_out = true;  // the SuD's transform takes values below 4q
     if (create_bconv(ctx, &fd.down, bconv_mode, e_idx.data(), E, ks->q_idx.data(), Lr, opt) != CERIUM_OK) {
       // a shape the converter cannot take (sum of products too wide): the plan simply has no fused variant
       fd.down = nullptr;
@@ -642,7 +669,7 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
       const uint64_t q = ctx->moduli[ks->q_idx[i]];
       fd.pinv[i] = host::invmod(host::product_mod(ctx->moduli, e_idx, q), q);
     }
-    std::vector<uint64_t> sc, scs;
+    std::vector<uint64_t> sc, scs, add;
     for (int p = 0; p < 2; p++)
       for (int k = 0; k < E; k++) {
         fd.ext_pos.push_back((uint32_t)(p * LK + Lr + k));
@@ -650,47 +677,55 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
         const uint64_t ek = ctx->moduli[e_idx[k]];
         sc.push_back(exact ? fd.down->inv_host[k] : 1);
         scs.push_back(host::shoup(sc.back(), ek, bits));
+        if (opt.round_half) add.push_back(fd.down->in_add_host[k]);
       }
+    std::vector<uint64_t> all;
     if (exact) {
-      std::vector<char> bytes(2 * sc.size() * wb);
-      for (size_t i = 0; i < 2 * sc.size(); i++) {
-        const uint64_t v = i < sc.size() ? sc[i] : scs[i - sc.size()];
-        if (bits == 32) reinterpret_cast<uint32_t*>(bytes.data())[i] = (uint32_t)v;
-        else reinterpret_cast<uint64_t*>(bytes.data())[i] = v;
-      }
-      if (cudaMalloc(&fd.d_scale, bytes.size()) != cudaSuccess ||
-          cudaMemcpy(fd.d_scale, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      all = sc;
+      all.insert(all.end(), scs.begin(), scs.end());
+    }
+    const size_t o_add = all.size() * wb;
+    all.insert(all.end(), add.begin(), add.end());
+    if (!all.empty()) {
+      if (!upload(all, &fd.d_block)) {
         cerium_bconv_destroy(fd.down);
         cerium_keyswitch_destroy(ks);
         return fail(CERIUM_ERR_CUDA, "keyswitch_create: scale upload failed");
       }
-      fd.d_scale_shoup = static_cast<char*>(fd.d_scale) + sc.size() * wb;
+      if (exact) {
+        fd.d_scale = fd.d_block;
+        fd.d_scale_shoup = static_cast<char*>(fd.d_block) + sc.size() * wb;
+      }
+      if (opt.round_half) fd.d_add = static_cast<char*>(fd.d_block) + o_add;
     }
     ks->fused.push_back(fd);
   }
-  if (exact) {
-    // [scale_q | scale_q_shoup | scale_p | scale_p_shoup]
+  {
+    // [scale_q | scale_q_shoup | scale_p | scale_p_shoup] (exact mode) [rounding term of the extension limbs]
     std::vector<uint64_t> all;
-    for (int i = 0; i < L; i++) all.push_back(scale_q[i]);
-    for (int i = 0; i < L; i++) all.push_back(host::shoup(scale_q[i], ctx->moduli[ks->q_idx[i]], bits));
-    for (int i = 0; i < 2 * Kl; i++) all.push_back(scale_p[i]);
-    for (int i = 0; i < 2 * Kl; i++) all.push_back(host::shoup(scale_p[i], ctx->moduli[ks->p_idx[i % Kl]], bits));
-    if (all.empty()) all.push_back(0);
-    std::vector<char> bytes(all.size() * wb);
-    for (size_t i = 0; i < all.size(); i++) {
-      if (bits == 32) reinterpret_cast<uint32_t*>(bytes.data())[i] = (uint32_t)all[i];
-      else reinterpret_cast<uint64_t*>(bytes.data())[i] = all[i];
+    if (exact) {
+      for (int i = 0; i < L; i++) all.push_back(scale_q[i]);
+      for (int i = 0; i < L; i++) all.push_back(host::shoup(scale_q[i], ctx->moduli[ks->q_idx[i]], bits));
+      for (int i = 0; i < 2 * Kl; i++) all.push_back(scale_p[i]);
+      for (int i = 0; i < 2 * Kl; i++) all.push_back(host::shoup(scale_p[i], ctx->moduli[ks->p_idx[i % Kl]], bits));
     }
-    if (cudaMalloc(&ks->d_scale, bytes.size()) != cudaSuccess ||
-        cudaMemcpy(ks->d_scale, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-      cerium_keyswitch_destroy(ks);
-      return fail(CERIUM_ERR_CUDA, "keyswitch_create: scale upload failed");
+    const size_t o_add = all.size() * wb;
+    if (round_mode == CERIUM_ROUND_HALF)
+      for (int i = 0; i < 2 * Kl; i++) all.push_back(add_p[i % Kl]);
+    if (!all.empty()) {
+      if (!upload(all, &ks->d_scale)) {
+        cerium_keyswitch_destroy(ks);
+        return fail(CERIUM_ERR_CUDA, "keyswitch_create: scale upload failed");
+      }
+      char* b = static_cast<char*>(ks->d_scale);
+      if (exact) {
+        ks->d_scale_q = b;
+        ks->d_scale_q_shoup = b + (size_t)L * wb;
+        ks->d_scale_p = b + (size_t)2 * L * wb;
+        ks->d_scale_p_shoup = b + (size_t)(2 * L + 2 * Kl) * wb;
+      }
+      if (round_mode == CERIUM_ROUND_HALF && Kl > 0) ks->d_add_p = b + o_add;
     }
-    char* b = static_cast<char*>(ks->d_scale);
-    ks->d_scale_q = b;
-    ks->d_scale_q_shoup = b + (size_t)L * wb;
-    ks->d_scale_p = b + (size_t)2 * L * wb;
-    ks->d_scale_p_shoup = b + (size_t)(2 * L + 2 * Kl) * wb;
   }
   // workspace layout (in words)
   size_t off = 0;
@@ -897,7 +932,7 @@ int cerium_keyswitch_destroy(cerium_keyswitch* ks) {
   if (ks->down) cerium_bconv_destroy(ks->down);
   for (auto& fd : ks->fused) {
     if (fd.down) cerium_bconv_destroy(fd.down);
-    cudaFree(fd.d_scale);
+    cudaFree(fd.d_block);
   }
   cudaFree(ks->d_scale);
   cudaFree(ks->ws);

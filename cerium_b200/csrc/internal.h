@@ -15,6 +15,7 @@
 
 #include "../../include/cerium_b200.h"
 #include "bconv_kernels.cuh"
+#include "bconv_mma.cuh"
 #include "bsgs_kernels.cuh"
 #include "ewise_kernels.cuh"
 #include "host_math.h"
@@ -119,21 +120,18 @@ struct cerium_bconv {
   std::vector<uint32_t> in_primes, out_primes;
   // one device allocation holding every table below
   void* d_block = nullptr;
-  void* d_factors = nullptr;    // W[O][I]
-  void* d_outc = nullptr;       // BconvOut<W>[O]
-  void* d_split_fac = nullptr;  // uint2[O][I] (64-bit words, at most 8 inputs)
-  void* d_fp_fac = nullptr;     // double2[O][I] (when fp_in)
+  int steps = 0;                // steps of 32 input bytes of the products
+  bool all_wide = true;         // every output prime is in the quotient class of the lazy kernel
+  void* d_table = nullptr;      // fragments of the tensor cores (bconv_mma.cuh)
+  void* d_outc = nullptr;       // BconvMmaOut<W>[O]
   void* d_inv = nullptr;        // W[I] (exact mode, unless the caller pre-scales)
   void* d_inv_shoup = nullptr;  // W[I]
-  void* d_in_add = nullptr;     // W[I]  rounding term, or null
-  void* d_out_sub = nullptr;    // W[O]  rounding term, or null
   uint32_t* d_in_prime = nullptr;
-  uint32_t* d_out_prime = nullptr;
-  uint32_t* d_out_pos = nullptr;  // or null
   uint32_t* d_in_pos = nullptr;   // or null
+  // rounding (round_half): what the caller adds to the inputs, modulo q_i, before they are converted
+  std::vector<uint64_t> in_add_host;
   bool lazy_out = false;
   std::vector<uint64_t> inv_host;  // [Qhat_i^-1]_{q_i}
-  bool fp_in = false;              // some outputs take their quotient from the FP64 pipe (d_fp_fac is present)
 };
 
 // Communicator of the limb collectives: the ranks of one job, one GPU each.  The transport is NCCL
@@ -163,7 +161,7 @@ int comm_subgroup(cerium_comm* comm, int size, cerium_comm** out);
 // Options of create_bconv beyond the public entry point.
 struct BconvOptions {
   bool prescaled = false;            // exact mode, inputs already multiplied by [Qhat_i^-1]
-  bool round_half = false;           // add floor(prod_in/2) to inputs, subtract it from outputs
+  bool round_half = false;           // the inputs come with floor(prod_in/2) added (in_add_host): subtract it from outputs
   std::vector<uint32_t> out_pos;     // output limb slots (empty = 0..O-1)
   std::vector<uint32_t> in_pos;      // input limb slots (empty = 0..I-1)
   bool lazy_out = false;             // outputs feed the forward NTT directly: skip the final corrections
@@ -203,9 +201,9 @@ struct NttCall {
 };
 // lazy_out: leave the results below 4q instead of canonical (internal buffers read by the inner product only)
 int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t stream, bool lazy_out = false);
-// scale / scale_shoup: device arrays with one word per batch entry, or null.
+// scale / scale_shoup / add: device arrays with one word per batch entry, or null: results * scale + add.
 int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale, const void* scale_shoup,
-                       cudaStream_t stream);
+                       cudaStream_t stream, const void* add = nullptr);
 
 // SuD over `count` limbs (count <= kSudMaxBatch per launch; chunked internally).
 struct SudCall {
@@ -228,6 +226,7 @@ struct SudCall {
   void* dst2 = nullptr;
   const void* minuend2 = nullptr;
   const void* addend2 = nullptr;
+  bool lazy_src = false;  // the source words are below 4q instead of canonical
   // source re-reduction (only when reduce_src): residues of modulus src_q, optional rounding
   bool reduce_src = false;
   uint64_t src_q = 0;

@@ -906,6 +906,7 @@ template <typename W>
 struct InvScale {
   const W* scale;        // per batch entry, may be null
   const W* scale_shoup;  // per batch entry
+  const W* add;          // per batch entry, added to the scaled value modulo q (rounding term), may be null
 };
 
 template <typename W, int kMode, typename Batch>
@@ -940,6 +941,11 @@ __device__ __forceinline__ void ntt_inv_cols_body(const Batch& batch, const InvS
     const W s = __ldg(sc.scale + b), ss = __ldg(sc.scale_shoup + b);
 #pragma unroll
     for (int j = 0; j < 16; j++) x[j] = csub<W>(mul_shoup_lazy<W>(x[j], s, ss, q), q);
+  }
+  if (sc.add != nullptr) {
+    const W a = __ldg(sc.add + b);
+#pragma unroll
+    for (int j = 0; j < 16; j++) x[j] = add_mod<W>(x[j], a, q);
   }
 #pragma unroll
   for (int j = 0; j < 16; j++) buf_strided[j * 16 * 256] = x[j];
