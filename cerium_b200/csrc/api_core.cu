@@ -98,8 +98,22 @@ int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t strea
   });
 }
 
-int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale, const void* scale_shoup,
-                       cudaStream_t stream, const void* add) {
+void inverse_last_words(const cerium_context* ctx, int k, uint64_t scale, uint64_t (&out)[4]) {
+  const uint64_t q = ctx->moduli[k];
+  for (int h = 0; h < 2; h++) {
+    const uint64_t w = host::mulmod(h == 0 ? ctx->ninv[k] : ctx->w1ninv[k], scale % q, q);
+    if (ctx->fp_ok[k]) {
+      const double wd = host::centred(w, q), wq = wd / (double)q;
+      std::memcpy(&out[2 * h], &wd, 8);
+      std::memcpy(&out[2 * h + 1], &wq, 8);
+    } else {
+      out[2 * h] = w;
+      out[2 * h + 1] = host::shoup(w, q, ctx->word_bits);
+    }
+  }
+}
+
+int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t stream, const void* last, const void* add) {
   if (c.count == 0) return CERIUM_OK;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
@@ -116,10 +130,7 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale,
       sb.in_elt = c.in_galois;
       if (int rc = fill_batch<W>(ctx, sb, c.pos, c.prime, first, cnt)) return rc;
       InvScale<W> sc{};
-      if (scale != nullptr) {
-        sc.scale = static_cast<const W*>(scale) + first;
-        sc.scale_shoup = static_cast<const W*>(scale_shoup) + first;
-      }
+      if (last != nullptr) sc.last = static_cast<const W*>(last) + 4 * (size_t)first;
       if (add != nullptr) sc.add = static_cast<const W*>(add) + first;
       if (c.src_pos != nullptr) {
         // entry b reads limb src_pos[b] of `in` and writes limb pos[b] of `out`
@@ -551,7 +562,7 @@ int cerium_context_create(cerium_context** out, int device, int log_n, int word_
       // twiddle and its correctly rounded quotient by q instead of the twiddle and its Shoup word
       const bool fp = word_bits == 64 && q < ((uint64_t)1 << 50) && ctx->allow_fp;
       auto fp_pair = [&](uint64_t w) {
-        const double wd = w > q / 2 ? -(double)(q - w) : (double)w;
+        const double wd = host::centred(w, q);
         const double wq = wd / (double)q;
         uint64_t a, b;
         std::memcpy(&a, &wd, 8);
@@ -607,6 +618,8 @@ int cerium_context_create(cerium_context** out, int device, int log_n, int word_
       ctx->mu_lo.push_back(t.mu_lo);
       ctx->lazy_ok.push_back(pc.lazy_ok != 0 ? 1 : 0);
       ctx->fp_ok.push_back(fp ? 1 : 0);
+      ctx->ninv.push_back(t.ninv);
+      ctx->w1ninv.push_back(w1);
       if (fp) {
         const double qinv = 1.0 / (double)q;
         uint64_t bits;
@@ -689,7 +702,7 @@ static int ntt_common(cerium_context* ctx, bool forward, void* out, size_t out_s
   DeviceGuard guard(ctx->device);
   NttCall c{in, out, in_stride, out_stride, nullptr, prime_idx, count};
   return forward ? launch_ntt_forward(ctx, c, (cudaStream_t)stream)
-                 : launch_ntt_inverse(ctx, c, nullptr, nullptr, (cudaStream_t)stream);
+                 : launch_ntt_inverse(ctx, c, (cudaStream_t)stream);
 }
 
 int cerium_ntt_forward(cerium_context* ctx, void* out, size_t out_stride, const void* in, size_t in_stride,

@@ -49,9 +49,8 @@ struct cerium_keyswitch {
     cerium_bconv* down = nullptr;
     std::vector<uint64_t> pinv;              // [L - r]
     std::vector<uint32_t> ext_pos, ext_prime;  // both accumulators: slots [L - r, LK) of each
-    void* d_block = nullptr;                 // what the next three point into
-    void* d_scale = nullptr;                 // exact mode: per entry of ext_pos, then the Shoup companions
-    void* d_scale_shoup = nullptr;
+    void* d_block = nullptr;                 // what the next two point into
+    void* d_last = nullptr;                  // exact mode: scaled last-layer constants per entry of ext_pos
     void* d_add = nullptr;                   // rounding term of the same entries, or null
   };
   std::vector<FusedDown> fused;
@@ -66,11 +65,9 @@ struct cerium_keyswitch {
   bool lifted = false;
   std::vector<uint32_t> ext_pos, ext_prime;  // extension limbs of both accumulators
   // exact mode: per-limb scalars folded into the inverse transforms (device, one word per entry)
-  void* d_scale = nullptr;  // [L] then [2K]: scale, and at +count their Shoup companions
-  void* d_scale_q = nullptr;
-  void* d_scale_q_shoup = nullptr;
-  void* d_scale_p = nullptr;
-  void* d_scale_p_shoup = nullptr;
+  void* d_consts = nullptr;  // what the next three point into
+  void* d_last_q = nullptr;  // [L] last-layer constants (inverse_last_words) of the switched polynomial's limbs
+  void* d_last_p = nullptr;  // [2K] ... and of the extension limbs of both accumulators
   void* d_add_p = nullptr;  // [2K] rounding term of the ModDown, added by the inverse transform, or null
   // workspace
   void* ws = nullptr;
@@ -118,7 +115,7 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
     c.pos = pos.data();
     c.prime = prime.data();
     c.count = n_polys;
-    if (int rc = launch_ntt_inverse(ctx, c, nullptr, nullptr, stream)) return rc;
+    if (int rc = launch_ntt_inverse(ctx, c, stream)) return rc;
   }
   // 2. SuD of the remaining limbs against the re-reduced last limb
   std::vector<uint64_t> factor(2 * R), post_sub(2 * R);
@@ -179,7 +176,7 @@ int keyswitch_begin(cerium_keyswitch* ks, void* dst, const void* cpoly, cudaStre
   const size_t n = kN;
   NttCall c{cpoly, dst, n, n, nullptr, ks->q_idx.data(), ks->L};
   c.in_galois = pre_elt;
-  return launch_ntt_inverse(ks->ctx, c, ks->d_scale_q, ks->d_scale_q_shoup, stream);
+  return launch_ntt_inverse(ks->ctx, c, stream, ks->d_last_q);
 }
 
 // Steps 2-7 from the coefficient-form limbs of ALL ranks (`gathered`: global limb i at slot
@@ -294,7 +291,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       // 5. iNTT of the extension limbs and the dropped Q limbs of both accumulators, in place
       {
         NttCall c{acc, acc, n, n, fd.ext_pos.data(), fd.ext_prime.data(), (int)fd.ext_pos.size()};
-        if (int rc = launch_ntt_inverse(ctx, c, fd.d_scale, fd.d_scale_shoup, stream, fd.d_add)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, stream, fd.d_last, fd.d_add)) return rc;
       }
       // 6. base conversion (dropped Q limbs, P) -> remaining Q limbs
       {
@@ -340,7 +337,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       if (!ks->ext_split) {
         // 5. iNTT of the extension limbs of both accumulators, in place
         NttCall c{acc, acc, n, n, ks->ext_pos.data(), ks->ext_prime.data(), 2 * K};
-        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream, ks->d_add_p)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, stream, ks->d_last_p, ks->d_add_p)) return rc;
       } else {
         // 5. iNTT of the LOCAL extension limbs into this rank's block of the gather buffer
         //    ([world][2][pgather_limbs]), then the all-gather: every rank needs all K limbs to convert
@@ -349,7 +346,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
         W* mine = pg + (size_t)ks->rank * block;
         NttCall c{acc, mine, n, n, ks->ext_dst.data(), ks->ext_prime.data(), 2 * K};
         c.src_pos = ks->ext_pos.data();
-        if (int rc = launch_ntt_inverse(ctx, c, ks->d_scale_p, ks->d_scale_p_shoup, stream, ks->d_add_p)) return rc;
+        if (int rc = launch_ntt_inverse(ctx, c, stream, ks->d_last_p, ks->d_add_p)) return rc;
         if (int rc = comm_allgather(comm, pg, mine, block * sizeof(W), stream)) return rc;
         p0 = pg;
         p1 = pg + (size_t)ks->pgather_limbs * n;
@@ -526,7 +523,6 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
   const int Kl = ks->K;  // local extension limbs
   ks->lifted = lifted;
   for (int e = 0; e < LK; e++) ks->own_digit.push_back((e < L && !lifted) ? ks->loc[e] % dnum : -1);
-  const int bits = ctx->word_bits;
   const bool exact = bconv_mode == CERIUM_BCONV_EXACT;
   std::vector<uint64_t> scale_q(std::max(L, 1), 1), scale_p(2 * std::max(Kl, 1), 1);
   ks->direct_raise = alpha == 1;
@@ -638,10 +634,15 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
   }
   const size_t wb = ctx->word_bytes();
   const size_t n = kN;
+  auto append_last = [&](std::vector<uint64_t>& v, uint32_t k, uint64_t scale) {
+    uint64_t w[4];
+    inverse_last_words(ctx, (int)k, scale, w);
+    v.insert(v.end(), w, w + 4);
+  };
   auto upload = [&](const std::vector<uint64_t>& v, void** dst) {
     std::vector<char> bytes(v.size() * wb);
     for (size_t i = 0; i < v.size(); i++) {
-      if (bits == 32) reinterpret_cast<uint32_t*>(bytes.data())[i] = (uint32_t)v[i];
+      if (ctx->word_bits == 32) reinterpret_cast<uint32_t*>(bytes.data())[i] = (uint32_t)v[i];
       else reinterpret_cast<uint64_t*>(bytes.data())[i] = v[i];
     }
     return cudaMalloc(dst, bytes.size()) == cudaSuccess &&
@@ -669,21 +670,14 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
       const uint64_t q = ctx->moduli[ks->q_idx[i]];
       fd.pinv[i] = host::invmod(host::product_mod(ctx->moduli, e_idx, q), q);
     }
-    std::vector<uint64_t> sc, scs, add;
+    std::vector<uint64_t> all, add;
     for (int p = 0; p < 2; p++)
       for (int k = 0; k < E; k++) {
         fd.ext_pos.push_back((uint32_t)(p * LK + Lr + k));
         fd.ext_prime.push_back(e_idx[k]);
-        const uint64_t ek = ctx->moduli[e_idx[k]];
-        sc.push_back(exact ? fd.down->inv_host[k] : 1);
-        scs.push_back(host::shoup(sc.back(), ek, bits));
+        if (exact) append_last(all, e_idx[k], fd.down->inv_host[k]);
         if (opt.round_half) add.push_back(fd.down->in_add_host[k]);
       }
-    std::vector<uint64_t> all;
-    if (exact) {
-      all = sc;
-      all.insert(all.end(), scs.begin(), scs.end());
-    }
     const size_t o_add = all.size() * wb;
     all.insert(all.end(), add.begin(), add.end());
     if (!all.empty()) {
@@ -692,37 +686,30 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
         cerium_keyswitch_destroy(ks);
         return fail(CERIUM_ERR_CUDA, "keyswitch_create: scale upload failed");
       }
-      if (exact) {
-        fd.d_scale = fd.d_block;
-        fd.d_scale_shoup = static_cast<char*>(fd.d_block) + sc.size() * wb;
-      }
+      if (exact) fd.d_last = fd.d_block;
       if (opt.round_half) fd.d_add = static_cast<char*>(fd.d_block) + o_add;
     }
     ks->fused.push_back(fd);
   }
   {
-    // [scale_q | scale_q_shoup | scale_p | scale_p_shoup] (exact mode) [rounding term of the extension limbs]
+    // [last-layer constants of the Q limbs, of the extension limbs twice] (exact mode) [rounding terms of the latter]
     std::vector<uint64_t> all;
     if (exact) {
-      for (int i = 0; i < L; i++) all.push_back(scale_q[i]);
-      for (int i = 0; i < L; i++) all.push_back(host::shoup(scale_q[i], ctx->moduli[ks->q_idx[i]], bits));
-      for (int i = 0; i < 2 * Kl; i++) all.push_back(scale_p[i]);
-      for (int i = 0; i < 2 * Kl; i++) all.push_back(host::shoup(scale_p[i], ctx->moduli[ks->p_idx[i % Kl]], bits));
+      for (int i = 0; i < L; i++) append_last(all, ks->q_idx[i], scale_q[i]);
+      for (int i = 0; i < 2 * Kl; i++) append_last(all, ks->p_idx[i % Kl], scale_p[i]);
     }
     const size_t o_add = all.size() * wb;
     if (round_mode == CERIUM_ROUND_HALF)
       for (int i = 0; i < 2 * Kl; i++) all.push_back(add_p[i % Kl]);
     if (!all.empty()) {
-      if (!upload(all, &ks->d_scale)) {
+      if (!upload(all, &ks->d_consts)) {
         cerium_keyswitch_destroy(ks);
         return fail(CERIUM_ERR_CUDA, "keyswitch_create: scale upload failed");
       }
-      char* b = static_cast<char*>(ks->d_scale);
+      char* b = static_cast<char*>(ks->d_consts);
       if (exact) {
-        ks->d_scale_q = b;
-        ks->d_scale_q_shoup = b + (size_t)L * wb;
-        ks->d_scale_p = b + (size_t)2 * L * wb;
-        ks->d_scale_p_shoup = b + (size_t)(2 * L + 2 * Kl) * wb;
+        ks->d_last_q = b;
+        ks->d_last_p = b + (size_t)4 * L * wb;
       }
       if (round_mode == CERIUM_ROUND_HALF && Kl > 0) ks->d_add_p = b + o_add;
     }
@@ -790,7 +777,7 @@ int cerium_mod_raise(cerium_keyswitch* ks, void* out0, void* out1, const void* c
   for (int k = 0; k < 2; k++) {
     const uint32_t prime[2] = {base0, base1};
     NttCall c{k == 0 ? c0 : c1, tmp + (size_t)2 * k * limb, n, n, nullptr, prime, 2};
-    if (int rc = launch_ntt_inverse(ctx, c, nullptr, nullptr, st)) return rc;
+    if (int rc = launch_ntt_inverse(ctx, c, st)) return rc;
   }
   // 2. exact CRT of each polynomial's pair of limbs: integers in [0, q_base0 * q_base1)
   if (int rc = cerium_resolve2(ctx, tmp + 4 * limb, tmp + 5 * limb, tmp, tmp + limb, 2 * n, base0, base1, 2, stream)) return rc;
@@ -903,7 +890,7 @@ int cerium_rescale_sharded(cerium_context* ctx, cerium_comm* comm, int round_mod
     c.pos = pos.data();
     c.prime = prime.data();
     c.count = n_polys;
-    if (int rc = launch_ntt_inverse(ctx, c, nullptr, nullptr, st)) return rc;
+    if (int rc = launch_ntt_inverse(ctx, c, st)) return rc;
   }
   if (int rc = comm_broadcast(comm, last_coef, (size_t)n_polys * n * wb, owner, st)) return rc;
   if (keep.empty()) return CERIUM_OK;
@@ -934,7 +921,7 @@ int cerium_keyswitch_destroy(cerium_keyswitch* ks) {
     if (fd.down) cerium_bconv_destroy(fd.down);
     cudaFree(fd.d_block);
   }
-  cudaFree(ks->d_scale);
+  cudaFree(ks->d_consts);
   cudaFree(ks->ws);
   delete ks;
   return CERIUM_OK;
@@ -1301,7 +1288,7 @@ int cerium_double_rescale(cerium_context* ctx, void* out, const void* in, const 
       c.pos = po.data();
       c.prime = pr.data();
       c.count = n_polys;
-      if (int rc = launch_ntt_inverse(ctx, c, nullptr, nullptr, st)) return rc;
+      if (int rc = launch_ntt_inverse(ctx, c, st)) return rc;
     }
   }
   // 2. exact CRT composition of the pair, every polynomial in one launch

@@ -88,7 +88,7 @@ extern "C" int cerium_rescale_static(cerium_context* ctx, int round_mode, void* 
   c.pos = pos;
   c.prime = prime;
   c.count = n_polys;
-  if (int rc = launch_ntt_inverse(ctx, c, nullptr, nullptr, s)) return rc;
+  if (int rc = launch_ntt_inverse(ctx, c, s)) return rc;
   uint64_t factor[kSudMaxBatch], post_sub[kSudMaxBatch];
   const uint64_t half = ql >> 1;
   for (int i = 0; i < L - 1; i++) {

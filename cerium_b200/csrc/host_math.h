@@ -107,6 +107,9 @@ inline u64 minimal_primitive_root(u64 q, int logn) {
 // floor(w * 2^bits / q)
 inline u64 shoup(u64 w, u64 q, int bits) { return (u64)((((u128)w) << bits) / q); }
 
+// residue in (-q/2, q/2) as a double (exact below 2^53)
+inline double centred(u64 w, u64 q) { return w > q / 2 ? -(double)(q - w) : (double)w; }
+
 struct PrimeTables {
   u64 q = 0, psi = 0, psi_inv = 0, ninv = 0, two_inv = 0;
   u64 mu_hi = 0, mu_lo = 0;       // floor(2^(2*bits) / q)

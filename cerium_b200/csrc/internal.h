@@ -98,6 +98,7 @@ struct cerium_context {
   int n_primes = 0;
   std::vector<uint64_t> moduli;
   std::vector<uint64_t> psi;
+  std::vector<uint64_t> ninv, w1ninv;  // N^-1, psi^-(N/2) N^-1
   void* d_tw_fwd = nullptr;  // Pair[n_primes][N], bit-reversed powers of psi
   void* d_tw_inv = nullptr;  // Pair[n_primes][N], bit-reversed powers of psi^-1
   void* d_twr_fwd = nullptr; // Pair[n_primes][256][15][16], lane-interleaved level-3 twiddles (row pass)
@@ -201,9 +202,12 @@ struct NttCall {
 };
 // lazy_out: leave the results below 4q instead of canonical (internal buffers read by the inner product only)
 int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t stream, bool lazy_out = false);
-// scale / scale_shoup / add: device arrays with one word per batch entry, or null: results * scale + add.
-int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, const void* scale, const void* scale_shoup,
-                       cudaStream_t stream, const void* add = nullptr);
+// last: device array of four words per batch entry (inverse_last_words: the results times a scale), or null.
+// add: device array of one word per batch entry, added to the results modulo q, or null.
+int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t stream, const void* last = nullptr,
+                       const void* add = nullptr);
+// The four words by which the last layer of an inverse transform of prime `k` scales its results by `scale` / N.
+void inverse_last_words(const cerium_context* ctx, int k, uint64_t scale, uint64_t (&out)[4]);
 
 // SuD over `count` limbs (count <= kSudMaxBatch per launch; chunked internally).
 struct SudCall {

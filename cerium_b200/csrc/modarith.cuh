@@ -290,22 +290,37 @@ __device__ __forceinline__ uint64_t fp_to_u64(double x) {
   return (uint64_t)__double_as_longlong(__dadd_rn(x, kFpTwo52)) & 0x000fffffffffffffull;
 }
 
-// Harvey forward butterfly: a, b in [0, 4q) -> [0, 4q).
-template <typename W>
-__device__ __forceinline__ void butterfly_fwd(W& a, W& b, W w, W ws, W q, W q2) {
-  W u = csub<W>(a, q2);
-  W v = mul_shoup_lazy<W>(b, w, ws, q);
+// Strict butterflies, one correction each.  32-bit words (Harvey): forward a, b in [0, 4q) -> [0, 4q), inverse a, b in
+// [0, 2q) -> [0, 2q).
+__device__ __forceinline__ void butterfly_fwd(uint32_t& a, uint32_t& b, uint32_t w, uint32_t ws, uint32_t q, uint32_t q2,
+                                              uint32_t /*nq*/, uint32_t /*q4*/) {
+  const uint32_t u = csub<uint32_t>(a, q2);
+  const uint32_t v = mul_shoup_lazy<uint32_t>(b, w, ws, q);
   a = u + v;
   b = u + q2 - v;
 }
-
-// Gentleman-Sande inverse butterfly: a, b in [0, 2q) -> [0, 2q).
-template <typename W>
-__device__ __forceinline__ void butterfly_inv(W& a, W& b, W w, W ws, W q, W q2) {
-  W s = csub<W>(a + b, q2);
-  W d = a + q2 - b;
+__device__ __forceinline__ void butterfly_inv(uint32_t& a, uint32_t& b, uint32_t w, uint32_t ws, uint32_t q, uint32_t q2,
+                                              uint32_t /*nq*/, uint32_t /*q4*/) {
+  const uint32_t s = csub<uint32_t>(a + b, q2);
+  const uint32_t d = a + q2 - b;
   a = s;
-  b = mul_shoup_lazy<W>(d, w, ws, q);
+  b = mul_shoup_lazy<uint32_t>(d, w, ws, q);
+}
+// 64-bit words (primes below 2^60, so 8q fits): the product in 32-bit pieces comes below 4q, which makes the ranges
+// twice as wide: forward a < 8q, b any -> below 8q; inverse a, b < 4q -> below 4q.
+__device__ __forceinline__ void butterfly_fwd(uint64_t& a, uint64_t& b, uint64_t w, uint64_t ws, uint64_t /*q*/, uint64_t /*q2*/,
+                                              uint64_t nq, uint64_t q4) {
+  const uint64_t u = csub<uint64_t>(a, q4);
+  const uint64_t v = mul_shoup_approx(b, w, ws, nq);
+  a = u + v;
+  b = u + q4 - v;
+}
+__device__ __forceinline__ void butterfly_inv(uint64_t& a, uint64_t& b, uint64_t w, uint64_t ws, uint64_t /*q*/, uint64_t /*q2*/,
+                                              uint64_t nq, uint64_t q4) {
+  const uint64_t s = csub<uint64_t>(a + b, q4);
+  const uint64_t d = a + q4 - b;
+  a = s;
+  b = mul_shoup_approx(d, w, ws, nq);
 }
 
 // NTT-domain Galois automorphism out[i] = in[pi(i)] with

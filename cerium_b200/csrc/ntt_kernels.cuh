@@ -96,7 +96,7 @@ struct PointerBatch {
 // arithmetic policies
 // ---------------------------------------------------------------------------------------
 
-// Strict (Harvey) butterflies keep every value below 4q (forward) / 2q (inverse) with one
+// Strict butterflies keep every value below 4q (forward) / 2q (inverse), twice that for 64-bit words, with one
 // correction per butterfly; they serve 32-bit words and 64-bit primes of 52 bits or more.
 // Lazy butterflies (64-bit words, primes below 2^52) use the headroom above the prime instead
 // of corrections and the 32-bit-piece products of modarith.cuh.
@@ -115,31 +115,34 @@ struct Arith {
   __device__ __forceinline__ W reduce(W x) const { return x; }
   __device__ __forceinline__ void fwd(W& a, W& b, W w, W ws) const {
     if (kLazy) butterfly_fwd_lazy<W>(a, b, w, ws, nq, q4);
-    else butterfly_fwd<W>(a, b, w, ws, q, q2);
+    else butterfly_fwd(a, b, w, ws, q, q2, nq, q4);
   }
   // k = layer number inside the pass (0..7)
   __device__ __forceinline__ void inv(W& a, W& b, W w, W ws, int k) const {
     if (kLazy) butterfly_inv_lazy<W>(a, b, w, ws, nq, q4 << k);
-    else butterfly_inv<W>(a, b, w, ws, q, q2);
+    else butterfly_inv(a, b, w, ws, q, q2, nq, q4);
   }
   // value at the end of a forward transform -> [0, q), or only below 4q when the consumer
   // takes lazy residues (kCanonical = false)
   template <bool kCanonical>
   __device__ __forceinline__ W finish_fwd(W x, W one_shoup) const {
     if (kLazy) x = reduce_lazy(x, one_shoup, nq);
+    else if (sizeof(W) == 8) x = csub<W>(x, q4);
     if (!kCanonical) return x;
     return csub<W>(csub<W>(x, q2), q);
   }
-  // last inverse layer: (a + b) * N^-1 and (a - b) * w1 * N^-1, reduced to [0, q)
-  __device__ __forceinline__ void inv_last(W& a, W& b, const PrimeConst<W>& pc) const {
+  // last inverse layer: (a + b) * last[0] and (a - b) * last[2], reduced to [0, q); last = {N^-1, Shoup companion,
+  // w1 * N^-1, Shoup companion}, times the caller's scale where there is one
+  __device__ __forceinline__ void inv_last(W& a, W& b, const W (&last)[4]) const {
     const W s = a + b;
-    const W d = a + (kLazy ? (q4 << 7) : q2) - b;
-    if (kLazy) {
-      a = csub<W>(csub<W>(mul_shoup_approx(s, pc.ninv, pc.ninv_shoup, nq), q2), q);
-      b = csub<W>(csub<W>(mul_shoup_approx(d, pc.w1ninv, pc.w1ninv_shoup, nq), q2), q);
+    if (kLazy || sizeof(W) == 8) {
+      const W d = a + (kLazy ? (q4 << 7) : q4) - b;
+      a = csub<W>(csub<W>(mul_shoup_approx(s, last[0], last[1], nq), q2), q);
+      b = csub<W>(csub<W>(mul_shoup_approx(d, last[2], last[3], nq), q2), q);
     } else {
-      a = csub<W>(mul_shoup_lazy<W>(s, pc.ninv, pc.ninv_shoup, q), q);
-      b = csub<W>(mul_shoup_lazy<W>(d, pc.w1ninv, pc.w1ninv_shoup, q), q);
+      const W d = a + q2 - b;
+      a = csub<W>(mul_shoup_lazy<W>(s, last[0], last[1], q), q);
+      b = csub<W>(mul_shoup_lazy<W>(d, last[2], last[3], q), q);
     }
   }
 };
@@ -180,10 +183,11 @@ struct Arith<uint64_t, kArithFp> {
     if (kCanonical) return canonical(r);
     return fp_to_u64(__dadd_rn(r, q));  // (0.49 q, 1.51 q): a lazy residue
   }
-  __device__ __forceinline__ void inv_last(W& a, W& b, const PrimeConst<W>& pc) const {
+  // last: the two constants of the last layer, each with its quotient by q
+  __device__ __forceinline__ void inv_last(W& a, W& b, const W (&last)[4]) const {
     const double x = d(a), y = d(b);
-    a = canonical(fp_mulmod(__dadd_rn(x, y), d(pc.fp_ninv), d(pc.fp_ninv_q), nq));
-    b = canonical(fp_mulmod(__dadd_rn(x, -y), d(pc.fp_w1ninv), d(pc.fp_w1ninv_q), nq));
+    a = canonical(fp_mulmod(__dadd_rn(x, y), d(last[0]), d(last[1]), nq));
+    b = canonical(fp_mulmod(__dadd_rn(x, -y), d(last[2]), d(last[3]), nq));
   }
 };
 
@@ -328,6 +332,14 @@ __device__ __forceinline__ W lane_tw_fp(const typename WordTraits<W>::Pair* tw, 
   return (slot & 1) ? pv.y : pv.x;
 }
 
+// 64-bit strict butterflies take ~25 instructions: unrolled, the two levels of a pass were 30 to 40 KB of straight-line
+// code, and a launch of one wave (the 60-bit extension limbs of a ModDown: 10 limbs, 160 CTAs) spent two thirds of its time
+// waiting for instructions (13 + 20 us for an inverse transform of 10 limbs against 16 + 16 us for 35 limbs of
+// 50-bit primes).  Their levels therefore loop over the layers: a perfect shuffle of the registers after every
+// layer makes every layer pair (k, k + 8), with the twiddle of group k mod 2^t, and four shuffles are the identity.
+template <typename W, int kMode>
+constexpr bool kRolled = sizeof(W) == 8 && kMode == kArithStrict;
+
 // Four forward layers on x[0..15]; layer t pairs (j, j + (8 >> t)).  kBin: bound of the inputs
 // (Fp arithmetic only).
 template <typename W, bool kGlobalTw, int kMode, bool kLaneTable = false, int kBin = 0>
@@ -335,6 +347,26 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
                                             uint32_t S, const Arith<W, kMode>& ar) {
   constexpr bool kPacked = kLaneTable && kMode == kArithFp;
   constexpr FpFwdPlan plan = fp_plan_fwd(kBin, kPacked ? kFpLaneK32 : 1);
+  if constexpr (kRolled<W, kMode>) {
+#pragma unroll 1
+    for (int t = 0; t < 4; t++) {
+      const int mask = (1 << t) - 1;
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, k & mask));
+        ar.fwd(x[k], x[k + 8], w.x, w.y);
+      }
+      W y[16];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        y[2 * k] = x[k];
+        y[2 * k + 1] = x[k + 8];
+      }
+#pragma unroll
+      for (int k = 0; k < 16; k++) x[k] = y[k];
+    }
+    return;
+  }
 #pragma unroll
   for (int t = 0; t < 4; t++) {
     const int half = 8 >> t;
@@ -359,6 +391,39 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
   }
 }
 
+// Inverse layers 3 .. last of a group, rolled; with last = 1 layer 0's pairs are left at (k, k + 8) in natural order.
+template <typename W, bool kGlobalTw, int kMode, bool kLaneTable>
+__device__ __forceinline__ void radix16_inv_rolled(W (&x)[16], const typename WordTraits<W>::Pair* twi, uint32_t S,
+                                                   const Arith<W, kMode>& ar, int last) {
+#pragma unroll 1
+  for (int t = 3; t >= last; t--) {
+    W y[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      y[k] = x[2 * k];
+      y[k + 8] = x[2 * k + 1];
+    }
+    const int mask = (1 << t) - 1;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, k & mask));
+      ar.inv(y[k], y[k + 8], w.x, w.y, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) x[k] = y[k];
+  }
+  if (last == 1) {
+    W y[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      y[k] = x[2 * k];
+      y[k + 8] = x[2 * k + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) x[k] = y[k];
+  }
+}
+
 // The four inverse layers of the same group, in reverse order; kLayer0 is the pass-local
 // number of the first layer executed (0 for the first level of a pass, 4 for the second).
 template <typename W, bool kGlobalTw, int kMode, int kLayer0, bool kLaneTable = false, int kBin = 0>
@@ -366,6 +431,10 @@ __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTrait
                                             uint32_t S, const Arith<W, kMode>& ar) {
   constexpr bool kPacked = kLaneTable && kMode == kArithFp;
   constexpr FpInvPlan plan = fp_plan_inv(kBin, kPacked ? kFpLaneK32 : 1);
+  if constexpr (kRolled<W, kMode>) {
+    radix16_inv_rolled<W, kGlobalTw, kMode, kLaneTable>(x, twi, S, ar, 0);
+    return;
+  }
 #pragma unroll
   for (int t = 3; t >= 0; t--) {
     const int half = 8 >> t;
@@ -394,10 +463,11 @@ __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTrait
 // also multiplies by N^-1 and reduces to [0, q).
 template <typename W, int kMode, int kBin = 0>
 __device__ __forceinline__ void radix16_inv_final(W (&x)[16], const typename WordTraits<W>::Pair* twi,
-                                                  const PrimeConst<W>& pc, const Arith<W, kMode>& ar) {
+                                                  const W (&last)[4], const Arith<W, kMode>& ar) {
   constexpr FpInvPlan plan = fp_plan_inv(kBin);
+  if constexpr (kRolled<W, kMode>) radix16_inv_rolled<W, false, kMode, false>(x, twi, 1u, ar, 1);
 #pragma unroll
-  for (int t = 3; t >= 1; t--) {
+  for (int t = kRolled<W, kMode> ? 0 : 3; t >= 1; t--) {
     const int half = 8 >> t;
     if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
 #pragma unroll
@@ -412,7 +482,7 @@ __device__ __forceinline__ void radix16_inv_final(W (&x)[16], const typename Wor
   }
   if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[0], ar);
 #pragma unroll
-  for (int j = 0; j < 8; j++) ar.inv_last(x[j], x[j + 8], pc);
+  for (int j = 0; j < 8; j++) ar.inv_last(x[j], x[j + 8], last);
 }
 
 // Row-pass exchange buffer: one pad word after every 16 keeps both the strided and the
@@ -882,7 +952,7 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
   for (int j = 0; j < 16; j++) dcol[j * 16] = x[j];
 }
 
-// Row pass (levels 3 and 2): in -> out; values leave in [0, 2q) (strict) or below 2^10 q (lazy).
+// Row pass (levels 3 and 2): in -> out; values leave below 2q (strict; 4q for 64-bit words) or below 2^10 q (lazy).
 template <typename W, typename Batch>
 __global__ void __launch_bounds__(kRowsPerCta * 16, 3)
     ntt_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
@@ -900,12 +970,11 @@ __global__ void __launch_bounds__(kRowsPerCta * 16, 3)
   CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, Batch, (batch, b, pc, tile, twi, twri));
 }
 
-// Optional per-limb scalar applied to the finished inverse transform (exact base
-// conversion wants x * [Qhat^-1] mod q; null = none).
+// Optional per-limb scalar of the finished inverse transform (exact base conversion wants x * [Qhat^-1] mod q):
+// it is folded into the two constants of the last layer, which every value passes anyway.
 template <typename W>
 struct InvScale {
-  const W* scale;        // per batch entry, may be null
-  const W* scale_shoup;  // per batch entry
+  const W* last;         // per batch entry the four words of Arith::inv_last, or null: plain N^-1
   const W* add;          // per batch entry, added to the scaled value modulo q (rounding term), may be null
 };
 
@@ -936,12 +1005,16 @@ __device__ __forceinline__ void ntt_inv_cols_body(const Batch& batch, const InvS
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_strided[j * 16 * kCols];
-  radix16_inv_final<W, kMode, kFpInvL1>(x, stw, pc, ar);
-  if (sc.scale != nullptr) {
-    const W s = __ldg(sc.scale + b), ss = __ldg(sc.scale_shoup + b);
+  W last[4];
+  if (sc.last != nullptr) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) x[j] = csub<W>(mul_shoup_lazy<W>(x[j], s, ss, q), q);
+    for (int e = 0; e < 4; e++) last[e] = __ldg(sc.last + 4 * b + e);
+  } else if (kMode == kArithFp) {
+    last[0] = pc.fp_ninv, last[1] = pc.fp_ninv_q, last[2] = pc.fp_w1ninv, last[3] = pc.fp_w1ninv_q;
+  } else {
+    last[0] = pc.ninv, last[1] = pc.ninv_shoup, last[2] = pc.w1ninv, last[3] = pc.w1ninv_shoup;
   }
+  radix16_inv_final<W, kMode, kFpInvL1>(x, stw, last, ar);
   if (sc.add != nullptr) {
     const W a = __ldg(sc.add + b);
 #pragma unroll
