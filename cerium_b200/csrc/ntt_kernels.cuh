@@ -652,14 +652,20 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 #endif
 }
 
-// What the row pass does with the finished NTT value.  kCanonicalInput says whether the
-// epilogue wants the value reduced to [0, q) first or takes it below 4q.
+// What the row pass does with the finished NTT values, 16 bytes at a time.  kCanonicalInput says whether the
+// epilogue wants the values reduced to [0, q) first or takes them below 4q.  load() fetches what the epilogue reads
+// itself: the row pass calls it for half of a thread's vectors at a time before it finishes any of them (with one
+// vector at a time the SuD tail waited for memory in 7 of 12 warp cycles: 43 us for 70 limbs against 18 us of traffic).
+template <typename W>
+struct NoOperands {};
 template <typename W>
 struct StoreEpilogue {
   static constexpr bool kCanonicalInput = true;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
+  using Operands = NoOperands<W>;
+  __device__ __forceinline__ Operands load(int, int) const { return {}; }
   template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&)[kWords], int, int, uint32_t, const PrimeConst<W>&) const {}
+  __device__ __forceinline__ void apply_vec(W (&)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>&) const {}
   __device__ __forceinline__ void prefetch(int /*b*/, int /*idx*/) const {}
 };
 
@@ -669,8 +675,10 @@ template <typename W>
 struct LazyStoreEpilogue {
   static constexpr bool kCanonicalInput = false;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
+  using Operands = NoOperands<W>;
+  __device__ __forceinline__ Operands load(int, int) const { return {}; }
   template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&)[kWords], int, int, uint32_t, const PrimeConst<W>&) const {}
+  __device__ __forceinline__ void apply_vec(W (&)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>&) const {}
   __device__ __forceinline__ void prefetch(int /*b*/, int /*idx*/) const {}
 };
 
@@ -702,37 +710,44 @@ struct SudEpilogue {
     const W* ap = second ? addend2 : addend;
     if (ap != nullptr && addend_elt == 0) prefetch_l2(ap + (size_t)e * addend_stride + idx);
   }
-  // The kWords results of one 16-byte vector (idx0 a multiple of kWords): minuend and addend come in
-  // as one 16-byte load each.  With an automorphism the aligned group idx0 .. idx0 + kWords - 1 is the
-  // image of ONE aligned group of the addend (the index map sends aligned 2^k blocks onto aligned 2^k
-  // blocks), so that is one load as well and the words are picked from it.
-  template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&w)[kWords], int b, int idx0, uint32_t /*pi*/,
-                                            const PrimeConst<W>& pc) const {
+  struct Operands {
+    typename RowVec<W>::Vec m, a;
+  };
+  // The operands of one 16-byte vector (idx0 a multiple of its words): minuend and addend come in as one 16-byte load
+  // each.  With an automorphism the aligned group idx0 .. idx0 + kWords - 1 is the image of ONE aligned group of the
+  // addend (the index map sends aligned 2^k blocks onto aligned 2^k blocks), so that is one load as well and the
+  // words are picked from it.
+  __device__ __forceinline__ Operands load(int b, int idx0) const {
     using Vec = typename RowVec<W>::Vec;
     const bool second = b >= split;
     const int e_ = second ? b - split : b;
     const W* mp = (second ? minuend2 : minuend) + (size_t)e_ * minuend_stride;
     const W* ap = second ? addend2 : addend;
-    W m[kWords], a[kWords] = {};
-    vec_unpack(*reinterpret_cast<const Vec*>(mp + idx0), m);
+    Operands o{};
+    o.m = *reinterpret_cast<const Vec*>(mp + idx0);
     if (ap != nullptr) {
-      ap += (size_t)e_ * addend_stride;
-      if (addend_elt != 0) {
-        uint32_t src[kWords];
+      const uint32_t at = addend_elt != 0 ? galois_source_index((uint32_t)idx0, addend_elt) & ~(uint32_t)(RowVec<W>::kWords - 1) : (uint32_t)idx0;
+      o.a = *reinterpret_cast<const Vec*>(ap + (size_t)e_ * addend_stride + at);
+    }
+    return o;
+  }
+  template <int kWords>
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int b, int idx0, uint32_t /*pi*/,
+                                            const PrimeConst<W>& pc) const {
+    const W* ap = b >= split ? addend2 : addend;
+    W m[kWords], a[kWords];
+    vec_unpack(o.m, m);
+    vec_unpack(o.a, a);
+    if (addend_elt != 0) {
+      W t[kWords];
+      vec_unpack(o.a, t);
 #pragma unroll
-        for (int e = 0; e < kWords; e++) src[e] = galois_source_index((uint32_t)(idx0 + e), addend_elt);
-        W t[kWords];
-        vec_unpack(*reinterpret_cast<const Vec*>(ap + (src[0] & ~(uint32_t)(kWords - 1))), t);
+      for (int e = 0; e < kWords; e++) {
+        const uint32_t src = galois_source_index((uint32_t)(idx0 + e), addend_elt);
+        a[e] = t[0];
 #pragma unroll
-        for (int e = 0; e < kWords; e++) {
-          a[e] = t[0];
-#pragma unroll
-          for (int k = 1; k < kWords; k++)
-            if ((src[e] & (uint32_t)(kWords - 1)) == (uint32_t)k) a[e] = t[k];
-        }
-      } else {
-        vec_unpack(*reinterpret_cast<const Vec*>(ap + idx0), a);
+        for (int k = 1; k < kWords; k++)
+          if ((src & (uint32_t)(kWords - 1)) == (uint32_t)k) a[e] = t[k];
       }
     }
 #pragma unroll
@@ -762,14 +777,22 @@ struct PtrSudEpilogue {
   const W* factors;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
   __device__ __forceinline__ void prefetch(int b, int idx) const { prefetch_l2(ins[2 * b] + idx); }
+  struct Operands {
+    W m[RowVec<W>::kWords];
+  };
+  __device__ __forceinline__ Operands load(int b, int idx0) const {
+    Operands o;
+#pragma unroll
+    for (int e = 0; e < RowVec<W>::kWords; e++) o.m[e] = ins[2 * b][idx0 + e];  // caller's limbs may be unaligned
+    return o;
+  }
   template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&w)[kWords], int b, int idx0, uint32_t pi,
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int /*b*/, int /*idx0*/, uint32_t pi,
                                             const PrimeConst<W>& pc) const {
 #pragma unroll
-    for (int e = 0; e < kWords; e++) w[e] = apply(w[e], b, idx0 + e, pi, pc);  // caller's limbs may be unaligned
+    for (int e = 0; e < kWords; e++) w[e] = apply(w[e], o.m[e], pi, pc);
   }
-  __device__ __forceinline__ W apply(W x, int b, int idx, uint32_t pi, const PrimeConst<W>& pc) const {
-    const W m = ins[2 * b][idx];
+  __device__ __forceinline__ W apply(W x, W m, uint32_t pi, const PrimeConst<W>& pc) const {
     // x < 4q and m < q: bring the difference to [0, q) before the Barrett product
     W d = m + pc.q2 - csub<W>(x, pc.q2);  // (m, m + 2q]
     d = csub<W>(csub<W>(d, pc.q2), pc.q);
@@ -829,6 +852,7 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
   const W* row = batch.in_limb(b) + (unsigned)(h * 256 + u);
   W* limb_out = batch.out_limb(b);
   W* drow = limb_out + (unsigned)(h * 256);
+  const int h_row = h * 256;
   const uint32_t selt = epi.scatter_elt();
   W* trow = tile + (unsigned)(r * kRowPitch);
   W* t_strided = trow + u;             // row_pos(j * 16 + u) = j * 17 + u
@@ -855,20 +879,26 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
   for (int jj = 0; jj < RV::kPerThread; jj++)
     vrow[row_vec_slot<W>(u * RV::kPerThread + jj)] = vec_pack(&x[jj * RV::kWords]);
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
+  constexpr int kHalf = sizeof(W) == 8 ? RV::kPerThread / 2 : 1;
 #pragma unroll
-  for (int k = 0; k < RV::kPerThread; k++) {
-    const int v = u + 16 * k;
-    W w[RV::kWords];
-    vec_unpack(vrow[row_vec_slot<W>(v)], w);
+  for (int h = 0; h < RV::kPerThread; h += kHalf) {
+    typename Epilogue::Operands ops[kHalf];
 #pragma unroll
-    epi.apply_vec(w, b, h * 256 + v * RV::kWords, pi, pc);
-    if (selt != 0) {
-      // the row's aligned 256-word block lands on one aligned block of the output limb
+    for (int k = 0; k < kHalf; k++) ops[k] = epi.load(b, h_row + (u + 16 * (h + k)) * RV::kWords);
 #pragma unroll
-      for (int e = 0; e < RV::kWords; e++)
-        limb_out[galois_source_index((uint32_t)(h * 256 + v * RV::kWords + e), selt)] = w[e];
-    } else {
-      reinterpret_cast<Vec*>(drow)[v] = vec_pack(w);
+    for (int k = 0; k < kHalf; k++) {
+      const int v = u + 16 * (h + k);
+      W w[RV::kWords];
+      vec_unpack(vrow[row_vec_slot<W>(v)], w);
+      epi.apply_vec(w, ops[k], b, h_row + v * RV::kWords, pi, pc);
+      if (selt != 0) {
+        // the row's aligned 256-word block lands on one aligned block of the output limb
+#pragma unroll
+        for (int e = 0; e < RV::kWords; e++)
+          limb_out[galois_source_index((uint32_t)(h_row + v * RV::kWords + e), selt)] = w[e];
+      } else {
+        reinterpret_cast<Vec*>(drow)[v] = vec_pack(w);
+      }
     }
   }
 }
