@@ -415,6 +415,21 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
   });
 }
 
+// Column sums of 28-bit pieces hold 16 products of residues below 2^56.
+template <typename W>
+bool pt_mac_in_pieces(const cerium_context* ctx, const uint32_t* prime_idx, int count) {
+  if (sizeof(W) == 4) return false;
+  for (int i = 0; i < count; i++)
+    if (ctx->moduli[prime_idx[i]] >> 56) return false;
+  return true;
+}
+
+template <typename W, int GI>
+void launch_pt_mac(const PtMacArgs<W>& a, bool pieces, dim3 grid, cudaStream_t stream, const PrimeConst<W>* pcs) {
+  auto kfn = pieces ? pt_mac_kernel<W, GI, sizeof(W) == 8> : pt_mac_kernel<W, GI, false>;
+  CERIUM_LAUNCH(kfn, grid, dim3(kEwThreads), 0, stream, a, pcs);
+}
+
 // Steps 4-7.  Can be repeated with different keys on the same raised digits (hoisting).
 int keyswitch_inner_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* cpoly, const void* evk,
                             const void* add0, const void* add1, cudaStream_t stream, uint32_t pre_elt = 0,
@@ -1064,6 +1079,7 @@ int cerium_plaintext_mac(cerium_context* ctx, int n_out, int n_src, void* const*
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+    const bool pieces = pt_mac_in_pieces<W>(ctx, prime_idx, count);
     for (int first = 0; first < n_out; first += kBsgsGroup) {
       const int cnt = std::min(kBsgsGroup, n_out - first);
       PtMacArgs<W> a{};
@@ -1084,10 +1100,10 @@ int cerium_plaintext_mac(cerium_context* ctx, int n_out, int n_src, void* const*
       for (int b = 0; b < count; b++) a.prime[b] = (uint8_t)prime_idx[b];
       const dim3 grid(kN / (kEwThreads * PtMacLanes<W>::kWords), count);
       switch (cnt) {
-        case 1: { auto kfn = pt_mac_kernel<W, 1>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        case 2: { auto kfn = pt_mac_kernel<W, 2>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        case 3: { auto kfn = pt_mac_kernel<W, 3>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        default: { auto kfn = pt_mac_kernel<W, 4>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
+        case 1: launch_pt_mac<W, 1>(a, pieces, grid, st, pcs); break;
+        case 2: launch_pt_mac<W, 2>(a, pieces, grid, st, pcs); break;
+        case 3: launch_pt_mac<W, 3>(a, pieces, grid, st, pcs); break;
+        default: launch_pt_mac<W, 4>(a, pieces, grid, st, pcs); break;
       }
     }
     CERIUM_LAUNCH_CHECK("plaintext_mac");
@@ -1154,6 +1170,7 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
     using W = decltype(tag);
     using V = Vec16<W>;
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+    const bool pieces = pt_mac_in_pieces<W>(ctx, ks->q_idx.data(), L);
     for (int first = 0; first < n_giant; first += kBsgsGroup) {
       const int cnt = std::min(kBsgsGroup, n_giant - first);
       PtMacArgs<W> a{};
@@ -1177,10 +1194,10 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       for (int b = 0; b < L; b++) a.prime[b] = (uint8_t)ks->q_idx[b];
       const dim3 grid(kN / (kEwThreads * PtMacLanes<W>::kWords), L);
       switch (cnt) {
-        case 1: { auto kfn = pt_mac_kernel<W, 1>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        case 2: { auto kfn = pt_mac_kernel<W, 2>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        case 3: { auto kfn = pt_mac_kernel<W, 3>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
-        default: { auto kfn = pt_mac_kernel<W, 4>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, st, a, pcs); } break;
+        case 1: launch_pt_mac<W, 1>(a, pieces, grid, st, pcs); break;
+        case 2: launch_pt_mac<W, 2>(a, pieces, grid, st, pcs); break;
+        case 3: launch_pt_mac<W, 3>(a, pieces, grid, st, pcs); break;
+        default: launch_pt_mac<W, 4>(a, pieces, grid, st, pcs); break;
       }
     }
     CERIUM_LAUNCH_CHECK("bsgs plaintext multiply-accumulate");
