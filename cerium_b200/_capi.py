@@ -7,6 +7,7 @@ Arguments that the C ABI takes as device pointers are plain integers here (``ten
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from typing import Optional, Sequence
 
@@ -127,14 +128,25 @@ class CeriumError(RuntimeError):
         self.message = message
 
 
+# Index and scalar lists as C arrays.  A program passes the same few prime lists over and over, and the conversion of
+# one (1.3 us for 6 entries, 40 us for 384) is a good part of what a small call costs: the last ones are kept.  The library
+# only reads them.
+@functools.lru_cache(maxsize=512)
+def _u32_array(values: tuple):
+    return (C.c_uint32 * len(values))(*[int(v) for v in values])
+
+
+@functools.lru_cache(maxsize=512)
+def _u64_array(values: tuple):
+    return (C.c_uint64 * len(values))(*[int(v) for v in values])
+
+
 def _u32(values: Sequence[int]):
-    arr = (C.c_uint32 * len(values))(*[int(v) for v in values])
-    return arr
+    return _u32_array(tuple(values))
 
 
 def _u64(values: Sequence[int]):
-    arr = (C.c_uint64 * len(values))(*[int(v) for v in values])
-    return arr
+    return _u64_array(tuple(values))
 
 
 class Library:

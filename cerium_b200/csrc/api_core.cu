@@ -542,6 +542,7 @@ int cerium_context_create(cerium_context** out, int device, int log_n, int word_
   ctx->n_primes = n_moduli;
   ctx->moduli.assign(moduli, moduli + n_moduli);
   ctx->psi.resize(n_moduli);
+  ctx->inverses.reset(new std::atomic<uint64_t>[(size_t)n_moduli * n_moduli]());
   if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || ctx->sm_count < 1) {
     delete ctx;
     return fail(CERIUM_ERR_CUDA, "context_create: cannot read the number of SMs");
@@ -837,7 +838,8 @@ int cerium_sud(cerium_context* ctx, void* out, size_t out_stride, const void* mi
     if (prime_idx[i] >= (uint32_t)ctx->n_primes) return fail(CERIUM_ERR_INVALID, "sud: prime index out of range");
     const uint64_t q = ctx->moduli[prime_idx[i]];
     // a prime that divides the product has no inverse: factor 0, as compute_sud_factors leaves it
-    factor[i] = host::invmod(host::product_mod(ctx->moduli, div, q), q);
+    factor[i] = 1 % q;
+    for (uint32_t d : div) factor[i] = host::mulmod(factor[i], d == prime_idx[i] ? 0 : ctx->inverse(d, prime_idx[i]), q);
   }
   DeviceGuard guard(ctx->device);
   SudCall c{};
@@ -888,6 +890,7 @@ int cerium_ewise(cerium_context* ctx, int op, void* out, size_t out_stride, cons
     for (int first = 0; first < count; first += kEwMaxLimbs) {
       const int cnt = std::min(kEwMaxLimbs, count - first);
       EwArgs<W> g{};
+      EwScalars<W> sc;
       g.out = {static_cast<W*>(out) + (size_t)first * out_stride, out_stride};
       g.a = {const_cast<W*>(static_cast<const W*>(a)) + (size_t)first * a_stride, a_stride};
       if (need_b) g.b = {const_cast<W*>(static_cast<const W*>(b)) + (size_t)first * b_stride, b_stride};
@@ -897,20 +900,20 @@ int cerium_ewise(cerium_context* ctx, int op, void* out, size_t out_stride, cons
         if (need_s) {
           const uint64_t q = ctx->moduli[prime_idx[first + k]];
           const uint64_t sv = scalars[first + k] % q;
-          g.scalar[k] = (W)sv;
-          g.scalar_shoup[k] = (W)host::shoup(sv, q, ctx->word_bits);
+          sc.scalar[k] = (W)sv;
+          sc.scalar_shoup[k] = (W)host::shoup(sv, q, ctx->word_bits);
         }
       }
       const dim3 grid(kN / (kEwThreads * V::kLanes), cnt);
       switch (op) {
-        case CERIUM_EW_ADD: { auto kfn = ewise_kernel<W, kEwAdd>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_SUB: { auto kfn = ewise_kernel<W, kEwSub>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_NEG: { auto kfn = ewise_kernel<W, kEwNeg>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_MUL: { auto kfn = ewise_kernel<W, kEwMul>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_MAD: { auto kfn = ewise_kernel<W, kEwMad>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_PMU: { auto kfn = ewise_kernel<W, kEwPmu>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        case CERIUM_EW_REDUCE: { auto kfn = ewise_kernel<W, kEwReduce>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
-        default: { auto kfn = ewise_kernel<W, kEwMulScalar>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); } break;
+        case CERIUM_EW_ADD: { auto kfn = ewise_kernel<W, kEwAdd>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        case CERIUM_EW_SUB: { auto kfn = ewise_kernel<W, kEwSub>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        case CERIUM_EW_NEG: { auto kfn = ewise_kernel<W, kEwNeg>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        case CERIUM_EW_MUL: { auto kfn = ewise_kernel<W, kEwMul>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        case CERIUM_EW_MAD: { auto kfn = ewise_kernel<W, kEwMad>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        case CERIUM_EW_PMU: { auto kfn = ewise_kernel<W, kEwPmu>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, sc, pcs); } break;
+        case CERIUM_EW_REDUCE: { auto kfn = ewise_kernel<W, kEwReduce>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); } break;
+        default: { auto kfn = ewise_kernel<W, kEwMulScalar>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, sc, pcs); } break;
       }
     }
     CERIUM_LAUNCH_CHECK("ewise");
@@ -951,8 +954,8 @@ int cerium_mul_plain_periodic(cerium_context* ctx, void* out, size_t out_stride,
       g.shift = log2_repeat;
       for (int k = 0; k < cnt; k++) g.prime[k] = (uint8_t)prime_idx[first + k];
       const dim3 grid(kN / (kEwThreads * V::kLanes), cnt);
-      if (addend) { auto kfn = ewise_kernel<W, kEwMadPeriodic>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); }
-      else { auto kfn = ewise_kernel<W, kEwMulPeriodic>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, pcs); }
+      if (addend) { auto kfn = ewise_kernel<W, kEwMadPeriodic>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); }
+      else { auto kfn = ewise_kernel<W, kEwMulPeriodic>; CERIUM_LAUNCH(kfn, grid, kEwThreads, 0, s, g, EwNone{}, pcs); }
     }
     CERIUM_LAUNCH_CHECK("mul_plain_periodic");
     return CERIUM_OK;
@@ -1067,7 +1070,7 @@ int cerium_resolve2(cerium_context* ctx, void* lo, void* hi, const void* x0, con
   for (const void* p : ptrs)
     if (int rc = check_stack(p, stride, wb, "resolve2: operand")) return rc;
   const uint64_t m0 = ctx->moduli[prime0], m1 = ctx->moduli[prime1];
-  const uint64_t inv = host::invmod(m0 % m1, m1);
+  const uint64_t inv = ctx->inverse(prime0, prime1);
   DeviceGuard guard(ctx->device);
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);

@@ -124,7 +124,7 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
   for (int i = 0; i < 2 * R; i++) {
     const uint64_t q = ctx->moduli[q_idx[i % R]];
     prime2[i] = q_idx[i % R];
-    factor[i] = host::invmod(ql % q, q);
+    factor[i] = ctx->inverse(last, q_idx[i % R]);
     post_sub[i] = round_mode == CERIUM_ROUND_HALF ? half % q : 0;
     src_pos[i] = i < R ? 0 : 1;
   }
@@ -418,10 +418,9 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
 // Column sums of 28-bit pieces hold 16 products of residues below 2^56.
 template <typename W>
 bool pt_mac_in_pieces(const cerium_context* ctx, const uint32_t* prime_idx, int count) {
-  if (sizeof(W) == 4) return false;
-  for (int i = 0; i < count; i++)
-    if (ctx->moduli[prime_idx[i]] >> 56) return false;
-  return true;
+  bool fits = sizeof(W) == 8;
+  for (int i = 0; i < count; i++) fits = fits && ctx->moduli[prime_idx[i]] >> 56 == 0;
+  return fits;
 }
 
 template <typename W, int GI>
@@ -1321,7 +1320,7 @@ int cerium_double_rescale(cerium_context* ctx, void* out, const void* in, const 
   for (int i = 0; i < 2 * R; i++) {
     const uint64_t q = ctx->moduli[q_idx[i % R]];
     prime2[i] = q_idx[i % R];
-    factor[i] = host::invmod(host::mulmod(ctx->moduli[pa] % q, ctx->moduli[pb] % q, q), q);
+    factor[i] = host::mulmod(ctx->inverse(pa, q_idx[i % R]), ctx->inverse(pb, q_idx[i % R]), q);
   }
   for (int p = 0; p < n_polys;) {
     char* o = static_cast<char*>(out) + (size_t)p * R * limb;

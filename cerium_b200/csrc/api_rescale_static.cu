@@ -93,7 +93,7 @@ extern "C" int cerium_rescale_static(cerium_context* ctx, int round_mode, void* 
   const uint64_t half = ql >> 1;
   for (int i = 0; i < L - 1; i++) {
     const uint64_t q = ctx->moduli[q_idx[i]];
-    factor[i] = host::invmod(ql % q, q);
+    factor[i] = ctx->inverse(q_idx[L - 1], q_idx[i]);
     post_sub[i] = round_mode == CERIUM_ROUND_HALF ? half % q : 0;
   }
   for (int p = 0; p < n_polys; p++) {

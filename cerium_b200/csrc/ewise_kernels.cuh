@@ -10,6 +10,8 @@
 // (two-word sums, one Barrett reduction at the end) instead of one Mul/Mad launch per digit
 // with a reduction mod q^2 after every term.
 #pragma once
+#include <type_traits>
+
 #include "modarith.cuh"
 
 namespace cerium {
@@ -76,16 +78,24 @@ enum EwOp : int {
 template <typename W>
 struct EwArgs {
   Limbs<W> out, a, b, c;
-  W scalar[kEwMaxLimbs];        // per limb (kEwPmu, kEwMulScalar)
-  W scalar_shoup[kEwMaxLimbs];  // per limb
   uint8_t prime[kEwMaxLimbs];
   int shift;                    // kEwMulPeriodic / kEwMadPeriodic: log2 of the repeat count
 };
 
+// Per-limb scalars (kEwPmu, kEwMulScalar): 2 KiB of parameters that the other operations do not carry.
+template <typename W>
+struct EwScalars {
+  W scalar[kEwMaxLimbs];
+  W scalar_shoup[kEwMaxLimbs];
+};
+struct EwNone {};
+template <typename W, int kOp>
+using EwScalarsOf = std::conditional_t<kOp == kEwPmu || kOp == kEwMulScalar, EwScalars<W>, EwNone>;
+
 // grid = (N / (256 * lanes), limbs), block = 256.
 template <typename W, int kOp>
 __global__ void __launch_bounds__(kEwThreads)
-    ewise_kernel(const EwArgs<W> g, const PrimeConst<W>* __restrict__ pcs) {
+    ewise_kernel(const EwArgs<W> g, const EwScalarsOf<W, kOp> sc, const PrimeConst<W>* __restrict__ pcs) {
   grid_dependency_launch();
   grid_dependency_wait();
   using V = Vec16<W>;
@@ -103,9 +113,9 @@ __global__ void __launch_bounds__(kEwThreads)
     for (int l = 0; l < V::kLanes; l++) bb.v[l] = *g.b.at(b, (idx + l) >> g.shift);
   }
   W s = 0, ss = 0;
-  if (kOp == kEwPmu || kOp == kEwMulScalar) {
-    s = g.scalar[b];
-    ss = g.scalar_shoup[b];
+  if constexpr (kOp == kEwPmu || kOp == kEwMulScalar) {
+    s = sc.scalar[b];
+    ss = sc.scalar_shoup[b];
   }
 #pragma unroll
   for (int l = 0; l < V::kLanes; l++) {

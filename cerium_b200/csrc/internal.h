@@ -6,9 +6,11 @@
 #include <cuda_runtime.h>
 #endif
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <memory>
 #include <string>
 #include <utility>
 #include <vector>
@@ -112,6 +114,18 @@ struct cerium_context {
   std::vector<uint64_t> mu_hi, mu_lo;  // Barrett constants per prime (host copy)
   std::vector<uint8_t> fp_ok, lazy_ok; // arithmetic of each prime's transforms (host copy)
   size_t word_bytes() const { return (size_t)word_bits / 8; }
+  // q_a^-1 mod q_b, found once per pair (the extended Euclid of a rescale's factors was most of its host time): a table
+  // of n_primes^2 words, 0 = not known yet; concurrent calls at worst find the same value twice
+  std::unique_ptr<std::atomic<uint64_t>[]> inverses;
+  uint64_t inverse(uint32_t a, uint32_t b) const {
+    std::atomic<uint64_t>& e = inverses[(size_t)a * n_primes + b];
+    uint64_t v = e.load(std::memory_order_relaxed);
+    if (v == 0) {
+      v = cerium::host::invmod(moduli[a] % moduli[b], moduli[b]);
+      e.store(v, std::memory_order_relaxed);
+    }
+    return v;
+  }
 };
 
 struct cerium_bconv {

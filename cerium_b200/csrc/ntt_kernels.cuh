@@ -365,27 +365,27 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
 #pragma unroll
       for (int k = 0; k < 16; k++) x[k] = y[k];
     }
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int t = 0; t < 4; t++) {
-    const int half = 8 >> t;
-    if (kMode == kArithFp && plan.before[t]) fp_reduce_masked<W, kMode>(x, 0xffffu, ar);
+    for (int t = 0; t < 4; t++) {
+      const int half = 8 >> t;
+      if (kMode == kArithFp && plan.before[t]) fp_reduce_masked<W, kMode>(x, 0xffffu, ar);
 #pragma unroll
-    for (int g = 0; g < (1 << t); g++) {
-      W w0, w1;
-      if constexpr (kPacked) {
-        w0 = lane_tw_fp<W>(tw, t, g);
-        w1 = ar.quotient(w0);
-      } else {
-        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, g));
-        w0 = w.x;
-        w1 = w.y;
-      }
+      for (int g = 0; g < (1 << t); g++) {
+        W w0, w1;
+        if constexpr (kPacked) {
+          w0 = lane_tw_fp<W>(tw, t, g);
+          w1 = ar.quotient(w0);
+        } else {
+          const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, g));
+          w0 = w.x;
+          w1 = w.y;
+        }
 #pragma unroll
-      for (int k = 0; k < half; k++) {
-        const int j = g * 2 * half + k;
-        ar.fwd(x[j], x[j + half], w0, w1);
+        for (int k = 0; k < half; k++) {
+          const int j = g * 2 * half + k;
+          ar.fwd(x[j], x[j + half], w0, w1);
+        }
       }
     }
   }
@@ -433,27 +433,27 @@ __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTrait
   constexpr FpInvPlan plan = fp_plan_inv(kBin, kPacked ? kFpLaneK32 : 1);
   if constexpr (kRolled<W, kMode>) {
     radix16_inv_rolled<W, kGlobalTw, kMode, kLaneTable>(x, twi, S, ar, 0);
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int t = 3; t >= 0; t--) {
-    const int half = 8 >> t;
-    if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
+    for (int t = 3; t >= 0; t--) {
+      const int half = 8 >> t;
+      if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
 #pragma unroll
-    for (int g = 0; g < (1 << t); g++) {
-      W w0, w1;
-      if constexpr (kPacked) {
-        w0 = lane_tw_fp<W>(twi, t, g);
-        w1 = ar.quotient(w0);
-      } else {
-        const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, g));
-        w0 = w.x;
-        w1 = w.y;
-      }
+      for (int g = 0; g < (1 << t); g++) {
+        W w0, w1;
+        if constexpr (kPacked) {
+          w0 = lane_tw_fp<W>(twi, t, g);
+          w1 = ar.quotient(w0);
+        } else {
+          const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, g));
+          w0 = w.x;
+          w1 = w.y;
+        }
 #pragma unroll
-      for (int k = 0; k < half; k++) {
-        const int j = g * 2 * half + k;
-        ar.inv(x[j], x[j + half], w0, w1, kLayer0 + 3 - t);
+        for (int k = 0; k < half; k++) {
+          const int j = g * 2 * half + k;
+          ar.inv(x[j], x[j + half], w0, w1, kLayer0 + 3 - t);
+        }
       }
     }
   }
