@@ -556,10 +556,6 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
       if (ks->own_digit[e] == d) continue;
       out_primes.push_back(ks->all_idx[e]);
       out_pos.push_back((uint32_t)e);
-      ks->ntt_pos.push_back((uint32_t)(d * LK + e));
-      ks->ntt_prime.push_back(ks->all_idx[e]);
-      ks->ntt_src.push_back(slot_of(d));
-      ks->ntt_src_prime.push_back(q_idx[d]);
     }
     if (in_primes.empty() || out_primes.empty() || ks->direct_raise) continue;
     BconvOptions opt;
@@ -573,6 +569,17 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
     if (rc != CERIUM_OK) break;
     ks->up.push_back(bc);
     ks->up_digit.push_back(d);
+  }
+  // the transforms of the converted limbs by output limb: those that run at the same time share a prime, so its twiddles
+  // (1.5 MiB) come from L2 (by digit, a rotation of 35 limbs took 381 us, now 376; of 12 limbs 144.4, now 140.5)
+  for (int e = 0; e < LK; e++) {
+    for (int d = 0; d < dnum && !lifted; d++) {
+      if (ks->own_digit[e] == d) continue;
+      ks->ntt_pos.push_back((uint32_t)(d * LK + e));
+      ks->ntt_prime.push_back(ks->all_idx[e]);
+      ks->ntt_src.push_back(slot_of(d));
+      ks->ntt_src_prime.push_back(q_idx[d]);
+    }
   }
   if (exact && !lifted && !ks->direct_raise) {
     // exact conversion: the inverse transform of local limb i leaves x_i * [Qhat_i^-1]_{q_i}, Qhat_i the
