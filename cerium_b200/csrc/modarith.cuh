@@ -336,5 +336,45 @@ __device__ __forceinline__ uint32_t galois_source_index(uint32_t i, uint32_t elt
   return __brev(raw) >> (32 - kLogN);
 }
 
+// The image of the aligned group of kWords (2 or 4) indices from i0 on is one aligned group; word e of the first comes
+// from word galois_pick(...) of the second.  With brev(i0 + e) = brev(i0) + brev(e), brev(e) in the top bits, the products
+// of the group differ in those bits only: pick = brev(top bits of the group's raw index + elt * brev(e)).
+template <int kWords>
+struct GaloisGroup {
+  static constexpr int kBits = kWords == 4 ? 2 : 1;
+  static_assert(kWords == 2 || kWords == 4, "group size");
+  uint32_t at;   // first index of the image group
+  uint32_t top;  // top bits of the raw index of i0
+  uint32_t elt;
+  __device__ __forceinline__ GaloisGroup(uint32_t i0, uint32_t e) : elt(e) {
+    const uint32_t r = (__brev(i0) >> (32 - kLogN)) * 2u + 1u;
+    const uint32_t raw = ((e * r) >> 1) & (uint32_t)(kN - 1);
+    at = (__brev(raw) >> (32 - kLogN)) & ~(uint32_t)(kWords - 1);
+    top = raw >> (kLogN - kBits);
+  }
+  static __device__ __forceinline__ uint32_t brev(uint32_t k) { return kWords == 4 ? (k & 1u) << 1 | k >> 1 : k; }
+  __device__ __forceinline__ uint32_t pick(int e) const {
+    return brev((top + elt * brev((uint32_t)e)) & (uint32_t)(kWords - 1));
+  }
+  // the word that pick() sends to k (an odd elt is its own inverse modulo 4)
+  __device__ __forceinline__ uint32_t unpick(int k) const {
+    return brev((elt * (brev((uint32_t)k) - top)) & (uint32_t)(kWords - 1));
+  }
+  // out[e] = in[pick(e)]; kInverse: out[pick(e)] = in[e]
+  template <bool kInverse = false, typename W>
+  __device__ __forceinline__ void permute(const W (&in)[kWords], W (&out)[kWords]) const {
+#pragma unroll
+    for (int e = 0; e < kWords; e++) {
+      const uint32_t k = kInverse ? unpick(e) : pick(e);
+      if (kWords == 2) {
+        out[e] = k != 0 ? in[kWords - 1] : in[0];
+      } else {
+        const W lo = (k & 1u) != 0 ? in[1] : in[0], hi = (k & 1u) != 0 ? in[kWords - 1] : in[kWords / 2];
+        out[e] = (k & 2u) != 0 ? hi : lo;
+      }
+    }
+  }
+};
+
 
 }  // namespace cerium

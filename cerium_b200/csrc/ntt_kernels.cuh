@@ -726,7 +726,7 @@ struct SudEpilogue {
     Operands o{};
     o.m = *reinterpret_cast<const Vec*>(mp + idx0);
     if (ap != nullptr) {
-      const uint32_t at = addend_elt != 0 ? galois_source_index((uint32_t)idx0, addend_elt) & ~(uint32_t)(RowVec<W>::kWords - 1) : (uint32_t)idx0;
+      const uint32_t at = addend_elt != 0 ? GaloisGroup<RowVec<W>::kWords>((uint32_t)idx0, addend_elt).at : (uint32_t)idx0;
       o.a = *reinterpret_cast<const Vec*>(ap + (size_t)e_ * addend_stride + at);
     }
     return o;
@@ -738,17 +738,10 @@ struct SudEpilogue {
     W m[kWords], a[kWords];
     vec_unpack(o.m, m);
     vec_unpack(o.a, a);
-    if (addend_elt != 0) {
+    if (ap != nullptr && addend_elt != 0) {
       W t[kWords];
       vec_unpack(o.a, t);
-#pragma unroll
-      for (int e = 0; e < kWords; e++) {
-        const uint32_t src = galois_source_index((uint32_t)(idx0 + e), addend_elt);
-        a[e] = t[0];
-#pragma unroll
-        for (int k = 1; k < kWords; k++)
-          if ((src & (uint32_t)(kWords - 1)) == (uint32_t)k) a[e] = t[k];
-      }
+      GaloisGroup<kWords>((uint32_t)idx0, addend_elt).permute(t, a);
     }
 #pragma unroll
     for (int e = 0; e < kWords; e++) {
@@ -892,10 +885,11 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
       vec_unpack(vrow[row_vec_slot<W>(v)], w);
       epi.apply_vec(w, ops[k], b, h_row + v * RV::kWords, pi, pc);
       if (selt != 0) {
-        // the row's aligned 256-word block lands on one aligned block of the output limb
-#pragma unroll
-        for (int e = 0; e < RV::kWords; e++)
-          limb_out[galois_source_index((uint32_t)(h_row + v * RV::kWords + e), selt)] = w[e];
+        // an aligned group of words lands on an aligned group of the output limb
+        const GaloisGroup<RV::kWords> gg((uint32_t)(h_row + v * RV::kWords), selt);
+        W t[RV::kWords];
+        gg.template permute<true>(w, t);
+        *reinterpret_cast<Vec*>(limb_out + gg.at) = vec_pack(t);
       } else {
         reinterpret_cast<Vec*>(drow)[v] = vec_pack(w);
       }
@@ -944,21 +938,25 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
   W* trow = tile + r * kRowPitch;
   // coalesced vectors -> swizzled staging -> own 16 consecutive words
   Vec* vrow = reinterpret_cast<Vec*>(tile + r * kRowPitch);  // same private region as the exchange rows
+  Vec in[RV::kPerThread];
+  if (elt == 0) {
 #pragma unroll
-  for (int k = 0; k < RV::kPerThread; k++) {
-    const int v = u + 16 * k;
-    if (elt != 0) {
-      // the automorphism maps the aligned 256-word block of this row onto one aligned block:
-      // the gathered words use whole sectors
-      W w[RV::kWords];
+    for (int k = 0; k < RV::kPerThread; k++) in[k] = reinterpret_cast<const Vec*>(src)[u + 16 * k];
+  } else {
+    // the automorphism maps aligned groups of words onto aligned groups: one vector, its words permuted
 #pragma unroll
-      for (int e = 0; e < RV::kWords; e++)
-        w[e] = limb_in[galois_source_index((uint32_t)(h * 256 + v * RV::kWords + e), elt)];
-      vrow[row_vec_slot<W>(v)] = vec_pack(w);
-    } else {
-      vrow[row_vec_slot<W>(v)] = reinterpret_cast<const Vec*>(src)[v];
+    for (int k = 0; k < RV::kPerThread; k++)
+      in[k] = *reinterpret_cast<const Vec*>(limb_in + GaloisGroup<RV::kWords>((uint32_t)(h * 256 + (u + 16 * k) * RV::kWords), elt).at);
+#pragma unroll
+    for (int k = 0; k < RV::kPerThread; k++) {
+      W t[RV::kWords], w[RV::kWords];
+      vec_unpack(in[k], t);
+      GaloisGroup<RV::kWords>((uint32_t)(h * 256 + (u + 16 * k) * RV::kWords), elt).permute(t, w);
+      in[k] = vec_pack(w);
     }
   }
+#pragma unroll
+  for (int k = 0; k < RV::kPerThread; k++) vrow[row_vec_slot<W>(u + 16 * k)] = in[k];
   __syncwarp();
   W x[16];
 #pragma unroll
