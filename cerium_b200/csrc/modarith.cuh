@@ -306,19 +306,34 @@ __device__ __forceinline__ void butterfly_inv(uint32_t& a, uint32_t& b, uint32_t
   a = s;
   b = mul_shoup_lazy<uint32_t>(d, w, ws, q);
 }
-// 64-bit words (primes below 2^60, so 8q fits): the product in 32-bit pieces comes below 4q, which makes the ranges
-// twice as wide: forward a < 8q, b any -> below 8q; inverse a, b < 4q -> below 4q.
+// 64-bit words (primes of 52 to 60 bits, so 9q fits): the product in 32-bit pieces comes below 4q, and the correction
+// looks at the high words only (three instructions, written out because the compiler selects on both words, where the
+// exact comparison takes six), which leaves up to 2^32 more:
+// with e = 2^32 a forward layer takes a < 8q + e, any b, to below 8q + e; an inverse layer takes a, b < 4q + d to below
+// 4q + max(e, 2d) and 4q, and sixteen layers of that stay below 5q.
+__device__ __forceinline__ uint64_t csub_high(uint64_t x, uint64_t c) {
+#if defined(CERIUM_EMU)
+  if ((uint32_t)(x >> 32) > (uint32_t)(c >> 32)) x -= c;
+#else
+  asm("{\n\t.reg .pred p;\n\t.reg .u32 a, b, c, d;\n\t"
+      "mov.b64 {a, b}, %0;\n\tmov.b64 {c, d}, %1;\n\t"
+      "setp.gt.u32 p, b, d;\n\t@p sub.cc.u32 a, a, c;\n\t@p subc.u32 b, b, d;\n\t"
+      "mov.b64 %0, {a, b};\n\t}"
+      : "+l"(x) : "l"(c));
+#endif
+  return x;
+}
 __device__ __forceinline__ void butterfly_fwd(uint64_t& a, uint64_t& b, uint64_t w, uint64_t ws, uint64_t /*q*/, uint64_t /*q2*/,
                                               uint64_t nq, uint64_t q4) {
-  const uint64_t u = csub<uint64_t>(a, q4);
+  const uint64_t u = csub_high(a, q4);
   const uint64_t v = mul_shoup_approx(b, w, ws, nq);
   a = u + v;
   b = u + q4 - v;
 }
 __device__ __forceinline__ void butterfly_inv(uint64_t& a, uint64_t& b, uint64_t w, uint64_t ws, uint64_t /*q*/, uint64_t /*q2*/,
                                               uint64_t nq, uint64_t q4) {
-  const uint64_t s = csub<uint64_t>(a + b, q4);
-  const uint64_t d = a + q4 - b;
+  const uint64_t s = csub_high(a + b, q4);
+  const uint64_t d = a + (q4 - nq) - b;
   a = s;
   b = mul_shoup_approx(d, w, ws, nq);
 }

@@ -127,7 +127,7 @@ struct Arith {
   template <bool kCanonical>
   __device__ __forceinline__ W finish_fwd(W x, W one_shoup) const {
     if (kLazy) x = reduce_lazy(x, one_shoup, nq);
-    else if (sizeof(W) == 8) x = csub<W>(x, q4);
+    else if constexpr (sizeof(W) == 8) x = csub<W>(csub_high(x, q4), q4);
     if (!kCanonical) return x;
     return csub<W>(csub<W>(x, q2), q);
   }
@@ -136,7 +136,7 @@ struct Arith {
   __device__ __forceinline__ void inv_last(W& a, W& b, const W (&last)[4]) const {
     const W s = a + b;
     if (kLazy || sizeof(W) == 8) {
-      const W d = a + (kLazy ? (q4 << 7) : q4) - b;
+      const W d = a + (kLazy ? (q4 << 7) : q4 + q) - b;
       a = csub<W>(csub<W>(mul_shoup_approx(s, last[0], last[1], nq), q2), q);
       b = csub<W>(csub<W>(mul_shoup_approx(d, last[2], last[3], nq), q2), q);
     } else {
@@ -332,14 +332,6 @@ __device__ __forceinline__ W lane_tw_fp(const typename WordTraits<W>::Pair* tw, 
   return (slot & 1) ? pv.y : pv.x;
 }
 
-// 64-bit strict butterflies take ~25 instructions: unrolled, the two levels of a pass were 30 to 40 KB of straight-line
-// code, and a launch of one wave (the 60-bit extension limbs of a ModDown: 10 limbs, 160 CTAs) spent two thirds of its time
-// waiting for instructions (13 + 20 us for an inverse transform of 10 limbs against 16 + 16 us for 35 limbs of
-// 50-bit primes).  Their levels therefore loop over the layers: a perfect shuffle of the registers after every
-// layer makes every layer pair (k, k + 8), with the twiddle of group k mod 2^t, and four shuffles are the identity.
-template <typename W, int kMode>
-constexpr bool kRolled = sizeof(W) == 8 && kMode == kArithStrict;
-
 // Four forward layers on x[0..15]; layer t pairs (j, j + (8 >> t)).  kBin: bound of the inputs
 // (Fp arithmetic only).
 template <typename W, bool kGlobalTw, int kMode, bool kLaneTable = false, int kBin = 0>
@@ -347,80 +339,27 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
                                             uint32_t S, const Arith<W, kMode>& ar) {
   constexpr bool kPacked = kLaneTable && kMode == kArithFp;
   constexpr FpFwdPlan plan = fp_plan_fwd(kBin, kPacked ? kFpLaneK32 : 1);
-  if constexpr (kRolled<W, kMode>) {
-#pragma unroll 1
-    for (int t = 0; t < 4; t++) {
-      const int mask = (1 << t) - 1;
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, k & mask));
-        ar.fwd(x[k], x[k + 8], w.x, w.y);
+  for (int t = 0; t < 4; t++) {
+    const int half = 8 >> t;
+    if (kMode == kArithFp && plan.before[t]) fp_reduce_masked<W, kMode>(x, 0xffffu, ar);
+#pragma unroll
+    for (int g = 0; g < (1 << t); g++) {
+      W w0, w1;
+      if constexpr (kPacked) {
+        w0 = lane_tw_fp<W>(tw, t, g);
+        w1 = ar.quotient(w0);
+      } else {
+        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, g));
+        w0 = w.x;
+        w1 = w.y;
       }
-      W y[16];
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        y[2 * k] = x[k];
-        y[2 * k + 1] = x[k + 8];
-      }
-#pragma unroll
-      for (int k = 0; k < 16; k++) x[k] = y[k];
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const int half = 8 >> t;
-      if (kMode == kArithFp && plan.before[t]) fp_reduce_masked<W, kMode>(x, 0xffffu, ar);
-#pragma unroll
-      for (int g = 0; g < (1 << t); g++) {
-        W w0, w1;
-        if constexpr (kPacked) {
-          w0 = lane_tw_fp<W>(tw, t, g);
-          w1 = ar.quotient(w0);
-        } else {
-          const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, g));
-          w0 = w.x;
-          w1 = w.y;
-        }
-#pragma unroll
-        for (int k = 0; k < half; k++) {
-          const int j = g * 2 * half + k;
-          ar.fwd(x[j], x[j + half], w0, w1);
-        }
+      for (int k = 0; k < half; k++) {
+        const int j = g * 2 * half + k;
+        ar.fwd(x[j], x[j + half], w0, w1);
       }
     }
-  }
-}
-
-// Inverse layers 3 .. last of a group, rolled; with last = 1 layer 0's pairs are left at (k, k + 8) in natural order.
-template <typename W, bool kGlobalTw, int kMode, bool kLaneTable>
-__device__ __forceinline__ void radix16_inv_rolled(W (&x)[16], const typename WordTraits<W>::Pair* twi, uint32_t S,
-                                                   const Arith<W, kMode>& ar, int last) {
-#pragma unroll 1
-  for (int t = 3; t >= last; t--) {
-    W y[16];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      y[k] = x[2 * k];
-      y[k + 8] = x[2 * k + 1];
-    }
-    const int mask = (1 << t) - 1;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, k & mask));
-      ar.inv(y[k], y[k + 8], w.x, w.y, 0);
-    }
-#pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = y[k];
-  }
-  if (last == 1) {
-    W y[16];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      y[k] = x[2 * k];
-      y[k + 8] = x[2 * k + 1];
-    }
-#pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = y[k];
   }
 }
 
@@ -431,29 +370,25 @@ __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTrait
                                             uint32_t S, const Arith<W, kMode>& ar) {
   constexpr bool kPacked = kLaneTable && kMode == kArithFp;
   constexpr FpInvPlan plan = fp_plan_inv(kBin, kPacked ? kFpLaneK32 : 1);
-  if constexpr (kRolled<W, kMode>) {
-    radix16_inv_rolled<W, kGlobalTw, kMode, kLaneTable>(x, twi, S, ar, 0);
-  } else {
 #pragma unroll
-    for (int t = 3; t >= 0; t--) {
-      const int half = 8 >> t;
-      if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
+  for (int t = 3; t >= 0; t--) {
+    const int half = 8 >> t;
+    if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
 #pragma unroll
-      for (int g = 0; g < (1 << t); g++) {
-        W w0, w1;
-        if constexpr (kPacked) {
-          w0 = lane_tw_fp<W>(twi, t, g);
-          w1 = ar.quotient(w0);
-        } else {
-          const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, g));
-          w0 = w.x;
-          w1 = w.y;
-        }
+    for (int g = 0; g < (1 << t); g++) {
+      W w0, w1;
+      if constexpr (kPacked) {
+        w0 = lane_tw_fp<W>(twi, t, g);
+        w1 = ar.quotient(w0);
+      } else {
+        const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, g));
+        w0 = w.x;
+        w1 = w.y;
+      }
 #pragma unroll
-        for (int k = 0; k < half; k++) {
-          const int j = g * 2 * half + k;
-          ar.inv(x[j], x[j + half], w0, w1, kLayer0 + 3 - t);
-        }
+      for (int k = 0; k < half; k++) {
+        const int j = g * 2 * half + k;
+        ar.inv(x[j], x[j + half], w0, w1, kLayer0 + 3 - t);
       }
     }
   }
@@ -465,9 +400,8 @@ template <typename W, int kMode, int kBin = 0>
 __device__ __forceinline__ void radix16_inv_final(W (&x)[16], const typename WordTraits<W>::Pair* twi,
                                                   const W (&last)[4], const Arith<W, kMode>& ar) {
   constexpr FpInvPlan plan = fp_plan_inv(kBin);
-  if constexpr (kRolled<W, kMode>) radix16_inv_rolled<W, false, kMode, false>(x, twi, 1u, ar, 1);
 #pragma unroll
-  for (int t = kRolled<W, kMode> ? 0 : 3; t >= 1; t--) {
+  for (int t = 3; t >= 1; t--) {
     const int half = 8 >> t;
     if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, plan.before[t], ar);
 #pragma unroll
