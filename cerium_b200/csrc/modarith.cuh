@@ -311,6 +311,8 @@ __device__ __forceinline__ void butterfly_inv(uint32_t& a, uint32_t& b, uint32_t
 // exact comparison takes six), which leaves up to 2^32 more:
 // with e = 2^32 a forward layer takes a < 8q + e, any b, to below 8q + e; an inverse layer takes a, b < 4q + d to below
 // 4q + max(e, 2d) and 4q, and sixteen layers of that stay below 5q.
+// 22 instructions a butterfly (30 with exact comparisons and layers rolled over shuffled registers): 245 limbs of 60-bit
+// primes forward 208 -> 171 us, 10 limbs inverse 28.3 -> 24.6 us.
 __device__ __forceinline__ uint64_t csub_high(uint64_t x, uint64_t c) {
 #if defined(CERIUM_EMU)
   if ((uint32_t)(x >> 32) > (uint32_t)(c >> 32)) x -= c;
