@@ -49,11 +49,34 @@ int fail(int code, const std::string& msg);
 #define CERIUM_LAUNCH(kfn, grid, block, smem, stream, ...) \
   ::cerium_emu::launch((grid), (block), (smem), [=]() { kfn(__VA_ARGS__); })
 #else
+// All kernels ask for one split of the SM's memory, 132 KB shared and 96 KB L1 (57 % of the 228 KB rounds up to it): what
+// three CTAs of a transform need.  Left to the driver every kernel gets the split that suits it alone, an SM has to drain
+// before it changes from one to the next, and the overlap of dependent launches is lost at every such boundary (a
+// rotation of 12 limbs, 11 launches: 132 us, 126 with one split; with 164 KB shared and more the transforms lose the L1
+// that holds their twiddles: 193 us for 384 limbs, 212 with 228 KB).  The attribute is set at a kernel's first
+// launch on a device.
+constexpr int kCarveoutPercent = 57;
+inline void prefer_carveout(const void* kfn) {
+  constexpr size_t kSlots = 1024;  // open addressing; a full table only means that the attribute is set again
+  static std::atomic<uintptr_t> seen[kSlots] = {};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return;
+  const uintptr_t key = reinterpret_cast<uintptr_t>(kfn) * kMaxDevices + (uintptr_t)device;
+  for (size_t k = 0, h = key / kMaxDevices / 16 % kSlots; k < kSlots; k++, h = (h + 1) % kSlots) {
+    uintptr_t at = seen[h].load(std::memory_order_relaxed);
+    if (at == key) return;
+    if (at == 0) {
+      cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent);  // a hint
+      if (seen[h].compare_exchange_strong(at, key, std::memory_order_relaxed) || at == key) return;
+    }
+  }
+}
 // Every kernel is launched with programmatic stream serialisation (see grid_dependency_wait in
 // modarith.cuh): its CTAs may be placed while the previous kernel of the stream drains.
 template <typename... KArgs, typename... Args>
 inline void launch_dependent(void (*kfn)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                              Args&&... args) {
+  prefer_carveout(reinterpret_cast<const void*>(kfn));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
