@@ -48,12 +48,68 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // NTT launchers
 // ---------------------------------------------------------------------------------------
 
+// The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
+static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm * ctx->sm_count; }
+
+template <typename W, typename Batch, typename Loader>
+static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loader& loader, int limbs, cudaStream_t stream) {
+  constexpr int kCols = NttCfg<W>::kCols;
+  const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
+  const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+  if (small_batch(ctx, limbs)) {
+    auto kfn = ntt_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
+    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, loader, tw, pcs);
+  } else {
+    auto kfn = ntt_fwd_cols_kernel<W, kCols, Batch, Loader>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
+  }
+}
+template <typename W, typename Batch>
+static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvScale<W>& scale, int limbs, cudaStream_t stream) {
+  constexpr int kCols = NttCfg<W>::kCols;
+  const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_inv);
+  const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+  if (small_batch(ctx, limbs)) {
+    auto kfn = ntt_inv_cols_kernel<W, kCols / 2, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, scale, tw, pcs);
+  } else {
+    auto kfn = ntt_inv_cols_kernel<W, kCols, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kCols, limbs), kCols * 16, 0, stream, batch, scale, tw, pcs);
+  }
+}
+template <typename W, typename Batch, typename Epilogue>
+static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilogue& epi, int limbs, cudaStream_t stream) {
+  using Pair = typename WordTraits<W>::Pair;
+  const auto* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
+  const auto* twr = static_cast<const Pair*>(ctx->d_twr_fwd);
+  const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+  if (small_batch(ctx, limbs)) {
+    auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, epi, tw, twr, pcs);
+  } else {
+    auto kfn = ntt_fwd_rows_kernel<W, kRowsPerCta, false, Batch, Epilogue>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, epi, tw, twr, pcs);
+  }
+}
+template <typename W, typename Batch>
+static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, cudaStream_t stream) {
+  using Pair = typename WordTraits<W>::Pair;
+  const auto* tw = static_cast<const Pair*>(ctx->d_tw_inv);
+  const auto* twr = static_cast<const Pair*>(ctx->d_twr_inv);
+  const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
+  if (small_batch(ctx, limbs)) {
+    auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
+  } else {
+    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
+  }
+}
+
 int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t stream, bool lazy_out) {
   if (c.count == 0) return CERIUM_OK;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    using Pair = typename WordTraits<W>::Pair;
-    constexpr int kCols = NttCfg<W>::kCols;
     for (int first = 0; first < c.count; first += kMaxBatch) {
       const int cnt = std::min(kMaxBatch, c.count - first);
       StridedBatch<W> cols{};
@@ -76,21 +132,16 @@ int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t strea
         ModLoader<W> ml{};
         for (int b = 0; b < cnt; b++)
           ml.small[b] = (c.src_prime != nullptr && ctx->moduli[c.src_prime[first + b]] < ((uint64_t)1 << 50)) ? 1 : 0;
-        auto kfn = ntt_fwd_cols_kernel<W, GatherBatch<W>, ModLoader<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, gb, ml, static_cast<const Pair*>(ctx->d_tw_fwd), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_fwd_cols<W>(ctx, gb, ml, cnt, stream);
       } else if (c.lazy_in) {
-        auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, LazyLoader<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, LazyLoader<W>{}, static_cast<const Pair*>(ctx->d_tw_fwd), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_fwd_cols<W>(ctx, cols, LazyLoader<W>{}, cnt, stream);
       } else {
-        auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, PlainLoader<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, PlainLoader<W>{}, static_cast<const Pair*>(ctx->d_tw_fwd), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, stream);
       }
       if (lazy_out) {
-        auto kfn = ntt_fwd_rows_kernel<W, StridedBatch<W>, LazyStoreEpilogue<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, stream, rows, LazyStoreEpilogue<W>{}, static_cast<const Pair*>(ctx->d_tw_fwd), static_cast<const Pair*>(ctx->d_twr_fwd), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_fwd_rows<W>(ctx, rows, LazyStoreEpilogue<W>{}, cnt, stream);
       } else {
-        auto kfn = ntt_fwd_rows_kernel<W, StridedBatch<W>, StoreEpilogue<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, stream, rows, StoreEpilogue<W>{}, static_cast<const Pair*>(ctx->d_tw_fwd), static_cast<const Pair*>(ctx->d_twr_fwd), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_fwd_rows<W>(ctx, rows, StoreEpilogue<W>{}, cnt, stream);
       }
     }
     CERIUM_LAUNCH_CHECK("ntt_forward");
@@ -117,8 +168,6 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t strea
   if (c.count == 0) return CERIUM_OK;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    using Pair = typename WordTraits<W>::Pair;
-    constexpr int kCols = NttCfg<W>::kCols;
     for (int first = 0; first < c.count; first += kMaxBatch) {
       const int cnt = std::min(kMaxBatch, c.count - first);
       StridedBatch<W> sb{};
@@ -140,13 +189,11 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t strea
           if (c.src_pos[first + b] > 0xffffu) return fail(CERIUM_ERR_INVALID, "limb slot exceeds 65535");
           gb.in_pos[b] = (uint16_t)c.src_pos[first + b];
         }
-        auto kfn = ntt_inv_rows_kernel<W, GatherBatch<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, stream, gb, static_cast<const Pair*>(ctx->d_tw_inv), static_cast<const Pair*>(ctx->d_twr_inv), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_inv_rows<W>(ctx, gb, cnt, stream);
       } else {
-        auto kfn = ntt_inv_rows_kernel<W, StridedBatch<W>>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, stream, sb, static_cast<const Pair*>(ctx->d_tw_inv), static_cast<const Pair*>(ctx->d_twr_inv), static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+        launch_inv_rows<W>(ctx, sb, cnt, stream);
       }
-      { auto kfn = ntt_inv_cols_kernel<W, StridedBatch<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, sb, sc, static_cast<const Pair*>(ctx->d_tw_inv), static_cast<const PrimeConst<W>*>(ctx->d_pcs)); }
+      launch_inv_cols<W>(ctx, sb, sc, cnt, stream);
     }
     CERIUM_LAUNCH_CHECK("ntt_inverse");
     return CERIUM_OK;
@@ -157,8 +204,6 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
   if (c.count == 0) return CERIUM_OK;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    using Pair = typename WordTraits<W>::Pair;
-    constexpr int kCols = NttCfg<W>::kCols;
     const int bits = ctx->word_bits;
     if (c.split > 0 && c.count > kSudMaxBatch) return fail(CERIUM_ERR_INVALID, "sud: a two-polynomial launch holds at most 96 limbs");
     {
@@ -205,8 +250,6 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
         epi.factor[b] = (W)f;
         epi.factor_shoup[b] = (W)host::shoup(f, q, bits);
       }
-      const Pair* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
-      const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
       if (c.reduce_src) {
         ReduceLoader<W> ld{};
         ld.src_q = (W)c.src_q;
@@ -217,18 +260,16 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
           static_cast<StridedBatch<W>&>(gb) = cols;
           gb.in = static_cast<const W*>(c.src);
           for (int b = 0; b < cnt; b++) gb.in_pos[b] = (uint16_t)c.src_pos[first + b];
-          auto kfn = ntt_fwd_cols_kernel<W, GatherBatch<W>, ReduceLoader<W>>;
-          CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, gb, ld, tw, pcs);
+          launch_fwd_cols<W>(ctx, gb, ld, cnt, stream);
         } else {
-          auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, ReduceLoader<W>>;
-          CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, ld, tw, pcs);
+          launch_fwd_cols<W>(ctx, cols, ld, cnt, stream);
         }
       } else if (c.lazy_src) {
-        { auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, LazyLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, LazyLoader<W>{}, tw, pcs); }
+        launch_fwd_cols<W>(ctx, cols, LazyLoader<W>{}, cnt, stream);
       } else {
-        { auto kfn = ntt_fwd_cols_kernel<W, StridedBatch<W>, PlainLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, stream, cols, PlainLoader<W>{}, tw, pcs); }
+        launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, stream);
       }
-      { auto kfn = ntt_fwd_rows_kernel<W, StridedBatch<W>, SudEpilogue<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, stream, rows, epi, tw, static_cast<const Pair*>(ctx->d_twr_fwd), pcs); }
+      launch_fwd_rows<W>(ctx, rows, epi, cnt, stream);
     }
     CERIUM_LAUNCH_CHECK("sud");
     return CERIUM_OK;
@@ -726,20 +767,15 @@ static int ntt_ptrs_common(cerium_context* ctx, bool forward, void* const* outs,
   cudaStream_t s = (cudaStream_t)stream;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    using Pair = typename WordTraits<W>::Pair;
-    constexpr int kCols = NttCfg<W>::kCols;
-    const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
     PointerBatch<W> pb{reinterpret_cast<W* const*>(outs), reinterpret_cast<const W* const*>(ins), bases, 1, 0};
     PointerBatch<W> inplace{reinterpret_cast<W* const*>(outs), reinterpret_cast<const W* const*>(outs), bases, 1, 0};
     const int cnt = (int)num_bases;
     if (forward) {
-      const Pair* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
-      { auto kfn = ntt_fwd_cols_kernel<W, PointerBatch<W>, PlainLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, s, pb, PlainLoader<W>{}, tw, pcs); }
-      { auto kfn = ntt_fwd_rows_kernel<W, PointerBatch<W>, StoreEpilogue<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, s, inplace, StoreEpilogue<W>{}, tw, static_cast<const Pair*>(ctx->d_twr_fwd), pcs); }
+      launch_fwd_cols<W>(ctx, pb, PlainLoader<W>{}, cnt, s);
+      launch_fwd_rows<W>(ctx, inplace, StoreEpilogue<W>{}, cnt, s);
     } else {
-      const Pair* tw = static_cast<const Pair*>(ctx->d_tw_inv);
-      { auto kfn = ntt_inv_rows_kernel<W, PointerBatch<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, s, pb, tw, static_cast<const Pair*>(ctx->d_twr_inv), pcs); }
-      { auto kfn = ntt_inv_cols_kernel<W, PointerBatch<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, s, pb, InvScale<W>{}, tw, pcs); }
+      launch_inv_rows<W>(ctx, pb, cnt, s);
+      launch_inv_cols<W>(ctx, pb, InvScale<W>{}, cnt, s);
     }
     CERIUM_LAUNCH_CHECK("ntt_ptrs");
     return CERIUM_OK;
@@ -766,17 +802,13 @@ int cerium_sud_ptrs(cerium_context* ctx, void* const* outs, const void* const* i
   cudaStream_t s = (cudaStream_t)stream;
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
-    using Pair = typename WordTraits<W>::Pair;
-    constexpr int kCols = NttCfg<W>::kCols;
-    const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-    const Pair* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
     const int cnt = (int)num_bases;
     // column pass: second input of every entry -> output limb; row pass in place on the output
     PointerBatch<W> cols{reinterpret_cast<W* const*>(outs), reinterpret_cast<const W* const*>(ins), bases, 2, 1};
     PointerBatch<W> rows{reinterpret_cast<W* const*>(outs), reinterpret_cast<const W* const*>(outs), bases, 1, 0};
     PtrSudEpilogue<W> epi{reinterpret_cast<const W* const*>(ins), static_cast<const W*>(factors)};
-    { auto kfn = ntt_fwd_cols_kernel<W, PointerBatch<W>, PlainLoader<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kCols, cnt), kCols * 16, 0, s, cols, PlainLoader<W>{}, tw, pcs); }
-    { auto kfn = ntt_fwd_rows_kernel<W, PointerBatch<W>, PtrSudEpilogue<W>>; CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, cnt), kRowsPerCta * 16, 0, s, rows, epi, tw, static_cast<const Pair*>(ctx->d_twr_fwd), pcs); }
+    launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, s);
+    launch_fwd_rows<W>(ctx, rows, epi, cnt, s);
     CERIUM_LAUNCH_CHECK("sud_ptrs");
     return CERIUM_OK;
   });

@@ -23,6 +23,8 @@
 //  * Values stay lazy inside a transform ([0,4q) forward, [0,2q) inverse) and are reduced to
 //    [0,q) by the last pass, so every buffer a caller sees is canonical.
 #pragma once
+#include <cstring>
+
 #include "modarith.cuh"
 
 namespace cerium {
@@ -38,7 +40,14 @@ struct NttCfg<uint32_t> {
   static constexpr int kCols = 32;  // 32 * 4 B = 128 B
 };
 
-constexpr int kRowsPerCta = 16;    // row pass: 16 rows of 256 coefficients, 256 threads
+// Tiles of the two passes: `kCols` columns on 16 kCols threads, or rows of 256 coefficients on 16 threads each.  Batches
+// that do not fill the GPU take smaller tiles (the work is spread over all SMs: 160 tiles of 256 threads on 148 SMs
+// leave twelve with twice the work of the others) and copy a row's twiddles into shared memory before they wait
+// for the previous kernel, so that a warp's chain has one memory latency less.  On full launches both cost more than
+// they give: the copies go through the same pipes as the data (71 -> 77 us for 245 limbs).
+constexpr int kRowsPerCta = 16;
+constexpr int kRowsSmall = 4;
+constexpr int kSmallBatchPerSm = 3;  // ... up to this many usual tiles per SM
 // Lane-interleaved level-3 twiddles: [row h (256)][e = 2^t - 1 + g (15)][thread u (16)] pairs per
 // prime; entry = bit-reversed table[((4096 + 16 h + u) << t) + g].
 constexpr int kRowTwPerPrime = 256 * 15 * 16;
@@ -315,29 +324,30 @@ __device__ __forceinline__ typename WordTraits<W>::Pair load_tw(const typename W
 }
 
 // Twiddle addressing of a radix-16 group.  Plain: entry (S << t) + g of the bit-reversed table.
-// Lane-interleaved (kLaneTable): the group's 15 twiddles sit at entries e * 16, e = 2^t - 1 + g,
-// of a table pre-permuted so that the 16 threads of a row read 16 consecutive entries.
-template <bool kLaneTable>
+// Lane-interleaved: the group's 15 twiddles sit at entries e * 16, e = 2^t - 1 + g,
+// of a table pre-permuted so that the 16 threads of a row read 16 consecutive entries.  Group: at entries e.
+enum : int { kTwPlain = 0, kTwLane = 1, kTwGroup = 2 };
+template <int kTw>
 __device__ __forceinline__ uint32_t tw_index(uint32_t S, int t, int g) {
-  return kLaneTable ? (uint32_t)(((1 << t) - 1 + g) * 16) : (S << t) + (uint32_t)g;
+  return kTw == kTwPlain ? (S << t) + (uint32_t)g : (uint32_t)(((1 << t) - 1 + g) * (kTw == kTwLane ? 16 : 1));
 }
 
 // Lane-interleaved table of a prime with double-precision butterflies: twiddles only, two per
 // 16-byte entry; twiddle e = 2^t - 1 + g sits in double number e + 1 of the group's 16 (number 0
 // is padding, so that every layer starts on an entry boundary), entry v of thread u at (v * 16).
-template <typename W>
+template <typename W, bool kGlobalTw>
 __device__ __forceinline__ W lane_tw_fp(const typename WordTraits<W>::Pair* tw, int t, int g) {
   const int slot = (1 << t) + g;
-  const auto pv = __ldg(tw + (slot >> 1) * 16);
+  const auto pv = load_tw<W, kGlobalTw>(tw, (slot >> 1) * 16);
   return (slot & 1) ? pv.y : pv.x;
 }
 
 // Four forward layers on x[0..15]; layer t pairs (j, j + (8 >> t)).  kBin: bound of the inputs
 // (Fp arithmetic only).
-template <typename W, bool kGlobalTw, int kMode, bool kLaneTable = false, int kBin = 0>
+template <typename W, bool kGlobalTw, int kMode, int kTw = kTwPlain, int kBin = 0>
 __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTraits<W>::Pair* tw,
                                             uint32_t S, const Arith<W, kMode>& ar) {
-  constexpr bool kPacked = kLaneTable && kMode == kArithFp;
+  constexpr bool kPacked = kTw == kTwLane && kMode == kArithFp;
   constexpr FpFwdPlan plan = fp_plan_fwd(kBin, kPacked ? kFpLaneK32 : 1);
 #pragma unroll
   for (int t = 0; t < 4; t++) {
@@ -347,10 +357,10 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
     for (int g = 0; g < (1 << t); g++) {
       W w0, w1;
       if constexpr (kPacked) {
-        w0 = lane_tw_fp<W>(tw, t, g);
+        w0 = lane_tw_fp<W, kGlobalTw>(tw, t, g);
         w1 = ar.quotient(w0);
       } else {
-        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kLaneTable>(S, t, g));
+        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kTw>(S, t, g));
         w0 = w.x;
         w1 = w.y;
       }
@@ -365,10 +375,10 @@ __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTrait
 
 // The four inverse layers of the same group, in reverse order; kLayer0 is the pass-local
 // number of the first layer executed (0 for the first level of a pass, 4 for the second).
-template <typename W, bool kGlobalTw, int kMode, int kLayer0, bool kLaneTable = false, int kBin = 0>
+template <typename W, bool kGlobalTw, int kMode, int kLayer0, int kTw = kTwPlain, int kBin = 0>
 __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTraits<W>::Pair* twi,
                                             uint32_t S, const Arith<W, kMode>& ar) {
-  constexpr bool kPacked = kLaneTable && kMode == kArithFp;
+  constexpr bool kPacked = kTw == kTwLane && kMode == kArithFp;
   constexpr FpInvPlan plan = fp_plan_inv(kBin, kPacked ? kFpLaneK32 : 1);
 #pragma unroll
   for (int t = 3; t >= 0; t--) {
@@ -378,10 +388,10 @@ __device__ __forceinline__ void radix16_inv(W (&x)[16], const typename WordTrait
     for (int g = 0; g < (1 << t); g++) {
       W w0, w1;
       if constexpr (kPacked) {
-        w0 = lane_tw_fp<W>(twi, t, g);
+        w0 = lane_tw_fp<W, kGlobalTw>(twi, t, g);
         w1 = ar.quotient(w0);
       } else {
-        const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kLaneTable>(S, t, g));
+        const auto w = load_tw<W, kGlobalTw>(twi, tw_index<kTw>(S, t, g));
         w0 = w.x;
         w1 = w.y;
       }
@@ -451,6 +461,62 @@ __device__ __forceinline__ void vec_unpack(const uint4& v, uint32_t* w) { w[0] =
 __device__ __forceinline__ ulonglong2 vec_pack(const uint64_t* w) { return make_ulonglong2(w[0], w[1]); }
 __device__ __forceinline__ uint4 vec_pack(const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); }
 
+// Twiddles of a row pass's rows in shared memory.  Tables of integer butterflies of 64-bit words are twice as long and
+// stay in global memory.
+template <typename W, int kRows>
+struct RowTwiddles {
+  using Pair = typename WordTraits<W>::Pair;
+  static constexpr int kLane = sizeof(W) == 8 ? 8 * 16 : 15 * 16;  // entries of a row's lane table
+  static constexpr int kGroupPitch = 17;                           // rows of a warp in different banks
+  Pair lane[kRows][kLane];
+  Pair group[kRows][kGroupPitch];
+};
+template <typename W, int kRows, bool kStage>
+struct alignas(16) RowsBuffer {
+  W tile[kRows * kRowPitch];
+  RowTwiddles<W, kStage ? kRows : 1> tw;
+};
+
+template <int kBytes>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+#if defined(CERIUM_EMU)
+  std::memcpy(dst, src, kBytes);
+#else
+  if constexpr (kBytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "n"(kBytes) : "memory");
+#endif
+}
+// Starts the copies of this warp's two rows (h0: first row of the CTA); row_twiddles_wait() before they are used.
+template <typename W, int kRows>
+__device__ __forceinline__ void row_twiddles_start(RowTwiddles<W, kRows>& to, const typename WordTraits<W>::Pair* tw,
+                                                   const typename WordTraits<W>::Pair* twr, int h0) {
+  using RT = RowTwiddles<W, kRows>;
+  using Pair = typename RT::Pair;
+  const int lane = threadIdx.x & 31, r0 = threadIdx.x >> 5 << 1;
+  constexpr int kChunks = 2 * RT::kLane * (int)sizeof(Pair) / 16;  // the lane tables of neighbouring rows adjoin
+  const char* src = reinterpret_cast<const char*>(twr + (size_t)(h0 + r0) * RT::kLane);
+  char* dst = reinterpret_cast<char*>(to.lane[r0]);
+#pragma unroll
+  for (int k = 0; k < (kChunks + 31) / 32; k++) {
+    const int i = lane + 32 * k;
+    if (kChunks % 32 == 0 || i < kChunks) copy_async<16>(dst + i * 16, src + i * 16);
+  }
+  // level 2: entry e = 2^t - 1 + g of row r is table entry ((256 + h) << t) + g
+  const int r = r0 + (lane >> 4), e = lane & 15;
+  if (e < 15) {
+    const int t = e < 1 ? 0 : e < 3 ? 1 : e < 7 ? 2 : 3;
+    copy_async<sizeof(Pair)>(&to.group[r][e], tw + (((uint32_t)(256 + h0 + r) << t) + (uint32_t)(e - ((1 << t) - 1))));
+  }
+}
+__device__ __forceinline__ void row_twiddles_wait() {
+#if !defined(CERIUM_EMU)
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+  __syncwarp();
+}
+
 // Runs one of the instantiations of a kernel body: the arithmetic policy of this CTA's prime
 // (BODY is a template name taking <W, mode, ...>; ARGS its call arguments in parentheses).
 #define CERIUM_TARGS(...) __VA_ARGS__
@@ -518,11 +584,10 @@ struct ReduceLoader {
   }
 };
 
-template <typename W, int kMode, typename Batch, typename Loader>
+template <typename W, int kMode, int kCols, typename Batch, typename Loader>
 __device__ __forceinline__ void ntt_fwd_cols_body(const Batch& batch, const Loader& loader, int b,
                                                   const PrimeConst<W>& pc, W* tile,
                                                   const typename WordTraits<W>::Pair* stw) {
-  constexpr int kCols = NttCfg<W>::kCols;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, c = tid % kCols, u = tid / kCols;
   const int col = blockIdx.x * kCols + c;
@@ -547,35 +612,34 @@ __device__ __forceinline__ void ntt_fwd_cols_body(const Batch& batch, const Load
     for (int j = 0; j < 16; j++) x[j] = ar.enter(loader.apply(x[j], b, pc));
   }
   __syncthreads();
-  radix16_fwd<W, false, kMode, false, Loader::kFpBound>(x, stw, 1u, ar);
+  radix16_fwd<W, false, kMode, kTwPlain, Loader::kFpBound>(x, stw, 1u, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) t_strided[j * 16 * kCols] = x[j];
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_own[j * kCols];
-  radix16_fwd<W, false, kMode, false, fp_plan_fwd(Loader::kFpBound).out>(x, stw, 16u + (uint32_t)u, ar);
+  radix16_fwd<W, false, kMode, kTwPlain, fp_plan_fwd(Loader::kFpBound).out>(x, stw, 16u + (uint32_t)u, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) out[j * 256] = x[j];
 }
 
 // Column pass (levels 0 and 1).  grid = (256 / kCols, limbs), block = 16 * kCols.
 // Element (h, l) of a limb is word h * 256 + l; the CTA owns kCols adjacent columns.
-template <typename W, typename Batch, typename Loader>
-__global__ void __launch_bounds__(NttCfg<W>::kCols * 16, sizeof(W) == 8 ? 3 : 2)
+template <typename W, int kCols, typename Batch, typename Loader>
+__global__ void __launch_bounds__(kCols * 16, (sizeof(W) == 8 ? 768 : 1024) / (kCols * 16))
     ntt_fwd_cols_kernel(const Batch batch, const Loader loader,
                         const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  constexpr int kCols = NttCfg<W>::kCols;
   __shared__ W tile[256 * kCols];
   __shared__ Pair stw[256];
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
-  if (threadIdx.x < 256) stw[threadIdx.x] = __ldg(tw_all + (size_t)pi * kN + threadIdx.x);
+  for (int k = threadIdx.x; k < 256; k += kCols * 16) stw[k] = __ldg(tw_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_cols_body, CERIUM_TARGS(Batch, Loader), (batch, loader, b, pc, tile, stw));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw));
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
@@ -766,16 +830,18 @@ __device__ __forceinline__ void load16<uint32_t>(const uint32_t* src, uint32_t (
   }
 }
 
-template <typename W, int kMode, typename Batch, typename Epilogue>
+template <typename W, int kMode, int kRows, bool kStage, typename Batch, typename Epilogue>
 __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epilogue& epi, int b, uint32_t pi,
-                                                  const PrimeConst<W>& pc, W* tile,
+                                                  const PrimeConst<W>& pc, RowsBuffer<W, kRows, kStage>& buf,
                                                   const typename WordTraits<W>::Pair* tw,
                                                   const typename WordTraits<W>::Pair* twr) {
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
+  constexpr bool kStaged = kStage && (sizeof(W) == 4 || kMode == kArithFp);
+  W* tile = buf.tile;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
-  const int h = blockIdx.x * kRowsPerCta + r;
+  const int h = blockIdx.x * kRows + r;
   const W* row = batch.in_limb(b) + (unsigned)(h * 256 + u);
   W* limb_out = batch.out_limb(b);
   W* drow = limb_out + (unsigned)(h * 256);
@@ -789,14 +855,16 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
   for (int j = 0; j < 16; j++) x[j] = row[j * 16];
 #pragma unroll
   for (int k = 0; k < RV::kPerThread; k++) epi.prefetch(b, h * 256 + (u + 16 * k) * RV::kWords);
-  radix16_fwd<W, true, kMode, false, kFpFwdMid>(x, tw, 256u + (uint32_t)h, ar);
+  if (kStaged) row_twiddles_wait();
+  radix16_fwd<W, !kStaged, kMode, kStaged ? kTwGroup : kTwPlain, kFpFwdMid>(x, kStaged ? buf.tw.group[kStaged ? r : 0] : tw, 256u + (uint32_t)h, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) t_strided[j * 17] = x[j];
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_own[j];
   // level 3: this thread's 15 twiddles from the lane-interleaved table of row h
-  radix16_fwd<W, true, kMode, true, kFpFwdL3>(x, twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  radix16_fwd<W, !kStaged, kMode, kTwLane, kFpFwdL3>(
+      x, kStaged ? buf.tw.lane[kStaged ? r : 0] + u : twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.template finish_fwd<Epilogue::kCanonicalInput>(x[j], pc.one_shoup);
   // own 16 words -> swizzled vectors -> coalesced vectors, then epilogue and store
@@ -833,38 +901,42 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
 
 // Row pass (levels 2 and 3): reads the column pass's result from the batch's `in` stack and
 // writes the finished transform to its `out` stack (the two may be the same buffer).
-// grid = (256 / kRowsPerCta, limbs), block = 16 * kRowsPerCta; 16 threads own one row.
-template <typename W, typename Batch, typename Epilogue>
-__global__ void __launch_bounds__(kRowsPerCta * 16, 3)
+// grid = (256 / kRows, limbs), block = 16 * kRows; 16 threads own one row.
+template <typename W, int kRows, bool kStage, typename Batch, typename Epilogue>
+__global__ void __launch_bounds__(kRows * 16, 768 / (kRows * 16))
     ntt_fwd_rows_kernel(const Batch batch, const Epilogue epi,
                         const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const typename WordTraits<W>::Pair* __restrict__ twr_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  __shared__ __align__(16) W tile[kRowsPerCta * kRowPitch];
+  __shared__ RowsBuffer<W, kRows, kStage> buf;
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   const Pair* tw = tw_all + (size_t)pi * kN;
   const Pair* twr = twr_all + (size_t)pi * kRowTwPerPrime;
+  if constexpr (kStage)
+    if (sizeof(W) == 4 || pc.fp_ok != 0) row_twiddles_start(buf.tw, tw, twr, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_rows_body, CERIUM_TARGS(Batch, Epilogue), (batch, epi, b, pi, pc, tile, tw, twr));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_rows_body, CERIUM_TARGS(kRows, kStage, Batch, Epilogue), (batch, epi, b, pi, pc, buf, tw, twr));
 }
 
 // ---------------------------------------------------------------------------------------
 // inverse transform
 // ---------------------------------------------------------------------------------------
 
-template <typename W, int kMode, typename Batch>
-__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, W* tile,
+template <typename W, int kMode, int kRows, bool kStage, typename Batch>
+__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, RowsBuffer<W, kRows, kStage>& buf,
                                                   const typename WordTraits<W>::Pair* twi,
                                                   const typename WordTraits<W>::Pair* twri) {
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
+  constexpr bool kStaged = kStage && (sizeof(W) == 4 || kMode == kArithFp);
+  W* tile = buf.tile;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
-  const int h = blockIdx.x * kRowsPerCta + r;
+  const int h = blockIdx.x * kRows + r;
   const W* limb_in = batch.in_limb(b);
   const W* src = limb_in + h * 256;
   const uint32_t elt = batch.gather_elt();
@@ -898,7 +970,9 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
     vec_unpack(vrow[row_vec_slot<W>(u * RV::kPerThread + jj)], &x[jj * RV::kWords]);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.enter(x[j]);
-  radix16_inv<W, true, kMode, 0, true, kFpCanon>(x, twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  if (kStaged) row_twiddles_wait();
+  radix16_inv<W, !kStaged, kMode, 0, kTwLane, kFpCanon>(
+      x, kStaged ? buf.tw.lane[kStaged ? r : 0] + u : twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
   if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, kFpInvRowsExMask, ar);
   __syncwarp();
   W* t_own = trow + (unsigned)(u * 17);  // row_pos(u * 16 + j) = u * 17 + j
@@ -908,28 +982,30 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_strided[j * 17];
-  radix16_inv<W, true, kMode, 4, false, kFpInvL3>(x, twi, 256u + (uint32_t)h, ar);
+  radix16_inv<W, !kStaged, kMode, 4, kStaged ? kTwGroup : kTwPlain, kFpInvL3>(x, kStaged ? buf.tw.group[kStaged ? r : 0] : twi, 256u + (uint32_t)h, ar);
   W* dcol = dst + u;
 #pragma unroll
   for (int j = 0; j < 16; j++) dcol[j * 16] = x[j];
 }
 
 // Row pass (levels 3 and 2): in -> out; values leave below 2q (strict; 4q for 64-bit words) or below 2^10 q (lazy).
-template <typename W, typename Batch>
-__global__ void __launch_bounds__(kRowsPerCta * 16, 3)
+template <typename W, int kRows, bool kStage, typename Batch>
+__global__ void __launch_bounds__(kRows * 16, 768 / (kRows * 16))
     ntt_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                         const typename WordTraits<W>::Pair* __restrict__ twri_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  __shared__ __align__(16) W tile[kRowsPerCta * kRowPitch];
+  __shared__ RowsBuffer<W, kRows, kStage> buf;
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   const Pair* twi = twi_all + (size_t)pi * kN;
   const Pair* twri = twri_all + (size_t)pi * kRowTwPerPrime;
+  if constexpr (kStage)
+    if (sizeof(W) == 4 || pc.fp_ok != 0) row_twiddles_start(buf.tw, twi, twri, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, Batch, (batch, b, pc, tile, twi, twri));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, CERIUM_TARGS(kRows, kStage, Batch), (batch, b, pc, buf, twi, twri));
 }
 
 // Optional per-limb scalar of the finished inverse transform (exact base conversion wants x * [Qhat^-1] mod q):
@@ -940,11 +1016,10 @@ struct InvScale {
   const W* add;          // per batch entry, added to the scaled value modulo q (rounding term), may be null
 };
 
-template <typename W, int kMode, typename Batch>
+template <typename W, int kMode, int kCols, typename Batch>
 __device__ __forceinline__ void ntt_inv_cols_body(const Batch& batch, const InvScale<W>& sc, int b,
                                                   const PrimeConst<W>& pc, W* tile,
                                                   const typename WordTraits<W>::Pair* stw) {
-  constexpr int kCols = NttCfg<W>::kCols;
   const Arith<W, kMode> ar(pc);
   const W q = pc.q;
   const int tid = threadIdx.x, c = tid % kCols, u = tid / kCols;
@@ -960,7 +1035,7 @@ __device__ __forceinline__ void ntt_inv_cols_body(const Batch& batch, const InvS
     if (kMode == kArithLazy) x[j] = reduce_lazy(x[j], pc.one_shoup, (W)0 - pc.q);  // back below 4q for the second pass
   }
   __syncthreads();
-  radix16_inv<W, false, kMode, 0, false, kFpInvMid>(x, stw, 16u + (uint32_t)u, ar);
+  radix16_inv<W, false, kMode, 0, kTwPlain, kFpInvMid>(x, stw, 16u + (uint32_t)u, ar);
   if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, kFpInvColsExMask, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) t_own[j * kCols] = x[j];
@@ -988,22 +1063,21 @@ __device__ __forceinline__ void ntt_inv_cols_body(const Batch& batch, const InvS
 
 // Column pass (levels 1 and 0), in place on the output limb of the row pass; scales by
 // N^-1 and reduces to [0, q).
-template <typename W, typename Batch>
-__global__ void __launch_bounds__(NttCfg<W>::kCols * 16, sizeof(W) == 8 ? 3 : 2)
+template <typename W, int kCols, typename Batch>
+__global__ void __launch_bounds__(kCols * 16, (sizeof(W) == 8 ? 768 : 1024) / (kCols * 16))
     ntt_inv_cols_kernel(const Batch batch, const InvScale<W> sc,
                         const typename WordTraits<W>::Pair* __restrict__ twi_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  constexpr int kCols = NttCfg<W>::kCols;
   __shared__ W tile[256 * kCols];
   __shared__ Pair stw[256];
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
-  if (threadIdx.x < 256) stw[threadIdx.x] = __ldg(twi_all + (size_t)pi * kN + threadIdx.x);
+  for (int k = threadIdx.x; k < 256; k += kCols * 16) stw[k] = __ldg(twi_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_cols_body, Batch, (batch, sc, b, pc, tile, stw));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_cols_body, CERIUM_TARGS(kCols, Batch), (batch, sc, b, pc, tile, stw));
 }
 
 }  // namespace cerium
