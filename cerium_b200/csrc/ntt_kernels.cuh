@@ -564,7 +564,10 @@ struct LazyLoader {
   __device__ __forceinline__ W apply(W x, int /*b*/, const PrimeConst<W>& /*pc*/) const { return x; }
 };
 
-constexpr int kSudMaxBatch = 96;  // limbs per launch when per-limb scalars travel as parameters
+// limbs per launch when per-limb scalars travel as parameters (4 KB of them at 128 limbs of 64-bit words).  Both
+// polynomials of a key switch over up to 64 limbs share one launch pair: a 32-bit rotation of 51 limbs took 213.8 us with
+// two launch pairs (limit 96), now 207.5
+constexpr int kSudMaxBatch = 128;
 
 // Source residues belong to another (possibly larger) modulus src_q: optionally add pre_add
 // mod src_q (rounding), reduce into [0, q) of the target prime, optionally subtract
