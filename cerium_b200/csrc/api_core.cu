@@ -205,7 +205,7 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     const int bits = ctx->word_bits;
-    if (c.split > 0 && c.count > kSudMaxBatch) return fail(CERIUM_ERR_INVALID, "sud: a two-polynomial launch holds at most 96 limbs");
+    if (c.split > 0 && c.count > kSudMaxBatch) return fail(CERIUM_ERR_INVALID, "sud: a two-polynomial launch holds at most 128 limbs");
     {
       // the tail reads minuend and addend as 16-byte vectors
       const size_t wb = sizeof(W);

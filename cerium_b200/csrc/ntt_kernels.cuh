@@ -914,7 +914,10 @@ __global__ void __launch_bounds__(kRows * 16, 768 / (kRows * 16))
   using Pair = typename WordTraits<W>::Pair;
   __shared__ RowsBuffer<W, kRows, kStage> buf;
   grid_dependency_launch();
-  const int b = blockIdx.y;
+  // From the last limb to the first, against the direction of the column pass: what that pass wrote last is still in L2
+  // and is read, and overwritten, before it goes to memory.  The reader of a result larger than L2 then starts at the
+  // first limb for the same reason.  (Rotation of 35 limbs 367 -> 355.6 us, transform of 384 limbs 190.6 -> 187.2 us.)
+  const int b = (int)(gridDim.y - 1 - blockIdx.y);
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   const Pair* tw = tw_all + (size_t)pi * kN;
@@ -1075,7 +1078,8 @@ __global__ void __launch_bounds__(kCols * 16, (sizeof(W) == 8 ? 768 : 1024) / (k
   __shared__ W tile[256 * kCols];
   __shared__ Pair stw[256];
   grid_dependency_launch();
-  const int b = blockIdx.y;
+  // against the direction of the row pass, as in the forward transform
+  const int b = (int)(gridDim.y - 1 - blockIdx.y);
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 16) stw[k] = __ldg(twi_all + (size_t)pi * kN + k);
