@@ -248,7 +248,6 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     }
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
     // every local extended limb (Q and extension) in one launch
-    g.first_limb = 0;
     { auto kfn = inner_product_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, pcs); }
     CERIUM_LAUNCH_CHECK("inner_product");
     return CERIUM_OK;

@@ -32,6 +32,14 @@ struct Vec16<uint64_t> {
     r.v[1] = t.y;
     return r;
   }
+  // words that nothing reads again soon: first to leave L2
+  static __device__ __forceinline__ Vec16 load_once(const uint64_t* p) {
+    const ulonglong2 t = __ldcs(reinterpret_cast<const ulonglong2*>(p));
+    Vec16 r;
+    r.v[0] = t.x;
+    r.v[1] = t.y;
+    return r;
+  }
   __device__ __forceinline__ void store(uint64_t* p) const {
     *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]);
   }
@@ -42,6 +50,15 @@ struct Vec16<uint32_t> {
   uint32_t v[4];
   static __device__ __forceinline__ Vec16 load(const uint32_t* p) {
     const uint4 t = *reinterpret_cast<const uint4*>(p);
+    Vec16 r;
+    r.v[0] = t.x;
+    r.v[1] = t.y;
+    r.v[2] = t.z;
+    r.v[3] = t.w;
+    return r;
+  }
+  static __device__ __forceinline__ Vec16 load_once(const uint32_t* p) {
+    const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p));
     Vec16 r;
     r.v[0] = t.x;
     r.v[1] = t.y;
@@ -263,6 +280,12 @@ __global__ void __launch_bounds__(kEwThreads) mod2_kernel(const Mod2Args<W> g, c
 // (own_digit[b] == d) the raised value is the NTT-form input limb, which is read in
 // place from `own` instead of from `raised` (cerium/compiler/backend/kernel_instruction.h:
 // 823-838 moves it; here it is never copied).
+// Bound by memory: 482 MB for 35 + 5 limbs and 7 digits of 64-bit words.  The key is more than half of that, and nobody
+// reads it or the raised limbs again before they would be gone: both are loaded to leave L2 first, so the raised limbs
+// that the transform wrote last are still there and the accumulators that the ModDown reads next stay.  Loads in flight
+// come from CTAs, not from the loop: 4 CTAs (64 registers) and a step at a time for 64-bit words, 5 and two steps for
+// 32-bit words.  With one step more or four registers over the limit a CTA is lost and a rotation of 35 limbs takes 364 us.
+// Against plain loads and no limit: 35 limbs 355.6 -> 349.2 us, 51 32-bit limbs 205.8 -> 200.0 us.
 // Restates the EVKMUL / EVKMUL_EXT groups of cerium/compiler/backend/compiler_keyswitch.cc:
 // 336-358 and :695-772 as one launch.
 template <typename W>
@@ -277,7 +300,6 @@ struct InnerProductArgs {
   size_t evk_poly_stride;
   size_t evk_limb_stride;
   Limbs<W> out0, out1;    // [LK][N]
-  int first_limb;         // grid.y covers extended limbs first_limb, first_limb + 1, ...
   int dnum;
   uint32_t own_elt;       // not 0: `own` is read through the Galois automorphism of this element
                           // (word i of a limb is own[pi(i)]), i.e. the rotation of the input is folded in
@@ -287,12 +309,12 @@ struct InnerProductArgs {
 };
 
 template <typename W>
-__global__ void __launch_bounds__(kEwThreads)
+__global__ void __launch_bounds__(kEwThreads, sizeof(W) == 8 ? 4 : 5)
     inner_product_kernel(const InnerProductArgs<W> g, const PrimeConst<W>* __restrict__ pcs) {
   grid_dependency_launch();
   grid_dependency_wait();
   using V = Vec16<W>;
-  const int b = g.first_limb + blockIdx.y;
+  const int b = blockIdx.y;
   const PrimeConst<W> pc = pcs[g.prime[b]];
   const int idx = (blockIdx.x * kEwThreads + threadIdx.x) * V::kLanes;
   Acc2<W> acc0[V::kLanes], acc1[V::kLanes];
@@ -302,7 +324,8 @@ __global__ void __launch_bounds__(kEwThreads)
     acc1[l].clear();
   }
   const int own_digit = g.own_digit[b];
-#pragma unroll 2
+  constexpr int kUnroll = sizeof(W) == 8 ? 1 : 2;
+#pragma unroll kUnroll
   for (int d = 0; d < g.dnum; d++) {
     const bool is_own = d == own_digit;
     const W* ap = is_own ? g.own + (size_t)b * g.own_stride + idx
@@ -315,10 +338,10 @@ __global__ void __launch_bounds__(kEwThreads)
 #pragma unroll
       for (int l = 0; l < V::kLanes; l++) a.v[l] = limb[galois_source_index((uint32_t)(idx + l), g.own_elt)];
     } else {
-      a = V::load(ap);
+      a = V::load_once(ap);
     }
-    const V k0 = V::load(kp);
-    const V k1 = V::load(kp + g.evk_poly_stride);
+    const V k0 = V::load_once(kp);
+    const V k1 = V::load_once(kp + g.evk_poly_stride);
 #pragma unroll
     for (int l = 0; l < V::kLanes; l++) {
       acc0[l].mad(a.v[l], k0.v[l]);
