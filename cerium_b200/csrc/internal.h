@@ -49,13 +49,13 @@ int fail(int code, const std::string& msg);
 #define CERIUM_LAUNCH(kfn, grid, block, smem, stream, ...) \
   ::cerium_emu::launch((grid), (block), (smem), [=]() { kfn(__VA_ARGS__); })
 #else
-// All kernels ask for one split of the SM's memory, 132 KB shared and 96 KB L1 (57 % of the 228 KB rounds up to it): what
-// three CTAs of a transform need.  Left to the driver every kernel gets the split that suits it alone, an SM has to drain
-// before it changes from one to the next, and the overlap of dependent launches is lost at every such boundary (a
-// rotation of 12 limbs, 11 launches: 132 us, 126 with one split; with 164 KB shared and more the transforms lose the L1
-// that holds their twiddles: 193 us for 384 limbs, 212 with 228 KB).  The attribute is set at a kernel's first
-// launch on a device.
-constexpr int kCarveoutPercent = 57;
+// All kernels ask for one split of the SM's memory, 164 KB shared and 64 KB L1 (71 % of the 228 KB rounds up to it): what
+// four CTAs of a transform's row pass need.  Left to the driver every kernel gets the split that suits it alone, an SM
+// has to drain before it changes from one to the next, and the overlap of dependent launches is lost at every such
+// boundary (a rotation of 12 limbs, 11 launches: 132 us; 127 with one split of 132 KB, then 119.5; 115.7 with 164 KB,
+// where the next kernel's CTAs find more room beside those that finish).  With 228 KB the transforms lose the L1 that
+// holds their twiddles (384 limbs: 212 us against 188).  The attribute is set at a kernel's first launch on a device.
+constexpr int kCarveoutPercent = 71;
 inline void prefer_carveout(const void* kfn) {
   constexpr size_t kSlots = 1024;  // open addressing; a full table only means that the attribute is set again
   static std::atomic<uintptr_t> seen[kSlots] = {};
