@@ -1,0 +1,23 @@
+"""Transforms on both sides of the batch size where the passes change from small tiles (up to three usual tiles per SM: 27
+limbs on 148 SMs) to usual ones, for every arithmetic: exact against the oracle, forward and inverse."""
+import numpy as np
+import pytest
+
+from tests import backends, parity_cases as pc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("word_bits", [64, 32])
+@pytest.mark.parametrize("count", [1, 27, 28, 61])
+def test_ntt_batch_sizes(word_bits, count):
+    mods = pc.moduli_for(word_bits, 3, 1)
+    h = pc.Harness(backends.CudaBackend(), word_bits, mods)
+    idx = [(count + b) % 3 for b in range(count)]
+    x = pc.rand_limbs(np.random.default_rng(count), mods, idx)
+    want = h.orc.ntt_forward(x, idx)
+    d = h.up(x)
+    h.ctx.ntt_forward(h.p(d), h.p(d), idx)
+    assert np.array_equal(h.down(d), want)
+    h.ctx.ntt_inverse(h.p(d), h.p(d), idx)
+    assert np.array_equal(h.down(d), x)
