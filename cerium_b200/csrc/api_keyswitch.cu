@@ -218,8 +218,11 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
 // Step 4 on the digits that keyswitch_raise left in the plan: inner product with `evk` into the
 // plan's accumulators (both polynomials, every local extended limb).  accumulate: add to what the
 // accumulators hold (the giant steps of a BSGS multiply-accumulate sum up in the extended basis).
+// add0 / add1: [P] times these join the Q limbs, what the reference's PMU group does before a ModDown that divides by
+// Q limbs as well.  As one more product of the sums they cost one read; as launches of their own they read and wrote the
+// accumulators again (7 us each at 24 limbs).
 int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cudaStream_t stream, uint32_t pre_elt = 0,
-                    bool accumulate = false) {
+                    bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr) {
   cerium_context* ctx = ks->ctx;
   const size_t n = kN;
   const int LK = ks->LK, dnum = ks->dnum;
@@ -242,6 +245,13 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     g.out0 = {acc, n};
     g.out1 = {acc + (size_t)LK * n, n};
     g.dnum = dnum;
+    if (add0 != nullptr || add1 != nullptr) {
+      g.add0 = static_cast<const W*>(add0);
+      g.add1 = static_cast<const W*>(add1);
+      g.add_stride = n;
+      g.add_limbs = ks->L;
+      for (int b = 0; b < ks->L; b++) g.add_factor[b] = (W)ks->pmod[b];
+    }
     for (int b = 0; b < LK; b++) {
       g.prime[b] = (uint8_t)ks->all_idx[b];
       g.own_digit[b] = (int8_t)ks->own_digit[b];
@@ -258,8 +268,8 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
 // comm: needed by plans with split extension limbs, whose accumulators' extension limbs are
 // all-gathered (coefficient form) between steps 5 and 6.
 // r > 0: the last r Q limbs are divided away in the same step (they join the extension limbs:
-// cerium/compiler/backend/compiler_keyswitch.cc:26-39, 402-412); add0 / add1 then enter as the
-// reference's PMU group does, acc += [P] * add on the Q limbs, and the outputs hold L - r limbs.
+// cerium/compiler/backend/compiler_keyswitch.cc:26-39, 402-412); additions have then entered the accumulators before
+// (keyswitch_inner), and the outputs hold L - r limbs.
 int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* add0, const void* add1,
                       cudaStream_t stream, uint32_t pre_elt = 0, uint32_t store_elt = 0, cerium_comm* comm = nullptr,
                       int r = 0) {
@@ -280,13 +290,6 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
     if (r > 0) {
       const cerium_keyswitch::FusedDown& fd = ks->fused[r - 1];
       const int Lr = L - r;
-      // PMU: acc_p += [P] * add_p on all Q limbs (the dropped ones as well: they are divided away below)
-      for (int p = 0; p < 2; p++) {
-        const void* add = p == 0 ? add0 : add1;
-        if (add == nullptr) continue;
-        W* ap = acc + (size_t)p * LK * n;
-        if (int rc = cerium_ewise(ctx, CERIUM_EW_PMU, ap, n, ap, n, add, n, nullptr, 0, ks->pmod.data(), ks->q_idx.data(), L, stream)) return rc;
-      }
       // 5. iNTT of the extension limbs and the dropped Q limbs of both accumulators, in place
       {
         NttCall c{acc, acc, n, n, fd.ext_pos.data(), fd.ext_prime.data(), (int)fd.ext_pos.size()};
@@ -434,8 +437,9 @@ int keyswitch_inner_moddown(cerium_keyswitch* ks, void* out0, void* out1, const 
                             uint32_t store_elt = 0, cerium_comm* comm = nullptr, int r = 0) {
   if (ks->ext_split && comm == nullptr)
     return fail(CERIUM_ERR_INVALID, "keyswitch: a plan with split extension limbs needs a communicator");
-  if (int rc = keyswitch_inner(ks, cpoly, evk, stream, pre_elt)) return rc;
-  return keyswitch_moddown(ks, out0, out1, add0, add1, stream, pre_elt, store_elt, comm, r);
+  const bool early = r > 0;  // all Q limbs get the additions (the dropped ones as well: they are divided away)
+  if (int rc = keyswitch_inner(ks, cpoly, evk, stream, pre_elt, false, early ? add0 : nullptr, early ? add1 : nullptr)) return rc;
+  return keyswitch_moddown(ks, out0, out1, early ? nullptr : add0, early ? nullptr : add1, stream, pre_elt, store_elt, comm, r);
 }
 
 int keyswitch_finish(cerium_keyswitch* ks, void* out0, void* out1, const void* gathered, const void* cpoly,
@@ -1228,12 +1232,16 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
   //    transform and of the digits' own limbs) and its product with the key, summed in the extended basis
   void* coef = static_cast<char*>(ks->ws) + ks->o_coef * wb;
   bool first = true;
+  int last = -1;
+  for (int i = 0; i < n_giant; i++)
+    if (have[i] && giant_elts[i] != 1) last = i;
   for (int i = 0; i < n_giant; i++) {
     if (!have[i] || giant_elts[i] == 1) continue;
     const char* s1 = inner + (size_t)i * 2 * poly + poly;
     if (int r2 = keyswitch_begin(ks, coef, s1, st, giant_elts[i])) return r2;
     if (int r2 = keyswitch_raise(ks, coef, st)) return r2;
-    if (int r2 = keyswitch_inner(ks, s1, giant_keys[i], st, giant_elts[i], !first)) return r2;
+    const bool add = i == last && rescale_levels > 0;
+    if (int r2 = keyswitch_inner(ks, s1, giant_keys[i], st, giant_elts[i], !first, add ? sum0 : nullptr, add ? sum1 : nullptr)) return r2;
     first = false;
   }
   if (first) {
@@ -1244,7 +1252,8 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
   }
   // 5. ONE ModDown (with the rescale levels in the same division); the sums enter as the PMU
   //    pre-addition: as addends of the last kernel when nothing else is divided away
-  return keyswitch_moddown(ks, out0, out1, sum0, sum1, st, 0, 0, nullptr, rescale_levels);
+  const bool late = rescale_levels == 0;
+  return keyswitch_moddown(ks, out0, out1, late ? sum0 : nullptr, late ? sum1 : nullptr, st, 0, 0, nullptr, rescale_levels);
 }
 
 int cerium_rescale(cerium_context* ctx, int round_mode, void* out, const void* in, const uint32_t* q_idx, int L,

@@ -304,6 +304,11 @@ struct InnerProductArgs {
   uint32_t own_elt;       // not 0: `own` is read through the Galois automorphism of this element
                           // (word i of a limb is own[pi(i)]), i.e. the rotation of the input is folded in
   int accumulate;         // not 0: the products are added to the (canonical) values out0 / out1 already hold
+  const W* add0;          // not null: add_factor[b] * add_p[b] joins the sums of the limbs b < add_limbs, each of which
+  const W* add1;          // belongs to a digit (its own term is below q^2, so the accumulator has room for one more)
+  size_t add_stride;
+  int add_limbs;
+  W add_factor[kEwMaxLimbs];
   uint8_t prime[kEwMaxLimbs];     // prime index of extended limb b
   int8_t own_digit[kEwMaxLimbs];  // digit that limb b belongs to (-1 for extension limbs)
 };
@@ -346,6 +351,20 @@ __global__ void __launch_bounds__(kEwThreads, sizeof(W) == 8 ? 4 : 5)
     for (int l = 0; l < V::kLanes; l++) {
       acc0[l].mad(a.v[l], k0.v[l]);
       acc1[l].mad(a.v[l], k1.v[l]);
+    }
+  }
+  if (b < g.add_limbs) {
+    const W f = g.add_factor[b];
+    const size_t at = (size_t)b * g.add_stride + idx;
+    if (g.add0 != nullptr) {
+      const V x = V::load_once(g.add0 + at);
+#pragma unroll
+      for (int l = 0; l < V::kLanes; l++) acc0[l].mad(x.v[l], f);
+    }
+    if (g.add1 != nullptr) {
+      const V x = V::load_once(g.add1 + at);
+#pragma unroll
+      for (int l = 0; l < V::kLanes; l++) acc1[l].mad(x.v[l], f);
     }
   }
   V o0, o1;
