@@ -79,6 +79,8 @@ static inline unsigned __brev(unsigned x) {
 }
 template <typename T>
 static inline T __ldg(const T* p) { return *p; }
+template <typename T>
+static inline T __ldcs(const T* p) { return *p; }
 static inline unsigned atomicOr(unsigned* p, unsigned v) { return __atomic_fetch_or(p, v, __ATOMIC_RELAXED); }
 
 // ---- runtime API subset ----
