@@ -49,14 +49,15 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // ---------------------------------------------------------------------------------------
 
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
-static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm * ctx->sm_count; }
+template <typename W>
+static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
 
 template <typename W, typename Batch, typename Loader>
 static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loader& loader, int limbs, cudaStream_t stream) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch(ctx, limbs)) {
+  if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, loader, tw, pcs);
   } else {
@@ -69,7 +70,7 @@ static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvSc
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch(ctx, limbs)) {
+  if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_inv_cols_kernel<W, kCols / 2, Batch>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, scale, tw, pcs);
   } else {
@@ -83,7 +84,7 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch(ctx, limbs)) {
+  if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, epi, tw, twr, pcs);
   } else {
@@ -97,7 +98,7 @@ static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, 
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_inv);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch(ctx, limbs)) {
+  if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
   } else {

@@ -1,5 +1,5 @@
-"""Transforms on both sides of the batch size where the passes change from small tiles (up to three usual tiles per SM: 27
-limbs on 148 SMs) to usual ones, for every arithmetic: exact against the oracle, forward and inverse."""
+"""Transforms on both sides of the batch size where the passes change from small tiles (64 limbs of 64-bit words, 74
+of 32-bit words on 148 SMs) to usual ones, for every arithmetic: exact against the oracle, forward and inverse."""
 import numpy as np
 import pytest
 
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("word_bits", [64, 32])
-@pytest.mark.parametrize("count", [1, 27, 28, 61])
+@pytest.mark.parametrize("count", [1, 27, 64, 65, 74, 75])
 def test_ntt_batch_sizes(word_bits, count):
     mods = pc.moduli_for(word_bits, 3, 1)
     h = pc.Harness(backends.CudaBackend(), word_bits, mods)
