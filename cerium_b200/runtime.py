@@ -309,8 +309,9 @@ class CKKSEncryptor:
             w[half].copy_(stage[half], non_blocking=True)
         m, a = w[:len(idx)], w[len(idx):]
         ew, st = ctx.handle.ewise, ctx.stream()
+        key = self._key_rows(idx)       # gathered rows are this call's own: held until the result is back on the host
         ew(_capi.EW_REDUCE, w.data_ptr(), w.data_ptr(), idx + idx, stream=st)     # a program's outputs may exceed q
-        ew(_capi.EW_MAD, m.data_ptr(), a.data_ptr(), idx, b=self._key_rows(idx).data_ptr(), c=m.data_ptr(), stream=st)
+        ew(_capi.EW_MAD, m.data_ptr(), a.data_ptr(), idx, b=key.data_ptr(), c=m.data_ptr(), stream=st)
         ctx.handle.ntt_inverse(m.data_ptr(), m.data_ptr(), idx, stream=st)
         centred = t.empty(ctx.n, dtype=t.float64, device=ctx.device)
         ctx.composer(idx).apply(centred.data_ptr(), m.data_ptr(), st)

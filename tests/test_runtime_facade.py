@@ -61,6 +61,15 @@ def emu():
     return context, ectx, enc
 
 
+@pytest.fixture(scope="module", params=["emu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def client(request):
+    """(context, keys, encryptor) in host memory (emulation build) and on the GPU."""
+    if request.param == "emu":
+        return request.getfixturevalue("emu")
+    context = runtime.Context(SLOTS, PRIMES)
+    return (context,) + _keys(context)
+
+
 def test_encrypt_decrypt_round_trip(emu):
     _context, _ectx, enc = emu
     x = sample_vector(1)
@@ -73,6 +82,35 @@ def test_encrypt_decrypt_round_trip(emu):
     assert _bits(enc.decrypt_and_decode(ct, 1 << 56), z) > 40
     ct = enc.encode_and_encrypt(2.5, 1 << 56, Q_IDX[:3])                  # a scalar fills every slot
     assert _bits(enc.decrypt_and_decode(ct, 1 << 56), np.full(SLOTS, 2.5)) > 40
+
+
+def test_decryption_on_primes_that_are_not_consecutive(client, monkeypatch):
+    """The gathered key rows stay alive until the product that reads them has been called."""
+    import gc
+    import weakref
+    context, _ectx, enc = client
+    x = sample_vector(3)
+    gathered = []
+    rows = enc._key_rows
+    ewise = context.handle.ewise
+
+    def watched_rows(idx):
+        t = rows(idx)
+        gathered.append(weakref.ref(t))
+        return t
+
+    def watched_ewise(op, *args, **kwargs):
+        gc.collect()
+        assert all(r() is not None for r in gathered), "the key rows are freed before the kernel is called"
+        return ewise(op, *args, **kwargs)
+
+    for idx in ([1, 3, 5, 7], [0, 2, 4, 6, 7], [5, 4, 3]):
+        ct = enc.encode_and_encrypt(x, 1 << 56, idx)
+        monkeypatch.setattr(enc, "_key_rows", watched_rows)
+        monkeypatch.setattr(context.handle, "ewise", watched_ewise)
+        assert _bits(enc.decrypt_and_decode(ct, 1 << 56), x) > 25
+        monkeypatch.undo()
+        gathered.clear()
 
 
 def _key_tensor(enc, key_type, rot):
