@@ -210,18 +210,14 @@ class CKKSEncryptor:
         self.context = encryptor_context.context
         self.rng = _rng(prng_seed if prng_seed is not None else encryptor_context.seed)
         self.encoder = _Encoder(self.context.n)
-        self._stage: Dict[str, object] = {}
 
     # -- staging ----------------------------------------------------------------------------------------
-    def _staging(self, name: str, rows: int):
-        """Page-locked host words [rows][n] (a plain array where the library computes in host memory), kept and grown
-        with this encryptor: copies to and from the device then run at the link's rate and beside the host's work."""
-        t = self._stage.get(name)
-        if t is None or t.shape[0] < rows:
-            torch = self.context.torch
-            t = torch.empty((rows, self.context.n), dtype=torch.int32, pin_memory=self.context.device.type == "cuda")
-            self._stage[name] = t
-        return t[:rows]
+    def _staging(self, rows: int):
+        """Page-locked host words [rows][n] (plain memory where the library computes in host memory): copies to and from
+        the device then run at the link's rate and beside the host's work.  A call's own, so calls may overlap; torch's
+        pool of such blocks is safe with threads and hands one out again only after the copies queued on it are done."""
+        torch = self.context.torch
+        return torch.empty((rows, self.context.n), dtype=torch.int32, pin_memory=self.context.device.type == "cuda")
 
     # -- sampling ---------------------------------------------------------------------------------------
     def _noise(self) -> np.ndarray:
@@ -233,7 +229,7 @@ class CKKSEncryptor:
     def _uniform(self, idx):
         """Uniform residues, (host, device) words: the draws of one limb go up while the next limb's are made."""
         ctx = self.context
-        stage = self._staging("uniform", len(idx))
+        stage = self._staging(len(idx))
         host = np.empty((len(idx), ctx.n), dtype=np.uint32)
         dev = ctx.torch.empty((len(idx), ctx.n), dtype=ctx.torch.int32, device=ctx.device)
         for k, p in enumerate(idx):
@@ -274,7 +270,7 @@ class CKKSEncryptor:
         ctx = self.context
         sel = ctx.torch.tensor(list(idx), dtype=ctx.torch.int64, device=ctx.device)
         c0, _, c1 = self._encrypt(key_rns[sel].to(ctx.torch.int32), list(idx))
-        ctx._sync()                             # the staging rows are free for the next draws
+        ctx._sync()
         return c0.to(ctx.torch.int64), c1.to(ctx.torch.int64)
 
     # -- messages ---------------------------------------------------------------------------------------
@@ -292,7 +288,7 @@ class CKKSEncryptor:
     def encode_and_encrypt(self, message, scale: float, rns_base_ids: Sequence[int]) -> Ciphertext:
         idx = list(rns_base_ids)
         c0, host1, _ = self._encrypt(self._key_rows(idx), idx, lambda: self.encoder.encode(message, scale))
-        stage = self._staging("result", len(idx))
+        stage = self._staging(len(idx))
         stage.copy_(c0, non_blocking=True)
         self.context._sync()
         return Ciphertext(stage.numpy().view(np.uint32).copy(), host1, idx)
@@ -301,7 +297,7 @@ class CKKSEncryptor:
         """Complex slot values of c0 + c1 s, composed over every limb of the ciphertext."""
         ctx, t = self.context, self.context.torch
         idx = ciphertext.rns_base_ids
-        stage = self._staging("input", 2 * len(idx))
+        stage = self._staging(2 * len(idx))
         w = t.empty((2 * len(idx), ctx.n), dtype=t.int32, device=ctx.device)
         for k, c in ((1, ciphertext.c1), (0, ciphertext.c0)):
             half = slice(k * len(idx), (k + 1) * len(idx))

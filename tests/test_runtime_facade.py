@@ -113,6 +113,21 @@ def test_decryption_on_primes_that_are_not_consecutive(client, monkeypatch):
         gathered.clear()
 
 
+def test_one_encryptor_serves_several_threads(client):
+    """Encryptions and decryptions that run at the same time through one encryptor do not see each other."""
+    from concurrent.futures import ThreadPoolExecutor
+    _context, _ectx, enc = client
+    messages = [sample_vector(20 + i) for i in range(24)]
+    idx = [list(range(2 + i % 5)) for i in range(24)]
+    with ThreadPoolExecutor(8) as pool:
+        cts = list(pool.map(lambda i: enc.encode_and_encrypt(messages[i], 1 << 50, idx[i]), range(24)))
+        back = list(pool.map(lambda i: enc.decrypt_and_decode(cts[i], 1 << 50), range(24)))
+    wrong = [i for i in range(24) if _bits(back[i], messages[i]) < 25]
+    assert not wrong, wrong
+    serial = [i for i in range(24) if _bits(enc.decrypt_and_decode(cts[i], 1 << 50), messages[i]) < 25]
+    assert not serial, serial
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
