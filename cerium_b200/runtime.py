@@ -65,6 +65,7 @@ class Context:
         self.handle = _capi.Context(self.lib, self.moduli, 32, device=device, logn=self.logn)
         self._q = torch.tensor(self.moduli, dtype=torch.int64, device=self.device)
         self._composers: Dict[Tuple[int, ...], _capi.Composer] = {}
+        self._composers_lock = threading.Lock()
 
     @property
     def coeff_count(self) -> int:
@@ -103,10 +104,11 @@ class Context:
     def composer(self, idx: Sequence[int]) -> "_capi.Composer":
         """CRT composition over these primes; the last few prime lists are kept."""
         key = tuple(idx)
-        c = self._composers.pop(key, None) or _capi.Composer(self.handle, key)
-        self._composers[key] = c
-        while len(self._composers) > 8:
-            self._composers.pop(next(iter(self._composers)))
+        with self._composers_lock:
+            c = self._composers.pop(key, None) or _capi.Composer(self.handle, key)
+            self._composers[key] = c
+            while len(self._composers) > 8:
+                self._composers.pop(next(iter(self._composers)))
         return c
 
     def words_ntt(self, idx: Sequence[int], values=None, small=None):
@@ -310,7 +312,8 @@ class CKKSEncryptor:
         ew(_capi.EW_MAD, m.data_ptr(), a.data_ptr(), idx, b=key.data_ptr(), c=m.data_ptr(), stream=st)
         ctx.handle.ntt_inverse(m.data_ptr(), m.data_ptr(), idx, stream=st)
         centred = t.empty(ctx.n, dtype=t.float64, device=ctx.device)
-        ctx.composer(idx).apply(centred.data_ptr(), m.data_ptr(), st)
+        composer = ctx.composer(idx)    # held, like the key: another thread may push it out of the table
+        composer.apply(centred.data_ptr(), m.data_ptr(), st)
         coeff = centred.cpu().numpy()
         if np.isinf(coeff).any():
             raise OverflowError("a composed coefficient passes the range of a double")

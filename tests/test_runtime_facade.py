@@ -128,6 +128,33 @@ def test_one_encryptor_serves_several_threads(client):
     assert not serial, serial
 
 
+def test_compositions_of_many_prime_lists_from_several_threads(emu, monkeypatch):
+    """The table of composition handles: bounded, one handle per prime list, unharmed by threads that use it at once."""
+    import sys
+    from concurrent.futures import ThreadPoolExecutor
+    context, _ectx, _enc = emu
+    made = []
+
+    class Handle:
+        def __init__(self, ctx, idx):
+            made.append(idx)
+
+    monkeypatch.setattr(runtime._capi, "Composer", Handle)
+    monkeypatch.setattr(context, "_composers", {})
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        with ThreadPoolExecutor(8) as pool:
+            for _ in range(20):     # few lists: a list in the table is not made twice
+                got = list(pool.map(lambda i: (i % 4, context.composer([i % 4])), range(400)))
+                assert len({id(h) for _i, h in got}) == 4 and len(made) == 4
+            for _ in range(20):     # more lists than the table keeps
+                list(pool.map(lambda i: context.composer([i % 24]), range(2000)))
+    finally:
+        sys.setswitchinterval(interval)
+    assert len(context._composers) <= 8
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
