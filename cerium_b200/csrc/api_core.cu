@@ -303,7 +303,7 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
                  const uint32_t* out_primes, int n_out, const BconvOptions& opt) {
   if (!ctx || !out || !in_primes || !out_primes) return fail(CERIUM_ERR_INVALID, "bconv_create: null argument");
   if (mode != CERIUM_BCONV_LAZY && mode != CERIUM_BCONV_EXACT) return fail(CERIUM_ERR_INVALID, "bconv_create: unknown mode");
-  if (n_in < 1 || n_in > 64 || n_out < 1 || n_out > 255) return fail(CERIUM_ERR_INVALID, "bconv_create: need 1..64 inputs and 1..255 outputs");
+  if (n_in < 1 || n_in > kMmaMaxInputs || n_out < 1 || n_out > 255) return fail(CERIUM_ERR_INVALID, "bconv_create: need 1..64 inputs and 1..255 outputs");
   if (!opt.out_pos.empty() && (int)opt.out_pos.size() != n_out) return fail(CERIUM_ERR_INVALID, "bconv_create: out_pos size");
   if (!opt.in_pos.empty() && (int)opt.in_pos.size() != n_in) return fail(CERIUM_ERR_INVALID, "bconv_create: in_pos size");
   for (int i = 0; i < n_in; i++)
@@ -529,7 +529,7 @@ static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int c
         stages = t;
       }
     }
-    if (smem > 48 * 1024) CERIUM_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) CERIUM_CUDA(allow_smem(kfn, bconv_mma_smem_bytes<W>(kMmaMaxInputs)));
     CERIUM_LAUNCH(kfn, dim3((kStages + stages - 1) / stages, cnt, slices), 32 * warps, smem, stream, batch, stages,
                   static_cast<const PrimeConst<W>*>(ctx->d_pcs));
     first += cnt;

@@ -41,6 +41,7 @@ template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
 constexpr int kMmaMaxBatch = 24;                  // conversions per launch (descriptors travel as parameters)
+constexpr int kMmaMaxInputs = 64;                 // of a conversion
 constexpr int kMmaPairInputs = 32;                // 64-bit inputs whose plane pairs c + 2^8 c' stay below 2^32:
                                                   // 8 I 255^2 257 < 2^32 (32-bit words: 4 I, so all 64 do)
 

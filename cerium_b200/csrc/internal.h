@@ -44,6 +44,41 @@ int fail(int code, const std::string& msg);
       return ::cerium::fail(CERIUM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e__)); \
   } while (0)
 
+// Kernels for which something has been set on a device.  Threads that come first together set it once each.
+class KernelTable {
+  static constexpr size_t kSlots = 1024;  // open addressing; a full table only means that it is set again
+  std::atomic<uintptr_t> seen_[kSlots] = {};
+
+ public:
+  template <typename Set>
+  cudaError_t once(const void* kfn, Set&& set) {
+    int device = 0;
+    if (cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
+    const uintptr_t key = reinterpret_cast<uintptr_t>(kfn) * kMaxDevices + (uintptr_t)device;
+    bool done = false;
+    for (size_t k = 0, h = key / kMaxDevices / 16 % kSlots; k < kSlots; k++, h = (h + 1) % kSlots) {
+      uintptr_t at = seen_[h].load(std::memory_order_acquire);
+      if (at == key) return cudaSuccess;
+      if (at != 0) continue;
+      if (!done)
+        if (cudaError_t e = set(); e != cudaSuccess) return e;
+      done = true;
+      if (seen_[h].compare_exchange_strong(at, key, std::memory_order_acq_rel) || at == key) return cudaSuccess;
+    }
+    return done ? cudaSuccess : set();
+  }
+};
+
+// Lets a kernel be launched with up to `bytes` of dynamic shared memory.  The limit belongs to the kernel and not to a
+// launch, so `bytes` is the most that any of its launches needs: one that lowered it would fail another thread's.
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel kfn, size_t bytes) {
+  static KernelTable seen;
+  return seen.once(reinterpret_cast<const void*>(kfn), [&] {
+    return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
+}
+
 // Kernel launch through a function pointer (template-ids with commas stay out of the macro).
 #if defined(CERIUM_EMU)
 #define CERIUM_LAUNCH(kfn, grid, block, smem, stream, ...) \
@@ -57,19 +92,11 @@ int fail(int code, const std::string& msg);
 // holds their twiddles (384 limbs: 212 us against 188).  The attribute is set at a kernel's first launch on a device.
 constexpr int kCarveoutPercent = 71;
 inline void prefer_carveout(const void* kfn) {
-  constexpr size_t kSlots = 1024;  // open addressing; a full table only means that the attribute is set again
-  static std::atomic<uintptr_t> seen[kSlots] = {};
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) return;
-  const uintptr_t key = reinterpret_cast<uintptr_t>(kfn) * kMaxDevices + (uintptr_t)device;
-  for (size_t k = 0, h = key / kMaxDevices / 16 % kSlots; k < kSlots; k++, h = (h + 1) % kSlots) {
-    uintptr_t at = seen[h].load(std::memory_order_relaxed);
-    if (at == key) return;
-    if (at == 0) {
-      cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent);  // a hint
-      if (seen[h].compare_exchange_strong(at, key, std::memory_order_relaxed) || at == key) return;
-    }
-  }
+  static KernelTable seen;
+  seen.once(kfn, [&] {
+    cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent);  // a hint
+    return cudaSuccess;
+  });
 }
 // Every kernel is launched with programmatic stream serialisation (see grid_dependency_wait in
 // modarith.cuh): its CTAs may be placed while the previous kernel of the stream drains.

@@ -51,6 +51,7 @@ void sync_threads();
 void sync_warp();
 void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()>& body);
 long launches();  // number of launches so far (tests use it to see that kernels ran)
+void set_smem_limit(const void* kernel, int bytes);
 }  // namespace cerium_emu
 
 #define threadIdx (::cerium_emu::t_threadIdx)
@@ -121,4 +122,7 @@ static inline cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigne
 template <typename T>
 static inline cudaError_t cudaGetSymbolAddress(void** p, T& symbol) { *p = (void*)&symbol; return cudaSuccess; }
 template <typename F>
-static inline cudaError_t cudaFuncSetAttribute(F, cudaFuncAttribute, int) { return cudaSuccess; }
+static inline cudaError_t cudaFuncSetAttribute(F kernel, cudaFuncAttribute, int bytes) {
+  ::cerium_emu::set_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
+  return cudaSuccess;
+}

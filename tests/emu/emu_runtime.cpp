@@ -2,6 +2,8 @@
 #include <ucontext.h>
 
 #include <atomic>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "emu_cuda.h"
@@ -110,6 +112,20 @@ void sync_warp() { yield_with(kWarp); }
 
 long launches() { return g_launches.load(); }
 
+// A kernel's limit of dynamic shared memory belongs to all threads of a process: one that lowers it can make another's
+// launch fail.
+namespace {
+std::mutex g_limits_lock;
+std::map<const void*, int> g_limits;
+long g_lowered = 0;
+}  // namespace
+void set_smem_limit(const void* kernel, int bytes) {
+  std::lock_guard<std::mutex> lock(g_limits_lock);
+  int& at = g_limits[kernel];
+  if (bytes < at) g_lowered++;
+  at = bytes;
+}
+
 void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()>& body) {
   g_launches++;
   const long nblocks = (long)grid.x * grid.y * grid.z;
@@ -129,3 +145,6 @@ void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()
 }
 
 }  // namespace cerium_emu
+
+// how often a kernel's limit was lowered
+extern "C" long cerium_emu_lowered_smem_limits() { return cerium_emu::g_lowered; }

@@ -50,3 +50,34 @@ def test_bconv_edges(be, word_bits, n_in, n_out, mode):
             else:
                 want = sum(int(x[i, c]) * invs[i] % ins[i] * hats[i] for i in range(n_in)) % p
             assert int(got[j, c]) == want, (j, c)
+
+
+def test_conversions_of_different_sizes_from_several_threads(be):
+    """Conversions that need more than 48 KB of shared memory, 30 and 20 inputs of 64-bit words: neither takes away the
+    limit that the other's launch counts on, and both are right when two threads launch them at once."""
+    from concurrent.futures import ThreadPoolExecutor
+    mods = params.ntt_primes_below(50, 31, 16)
+    ctx = _capi.Context(be.lib, mods, 64)
+    rng = np.random.default_rng(7)
+    x = np.stack([rng.integers(0, q, N, dtype=np.uint64) for q in mods[:30]])
+    dx = be.to_dev(x)
+    made = [(_capi.BaseConverter(ctx, range(n), [30], _capi.BCONV_LAZY), be.empty((1, N), np.uint64)) for n in (30, 20)]
+
+    def run(k, times):
+        for _ in range(times):
+            made[k][0].apply(be.ptr(made[k][1]), be.ptr(dx))
+
+    for k in (0, 1, 0):
+        run(k, 1)
+    if be.name == "emu":
+        assert be.lib.dll.cerium_emu_lowered_smem_limits() == 0
+    else:
+        with ThreadPoolExecutor(2) as pool:
+            list(pool.map(run, (0, 1), (2000, 2000)))
+    for n, (_bc, out) in zip((30, 20), made):
+        got, big = be.to_host(out), 1
+        for q in mods[:n]:
+            big *= q
+        f = [big // q * pow(big // q, -1, q) % mods[30] for q in mods[:n]]
+        for c in (0, 1, 127, 128, N - 1):
+            assert int(got[0, c]) == sum(int(x[i, c]) * f[i] for i in range(n)) % mods[30]
