@@ -409,22 +409,9 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
             bytes[entry * 16 + reg * 4 + col % 4] = (unsigned char)(g >> (8 * b));
           }
         }
-      BconvMmaOut<W>& o = outc[j];
-      std::memset(&o, 0, sizeof(o));
-      o.nq = (W)0 - (W)q;
-      o.add = out_sub.empty() ? (W)0 : (W)(q - out_sub[j]);
-      o.pos = opt.out_pos.empty() ? (uint32_t)j : opt.out_pos[j];
-      o.cls = sizeof(W) == 4 || q >= ((uint64_t)1 << 48) ? kMmaWide : q >= ((uint64_t)1 << 40) ? kMmaNarrow : kMmaTiny;
-      bc->all_wide = bc->all_wide && o.cls == kMmaWide;
-      if (o.cls == kMmaTiny) {
-        o.mu = (W)host::shoup(1, q, 64);
-      } else if (o.cls == kMmaNarrow) {
-        uint64_t mu = 0;
-        while ((mu = (uint64_t)(((unsigned __int128)1 << (64 + o.shift)) / q)) < ((uint64_t)1 << 31)) o.shift++;
-        o.mu = (W)mu;
-      } else {
-        o.mu = (W)(((unsigned __int128)1 << (sizeof(W) == 8 ? 80 : 48)) / q);
-      }
+      outc[j] = bconv_mma_constants<W>(q, out_sub.empty() ? 0 : out_sub[j]);
+      outc[j].pos = opt.out_pos.empty() ? (uint32_t)j : opt.out_pos[j];
+      bc->all_wide = bc->all_wide && outc[j].cls == kMmaWide;
     }
     o_outc = blob.append(outc.data(), outc.size() * sizeof(BconvMmaOut<W>));
     o_table = blob.append(table.data(), table.size() * sizeof(uint4));

@@ -50,7 +50,8 @@ constexpr int kMmaPairInputs = 32;                // 64-bit inputs whose plane p
 // The quotient c of the recombined sum x <= 255 b I (q - 1) (b = bytes of a word) comes from the bits of x above
 // 2^base, t, times floor(2^(base + 32 + shift) / q):
 //   64-bit words, wide    q >= 2^48, base = 48, shift = 0: x - c q is below 2.3 q, and taken modulo 2^64 (x itself may pass it)
-//   64-bit words, narrow  2^40 <= q < 2^48, base = 32 (x fits 64 bits): below 1.1 q
+//   64-bit words, narrow  2^40 <= q < 2^48, base = 32 (x fits 64 bits up to kMmaPairInputs inputs; beyond them base = 34,
+//                         from the plane sums): below 1.1 q
 //   64-bit words, tiny    q < 2^40: 64-bit high product with floor(2^64 / q); below 4 q
 //   32-bit words          base = 16, shift = 0: q > 2^17, so below 1.3 q
 template <typename W>
@@ -63,6 +64,25 @@ struct alignas(16) BconvMmaOut {
   uint16_t cls;
 };
 enum : int { kMmaWide = 0, kMmaNarrow = 1, kMmaTiny = 2 };
+
+// The constants of an output of modulus q (its slot aside); sub = rounding term that leaves the result.
+template <typename W>
+inline BconvMmaOut<W> bconv_mma_constants(uint64_t q, uint64_t sub) {
+  BconvMmaOut<W> o{};
+  o.nq = (W)0 - (W)q;
+  o.add = sub != 0 ? (W)(q - sub) : (W)0;
+  o.cls = sizeof(W) == 4 || q >= ((uint64_t)1 << 48) ? kMmaWide : q >= ((uint64_t)1 << 40) ? kMmaNarrow : kMmaTiny;
+  if (o.cls == kMmaTiny) {
+    o.mu = (W)(((unsigned __int128)1 << 64) / q);
+  } else if (o.cls == kMmaNarrow) {
+    uint64_t mu = 0;
+    while ((mu = (uint64_t)(((unsigned __int128)1 << (64 + o.shift)) / q)) < ((uint64_t)1 << 31)) o.shift++;
+    o.mu = (W)mu;
+  } else {
+    o.mu = (W)(((unsigned __int128)1 << (sizeof(W) == 8 ? 80 : 48)) / q);
+  }
+  return o;
+}
 
 template <typename W>
 struct BconvMmaDesc {
@@ -112,7 +132,8 @@ __device__ __forceinline__ uint64_t bconv_mma_finish(const uint32_t (&c)[8], con
   using Sum = std::conditional_t<kFinish == kMmaBig, uint64_t, uint32_t>;
   const Sum a = c[0] + ((Sum)c[1] << 8), b = c[2] + ((Sum)c[3] << 8), cc = c[4] + ((Sum)c[5] << 8), d = c[6] + ((Sum)c[7] << 8);
   const Sum u = cc + (b >> 16);
-  const uint64_t x = (uint64_t)a + ((uint64_t)(b & 0xffffu) << 16) + ((uint64_t)(u + (d << 16)) << 32);  // modulo 2^64
+  const uint64_t low = (uint64_t)a + ((uint64_t)(b & 0xffffu) << 16);
+  const uint64_t x = low + ((uint64_t)(u + (d << 16)) << 32);  // modulo 2^64
   if (kFinish <= kMmaLazyAdd) {
     const uint32_t t = (uint32_t)(d + (u >> 16));
     const uint64_t r = x + (uint64_t)__umulhi(t, (uint32_t)o.mu) * o.nq;
@@ -123,8 +144,13 @@ __device__ __forceinline__ uint64_t bconv_mma_finish(const uint32_t (&c)[8], con
   if (o.cls == kMmaTiny) {
     r = x + mulhi_approx64(x, o.mu) * o.nq;
   } else {
-    const uint32_t t = o.cls == kMmaWide ? (uint32_t)(d + (u >> 16)) : (uint32_t)(x >> 32);
-    r = x + (uint64_t)(__umulhi(t, (uint32_t)o.mu) >> o.shift) * o.nq;
+    // narrow, more than kMmaPairInputs inputs: x may pass 2^64 (below 2^65), so the bits above 2^32 come from the sums,
+    // two fewer of them
+    const uint32_t t = o.cls == kMmaWide     ? (uint32_t)(d + (u >> 16))
+                       : kFinish == kMmaBig ? (uint32_t)((u + (d << 16) + (low >> 32)) >> 2)
+                                            : (uint32_t)(x >> 32);
+    const int shift = kFinish == kMmaBig && o.cls == kMmaNarrow ? o.shift - 2 : o.shift;  // narrow: at least 7
+    r = x + (uint64_t)(__umulhi(t, (uint32_t)o.mu) >> shift) * o.nq;
   }
   r = csub<uint64_t>(csub<uint64_t>(r, q + q), q);
   return csub<uint64_t>(r + o.add, q);

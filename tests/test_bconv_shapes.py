@@ -17,13 +17,14 @@ def be(request):
 
 @pytest.mark.parametrize("word_bits,n_in,n_out,mode", [
     (64, 1, 1, _capi.BCONV_LAZY), (64, 4, 8, _capi.BCONV_EXACT), (64, 5, 9, _capi.BCONV_LAZY), (64, 9, 17, _capi.BCONV_EXACT),
-    (64, 33, 3, _capi.BCONV_LAZY),
+    (64, 33, 3, _capi.BCONV_LAZY), (64, 64, 6, _capi.BCONV_LAZY),
     (32, 1, 1, _capi.BCONV_LAZY), (32, 8, 9, _capi.BCONV_EXACT), (32, 17, 16, _capi.BCONV_LAZY), (32, 21, 25, _capi.BCONV_EXACT),
 ])
 def test_bconv_edges(be, word_bits, n_in, n_out, mode):
     if word_bits == 64:     # outputs of 30 to 60 bits in one conversion, inputs of 60 and 50 bits
+        widths = (59, 49, 47, 39, 30) if n_in < 64 else (59, 49, 48, 40, 30)    # most inputs: classes at their upper ends
         ins = params.ntt_primes_below(60, (n_in + 1) // 2, 16) + params.ntt_primes_below(50, n_in // 2, 16)
-        pools = [params.ntt_primes_below(b, n_out, 16, exclude=ins) for b in (59, 49, 47, 39, 30)]
+        pools = [params.ntt_primes_below(b, n_out, 16, exclude=ins) for b in widths]
         outs = [pools[j % 5][j] for j in range(n_out)]
     else:
         mods = params.reference_primes_28bit(n_in + n_out)
@@ -34,6 +35,7 @@ def test_bconv_edges(be, word_bits, n_in, n_out, mode):
     rng = np.random.default_rng(n_in * 100 + n_out)
     x = np.stack([rng.integers(0, q, N, dtype=dt) for q in ins])
     x[:, 0], x[:, 1] = 0, [q - 1 for q in ins]
+    x[:, 2] = [(1 << (q.bit_length() - 1)) - 1 for q in ins]    # low bytes of 255
     dx, out = be.to_dev(x), be.empty((n_out, N), dt)
     bc.apply(be.ptr(out), be.ptr(dx))
     got = be.to_host(out)
@@ -42,7 +44,7 @@ def test_bconv_edges(be, word_bits, n_in, n_out, mode):
         big *= q
     hats = [big // q for q in ins]
     invs = [pow(h % q, -1, q) for h, q in zip(hats, ins)]
-    at = sorted({0, 1, 7, 8, 127, 128, 383, 384, N - 129, N - 1} | set(int(c) for c in rng.integers(0, N, 200)))
+    at = sorted({0, 1, 2, 7, 8, 127, 128, 383, 384, N - 129, N - 1} | set(int(c) for c in rng.integers(0, N, 200)))
     for j, p in enumerate(outs):
         for c in at:
             if mode == _capi.BCONV_LAZY:
