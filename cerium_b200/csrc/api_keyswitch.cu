@@ -223,6 +223,7 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
 // accumulators again (7 us each at 24 limbs).
 int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cudaStream_t stream, uint32_t pre_elt = 0,
                     bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr) {
+  if (((uintptr_t)add0 | (uintptr_t)add1) & 15u) return fail(CERIUM_ERR_INVALID, "keyswitch: additions must be 16-byte aligned");
   cerium_context* ctx = ks->ctx;
   const size_t n = kN;
   const int LK = ks->LK, dnum = ks->dnum;

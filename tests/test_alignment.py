@@ -1,0 +1,41 @@
+"""Operands that are not 16-byte aligned: the kernels move 16 bytes at a time, so a call refuses such an operand or takes a
+way that does not."""
+import numpy as np
+import pytest
+
+import oracle
+from cerium_b200 import _capi
+from tests import parity_cases as pc
+
+L, K, DNUM = 3, 2, 2
+
+
+@pytest.fixture(scope="module", params=["emu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def be(request):
+    from tests import backends
+    return backends.EmuBackend() if request.param == "emu" else backends.CudaBackend()
+
+
+class Plan:
+    def __init__(self, be, word_bits):
+        prm = self.prm = pc.small_params(word_bits, L, K, DNUM)
+        self.h = pc.Harness(be, word_bits, prm.moduli)
+        self.c0, self.c1, self.evk = pc.make_keyswitch_inputs(np.random.default_rng(5), prm)
+        self.d_c0, self.d_c1, self.d_evk = self.h.up(self.c0), self.h.up(self.c1), self.h.up(self.evk)
+        self.ks = _capi.KeySwitch(self.h.ctx, prm.q_idx, prm.p_idx, DNUM, _capi.BCONV_LAZY, _capi.ROUND_FLOOR)
+
+
+@pytest.mark.parametrize("word_bits", [64, 32])
+@pytest.mark.parametrize("levels", [0, 1, 2])
+def test_additions_of_a_key_switch_are_refused(be, word_bits, levels):
+    t = Plan(be, word_bits)
+    h, word = t.h, word_bits // 8
+    o = h.new(2, L - levels, pc.N)
+    spare = h.new(L + 1, pc.N)
+    o1 = h.p(o) + (L - levels) * pc.N * word
+    for add0, add1 in ((h.p(spare) + word, 0), (0, h.p(spare) + 8), (h.p(t.d_c0), h.p(spare) + word)):
+        with pytest.raises(_capi.CeriumError) as e:
+            t.ks.apply_rescale(h.p(o), o1, h.p(t.d_c1), h.p(t.d_evk), levels, add0, add1)
+        assert e.value.code == _capi.ERR_INVALID
+    be.sync()
+    t.ks.close()
