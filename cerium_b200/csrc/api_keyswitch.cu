@@ -1020,14 +1020,17 @@ int cerium_hoisted_rotate(cerium_keyswitch* ks, void* out0, void* out1, const vo
   void* t1 = tmp + (size_t)ks->L * n * wb;
   // (t0, t1) = KeySwitch(c1) + (c0, 0) on the un-rotated digits, then the automorphism: as the store
   // pattern of the last kernel (out[i] = t[pi_g(i)] is t[i] -> out[pi_{1/g}(i)]), unless an output
-  // overlaps an input that kernel still reads
+  // overlaps an input that kernel still reads, or is aligned to words only (that kernel stores 16 bytes at a time)
+  const bool aligned = (((uintptr_t)out0 | (uintptr_t)out1) & 15u) == 0;
   {
     const size_t poly_bytes = (size_t)ks->L * n * wb;
     auto overlaps = [&](const void* a, const void* b) {
       const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
       return x < y + poly_bytes && y < x + poly_bytes;
     };
-    if (!overlaps(out0, c0) && !overlaps(out1, c0) && !overlaps(out0, c1) && !overlaps(out1, c1)) {
+    const bool apart = !overlaps(out0, c0) && !overlaps(out1, c0) && !overlaps(out0, c1) && !overlaps(out1, c1);
+    if (!apart && !aligned) return fail(CERIUM_ERR_INVALID, "hoisted_rotate: pointers must be 16-byte aligned");
+    if (apart && aligned) {
       // inverse of the element modulo 2N (odd, so it exists): Newton steps double the valid bits
       uint32_t inv = galois_elt;
       for (int k = 0; k < 5; k++) inv *= 2u - galois_elt * inv;
@@ -1036,7 +1039,6 @@ int cerium_hoisted_rotate(cerium_keyswitch* ks, void* out0, void* out1, const vo
     }
   }
   if (int rc = keyswitch_inner_moddown(ks, t0, t1, c1, evk_pre, c0, nullptr, (cudaStream_t)stream)) return rc;
-  if (((uintptr_t)out0 | (uintptr_t)out1) & 15u) return fail(CERIUM_ERR_INVALID, "hoisted_rotate: pointers must be 16-byte aligned");
   return launch_automorph_pair(ctx, out0, t0, out1, t1, galois_elt, ks->L, (cudaStream_t)stream);
 }
 

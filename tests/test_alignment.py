@@ -39,3 +39,24 @@ def test_additions_of_a_key_switch_are_refused(be, word_bits, levels):
         assert e.value.code == _capi.ERR_INVALID
     be.sync()
     t.ks.close()
+
+
+@pytest.mark.parametrize("word_bits", [64, 32])
+def test_hoisted_rotation_into_outputs_aligned_to_words(be, word_bits):
+    t = Plan(be, word_bits)
+    h, word, prm = t.h, word_bits // 8, t.prm
+    elt = be.lib.galois_elt_from_step(-3, pc.LOGN)
+    k0, k1 = h.orc.keyswitch(_capi.BCONV_LAZY, _capi.ROUND_FLOOR, prm.q_idx, prm.p_idx, DNUM, t.c1, t.evk)
+    k0 = np.stack([oracle.ew("add", prm.moduli[p], k0[i], t.c0[i]) for i, p in enumerate(prm.q_idx)])
+    want = [np.stack([oracle.apply_galois_ntt(elt, pc.LOGN, k[i]) for i in range(L)]) for k in (k0, k1)]
+    buf = [h.new((L + 1) * pc.N) for _ in range(2)]
+    t.ks.hoisted_begin(h.p(t.d_c1))
+    t.ks.hoisted_rotate(h.p(buf[0]) + word, h.p(buf[1]) + 3 * word, h.p(t.d_c0), h.p(t.d_c1), h.p(t.d_evk), elt)
+    for b, at, w in zip(buf, (1, 3), want):
+        assert np.array_equal(h.down(b)[at:at + L * pc.N].reshape(L, pc.N), w)
+    # outputs on top of the inputs: refused
+    with pytest.raises(_capi.CeriumError) as e:
+        t.ks.hoisted_rotate(h.p(t.d_c0) + word, h.p(t.d_c1), h.p(t.d_c0), h.p(t.d_c1), h.p(t.d_evk), elt)
+    assert e.value.code == _capi.ERR_INVALID
+    be.sync()
+    t.ks.close()
