@@ -844,6 +844,13 @@ int cerium_keyswitch_sharded_finish(cerium_keyswitch* ks, void* out0, void* out1
   if (ks->L > 0 && (!out0 || !out1 || !cpoly_local)) return fail(CERIUM_ERR_INVALID, "keyswitch_sharded_finish: null argument");
   if (ks->ext_split) return fail(CERIUM_ERR_INVALID, "keyswitch_sharded_finish: plans with split extension limbs exchange twice; use cerium_keyswitch_sharded_apply");
   DeviceGuard guard(ks->ctx->device);
+  if (((uintptr_t)gathered & 15u) && !ks->direct_raise) {
+    // the conversion copies 16 bytes at a time: from the plan's own gather buffer then
+    const size_t wb = ks->ctx->word_bytes();
+    void* own = static_cast<char*>(ks->ws) + (ks->world == 1 ? ks->o_coef : ks->o_gathered) * wb;
+    CERIUM_CUDA(cudaMemcpyAsync(own, gathered, (size_t)ks->world * ks->gather_limbs * kN * wb, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+    gathered = own;
+  }
   return keyswitch_finish(ks, out0, out1, gathered, cpoly_local, evk_local, add0, add1, (cudaStream_t)stream);
 }
 

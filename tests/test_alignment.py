@@ -60,3 +60,28 @@ def test_hoisted_rotation_into_outputs_aligned_to_words(be, word_bits):
     assert e.value.code == _capi.ERR_INVALID
     be.sync()
     t.ks.close()
+
+
+@pytest.mark.parametrize("word_bits,world", [(64, 2), (32, 2), (64, 1)])
+def test_sharded_key_switch_from_a_gather_buffer_aligned_to_words(be, word_bits, world):
+    prm = pc.small_params(word_bits, 4, 2, 2)
+    h, word = pc.Harness(be, word_bits, prm.moduli), word_bits // 8
+    _c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(6), prm)
+    want = h.orc.keyswitch(_capi.BCONV_EXACT, _capi.ROUND_HALF, prm.q_idx, prm.p_idx, 2, c1, evk)
+    plans = [_capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, 2, _capi.BCONV_EXACT, _capi.ROUND_HALF, rank=r, world=world) for r in range(world)]
+    g = -(-4 // world)
+    gathered = np.zeros((world * g, pc.N), dtype=h.dt)
+    for r, ks in enumerate(plans):     # what the ranks send, one after another
+        send, mine = h.new(g, pc.N), h.up(c1[r::world])
+        ks.sharded_begin(h.p(send), h.p(mine))
+        gathered[r * g:(r + 1) * g] = be.to_host(send)
+    flat = be.to_dev(np.concatenate([np.zeros(1, dtype=h.dt), gathered.ravel(), np.zeros(3, dtype=h.dt)]))
+    for r, ks in enumerate(plans):
+        local = list(range(r, 4, world))
+        key = evk[:, :, local + [4, 5]]
+        o = [h.new(len(local), pc.N) for _ in range(2)]
+        d_c1, d_key = h.up(c1[local]), h.up(key)
+        ks.sharded_finish(h.p(o[0]), h.p(o[1]), h.p(flat) + word, h.p(d_c1), h.p(d_key))
+        for out, w in zip(o, want):
+            assert np.array_equal(h.down(out), w[local])
+        ks.close()
