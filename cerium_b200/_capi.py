@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import numbers
 import os
 from typing import Optional, Sequence
 
@@ -129,24 +130,42 @@ class CeriumError(RuntimeError):
 
 
 # Index and scalar lists as C arrays.  A program passes the same few prime lists over and over, and the conversion of
-# one (1.3 us for 6 entries, 40 us for 384) is a good part of what a small call costs: the last ones are kept.  The library
-# only reads them.
+# one (1.3 us for 6 entries, 40 us for 384) is a good part of what a small call costs: the last ones are kept, by value.  The
+# library only reads them.  Lists of anything but whole numbers (0-d tensors and arrays: hashed by identity or not
+# at all, and changed in place) are converted every time.
+def _array_of(element, values):
+    return (element * len(values))(*[int(v) for v in values])
+
+
+def _check_whole(values):
+    if not all(isinstance(v, numbers.Integral) for v in values):
+        raise TypeError("not kept")
+
+
 @functools.lru_cache(maxsize=512)
 def _u32_array(values: tuple):
-    return (C.c_uint32 * len(values))(*[int(v) for v in values])
+    _check_whole(values)
+    return _array_of(C.c_uint32, values)
 
 
 @functools.lru_cache(maxsize=512)
 def _u64_array(values: tuple):
-    return (C.c_uint64 * len(values))(*[int(v) for v in values])
+    _check_whole(values)
+    return _array_of(C.c_uint64, values)
 
 
 def _u32(values: Sequence[int]):
-    return _u32_array(tuple(values))
+    try:
+        return _u32_array(tuple(values))
+    except TypeError:
+        return _array_of(C.c_uint32, values)
 
 
 def _u64(values: Sequence[int]):
-    return _u64_array(tuple(values))
+    try:
+        return _u64_array(tuple(values))
+    except TypeError:
+        return _array_of(C.c_uint64, values)
 
 
 class Library:
