@@ -195,7 +195,6 @@ class CKKSEncryptorContext:
         self.secret_key_rns = context.ntt(context.signed_to_rns(sk, all_idx), all_idx)
         self.ephemeral_key_rns = context.ntt(context.signed_to_rns(ek, all_idx), all_idx)
         self.secret_key_squared_rns = self.secret_key_rns * self.secret_key_rns % context.q(all_idx)
-        self.secret_key_words = self.secret_key_rns.to(context.torch.int32)     # the form the kernels multiply with
 
 
 def _rng(seed):
@@ -281,11 +280,11 @@ class CKKSEncryptor:
         return self.context.words_ntt(list(rns_base_ids), self.encoder.encode(message, scale)).to(self.context.torch.int64)
 
     def _key_rows(self, idx):
-        """Rows of the secret key for these primes: a view where they are consecutive."""
-        w = self.ectx.secret_key_words
+        """Rows of the secret key for these primes, words."""
+        s, t = self.ectx.secret_key_rns, self.context.torch
         if list(idx) == list(range(idx[0], idx[0] + len(idx))):
-            return w[idx[0]:idx[0] + len(idx)]
-        return w[self.context.torch.tensor(list(idx), dtype=self.context.torch.int64, device=self.context.device)]
+            return s[idx[0]:idx[0] + len(idx)].to(t.int32)
+        return s[t.tensor(list(idx), dtype=t.int64, device=self.context.device)].to(t.int32)
 
     def encode_and_encrypt(self, message, scale: float, rns_base_ids: Sequence[int]) -> Ciphertext:
         idx = list(rns_base_ids)
@@ -307,7 +306,7 @@ class CKKSEncryptor:
             w[half].copy_(stage[half], non_blocking=True)
         m, a = w[:len(idx)], w[len(idx):]
         ew, st = ctx.handle.ewise, ctx.stream()
-        key = self._key_rows(idx)       # gathered rows are this call's own: held until the result is back on the host
+        key = self._key_rows(idx)       # this call's own: held until the result is back on the host
         ew(_capi.EW_REDUCE, w.data_ptr(), w.data_ptr(), idx + idx, stream=st)     # a program's outputs may exceed q
         ew(_capi.EW_MAD, m.data_ptr(), a.data_ptr(), idx, b=key.data_ptr(), c=m.data_ptr(), stream=st)
         ctx.handle.ntt_inverse(m.data_ptr(), m.data_ptr(), idx, stream=st)

@@ -155,6 +155,23 @@ def test_compositions_of_many_prime_lists_from_several_threads(emu, monkeypatch)
     assert len(context._composers) <= 8
 
 
+def test_the_key_is_what_the_encryptor_context_holds_now(client):
+    """A secret key that is replaced, or changed in place, is the one that the next call uses."""
+    context, _ectx, _enc = client
+    ectx, enc = _keys(context)
+    x = sample_vector(4)
+    other = runtime.CKKSEncryptorContext(context, _secret_key(random.Random(11), 64), None, 3)
+    ours, theirs = ectx.secret_key_rns, other.secret_key_rns
+    ct = enc.encode_and_encrypt(x, 1 << 50, [0, 1])
+    ectx.secret_key_rns = theirs
+    ct2 = enc.encode_and_encrypt(x, 1 << 50, [2, 3])
+    assert _bits(enc.decrypt_and_decode(ct, 1 << 50), x) < 0 and _bits(enc.decrypt_and_decode(ct2, 1 << 50), x) > 25
+    ectx.secret_key_rns = ours.clone()
+    assert _bits(enc.decrypt_and_decode(ct, 1 << 50), x) > 25
+    ectx.secret_key_rns.copy_(theirs)
+    assert _bits(enc.decrypt_and_decode(ct, 1 << 50), x) < 0 and _bits(enc.decrypt_and_decode(ct2, 1 << 50), x) > 25
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
