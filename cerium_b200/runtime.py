@@ -302,6 +302,8 @@ class CKKSEncryptor:
         w = t.empty((2 * len(idx), ctx.n), dtype=t.int32, device=ctx.device)
         for k, c in ((1, ciphertext.c1), (0, ciphertext.c0)):
             half = slice(k * len(idx), (k + 1) * len(idx))
+            if c.dtype != np.uint32:        # any whole numbers: their residues
+                c = c.astype(np.int64) % np.array([ctx.moduli[p] for p in idx], dtype=np.int64).reshape(-1, 1)
             stage[half].numpy().view(np.uint32)[:] = c
             w[half].copy_(stage[half], non_blocking=True)
         m, a = w[:len(idx)], w[len(idx):]

@@ -172,6 +172,20 @@ def test_the_key_is_what_the_encryptor_context_holds_now(client):
     assert _bits(enc.decrypt_and_decode(ct, 1 << 50), x) < 0 and _bits(enc.decrypt_and_decode(ct2, 1 << 50), x) > 25
 
 
+def test_ciphertext_words_of_other_types(client):
+    """Residues in a wider type, reduced or not, negative ones among them, decrypt as the words they stand for."""
+    _context, _ectx, enc = client
+    x = sample_vector(5)
+    idx = [4, 0, 2]
+    ct = enc.encode_and_encrypt(x, 1 << 50, idx)
+    q = np.array([PRIMES[i] for i in idx], dtype=np.int64).reshape(-1, 1)
+    want = enc.decrypt_and_decode(ct, 1 << 50)
+    assert _bits(want, x) > 25
+    wide0, wide1 = ct.c0.astype(np.int64), ct.c1.astype(np.int64)
+    for c0, c1 in ((wide0 - q, wide1 - 5 * q), (wide0 + (q << 20), wide1), (ct.c0.astype(np.uint64), ct.c1.astype(np.float64))):
+        assert np.array_equal(enc.decrypt_and_decode(runtime.Ciphertext(c0, c1, idx), 1 << 50), want)
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
