@@ -115,6 +115,8 @@ class Context:
         """NTT form of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
         on the device."""
         t = self.torch
+        if len(idx) == 0:
+            return t.empty((0, self.n), dtype=t.int32, device=self.device)
         v = t.from_numpy(values).to(self.device) if values is not None else t.zeros(self.n, dtype=t.float64, device=self.device)
         e = t.from_numpy(small).to(self.device) if small is not None else None
         w = t.empty((len(idx), self.n), dtype=t.int32, device=self.device)
@@ -288,6 +290,8 @@ class CKKSEncryptor:
 
     def encode_and_encrypt(self, message, scale: float, rns_base_ids: Sequence[int]) -> Ciphertext:
         idx = list(rns_base_ids)
+        if not idx:
+            raise ValueError("encryption needs at least one prime")
         c0, host1, _ = self._encrypt(self._key_rows(idx), idx, lambda: self.encoder.encode(message, scale))
         stage = self._staging(len(idx))
         stage.copy_(c0, non_blocking=True)
@@ -298,6 +302,8 @@ class CKKSEncryptor:
         """Complex slot values of c0 + c1 s, composed over every limb of the ciphertext."""
         ctx, t = self.context, self.context.torch
         idx = ciphertext.rns_base_ids
+        if not idx:
+            return self.encoder.decode(np.zeros(ctx.n), scale)
         stage = self._staging(2 * len(idx))
         w = t.empty((2 * len(idx), ctx.n), dtype=t.int32, device=ctx.device)
         for k, c in ((1, ciphertext.c1), (0, ciphertext.c0)):

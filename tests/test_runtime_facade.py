@@ -186,6 +186,15 @@ def test_ciphertext_words_of_other_types(client):
         assert np.array_equal(enc.decrypt_and_decode(runtime.Ciphertext(c0, c1, idx), 1 << 50), want)
 
 
+def test_no_primes_at_all(client):
+    context, _ectx, enc = client
+    assert tuple(enc.encode(sample_vector(1), 1 << 40, []).shape) == (0, context.n)
+    none = np.empty((0, context.n), dtype=np.uint32)
+    assert np.array_equal(enc.decrypt_and_decode(runtime.Ciphertext(none, none, []), 1 << 40), np.zeros(SLOTS))
+    with pytest.raises(ValueError):
+        enc.encode_and_encrypt(sample_vector(1), 1 << 40, [])
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
