@@ -23,6 +23,7 @@ equivalent, not byte-identical.  One process drives one GPU; a function compiled
 """
 from __future__ import annotations
 
+import contextvars
 import os
 import threading
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -253,7 +254,7 @@ class CKKSEncryptor:
                     values.append(message())
                 except Exception:           # met again, and raised, by the caller below
                     pass
-            worker = threading.Thread(target=work)
+            worker = threading.Thread(target=contextvars.copy_context().run, args=(work,))  # with the caller's np.errstate
             worker.start()
         host1, dev1 = self._uniform(idx)
         noise = self._noise()

@@ -195,6 +195,13 @@ def test_no_primes_at_all(client):
         enc.encode_and_encrypt(sample_vector(1), 1 << 40, [])
 
 
+def test_encoding_beside_the_draws_keeps_the_callers_error_state(emu):
+    _context, _ectx, enc = emu
+    huge = np.full(SLOTS, 1e300)
+    with np.errstate(over="raise"), pytest.raises(FloatingPointError):
+        enc.encode_and_encrypt(huge, 1e300, [0, 1])
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
