@@ -112,8 +112,8 @@ class Context:
                 self._composers.pop(next(iter(self._composers)))
         return c
 
-    def words_ntt(self, idx: Sequence[int], values=None, small=None):
-        """NTT form of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
+    def _words(self, idx: Sequence[int], values=None, small=None):
+        """Residues of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
         on the device."""
         t = self.torch
         if len(idx) == 0:
@@ -122,7 +122,18 @@ class Context:
         e = t.from_numpy(small).to(self.device) if small is not None else None
         w = t.empty((len(idx), self.n), dtype=t.int32, device=self.device)
         self.handle.residues(w.data_ptr(), v.data_ptr(), idx, small=e.data_ptr() if e is not None else 0, stream=self.stream())
-        self.handle.ntt_forward(w.data_ptr(), w.data_ptr(), idx, stream=self.stream())
+        return w
+
+    def float_to_rns(self, c: np.ndarray, idx: Sequence[int]):
+        """Integer-valued doubles of any magnitude -> exact residues, [k][n] int64."""
+        return self._words(idx, np.ascontiguousarray(c, dtype=np.float64)).to(self.torch.int64)
+
+    def words_ntt(self, idx: Sequence[int], values=None, small=None):
+        """NTT form of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
+        on the device."""
+        w = self._words(idx, values, small)
+        if len(idx):
+            self.handle.ntt_forward(w.data_ptr(), w.data_ptr(), idx, stream=self.stream())
         return w
 
 

@@ -202,6 +202,19 @@ def test_encoding_beside_the_draws_keeps_the_callers_error_state(emu):
         enc.encode_and_encrypt(huge, 1e300, [0, 1])
 
 
+def test_residues_of_integer_valued_doubles(client):
+    context, _ectx, _enc = client
+    v = np.rint(np.random.default_rng(8).standard_normal(context.n) * 2.0 ** 60)
+    v[:4] = [0.0, -1.0, 2.0 ** 70, -(2.0 ** 1000)]
+    idx = [7, 0, 63]
+    got = context.float_to_rns(v, idx)
+    assert got.dtype == context.torch.int64 and tuple(got.shape) == (3, context.n)
+    got = got.cpu().numpy()
+    for row, p in zip(got, idx):
+        assert [int(r) for r in row] == [int(x) % PRIMES[p] for x in v]
+    assert tuple(context.float_to_rns(v, []).shape) == (0, context.n)
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
