@@ -217,6 +217,14 @@ def _rng(seed):
     return np.random.default_rng([int(s) & 0xFFFFFFFFFFFFFFFF for s in np.atleast_1d(seed)])
 
 
+def _bit_count(x: np.ndarray) -> np.ndarray:
+    """Bits set in each word below 2^21."""
+    if hasattr(np, "bitwise_count"):        # numpy 2
+        return np.bitwise_count(x)
+    table = np.array([bin(v).count("1") for v in range(1 << 11)], dtype=np.uint8)
+    return table[x & 0x7ff] + table[x >> 11]
+
+
 class CKKSEncryptor:
     """``runtime.CKKSEncryptor(encryptor_context[, prng_seed])`` (wrapper.cpp:78-116)."""
 
@@ -238,7 +246,7 @@ class CKKSEncryptor:
     def _noise(self) -> np.ndarray:
         """Centred binomial error, 21 coin pairs per coefficient (standard deviation 3.24)."""
         bits = self.rng.integers(0, 1 << 21, size=(2, self.context.n), dtype=np.uint32)
-        pop = np.bitwise_count(bits).astype(np.int32)
+        pop = _bit_count(bits).astype(np.int32)
         return pop[0] - pop[1]
 
     def _uniform(self, idx):

@@ -215,6 +215,16 @@ def test_residues_of_integer_valued_doubles(client):
     assert tuple(context.float_to_rns(v, []).shape) == (0, context.n)
 
 
+def test_noise_without_the_bit_count_of_numpy_2(emu, monkeypatch):
+    _context, _ectx, enc = emu
+    monkeypatch.setattr(enc, "rng", np.random.default_rng(9))
+    want = enc._noise()
+    assert want.dtype == np.int32 and 3 < want.std() < 3.5
+    monkeypatch.delattr(np, "bitwise_count", raising=False)
+    monkeypatch.setattr(enc, "rng", np.random.default_rng(9))
+    assert np.array_equal(enc._noise(), want)
+
+
 def _key_tensor(enc, key_type, rot):
     """One-digit key in the oracle's layout [1][2][Q limbs, extension limbs ascending][n]."""
     c0, c1 = enc.generate_evalkey(key_type, LEVEL, LEVEL, rot, Q_IDX)
