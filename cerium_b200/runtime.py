@@ -116,6 +116,8 @@ class Context:
         """Residues of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words
         on the device."""
         t = self.torch
+        if any(a is not None and a.shape != (self.n,) for a in (values, small)):
+            raise ValueError("a polynomial has %d coefficients" % self.n)
         if len(idx) == 0:
             return t.empty((0, self.n), dtype=t.int32, device=self.device)
         v = t.from_numpy(values).to(self.device) if values is not None else t.zeros(self.n, dtype=t.float64, device=self.device)
@@ -125,8 +127,15 @@ class Context:
         return w
 
     def float_to_rns(self, c: np.ndarray, idx: Sequence[int]):
-        """Integer-valued doubles of any magnitude -> exact residues, [k][n] int64."""
-        return self._words(idx, np.ascontiguousarray(c, dtype=np.float64)).to(self.torch.int64)
+        """Integer-valued doubles of any magnitude and number -> exact residues, [len(idx)][c.size] int64."""
+        c = np.asarray(c, dtype=np.float64).ravel()
+        out = []
+        for first in range(0, c.size, self.n):      # the kernel takes whole polynomials
+            block = np.zeros(self.n)
+            part = c[first:first + self.n]
+            block[:part.size] = part
+            out.append(self._words(idx, block)[:, :part.size].to(self.torch.int64))
+        return self.torch.cat(out, 1) if out else self.torch.empty((len(idx), 0), dtype=self.torch.int64, device=self.device)
 
     def words_ntt(self, idx: Sequence[int], values=None, small=None):
         """NTT form of integer-valued doubles plus small integers (host arrays, either may be missing): [k][n] int32 words

@@ -213,6 +213,12 @@ def test_residues_of_integer_valued_doubles(client):
     for row, p in zip(got, idx):
         assert [int(r) for r in row] == [int(x) % PRIMES[p] for x in v]
     assert tuple(context.float_to_rns(v, []).shape) == (0, context.n)
+    for size in (0, 5, context.n + 7):
+        w = np.resize(v, size)
+        got = context.float_to_rns(w, idx).cpu().numpy()
+        assert got.shape == (3, size) and [int(r) for r in got[1]] == [int(x) % PRIMES[0] for x in w]
+    with pytest.raises(ValueError):
+        context.words_ntt(idx, v[:100])
 
 
 def test_noise_without_the_bit_count_of_numpy_2(emu, monkeypatch):
