@@ -326,7 +326,6 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
   bc->I = n_in;
   bc->O = n_out;
   bc->in_primes.assign(in_primes, in_primes + n_in);
-  bc->out_primes.assign(out_primes, out_primes + n_out);
   const auto& m = ctx->moduli;
   const int bits = ctx->word_bits;
   // [Qhat_i^-1]_{q_i}
@@ -644,9 +643,6 @@ int cerium_context_create(cerium_context** out, int device, int log_n, int word_
       pc.w1ninv = (W)w1;
       pc.w1ninv_shoup = (W)host::shoup(w1, q, word_bits);
       pc.lazy_ok = (W)((word_bits == 64 && q < ((uint64_t)1 << 52)) ? 1 : 0);
-      ctx->mu_hi.push_back(t.mu_hi);
-      ctx->mu_lo.push_back(t.mu_lo);
-      ctx->lazy_ok.push_back(pc.lazy_ok != 0 ? 1 : 0);
       ctx->fp_ok.push_back(fp ? 1 : 0);
       ctx->ninv.push_back(t.ninv);
       ctx->w1ninv.push_back(w1);

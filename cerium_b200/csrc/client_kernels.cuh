@@ -61,8 +61,8 @@ __global__ void __launch_bounds__(kClientThreads) residues_kernel(const ResidueA
 
 // Exact CRT composition of `limbs` 32-bit residues per coefficient.  With y_i = x_i [Qhat_i^-1] mod q_i the
 // value is v = sum_i y_i Qhat_i - k Q, k the integer next to sum_i y_i / q_i: that is the centred representative
-// (a double holds the sum to 2^-44, and where it is that close to a half the comparison with Q / 2 below
-// decides), kept in two's complement over `words` 32-bit words, one column at a time.
+// (the sum of L terms below 1 is off by at most (L^2 + L) 2^-53 as a double, 2^-44 for 17 limbs and 2^-37 for 255, and where
+// it is that close to a half the comparison with Q / 2 below decides), kept in two's complement over `words` 32-bit words, one column at a time.
 struct ComposeArgs {
   const uint32_t* in;        // [limbs][N], coefficient form, canonical
   size_t in_stride;

@@ -280,9 +280,11 @@ __global__ void __launch_bounds__(kEwThreads) mod2_kernel(const Mod2Args<W> g, c
 // (own_digit[b] == d) the raised value is the NTT-form input limb, which is read in
 // place from `own` instead of from `raised` (cerium/compiler/backend/kernel_instruction.h:
 // 823-838 moves it; here it is never copied).
-// Bound by memory: 482 MB for 35 + 5 limbs and 7 digits of 64-bit words.  The key is more than half of that, and nobody
-// reads it or the raised limbs again before they would be gone: both are loaded to leave L2 first, so the raised limbs
-// that the transform wrote last are still there and the accumulators that the ModDown reads next stay.  Loads in flight
+// Bound by memory: 482 MB for 35 + 5 limbs and 7 digits of 64-bit words.  The key is more than half of that, and is
+// read once; key and raised limbs are loaded to leave L2 first, so the raised limbs that the transform wrote last are
+// still there and the accumulators that the ModDown reads next stay.  That holds for hoisted rotations as well, which
+// read the raised limbs again for every key: with plain loads of them one ModUp and 7 rotations take 1371 us against
+// 1343 at 35 limbs, 803 / 790 at 20, 544 / 536 at 12, and the same at 6 (430); 841 / 835 at 51 32-bit limbs.  Loads in flight
 // come from CTAs, not from the loop: 4 CTAs (64 registers) and a step at a time for 64-bit words, 5 and two steps for
 // 32-bit words.  With one step more or four registers over the limit a CTA is lost and a rotation of 35 limbs takes 364 us.
 // Against plain loads and no limit: 35 limbs 355.6 -> 349.2 us, 51 32-bit limbs 205.8 -> 200.0 us.

@@ -161,8 +161,7 @@ struct cerium_context {
   // CERIUM_B200_NTT_ARITH is "int" when the context is created (for comparisons)
   bool allow_fp = true;
   int sm_count = 1;  // SMs of the device (launch shapes are sized in multiples of it)
-  std::vector<uint64_t> mu_hi, mu_lo;  // Barrett constants per prime (host copy)
-  std::vector<uint8_t> fp_ok, lazy_ok; // arithmetic of each prime's transforms (host copy)
+  std::vector<uint8_t> fp_ok;  // primes whose transforms run on doubles (host copy)
   size_t word_bytes() const { return (size_t)word_bits / 8; }
   // q_a^-1 mod q_b, found once per pair (the extended Euclid of a rescale's factors was most of its host time): a table
   // of n_primes^2 words, 0 = not known yet; concurrent calls at worst find the same value twice
@@ -182,7 +181,7 @@ struct cerium_bconv {
   cerium_context* ctx = nullptr;
   int mode = 0;
   int I = 0, O = 0;
-  std::vector<uint32_t> in_primes, out_primes;
+  std::vector<uint32_t> in_primes;
   // one device allocation holding every table below
   void* d_block = nullptr;
   int steps = 0;                // steps of 32 input bytes of the products
