@@ -17,8 +17,9 @@ def be(request):
 
 @pytest.mark.parametrize("word_bits,n_in,n_out,mode", [
     (64, 1, 1, _capi.BCONV_LAZY), (64, 4, 8, _capi.BCONV_EXACT), (64, 5, 9, _capi.BCONV_LAZY), (64, 9, 17, _capi.BCONV_EXACT),
-    (64, 33, 3, _capi.BCONV_LAZY), (64, 64, 6, _capi.BCONV_LAZY),
+    (64, 33, 3, _capi.BCONV_LAZY), (64, 64, 6, _capi.BCONV_LAZY), (64, 8, 16, _capi.BCONV_LAZY), (64, 32, 7, _capi.BCONV_EXACT),
     (32, 1, 1, _capi.BCONV_LAZY), (32, 8, 9, _capi.BCONV_EXACT), (32, 17, 16, _capi.BCONV_LAZY), (32, 21, 25, _capi.BCONV_EXACT),
+    (32, 32, 17, _capi.BCONV_LAZY), (32, 33, 8, _capi.BCONV_EXACT),
 ])
 def test_bconv_edges(be, word_bits, n_in, n_out, mode):
     if word_bits == 64:     # outputs of 30 to 60 bits in one conversion, inputs of 60 and 50 bits

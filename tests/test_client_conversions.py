@@ -38,16 +38,17 @@ def test_residues(be, word_bits):
             assert np.array_equal(got[l], np.array(want, dtype=np.uint64))
 
 
-@pytest.mark.parametrize("limbs", [1, 2, 17, 64])
+@pytest.mark.parametrize("limbs", [1, 2, 17, 64, 255])
 def test_compose(be, limbs):
-    mods = params.reference_primes_28bit(64)[:limbs]
+    mods = params.reference_primes_28bit(64)[:limbs] if limbs <= 64 else params.ntt_primes_below(30, limbs, 16)
     ctx = _capi.Context(be.lib, mods, 32)
     big = 1
     for q in mods:
         big *= q
     rng = np.random.default_rng(limbs)
     # magnitudes from a few bits up to the whole range, and the values where the rounding or the sign turns
-    vals = [int.from_bytes(rng.bytes(240), "little") % max(2, big >> int(rng.integers(0, big.bit_length()))) for _ in range(N)]
+    vals = [int.from_bytes(rng.bytes(240 if limbs <= 64 else 1000), "little") % max(2, big >> int(rng.integers(0, big.bit_length())))
+            for _ in range(N if limbs <= 64 else 1024)] * (1 if limbs <= 64 else N // 1024)
     vals = [(-x if i & 1 else x) for i, x in enumerate(vals)]
     vals[:6] = [0, 1, -1, big // 2, -(big // 2), big // 2 - 1]
     if limbs > 2:
