@@ -115,6 +115,9 @@ class Watchdog:
                 os._exit(3)
 
 
+MIN_SAMPLED_MS = 500.0   # of timed blocks: ten samples 50 ms apart
+
+
 class ClockSampler:
     """Samples SM clocks and throttle reasons with nvidia-smi while the timed region runs."""
 
@@ -1065,11 +1068,12 @@ def bind_to_gpu_numa(torch, local_rank):
         return None
 
 
-def time_blocks(torch, dist, world, wl, steps, blocks, barrier):
+def time_blocks(torch, dist, world, wl, steps, blocks, barrier, at_least_ms=0.0):
     """`blocks` timed regions of `steps` steps each (CUDA events on the current stream, side streams
-    forked and joined inside, max over ranks); returns the list of milliseconds."""
+    forked and joined inside, max over ranks), and as many more as make `at_least_ms` in all by the time of
+    the first; returns the list of milliseconds."""
     out = []
-    for _ in range(blocks):
+    while len(out) < blocks or len(out) * out[0] < at_least_ms:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         barrier()
         e0.record()
@@ -1248,7 +1252,9 @@ def main():
     if profile_range:
         torch.cuda.profiler.start()
     dog.at("timed blocks")
-    block_ms = time_blocks(torch, dist, world, wl, args.steps, max(1, args.blocks), barrier)
+    # short steps are repeated until the clocks have been sampled under load a few times
+    block_ms = time_blocks(torch, dist, world, wl, args.steps, max(1, args.blocks), barrier,
+                           at_least_ms=0.0 if profile_range or args.blocks < 2 else MIN_SAMPLED_MS)
     if profile_range:
         torch.cuda.synchronize()
         torch.cuda.profiler.stop()
