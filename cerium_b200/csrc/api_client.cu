@@ -106,7 +106,7 @@ int cerium_compose_create(cerium_context* ctx, cerium_compose** out, const uint3
   std::memcpy(bytes.data() + c->o_inv, inv.data(), inv.size() * 4);
   std::memcpy(bytes.data() + c->o_table, table.data(), table.size() * 4);
   if (cudaMalloc(&c->d_block, bytes.size()) != cudaSuccess ||
-      cudaMemcpy(c->d_block, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaMemcpy(c->d_block, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess || uploads_done() != cudaSuccess) {
     cerium_compose_destroy(c);
     return fail(CERIUM_ERR_CUDA, "compose_create: table upload failed");
   }

@@ -422,7 +422,8 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
     delete bc;
     return fail(CERIUM_ERR_CUDA, "bconv_create: cudaMalloc failed");
   }
-  if (cudaMemcpy(bc->d_block, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpy(bc->d_block, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      uploads_done() != cudaSuccess) {
     cudaFree(bc->d_block);
     delete bc;
     return fail(CERIUM_ERR_CUDA, "bconv_create: upload failed");
@@ -671,6 +672,7 @@ int cerium_context_create(cerium_context** out, int device, int log_n, int word_
     CERIUM_CUDA(cudaMemcpy(ctx->d_tw_fwd, fwd.data(), fwd.size() * sizeof(Pair), cudaMemcpyHostToDevice));
     CERIUM_CUDA(cudaMemcpy(ctx->d_tw_inv, inv.data(), inv.size() * sizeof(Pair), cudaMemcpyHostToDevice));
     CERIUM_CUDA(cudaMemcpy(ctx->d_pcs, pcs.data(), pcs.size() * sizeof(PrimeConst<W>), cudaMemcpyHostToDevice));
+    CERIUM_CUDA(uploads_done());
     return CERIUM_OK;
   });
   if (rc != CERIUM_OK) {
@@ -701,6 +703,7 @@ int cerium_context_check(cerium_context* ctx) {
   CERIUM_CUDA(cudaMemcpy(&st, ctx->d_status, sizeof(st), cudaMemcpyDeviceToHost));  // waits for the device's work
   if (st == 0) return CERIUM_OK;
   CERIUM_CUDA(cudaMemset(ctx->d_status, 0, sizeof(st)));
+  CERIUM_CUDA(uploads_done());
   std::string msg = "context_check:";
   if (st & kStatusBconvShape) msg += " a base-conversion table entry exceeded the shape bounds of its launch (that conversion was skipped);";
   if (st & ~kStatusBconvShape) msg += " unknown status bits;";

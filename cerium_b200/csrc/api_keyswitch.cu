@@ -671,7 +671,7 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
       else reinterpret_cast<uint64_t*>(bytes.data())[i] = v[i];
     }
     return cudaMalloc(dst, bytes.size()) == cudaSuccess &&
-           cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+           cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice) == cudaSuccess && uploads_done() == cudaSuccess;
   };
   // ModDown with rescale levels folded in (one-GPU plans only)
   for (int r = 1; r <= 2 && world == 1 && !lifted && L - r >= 1; r++) {

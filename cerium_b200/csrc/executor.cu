@@ -814,6 +814,7 @@ cerium_program* load_program(cerium_context* ctx, const std::string& functions_p
     const FunctionMapType& fmap = getter();
     Loader ld{p, ctx, {}};
     ld.build(recs, fmap, scalars);
+    if (uploads_done() != cudaSuccess) throw std::runtime_error("upload failed");
   } catch (...) {
     cerium_program_destroy(p);
     throw;

@@ -127,6 +127,11 @@ inline int dispatch_word(int word_bits, F&& fn) {
   return fn(uint64_t{});
 }
 
+// The end of every call that makes a handle: what it copied from pageable memory, or set, is in place.  cudaMemcpy may
+// return when the bytes have left the caller's buffer, with the copy to the device still queued on the default
+// stream, and a stream created without blocking does not wait for that one.
+inline cudaError_t uploads_done() { return cudaStreamSynchronize(nullptr); }
+
 // RAII switch to the context's device for the duration of a call.
 struct DeviceGuard {
   int prev = -1;

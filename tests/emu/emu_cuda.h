@@ -52,6 +52,7 @@ void sync_warp();
 void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()>& body);
 long launches();  // number of launches so far (tests use it to see that kernels ran)
 void set_smem_limit(const void* kernel, int bytes);
+void default_stream(bool pending);  // something was queued on the default stream / the host has waited for it
 }  // namespace cerium_emu
 
 #define threadIdx (::cerium_emu::t_threadIdx)
@@ -98,11 +99,22 @@ static inline cudaError_t cudaMalloc(void** p, size_t n) {
 template <typename T>
 static inline cudaError_t cudaMalloc(T** p, size_t n) { return cudaMalloc(reinterpret_cast<void**>(p), n); }
 static inline cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
-static inline cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
+static inline cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind kind) {
+  std::memcpy(d, s, n);
+  ::cerium_emu::default_stream(kind == cudaMemcpyHostToDevice);
+  return cudaSuccess;
+}
 static inline cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { std::memmove(d, s, n); return cudaSuccess; }
-static inline cudaError_t cudaMemset(void* d, int v, size_t n) { std::memset(d, v, n); return cudaSuccess; }
+static inline cudaError_t cudaMemset(void* d, int v, size_t n) {
+  std::memset(d, v, n);
+  ::cerium_emu::default_stream(true);
+  return cudaSuccess;
+}
 static inline cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { std::memset(d, v, n); return cudaSuccess; }
-static inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+static inline cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  if (s == nullptr) ::cerium_emu::default_stream(false);
+  return cudaSuccess;
+}
 static inline cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 enum cudaDeviceAttr { cudaDevAttrMultiProcessorCount = 16 };
 static inline cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 2; return cudaSuccess; }

@@ -126,8 +126,17 @@ void set_smem_limit(const void* kernel, int bytes) {
   at = bytes;
 }
 
+// Host-to-device copies and fills of the synchronous calls may still be queued when the call returns; a kernel of a
+// non-blocking stream that is launched before the host has waited may read what was there before.
+namespace {
+std::atomic<bool> g_pending{false};
+std::atomic<long> g_early{0};
+}  // namespace
+void default_stream(bool pending) { g_pending = pending; }
+
 void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()>& body) {
   g_launches++;
+  if (g_pending) g_early++;
   const long nblocks = (long)grid.x * grid.y * grid.z;
 #pragma omp parallel
   {
@@ -148,3 +157,5 @@ void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()
 
 // how often a kernel's limit was lowered
 extern "C" long cerium_emu_lowered_smem_limits() { return cerium_emu::g_lowered; }
+// launches before the default stream's copies were waited for
+extern "C" long cerium_emu_early_launches() { return cerium_emu::g_early; }
