@@ -46,10 +46,10 @@ from cerium_b200 import params  # noqa: E402
 
 LOGN = 16
 N = 1 << LOGN
-# dram__bytes_read.sum + dram__bytes_write.sum of the forward-NTT launch pair from the ncu capture
-# summarised in profiles/hrot_u64_top_kernels_ncu_full.md: 443.2 MB for 245 u64 limbs (traffic grows
-# in proportion to the limbs transformed)
-NTT_PAIR_DRAM_BYTES_PER_LIMB = 443.2e6 / 245
+# dram__bytes_read.sum + dram__bytes_write.sum of the forward-NTT launch pair by number of u64 limbs, repeated on the same
+# buffers with the caches left alone (profiles/key_switch_u64_traffic_and_pipes.md).  Measured, not scaled: the second
+# pass starts where the first ended, so the share that L2 serves depends on the size.
+NTT_PAIR_DRAM_BYTES = {245: 354.2e6, 384: 770.9e6, 576: 1015.9e6}
 # what the CPU figure is: the checker, not a tuned evaluator
 PORT_QUALITY = ("unoptimised checker: plain-C restatement with a 128-bit remainder in every modular product outside "
                 "the transforms; a Barrett/Shoup CPU evaluator would be several times faster")
@@ -453,9 +453,8 @@ class HMultWorkload(Workload):
         self.host_in[1].copy_(self.b.cpu())
         self.host_out = torch.empty(self.out.shape, dtype=torch.int64).pin_memory()
         # tensor; key switch: iNTT pair, NTT pair x2 (576 limbs in two batches), inner product, iNTT pair,
-        # BConv, SuD pair; then either the rescale of both polynomials (iNTT pair, SuD pair) or, folded
-        # into the ModDown, two PMU launches
-        self.gpu_launches_per_step = 1 + (2 + 4 + 1 + 2 + 1 + 2) + (2 if self.rescale_mode == 2 else 4)
+        # BConv, SuD pair; then the rescale of both polynomials (iNTT pair, SuD pair) unless it is folded into the ModDown
+        self.gpu_launches_per_step = 1 + (2 + 4 + 1 + 2 + 1 + 2) + (0 if self.rescale_mode == 2 else 4)
 
     def step(self):
         s = self.torch.cuda.current_stream().cuda_stream
@@ -764,10 +763,10 @@ class BootstrapWorkload(Workload):
         torch.cuda.synchronize()
         n = self.ev.count.n
         self.op_counts = dict(n)
-        # launches: ModRaise 19; a BSGS stage 5 + 7 * 6 + 2 + 2 + 8 * 6 + 5; an HMult 15; a conjugation 11;
-        # a rescale 4; every other pass 1
-        self.gpu_launches_per_step = (19 * n["mod_raise"] + 104 * n["bsgs"] + 15 * n["hmult"] + 11 + 4 * n["rescale"]
-                                      + n["ewise"] + 2 * n["pt_mac"])
+        # launches: ModRaise 21; a BSGS stage 5 + 7 * 6 + 2 + 2 + 8 * 6 + 5; an HMult 12; a conjugation 11;
+        # a rescale 4; every other pass 1, and ModUps that convert their digits in two launches
+        self.gpu_launches_per_step = (21 * n["mod_raise"] + 104 * n["bsgs"] + 12 * n["hmult"] + 11 + 4 * n["rescale"]
+                                      + n["ewise"] + 2 * n["pt_mac"] + n["split_mod_up"])
         self.ev.count.n = {}
         self.alg_bytes = 0
 
@@ -1108,9 +1107,9 @@ def roofline_of(torch, wl, peak, peak_kind, iters=20):
     u32 = getattr(wl, "dtype", "u64") == "u32"
     limbs = wl.rl_bytes // (2 * N * (4 if u32 else 8))
     return {"bound": "hbm", "kernel": wl.rl_name, "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "traffic": None if u32 else NTT_PAIR_DRAM_BYTES_PER_LIMB * limbs,
-            "traffic_source": ("no ncu capture of the 32-bit transform pair" if u32 else
-                               "profiles/ (ncu capture of the forward NTT pair, scaled by limbs)"),
+            "frac": achieved / peak, "traffic": None if u32 else NTT_PAIR_DRAM_BYTES.get(limbs),
+            "traffic_source": ("no ncu capture of the transform pair at this size" if u32 or limbs not in NTT_PAIR_DRAM_BYTES else
+                               "profiles/ (ncu capture of this launch pair)"),
             "peak_kind": peak_kind, "ms_per_launch_pair": rl_ms, "algorithmic_bytes": wl.rl_bytes}, rl_ms, limbs
 
 
