@@ -365,7 +365,15 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       }
     }
     // 7. SuD: out = (acc_Q - NTT(conv)) * P^-1 (+ add); both polynomials in one launch pair
-    if (2 * L <= kSudMaxBatch) {
+    // An output that lies on the other polynomial's addition is written after that has been read: one polynomial at a
+    // time then, the reader first.
+    const size_t poly_bytes = (size_t)L * n * sizeof(W);
+    auto onto = [&](const void* out, const void* add) {
+      const uintptr_t x = (uintptr_t)out, y = (uintptr_t)add;
+      return add != nullptr && x < y + poly_bytes && y < x + poly_bytes;
+    };
+    const bool second_first = onto(out0, add1) && !onto(out1, add0);
+    if (2 * L <= kSudMaxBatch && !onto(out0, add1) && !onto(out1, add0)) {
       std::vector<uint32_t> prime2(ks->q_idx);
       prime2.insert(prime2.end(), ks->q_idx.begin(), ks->q_idx.end());
       std::vector<uint64_t> factor2(ks->pinv);
@@ -393,7 +401,8 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       s.store_galois = store_elt;
       if (int rc = launch_sud(ctx, s, stream)) return rc;
     } else {
-      for (int p = 0; p < 2; p++) {
+      for (int k = 0; k < 2; k++) {
+        const int p = second_first ? 1 - k : k;
         SudCall s{};
         s.src = conv + (size_t)p * L * n;
         s.src_stride = n;
