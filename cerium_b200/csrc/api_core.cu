@@ -139,6 +139,7 @@ int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t strea
       } else {
         launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, stream);
       }
+      if (c.cols_only) continue;
       if (lazy_out) {
         launch_fwd_rows<W>(ctx, rows, LazyStoreEpilogue<W>{}, cnt, stream);
       } else {

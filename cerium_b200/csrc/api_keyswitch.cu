@@ -6,8 +6,8 @@
 // instead of being compiled per program:
 //   1 launch pair  iNTT of the switched polynomial            (L limbs)
 //   1 launch       base conversion of every digit             (dnum conversions in one grid)
-//   1 launch pair  NTT of all converted limbs of all digits   (dnum*(L+K) - L limbs)
-//   1 launch       inner product with the key over all digits (L+K limbs, 2 outputs)
+//   1 launch       column pass of the NTT of all converted limbs of all digits (dnum*(L+K) - L limbs)
+//   1 launch       row pass and inner product with the key over all digits (L+K limbs, 2 outputs)
 //   1 launch pair  iNTT of the 2*K extension limbs
 //   1 launch       base conversion P -> Q for both outputs
 //   2 launch pairs SuD (NTT fused with subtract, multiply by P^-1 and the final addition)
@@ -167,6 +167,13 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
   return CERIUM_OK;
 }
 
+// Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where it can read the key
+// and the polynomials four words at a time.  Hoisted rotations transform the digits once for many keys instead.
+bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* evk, const void* add0, const void* add1) {
+  const uintptr_t ptrs = (uintptr_t)cpoly | (uintptr_t)evk | (uintptr_t)add0 | (uintptr_t)add1;
+  return ptrs % (4 * ks->ctx->word_bytes()) == 0;
+}
+
 // Step 1: inverse transform of the local limbs of the switched polynomial into `dst`
 // ([gather_limbs][N]; exact mode: times [Qhat_i^-1] of the limb's digit).
 // pre_elt (here and below), not 0: the key switch runs on the Galois automorphism of this element
@@ -183,7 +190,8 @@ int keyswitch_begin(cerium_keyswitch* ks, void* dst, const void* cpoly, cudaStre
 // (i % world) * gather_limbs + i / world).
 // Steps 2-3: base conversion of every digit and forward transform of the converted limbs into
 // the plan's `raised` buffer.
-int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t stream) {
+// rows_left: the transforms stop after their column pass, keyswitch_inner with the same argument does the rest.
+int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t stream, bool rows_left = false) {
   cerium_context* ctx = ks->ctx;
   const size_t n = kN;
   const int LK = ks->LK;
@@ -194,6 +202,7 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
       NttCall c{gathered, raised, n, n, ks->ntt_pos.data(), ks->ntt_prime.data(), (int)ks->ntt_pos.size()};
       c.src_pos = ks->ntt_src.data();
       c.src_prime = ks->ntt_src_prime.data();
+      c.cols_only = rows_left;
       return launch_ntt_forward(ctx, c, stream, /*lazy_out=*/true);
     }
     // 2. ModUp base conversion, every digit in one launch
@@ -209,6 +218,7 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
     {
       NttCall c{raised, raised, n, n, ks->ntt_pos.data(), ks->ntt_prime.data(), (int)ks->ntt_pos.size()};
       c.lazy_in = true;  // the converters of step 2 are created with lazy_out
+      c.cols_only = rows_left;
       if (int rc = launch_ntt_forward(ctx, c, stream, /*lazy_out=*/true)) return rc;
     }
     return CERIUM_OK;
@@ -222,7 +232,7 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
 // Q limbs as well.  As one more product of the sums they cost one read; as launches of their own they read and wrote the
 // accumulators again (7 us each at 24 limbs).
 int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cudaStream_t stream, uint32_t pre_elt = 0,
-                    bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr) {
+                    bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr, bool rows_left = false) {
   if (((uintptr_t)add0 | (uintptr_t)add1) & 15u) return fail(CERIUM_ERR_INVALID, "keyswitch: additions must be 16-byte aligned");
   cerium_context* ctx = ks->ctx;
   const size_t n = kN;
@@ -259,7 +269,11 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     }
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
     // every local extended limb (Q and extension) in one launch
-    { auto kfn = inner_product_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, pcs); }
+    if (rows_left) {
+      auto kfn = raised_inner_kernel<W, kRaisedRows>;
+      CERIUM_LAUNCH(kfn, dim3(256 / kRaisedRows, LK), dim3(32 * kRaisedRows), 0, stream, g,
+                    static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd), pcs);
+    } else { auto kfn = inner_product_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, pcs); }
     CERIUM_LAUNCH_CHECK("inner_product");
     return CERIUM_OK;
   });
@@ -444,19 +458,20 @@ void launch_pt_mac(const PtMacArgs<W>& a, bool pieces, dim3 grid, cudaStream_t s
 // Steps 4-7.  Can be repeated with different keys on the same raised digits (hoisting).
 int keyswitch_inner_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* cpoly, const void* evk,
                             const void* add0, const void* add1, cudaStream_t stream, uint32_t pre_elt = 0,
-                            uint32_t store_elt = 0, cerium_comm* comm = nullptr, int r = 0) {
+                            uint32_t store_elt = 0, cerium_comm* comm = nullptr, int r = 0, bool rows_left = false) {
   if (ks->ext_split && comm == nullptr)
     return fail(CERIUM_ERR_INVALID, "keyswitch: a plan with split extension limbs needs a communicator");
   const bool early = r > 0;  // all Q limbs get the additions (the dropped ones as well: they are divided away)
-  if (int rc = keyswitch_inner(ks, cpoly, evk, stream, pre_elt, false, early ? add0 : nullptr, early ? add1 : nullptr)) return rc;
+  if (int rc = keyswitch_inner(ks, cpoly, evk, stream, pre_elt, false, early ? add0 : nullptr, early ? add1 : nullptr, rows_left)) return rc;
   return keyswitch_moddown(ks, out0, out1, early ? nullptr : add0, early ? nullptr : add1, stream, pre_elt, store_elt, comm, r);
 }
 
 int keyswitch_finish(cerium_keyswitch* ks, void* out0, void* out1, const void* gathered, const void* cpoly,
                      const void* evk, const void* add0, const void* add1, cudaStream_t stream, uint32_t pre_elt = 0,
                      cerium_comm* comm = nullptr) {
-  if (int rc = keyswitch_raise(ks, gathered, stream)) return rc;
-  return keyswitch_inner_moddown(ks, out0, out1, cpoly, evk, add0, add1, stream, pre_elt, 0, comm);
+  const bool fused = rows_with_inner(ks, cpoly, evk, add0, add1);
+  if (int rc = keyswitch_raise(ks, gathered, stream, fused)) return rc;
+  return keyswitch_inner_moddown(ks, out0, out1, cpoly, evk, add0, add1, stream, pre_elt, 0, comm, 0, fused);
 }
 
 // The whole key switch of a limb-sharded plan: inverse transform of the local limbs straight into
@@ -482,8 +497,9 @@ int keyswitch_impl(cerium_keyswitch* ks, void* out0, void* out1, const void* cpo
   if (ks->lifted) return fail(CERIUM_ERR_INVALID, "keyswitch: a lifted plan only serves cerium_mod_raise");
   void* coef = static_cast<char*>(ks->ws) + ks->o_coef * ks->ctx->word_bytes();
   if (int rc = keyswitch_begin(ks, coef, cpoly, stream, pre_elt)) return rc;
-  if (int rc = keyswitch_raise(ks, coef, stream)) return rc;
-  return keyswitch_inner_moddown(ks, out0, out1, cpoly, evk, add0, add1, stream, pre_elt, 0, nullptr, r);
+  const bool fused = rows_with_inner(ks, cpoly, evk, add0, add1);
+  if (int rc = keyswitch_raise(ks, coef, stream, fused)) return rc;
+  return keyswitch_inner_moddown(ks, out0, out1, cpoly, evk, add0, add1, stream, pre_elt, 0, nullptr, r, fused);
 }
 
 }  // namespace
@@ -822,13 +838,15 @@ int cerium_mod_raise(cerium_keyswitch* ks, void* out0, void* out1, const void* c
     if (int rc = launch_ntt_forward(ctx, c, st)) return rc;
   }
   // 4. c1 lifted to every prime of the plan: the one digit of the key switch
+  const bool fused = rows_with_inner(ks, nullptr, evk, nullptr, nullptr);
   if (int rc = cerium_mod2(ctx, raised, n, tmp + 6 * limb, tmp + 7 * limb, ks->all_idx.data(), LK, stream)) return rc;
   {
     NttCall c{raised, raised, n, n, nullptr, ks->all_idx.data(), LK};
+    c.cols_only = fused;
     if (int rc = launch_ntt_forward(ctx, c, st, /*lazy_out=*/true)) return rc;
   }
   // 5-6. product with the key, ModDown
-  if (int rc = keyswitch_inner_moddown(ks, kso, kso + (size_t)L * limb, nullptr, evk, nullptr, nullptr, st)) return rc;
+  if (int rc = keyswitch_inner_moddown(ks, kso, kso + (size_t)L * limb, nullptr, evk, nullptr, nullptr, st, 0, 0, nullptr, 0, fused)) return rc;
   // 7-8. drop the plan's last Q limb; add the lifted c0
   void* outs[2] = {out0, out1};
   void* scratch = ws + ks->o_scratch * wb;
@@ -1258,9 +1276,9 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
     if (!have[i] || giant_elts[i] == 1) continue;
     const char* s1 = inner + (size_t)i * 2 * poly + poly;
     if (int r2 = keyswitch_begin(ks, coef, s1, st, giant_elts[i])) return r2;
-    if (int r2 = keyswitch_raise(ks, coef, st)) return r2;
-    const bool add = i == last && rescale_levels > 0;
-    if (int r2 = keyswitch_inner(ks, s1, giant_keys[i], st, giant_elts[i], !first, add ? sum0 : nullptr, add ? sum1 : nullptr)) return r2;
+    const bool add = i == last && rescale_levels > 0, fused = rows_with_inner(ks, s1, giant_keys[i], sum0, sum1);
+    if (int r2 = keyswitch_raise(ks, coef, st, fused)) return r2;
+    if (int r2 = keyswitch_inner(ks, s1, giant_keys[i], st, giant_elts[i], !first, add ? sum0 : nullptr, add ? sum1 : nullptr, fused)) return r2;
     first = false;
   }
   if (first) {

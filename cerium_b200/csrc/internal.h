@@ -22,6 +22,7 @@
 #include "ewise_kernels.cuh"
 #include "host_math.h"
 #include "ntt_kernels.cuh"
+#include "raised_inner.cuh"
 
 namespace cerium {
 
@@ -267,6 +268,8 @@ struct NttCall {
   bool lazy_in = false;
   // inverse transform only, not 0: the input limbs are read through the Galois automorphism of this element
   uint32_t in_galois = 0;
+  // forward transform only: the column pass alone; raised_inner_kernel does the rows
+  bool cols_only = false;
 };
 // lazy_out: leave the results below 4q instead of canonical (internal buffers read by the inner product only)
 int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t stream, bool lazy_out = false);

@@ -1,0 +1,352 @@
+// Row pass of the raised digits and their inner product with the evaluation key in one kernel.
+//
+// A warp owns one row (256 words) of one output limb.  It walks the digits: takes the row of the digit's column pass through
+// the last eight layers and multiplies the result with the two key rows into sums that stay in its registers, so the raised
+// digits are never written in transformed form (302 MB written and read again for 24 digits of 24 limbs).
+//
+// Bound by memory: 482 MB for 7 digits on 40 limbs of 64-bit words, 945 MB for 24 digits on 25.  The twiddles of a row serve
+// every digit from shared memory (read through L1 for every digit they took the gain away: 147 us for the first shape, the
+// two kernels 143).  A lane keeps 8 words and 16 sums, so that 16 warps fit an SM at 128 registers; with 16 words to a lane
+// it would be 8.  The next digit's row is on its way (cp.async) while one is worked on, and the key rows are asked for before
+// the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against 301).
+// Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 118.8 us against 122.4).
+// Measured, row pass + inner product -> this kernel: rotation of 35 limbs 340.6 -> 301.3 us, multiplication of 24 limbs with
+// one-limb digits 536 -> 471, rotation of 51 32-bit limbs 197.2 -> 182.9, of 12 64-bit limbs 119.2 -> 118.8.
+#pragma once
+#include "ewise_kernels.cuh"
+#include "ntt_kernels.cuh"
+
+namespace cerium {
+
+// Four consecutive words, one access of 32 bytes (64-bit words) or 16.
+template <typename W>
+struct Quad {
+  W v[4];
+};
+__device__ __forceinline__ Quad<uint32_t> quad_load(const uint32_t* p) {
+  const uint4 t = *reinterpret_cast<const uint4*>(p);
+  return {{t.x, t.y, t.z, t.w}};
+}
+// words that nothing reads again soon
+__device__ __forceinline__ Quad<uint32_t> quad_load_once(const uint32_t* p) {
+  const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p));
+  return {{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ void quad_store(uint32_t* p, const Quad<uint32_t>& q) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+#if defined(CERIUM_EMU)
+inline Quad<uint64_t> quad_load(const uint64_t* p) { return {{p[0], p[1], p[2], p[3]}}; }
+inline Quad<uint64_t> quad_load_once(const uint64_t* p) { return quad_load(p); }
+inline void quad_store(uint64_t* p, const Quad<uint64_t>& q) {
+  for (int e = 0; e < 4; e++) p[e] = q.v[e];
+}
+#else
+__device__ __forceinline__ Quad<uint64_t> quad_load(const uint64_t* p) {
+  Quad<uint64_t> q;
+  asm volatile("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
+  return q;
+}
+__device__ __forceinline__ Quad<uint64_t> quad_load_once(const uint64_t* p) {
+  Quad<uint64_t> q;
+  asm volatile("ld.global.cs.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
+  return q;
+}
+__device__ __forceinline__ void quad_store(uint64_t* p, const Quad<uint64_t>& q) {
+  asm volatile("st.global.v4.b64 [%0], {%1,%2,%3,%4};" ::"l"(p), "l"(q.v[0]), "l"(q.v[1]), "l"(q.v[2]), "l"(q.v[3]) : "memory");
+}
+#endif
+
+// Bounds of the Fp butterflies over the eight layers of a row, as fp_plan_fwd has them for four.
+struct FpRowPlan {
+  bool before[8];
+  int out;
+};
+__host__ __device__ constexpr FpRowPlan fp_plan_row(int bin) {
+  FpRowPlan p{};
+  int b = bin;
+  for (int t = 0; t < 8; t++) {
+    p.before[t] = b > kFpOperandMax;
+    if (p.before[t]) b = kFpReduced;
+    b += fp_product_bound(b, t < 6 ? 1 : kFpLaneK32);  // the last two layers compute their quotients
+  }
+  p.out = b;
+  return p;
+}
+static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values must stay exact integers");
+
+// Sums of products of residues with key words.  Integer arithmetic: two words, one reduction at the end.  Fp: every product
+// comes back as y k - c q, c the rounded quotient.  With |y| <= q, 0 <= k < q < 2^50 the quotient RN(RN(y k) RN(1/q)) is off
+// by 3/2^53 * 2^50 = 3/8 at most before it is rounded, so a product is below 7/8 q, and eight of them on a reduced sum stay
+// below 8 q: exact (RN(y k) - c q is an integer below 2^53, as in fp_mulmod).
+template <typename W, int kMode>
+struct KeySum {
+  static constexpr int kTerms = 1 << 30;           // on a reduced sum
+  static constexpr bool kEarly = sizeof(W) == 4;  // registers for a digit's key words during the butterflies
+  Acc2<W> acc;
+  __device__ __forceinline__ void clear() { acc.clear(); }
+  __device__ __forceinline__ void add(const Arith<W, kMode>&, W y, W k) { acc.mad(y, k); }
+  __device__ __forceinline__ void reduce(const Arith<W, kMode>&) {}
+  __device__ __forceinline__ W finish(const Arith<W, kMode>&, const PrimeConst<W>& pc) const { return barrett2<W>(acc.hi(), acc.lo(), pc); }
+};
+template <>
+struct KeySum<uint64_t, kArithFp> {
+  using A = Arith<uint64_t, kArithFp>;
+  static constexpr int kTerms = 8;
+  static constexpr bool kEarly = true;
+  double s;
+  __device__ __forceinline__ void clear() { s = 0.0; }
+  __device__ __forceinline__ void add(const A& ar, uint64_t y, uint64_t k) {
+    const double yd = A::d(y), kd = fp_from_u64(k);
+    const double h = __dmul_rn(yd, kd);
+    const double l = __fma_rn(yd, kd, -h);
+    const double c = __dadd_rn(__fma_rn(h, ar.qinv, kFpMagic), -kFpMagic);
+    s = __dadd_rn(s, __dadd_rn(__fma_rn(c, ar.nq, h), l));
+  }
+  __device__ __forceinline__ void reduce(const A& ar) { s = fp_reduce(s, ar.qinv, ar.nq); }
+  __device__ __forceinline__ uint64_t finish(const A& ar, const PrimeConst<uint64_t>&) const {
+    return ar.canonical(fp_reduce(s, ar.qinv, ar.nq));
+  }
+};
+
+constexpr int kRaisedRows = 2;  // rows of a CTA, one warp each
+
+// Exchange buffer of a row: word i at i + 4 (i / 32), 64-bit words with bit 1 of i flipped where bit 4 is set.  The three
+// patterns (a run of 32; 8 runs of 4 at a distance of 32; 4 words of each of 32 neighbouring lanes, 16 bytes at a time) are
+// then free of bank conflicts.
+constexpr int kRaisedPitch = 256 + 8 * 4;
+template <typename W>
+__device__ __forceinline__ int raised_pos(int i) {
+  return (sizeof(W) == 8 ? i ^ ((i >> 3) & 2) : i) + (i >> 5) * 4;
+}
+
+// A row's shared memory: the digit that is worked on and the next one on its way, and the twiddles of the row, which serve
+// every digit.  Pair (1 << t) + g is entry ((256 + h) << t) + g of the table, layers t = 0..7.  64-bit words: layers 0..5
+// only; Fp has the last two without their quotients after them, word (1 << t) + g - 64 of `late`.  The integer butterflies of
+// 64-bit words read those from global memory.
+template <typename W>
+struct alignas(16) RaisedRow {
+  static constexpr int kPairs = sizeof(W) == 8 ? 64 : 256;
+  W buf[2][kRaisedPitch];
+  typename WordTraits<W>::Pair tw[kPairs];
+  W late[sizeof(W) == 8 ? 192 : 2];
+};
+template <typename W, bool kFp>
+__device__ __forceinline__ void raised_twiddles(RaisedRow<W>& row, const typename WordTraits<W>::Pair* tw, int h) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t S = 256u + (uint32_t)h;
+#pragma unroll
+  for (int k = 0; k < (sizeof(W) == 8 && !kFp ? 2 : 8); k++) {
+    const int i = k * 32 + lane;
+    if (i == 0) continue;
+    const int t = 31 - __clz(i);
+    const auto w = __ldg(tw + ((S << t) + (uint32_t)(i - (1 << t))));
+    if (i < RaisedRow<W>::kPairs) row.tw[i] = w;
+    else row.late[sizeof(W) == 8 ? i - 64 : 0] = w.x;
+  }
+}
+
+// Three layers on x[0..7]; layer t pairs (j, j + (4 >> t)) with twiddle (S << t) + (j >> (3 - t)).  kLayer: number of the
+// first one inside the row.
+template <typename W, int kMode, int kLayer>
+__device__ __forceinline__ void radix8_fwd(W (&x)[8], const typename WordTraits<W>::Pair* tw, int S, const Arith<W, kMode>& ar) {
+  constexpr FpRowPlan plan = fp_plan_row(kFpFwdMid);
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    const int half = 4 >> t;
+    if (kMode == kArithFp && plan.before[kLayer + t]) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) x[j] = ar.reduce(x[j]);
+    }
+#pragma unroll
+    for (int g = 0; g < (1 << t); g++) {
+      const auto w = tw[(S << t) + g];
+#pragma unroll
+      for (int k = 0; k < half; k++) ar.fwd(x[g * 2 * half + k], x[g * 2 * half + k + half], w.x, w.y);
+    }
+  }
+}
+
+// The eight layers of row h.  In: x[j] = word j * 32 + lane.  Out: x[r] = word (r / 4) * 128 + lane * 4 + r % 4, Fp:
+// |x| <= 0.51 q, integers: below 4q.
+template <typename W, int kMode>
+__device__ __forceinline__ void raised_row(W (&x)[8], W* ex, const RaisedRow<W>& row, const typename WordTraits<W>::Pair* tw, int h,
+                                           const Arith<W, kMode>& ar, const PrimeConst<W>& pc) {
+  using RV = RowVec<W>;
+  constexpr FpRowPlan plan = fp_plan_row(kFpFwdMid);
+  const int lane = threadIdx.x & 31;
+  radix8_fwd<W, kMode, 0>(x, row.tw, 1, ar);
+#pragma unroll
+  for (int j = 0; j < 8; j++) ex[raised_pos<W>(j * 32 + lane)] = x[j];
+  __syncwarp();
+  const int own = (lane >> 2) * 32 + (lane & 3);
+#pragma unroll
+  for (int j = 0; j < 8; j++) x[j] = ex[raised_pos<W>(own + 4 * j)];
+  radix8_fwd<W, kMode, 3>(x, row.tw, 8 + (lane >> 2), ar);
+#pragma unroll
+  for (int j = 0; j < 8; j++) ex[raised_pos<W>(own + 4 * j)] = x[j];
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; k += RV::kWords)
+    vec_unpack(*reinterpret_cast<const typename RV::Vec*>(ex + raised_pos<W>((k >> 2) * 128 + lane * 4 + (k & 3))), &x[k]);
+  __syncwarp();  // the buffer is free for the digit after the next
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int g = k * 32 + lane;
+    W w6[2], w7[4];  // twiddles, each with its companion
+    if constexpr (kMode == kArithFp) {
+      W v[2];
+      vec_unpack(*reinterpret_cast<const typename RV::Vec*>(row.late + 64 + 2 * g), v);
+      w6[0] = row.late[g], w6[1] = ar.quotient(w6[0]);
+      w7[0] = v[0], w7[1] = ar.quotient(v[0]), w7[2] = v[1], w7[3] = ar.quotient(v[1]);
+    } else {
+      constexpr bool kNear = sizeof(W) == 4;
+      const auto* at6 = kNear ? row.tw + (64 + g) % RaisedRow<W>::kPairs : tw + ((256 + h) * 64 + g);
+      const auto* at7 = kNear ? row.tw + (128 + 2 * g) % RaisedRow<W>::kPairs : tw + ((256 + h) * 128 + 2 * g);
+      const auto a = at6[0], b = at7[0], c = at7[1];
+      w6[0] = a.x, w6[1] = a.y, w7[0] = b.x, w7[1] = b.y, w7[2] = c.x, w7[3] = c.y;
+    }
+    if (kMode == kArithFp && plan.before[6]) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) x[4 * k + j] = ar.reduce(x[4 * k + j]);
+    }
+    ar.fwd(x[4 * k], x[4 * k + 2], w6[0], w6[1]);
+    ar.fwd(x[4 * k + 1], x[4 * k + 3], w6[0], w6[1]);
+    if (kMode == kArithFp && plan.before[7]) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) x[4 * k + j] = ar.reduce(x[4 * k + j]);
+    }
+    ar.fwd(x[4 * k], x[4 * k + 1], w7[0], w7[1]);
+    ar.fwd(x[4 * k + 2], x[4 * k + 3], w7[2], w7[3]);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    if constexpr (kMode == kArithFp) x[j] = ar.reduce(x[j]);
+    else x[j] = ar.template finish_fwd<false>(x[j], pc.one_shoup);
+  }
+}
+
+template <typename W, int kMode, int kRows>
+__device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, int b, int h, const PrimeConst<W>& pc, RaisedRow<W>& row,
+                                                  const typename WordTraits<W>::Pair* tw) {
+  const Arith<W, kMode> ar(pc);
+  using Sum = KeySum<W, kMode>;
+  constexpr int kWords = RowVec<W>::kWords;
+  const int lane = threadIdx.x & 31;
+  raised_twiddles<W, kMode == kArithFp>(row, tw, h);
+  grid_dependency_wait();
+  const size_t at = (size_t)(h * 256 + lane * 4);  // this lane's first quad; the second one is 128 words on
+  const W* rp = g.raised + (size_t)b * g.raised_limb_stride + h * 256;
+  const W* kp = g.evk + (size_t)b * g.evk_limb_stride + at;
+  const int own_digit = g.own_digit[b];
+  Sum sum[2][8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    sum[0][j].clear();
+    sum[1][j].clear();
+  }
+  auto fetch = [&](int d) {
+    if (d < g.dnum && d != own_digit) {
+#pragma unroll
+      for (int j = 0; j < 8 / kWords; j++)
+        copy_async<16>(row.buf[d & 1] + (j * 32 + lane) * kWords, rp + (size_t)d * g.raised_digit_stride + (j * 32 + lane) * kWords);
+    }
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int d = 0; d < g.dnum; d++) {
+    Quad<W> key[2][2];
+    auto fetch_key = [&](int p) {
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        key[p][k] = quad_load_once(kp + (size_t)d * g.evk_digit_stride + (size_t)p * g.evk_poly_stride + k * 128);
+    };
+    if (Sum::kEarly) {
+      fetch_key(0);
+      fetch_key(1);
+    }
+    W y[8];
+    row_twiddles_wait();  // digit d is here, and the first time the twiddles
+    fetch(d + 1);         // its buffer was the previous digit's
+    if (d != own_digit) {
+      W* ex = row.buf[d & 1];
+#pragma unroll
+      for (int j = 0; j < 8; j++) y[j] = ex[j * 32 + lane];
+      __syncwarp();
+      raised_row<W, kMode>(y, ex, row, tw, h, ar, pc);
+    } else {
+      const W* limb = g.own + (size_t)b * g.own_stride;
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        if (g.own_elt != 0) {
+          // the automorphism maps aligned groups of words onto aligned groups
+          const GaloisGroup<4> gg((uint32_t)at + 128u * (uint32_t)k, g.own_elt);
+          const Quad<W> t = quad_load(limb + gg.at);
+          W w[4];
+          gg.permute(t.v, w);
+#pragma unroll
+          for (int e = 0; e < 4; e++) y[4 * k + e] = ar.enter(w[e]);
+        } else {
+          const Quad<W> t = quad_load_once(limb + at + 128 * k);
+#pragma unroll
+          for (int e = 0; e < 4; e++) y[4 * k + e] = ar.enter(t.v[e]);
+        }
+      }
+    }
+    if (d != 0 && d % Sum::kTerms == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        sum[0][j].reduce(ar);
+        sum[1][j].reduce(ar);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      if (!Sum::kEarly) fetch_key(p);
+#pragma unroll
+      for (int j = 0; j < 8; j++) sum[p][j].add(ar, y[j], key[p][j >> 2].v[j & 3]);
+    }
+  }
+  const W* adds[2] = {g.add0, g.add1};
+  W* outs[2] = {g.out0.at(b, (int)at), g.out1.at(b, (int)at)};
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      if (b < g.add_limbs && adds[p] != nullptr) {
+        const Quad<W> t = quad_load_once(adds[p] + (size_t)b * g.add_stride + at + 128 * k);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          sum[p][4 * k + e].reduce(ar);
+          sum[p][4 * k + e].add(ar, ar.enter(t.v[e]), g.add_factor[b]);
+        }
+      }
+      Quad<W> o;
+#pragma unroll
+      for (int e = 0; e < 4; e++) o.v[e] = sum[p][4 * k + e].finish(ar, pc);
+      if (g.accumulate != 0) {
+        const Quad<W> t = quad_load(outs[p] + 128 * k);
+#pragma unroll
+        for (int e = 0; e < 4; e++) o.v[e] = add_mod<W>(o.v[e], t.v[e], pc.q);
+      }
+      quad_store(outs[p] + 128 * k, o);
+    }
+  }
+}
+
+// grid = (256 / kRows, limbs), block = 32 kRows.
+template <typename W, int kRows>
+__global__ void __launch_bounds__(32 * kRows, (sizeof(W) == 8 ? 16 : 20) / kRows)
+    raised_inner_kernel(const InnerProductArgs<W> g, const typename WordTraits<W>::Pair* __restrict__ tw_all,
+                        const PrimeConst<W>* __restrict__ pcs) {
+  __shared__ RaisedRow<W> rows[kRows];
+  grid_dependency_launch();
+  const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
+  const int warp = threadIdx.x >> 5, h = blockIdx.x * kRows + warp;
+  const uint32_t pi = g.prime[b];
+  const PrimeConst<W> pc = pcs[pi];
+  const auto* tw = tw_all + (size_t)pi * kN;
+  CERIUM_DISPATCH_ARITH(W, pc, raised_inner_body, kRows, (g, b, h, pc, rows[warp], tw));
+}
+
+}  // namespace cerium

@@ -79,6 +79,7 @@ static inline unsigned __brev(unsigned x) {
   for (int i = 0; i < 32; i++) { r = (r << 1) | (x & 1); x >>= 1; }
   return r;
 }
+static inline int __clz(int x) { return x == 0 ? 32 : __builtin_clz((unsigned)x); }
 template <typename T>
 static inline T __ldg(const T* p) { return *p; }
 template <typename T>
