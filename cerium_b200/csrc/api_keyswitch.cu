@@ -167,11 +167,22 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
   return CERIUM_OK;
 }
 
+// Digits from which on two warps share a row of raised_inner_kernel<uint64_t>: whole rounds of CTAs are shorter (24 limbs
+// with as many digits 467 -> 452 us, 15 limbs 257.5 -> 256.5); 7 digits on 40 limbs lose (301 -> 320 us).  32-bit words are never split:
+// rotations of 3 to 51 limbs lose 5 to 10 %.
+constexpr int kSplitDigits = 12;
 // Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where it can read the key
-// and the polynomials four words at a time.  Hoisted rotations transform the digits once for many keys instead.
+// and the polynomials four words at a time, and 64-bit words have the rows that keep the resident warps (16 to an SM) busy.
+// With fewer the serial walk over the digits shows: rotation of 10 limbs (15 with the extension) 102.9 us in two kernels and
+// 110.6 in one, 11 limbs 113.6 / 115.4, 12 limbs 118.0 / 117.3, 13 limbs 138.2 / 129.2; digits of one limb, 10 limbs
+// 180.1 / 183.6, 12 limbs 220.9 / 216.0.  32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 197.4 / 182.8).
+// Hoisted rotations transform the digits once for many keys and keep the two kernels.
 bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* evk, const void* add0, const void* add1) {
   const uintptr_t ptrs = (uintptr_t)cpoly | (uintptr_t)evk | (uintptr_t)add0 | (uintptr_t)add1;
-  return ptrs % (4 * ks->ctx->word_bytes()) == 0;
+  if (ptrs % (4 * ks->ctx->word_bytes()) != 0) return false;
+  if (ks->ctx->word_bits == 32) return true;
+  const double rows_per_warp = 256.0 * ks->LK / (16.0 * ks->ctx->sm_count);
+  return rows_per_warp >= (ks->dnum >= kSplitDigits ? 1.4 : 1.8);
 }
 
 // Step 1: inverse transform of the local limbs of the switched polynomial into `dst`
@@ -270,9 +281,12 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
     // every local extended limb (Q and extension) in one launch
     if (rows_left) {
-      auto kfn = raised_inner_kernel<W, kRaisedRows>;
-      CERIUM_LAUNCH(kfn, dim3(256 / kRaisedRows, LK), dim3(32 * kRaisedRows), 0, stream, g,
-                    static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd), pcs);
+      const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
+      const int split = sizeof(W) == 8 && dnum >= kSplitDigits ? 2 : 1;
+      auto kfn = raised_inner_kernel<W, 2, 1>;
+      if constexpr (sizeof(W) == 8)
+        if (split == 2) kfn = raised_inner_kernel<W, 2, 2>;
+      CERIUM_LAUNCH(kfn, dim3(128 * split, LK), dim3(64), 0, stream, g, tw, pcs);
     } else { auto kfn = inner_product_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, pcs); }
     CERIUM_LAUNCH_CHECK("inner_product");
     return CERIUM_OK;

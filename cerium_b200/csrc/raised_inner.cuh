@@ -1,17 +1,19 @@
 // Row pass of the raised digits and their inner product with the evaluation key in one kernel.
 //
-// A warp owns one row (256 words) of one output limb.  It walks the digits: takes the row of the digit's column pass through
-// the last eight layers and multiplies the result with the two key rows into sums that stay in its registers, so the raised
-// digits are never written in transformed form (302 MB written and read again for 24 digits of 24 limbs).
+// A warp (two of them where there are many digits) owns one row (256 words) of one output limb.  It walks the digits: takes
+// the row of the digit's column pass through the last eight layers and multiplies the result with the two key rows into
+// sums that stay in its registers, so the raised digits are never written in transformed form (302 MB written and read again
+// for 24 digits of 24 limbs).
 //
 // Bound by memory: 482 MB for 7 digits on 40 limbs of 64-bit words, 945 MB for 24 digits on 25.  The twiddles of a row serve
 // every digit from shared memory (read through L1 for every digit they took the gain away: 147 us for the first shape, the
 // two kernels 143).  A lane keeps 8 words and 16 sums, so that 16 warps fit an SM at 128 registers; with 16 words to a lane
 // it would be 8.  The next digit's row is on its way (cp.async) while one is worked on, and the key rows are asked for before
 // the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against 301).
-// Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 118.8 us against 122.4).
+// Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 117.3 us against 122.4).
 // Measured, row pass + inner product -> this kernel: rotation of 35 limbs 340.6 -> 301.3 us, multiplication of 24 limbs with
-// one-limb digits 536 -> 471, rotation of 51 32-bit limbs 197.2 -> 182.9, of 12 64-bit limbs 119.2 -> 118.8.
+// one-limb digits 540 -> 452, rotation of 51 32-bit limbs 197.2 -> 182.9.  When it is used: rows_with_inner
+// (api_keyswitch.cu).
 #pragma once
 #include "ewise_kernels.cuh"
 #include "ntt_kernels.cuh"
@@ -75,41 +77,69 @@ __host__ __device__ constexpr FpRowPlan fp_plan_row(int bin) {
 }
 static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values must stay exact integers");
 
-// Sums of products of residues with key words.  Integer arithmetic: two words, one reduction at the end.  Fp: every product
-// comes back as y k - c q, c the rounded quotient.  With |y| <= q, 0 <= k < q < 2^50 the quotient RN(RN(y k) RN(1/q)) is off
-// by 3/2^53 * 2^50 = 3/8 at most before it is rounded, so a product is below 7/8 q, and eight of them on a reduced sum stay
-// below 8 q: exact (RN(y k) - c q is an integer below 2^53, as in fp_mulmod).
+// Sums of products of residues (integers: below 4q) with key words; 64 bits, so that partial sums of a row can be put
+// together.
+//   32-bit words: the products themselves, one reduction at the end.
+//   64-bit integers: every product x = y k < 4 q^2 is reduced: t = x / 2^(b - 2), q of b bits (52 to 60), is below 2^64, the quotient
+//   hi(t * floor(2^(b + 62) / q)) is short by less than 1/2 + 1 + 1 + 2 (t, the factor, the product, mulhi_approx64), so the
+//   remainder is below 4.5 q, and a sum below 5q + 2^32 stays there when 5q leaves it where its high word says so (csub_high).
+//   Sums of two words take 64 registers and leave none for the key words that are on their way.
+//   Fp: every product comes back as y k - c q, c the rounded quotient.  With |y| <= q, 0 <= k < q < 2^50 the quotient
+//   RN(RN(y k) RN(1/q)) is off by 3/2^53 * 2^50 = 3/8 at most before it is rounded, so a product is below 7/8 q, and eight of
+//   them on a reduced sum stay below 8 q: exact (RN(y k) - c q is an integer below 2^53, as in fp_mulmod).
 template <typename W, int kMode>
 struct KeySum {
-  static constexpr int kTerms = 1 << 30;           // on a reduced sum
-  static constexpr bool kEarly = sizeof(W) == 4;  // registers for a digit's key words during the butterflies
-  Acc2<W> acc;
-  __device__ __forceinline__ void clear() { acc.clear(); }
-  __device__ __forceinline__ void add(const Arith<W, kMode>&, W y, W k) { acc.mad(y, k); }
-  __device__ __forceinline__ void reduce(const Arith<W, kMode>&) {}
-  __device__ __forceinline__ W finish(const Arith<W, kMode>&, const PrimeConst<W>& pc) const { return barrett2<W>(acc.hi(), acc.lo(), pc); }
+  static constexpr int kTerms = 1 << 30;  // on a reduced sum
+  using A = Arith<W, kMode>;
+  const A& ar;
+  uint64_t mu;  // 64-bit integers
+  int shift;    // ... what is left of b - 2 when a word has been passed over
+  __device__ __forceinline__ KeySum(const A& a, const PrimeConst<W>& pc) : ar(a), mu(0), shift(0) {
+    if constexpr (sizeof(W) == 8) {
+      const int bits = 64 - __clzll((long long)pc.q);
+      mu = pc.mu_hi << (bits - 2) | pc.mu_lo >> (66 - bits);
+      shift = bits - 2 - 32;
+    }
+  }
+  __device__ __forceinline__ void add(uint64_t& s, W y, W k) const {
+    if constexpr (sizeof(W) == 4) {
+      s += (uint64_t)y * k;
+    } else {
+      const uint64_t lo = y * k, hi = WordTraits<W>::mulhi(y, k);
+      const uint64_t t = (uint64_t)__funnelshift_r((uint32_t)hi, (uint32_t)(hi >> 32), shift) << 32 |
+                         __funnelshift_r((uint32_t)(lo >> 32), (uint32_t)hi, shift);
+      s = csub_high(s + (lo + mulhi_approx64(t, mu) * ar.nq), ar.q4 + ar.q);
+    }
+  }
+  __device__ __forceinline__ void reduce(uint64_t&) const {}
+  __device__ __forceinline__ void join(uint64_t& s, uint64_t t) const {
+    if constexpr (sizeof(W) == 4) s += t;
+    else s = csub_high(s + t, ar.q4 + ar.q);
+  }
+  __device__ __forceinline__ W finish(uint64_t s, const PrimeConst<W>& pc) const {
+    if constexpr (sizeof(W) == 4) return barrett2<W>((W)(s >> 32), (W)s, pc);
+    else return reduce_word<W>(s, pc);
+  }
 };
 template <>
 struct KeySum<uint64_t, kArithFp> {
-  using A = Arith<uint64_t, kArithFp>;
   static constexpr int kTerms = 8;
-  static constexpr bool kEarly = true;
-  double s;
-  __device__ __forceinline__ void clear() { s = 0.0; }
-  __device__ __forceinline__ void add(const A& ar, uint64_t y, uint64_t k) {
+  using A = Arith<uint64_t, kArithFp>;
+  const A& ar;
+  __device__ __forceinline__ KeySum(const A& a, const PrimeConst<uint64_t>&) : ar(a) {}
+  __device__ __forceinline__ void add(uint64_t& s, uint64_t y, uint64_t k) const {
     const double yd = A::d(y), kd = fp_from_u64(k);
     const double h = __dmul_rn(yd, kd);
     const double l = __fma_rn(yd, kd, -h);
     const double c = __dadd_rn(__fma_rn(h, ar.qinv, kFpMagic), -kFpMagic);
-    s = __dadd_rn(s, __dadd_rn(__fma_rn(c, ar.nq, h), l));
+    s = A::u(__dadd_rn(A::d(s), __dadd_rn(__fma_rn(c, ar.nq, h), l)));
   }
-  __device__ __forceinline__ void reduce(const A& ar) { s = fp_reduce(s, ar.qinv, ar.nq); }
-  __device__ __forceinline__ uint64_t finish(const A& ar, const PrimeConst<uint64_t>&) const {
-    return ar.canonical(fp_reduce(s, ar.qinv, ar.nq));
+  __device__ __forceinline__ void reduce(uint64_t& s) const { s = ar.reduce(s); }
+  __device__ __forceinline__ void join(uint64_t& s, uint64_t t) const { s = A::u(__dadd_rn(A::d(s), A::d(t))); }
+  __device__ __forceinline__ uint64_t finish(uint64_t s, const PrimeConst<uint64_t>&) const {
+    return ar.canonical(fp_reduce(A::d(s), ar.qinv, ar.nq));
   }
 };
-
-constexpr int kRaisedRows = 2;  // rows of a CTA, one warp each
 
 // Exchange buffer of a row: word i at i + 4 (i / 32), 64-bit words with bit 1 of i flipped where bit 4 is set.  The three
 // patterns (a run of 32; 8 runs of 4 at a distance of 32; 4 words of each of 32 neighbouring lanes, 16 bytes at a time) are
@@ -144,6 +174,8 @@ __device__ __forceinline__ void raised_twiddles(RaisedRow<W>& row, const typenam
     if (i < RaisedRow<W>::kPairs) row.tw[i] = w;
     else row.late[sizeof(W) == 8 ? i - 64 : 0] = w.x;
   }
+  if (sizeof(W) == 8 && !kFp && lane < 24)  // the others on their way: lines of 128 bytes, 8 of layer 6 and 16 of layer 7
+    prefetch_l2(lane < 8 ? tw + (S * 64u + 8u * (uint32_t)lane) : tw + (S * 128u + 8u * (uint32_t)(lane - 8)));
 }
 
 // Three layers on x[0..7]; layer t pairs (j, j + (4 >> t)) with twiddle (S << t) + (j >> (3 - t)).  kLayer: number of the
@@ -226,50 +258,48 @@ __device__ __forceinline__ void raised_row(W (&x)[8], W* ex, const RaisedRow<W>&
   }
 }
 
-template <typename W, int kMode, int kRows>
-__device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, int b, int h, const PrimeConst<W>& pc, RaisedRow<W>& row,
-                                                  const typename WordTraits<W>::Pair* tw) {
+// kSplit warps share a row: warp `part` takes digits part, part + kSplit, ..., and finishes polynomial `part` from the sums of
+// all of them (kSplit = 1: both).
+template <typename W, int kMode, int kSplit>
+__device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, int b, int h, int part, const PrimeConst<W>& pc,
+                                                  RaisedRow<W>* rows, const typename WordTraits<W>::Pair* tw) {
   const Arith<W, kMode> ar(pc);
   using Sum = KeySum<W, kMode>;
+  const Sum ks(ar, pc);
   constexpr int kWords = RowVec<W>::kWords;
   const int lane = threadIdx.x & 31;
+  RaisedRow<W>& row = rows[part];
   raised_twiddles<W, kMode == kArithFp>(row, tw, h);
   grid_dependency_wait();
   const size_t at = (size_t)(h * 256 + lane * 4);  // this lane's first quad; the second one is 128 words on
   const W* rp = g.raised + (size_t)b * g.raised_limb_stride + h * 256;
   const W* kp = g.evk + (size_t)b * g.evk_limb_stride + at;
   const int own_digit = g.own_digit[b];
-  Sum sum[2][8];
+  uint64_t sum[2][8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    sum[0][j].clear();
-    sum[1][j].clear();
-  }
-  auto fetch = [&](int d) {
+  for (int j = 0; j < 8; j++) sum[0][j] = sum[1][j] = 0;  // 0.0 as well
+  auto fetch = [&](int d, int into) {
     if (d < g.dnum && d != own_digit) {
 #pragma unroll
       for (int j = 0; j < 8 / kWords; j++)
-        copy_async<16>(row.buf[d & 1] + (j * 32 + lane) * kWords, rp + (size_t)d * g.raised_digit_stride + (j * 32 + lane) * kWords);
+        copy_async<16>(row.buf[into] + (j * 32 + lane) * kWords, rp + (size_t)d * g.raised_digit_stride + (j * 32 + lane) * kWords);
     }
   };
-  fetch(0);
+  fetch(part, 0);
+  int n = 0;  // terms so far
 #pragma unroll 1
-  for (int d = 0; d < g.dnum; d++) {
+  for (int d = part; d < g.dnum; d += kSplit, n++) {
     Quad<W> key[2][2];
-    auto fetch_key = [&](int p) {
+#pragma unroll
+    for (int p = 0; p < 2; p++)
 #pragma unroll
       for (int k = 0; k < 2; k++)
         key[p][k] = quad_load_once(kp + (size_t)d * g.evk_digit_stride + (size_t)p * g.evk_poly_stride + k * 128);
-    };
-    if (Sum::kEarly) {
-      fetch_key(0);
-      fetch_key(1);
-    }
     W y[8];
-    row_twiddles_wait();  // digit d is here, and the first time the twiddles
-    fetch(d + 1);         // its buffer was the previous digit's
+    row_twiddles_wait();             // this digit is here, and the first time the twiddles
+    fetch(d + kSplit, (n & 1) ^ 1);  // its buffer was the previous digit's
     if (d != own_digit) {
-      W* ex = row.buf[d & 1];
+      W* ex = row.buf[n & 1];
 #pragma unroll
       for (int j = 0; j < 8; j++) y[j] = ex[j * 32 + lane];
       __syncwarp();
@@ -293,60 +323,87 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
         }
       }
     }
-    if (d != 0 && d % Sum::kTerms == 0) {
+    if (n != 0 && n % Sum::kTerms == 0) {
 #pragma unroll
       for (int j = 0; j < 8; j++) {
-        sum[0][j].reduce(ar);
-        sum[1][j].reduce(ar);
+        ks.reduce(sum[0][j]);
+        ks.reduce(sum[1][j]);
       }
     }
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-      if (!Sum::kEarly) fetch_key(p);
+    for (int p = 0; p < 2; p++)
 #pragma unroll
-      for (int j = 0; j < 8; j++) sum[p][j].add(ar, y[j], key[p][j >> 2].v[j & 3]);
-    }
+      for (int j = 0; j < 8; j++) ks.add(sum[p][j], y[j], key[p][j >> 2].v[j & 3]);
   }
-  const W* adds[2] = {g.add0, g.add1};
-  W* outs[2] = {g.out0.at(b, (int)at), g.out1.at(b, (int)at)};
-#pragma unroll
-  for (int p = 0; p < 2; p++) {
+  // adds what joins the sums, and stores
+  auto finish = [&](uint64_t (&s)[8], const W* add, W* out) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      if (b < g.add_limbs && adds[p] != nullptr) {
-        const Quad<W> t = quad_load_once(adds[p] + (size_t)b * g.add_stride + at + 128 * k);
+      if (b < g.add_limbs && add != nullptr) {
+        const Quad<W> t = quad_load_once(add + (size_t)b * g.add_stride + at + 128 * k);
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          sum[p][4 * k + e].reduce(ar);
-          sum[p][4 * k + e].add(ar, ar.enter(t.v[e]), g.add_factor[b]);
+          ks.reduce(s[4 * k + e]);
+          ks.add(s[4 * k + e], ar.enter(t.v[e]), g.add_factor[b]);
         }
       }
       Quad<W> o;
 #pragma unroll
-      for (int e = 0; e < 4; e++) o.v[e] = sum[p][4 * k + e].finish(ar, pc);
+      for (int e = 0; e < 4; e++) o.v[e] = ks.finish(s[4 * k + e], pc);
+      W* to = out + 128 * k;
       if (g.accumulate != 0) {
-        const Quad<W> t = quad_load(outs[p] + 128 * k);
+        const Quad<W> t = quad_load(to);
 #pragma unroll
         for (int e = 0; e < 4; e++) o.v[e] = add_mod<W>(o.v[e], t.v[e], pc.q);
       }
-      quad_store(outs[p] + 128 * k, o);
+      quad_store(to, o);
+    }
+  };
+  if constexpr (kSplit == 1) {
+    finish(sum[0], g.add0, g.out0.at(b, (int)at));
+    finish(sum[1], g.add1, g.out1.at(b, (int)at));
+  } else {
+    // the sums take the place of the digits and the twiddles; words of a lane 256 bytes apart
+    static_assert(sizeof(RaisedRow<W>) >= 2 * 8 * 32 * 8, "room for the sums of a warp");
+    uint64_t* mine = reinterpret_cast<uint64_t*>(&row) + lane;
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        ks.reduce(sum[p][j]);
+        mine[(p * 8 + j) * 32] = sum[p][j];
+      }
+    __syncthreads();
+    if (part < 2) {
+      uint64_t total[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        total[j] = 0;
+#pragma unroll
+        for (int o = 0; o < kSplit; o++) ks.join(total[j], (reinterpret_cast<const uint64_t*>(rows + o) + lane)[(part * 8 + j) * 32]);
+      }
+      finish(total, part == 0 ? g.add0 : g.add1, (part == 0 ? g.out0 : g.out1).at(b, (int)at));
     }
   }
 }
 
-// grid = (256 / kRows, limbs), block = 32 kRows.
-template <typename W, int kRows>
-__global__ void __launch_bounds__(32 * kRows, (sizeof(W) == 8 ? 16 : 20) / kRows)
+// A CTA has kWarps warps.  grid = (256 kSplit / kWarps, limbs), block = 32 kWarps.
+template <typename W, int kWarps, int kSplit>
+__global__ void __launch_bounds__(32 * kWarps, (sizeof(W) == 8 ? 16 : 20) / kWarps)
     raised_inner_kernel(const InnerProductArgs<W> g, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const PrimeConst<W>* __restrict__ pcs) {
-  __shared__ RaisedRow<W> rows[kRows];
+  static_assert(kSplit == 1 || kSplit == kWarps, "warps that share a row are the CTA");
+  __shared__ RaisedRow<W> rows[kWarps];
   grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
-  const int warp = threadIdx.x >> 5, h = blockIdx.x * kRows + warp;
+  const int warp = threadIdx.x >> 5;
+  const int h = kSplit == 1 ? blockIdx.x * kWarps + warp : blockIdx.x, part = kSplit == 1 ? 0 : warp;
+  RaisedRow<W>* mine = kSplit == 1 ? rows + warp : rows;
   const uint32_t pi = g.prime[b];
   const PrimeConst<W> pc = pcs[pi];
   const auto* tw = tw_all + (size_t)pi * kN;
-  CERIUM_DISPATCH_ARITH(W, pc, raised_inner_body, kRows, (g, b, h, pc, rows[warp], tw));
+  CERIUM_DISPATCH_ARITH(W, pc, raised_inner_body, kSplit, (g, b, h, part, pc, mine, tw));
 }
 
 }  // namespace cerium

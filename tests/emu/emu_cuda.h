@@ -79,6 +79,8 @@ static inline unsigned __brev(unsigned x) {
   for (int i = 0; i < 32; i++) { r = (r << 1) | (x & 1); x >>= 1; }
   return r;
 }
+static inline int __clzll(long long x) { return x == 0 ? 64 : __builtin_clzll((unsigned long long)x); }
+static inline unsigned __funnelshift_r(unsigned lo, unsigned hi, unsigned s) { return (unsigned)(((uint64_t)hi << 32 | lo) >> (s & 31)); }
 static inline int __clz(int x) { return x == 0 ? 32 : __builtin_clz((unsigned)x); }
 template <typename T>
 static inline T __ldg(const T* p) { return *p; }

@@ -22,7 +22,7 @@ def _params(word_bits, L, K, dnum):
     return params.CkksParams(pc.LOGN, 64, q + p60[1:], L, K, dnum)
 
 
-@pytest.mark.parametrize("word_bits,L,K,dnum", [(64, 3, 1, 3), (64, 10, 1, 10), (64, 5, 2, 3), (32, 9, 2, 5)])
+@pytest.mark.parametrize("word_bits,L,K,dnum", [(64, 3, 1, 3), (64, 12, 1, 12), (64, 15, 2, 10), (32, 9, 2, 5)])
 @pytest.mark.parametrize("offset", [0, 16])
 def test_key_switch(be, word_bits, L, K, dnum, offset):
     prm = _params(word_bits, L, K, dnum)
