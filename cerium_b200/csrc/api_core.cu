@@ -192,6 +192,11 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t strea
           gb.in_pos[b] = (uint16_t)c.src_pos[first + b];
         }
         launch_inv_rows<W>(ctx, gb, cnt, stream);
+      } else if (c.factor != nullptr) {
+        ProductBatch<W> pb{};
+        static_cast<StridedBatch<W>&>(pb) = sb;
+        pb.factor = static_cast<const W*>(c.factor);
+        launch_inv_rows<W>(ctx, pb, cnt, stream);
       } else {
         launch_inv_rows<W>(ctx, sb, cnt, stream);
       }

@@ -190,10 +190,13 @@ bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* 
 // pre_elt (here and below), not 0: the key switch runs on the Galois automorphism of this element
 // applied to cpoly and to add0 / add1, which are read through the index map wherever they are used
 // (a rotation then needs no pass and no copy of its own).
-int keyswitch_begin(cerium_keyswitch* ks, void* dst, const void* cpoly, cudaStream_t stream, uint32_t pre_elt = 0) {
+// factor: the switched polynomial is the product of cpoly and this one.
+int keyswitch_begin(cerium_keyswitch* ks, void* dst, const void* cpoly, cudaStream_t stream, uint32_t pre_elt = 0,
+                    const void* factor = nullptr) {
   const size_t n = kN;
   NttCall c{cpoly, dst, n, n, nullptr, ks->q_idx.data(), ks->L};
   c.in_galois = pre_elt;
+  c.factor = factor;
   return launch_ntt_inverse(ks->ctx, c, stream, ks->d_last_q);
 }
 
@@ -236,6 +239,11 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
   });
 }
 
+// Of a multiplication (a0, a1) (b0, b1) whose a1 is the polynomial that the steps are given.
+struct TensorInputs {
+  const void *a0, *b0, *b1;
+};
+
 // Step 4 on the digits that keyswitch_raise left in the plan: inner product with `evk` into the
 // plan's accumulators (both polynomials, every local extended limb).  accumulate: add to what the
 // accumulators hold (the giant steps of a BSGS multiply-accumulate sum up in the extended basis).
@@ -243,7 +251,8 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
 // Q limbs as well.  As one more product of the sums they cost one read; as launches of their own they read and wrote the
 // accumulators again (7 us each at 24 limbs).
 int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cudaStream_t stream, uint32_t pre_elt = 0,
-                    bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr, bool rows_left = false) {
+                    bool accumulate = false, const void* add0 = nullptr, const void* add1 = nullptr, bool rows_left = false,
+                    const TensorInputs* tensor = nullptr) {
   if (((uintptr_t)add0 | (uintptr_t)add1) & 15u) return fail(CERIUM_ERR_INVALID, "keyswitch: additions must be 16-byte aligned");
   cerium_context* ctx = ks->ctx;
   const size_t n = kN;
@@ -267,7 +276,7 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     g.out0 = {acc, n};
     g.out1 = {acc + (size_t)LK * n, n};
     g.dnum = dnum;
-    if (add0 != nullptr || add1 != nullptr) {
+    if (add0 != nullptr || add1 != nullptr || tensor != nullptr) {
       g.add0 = static_cast<const W*>(add0);
       g.add1 = static_cast<const W*>(add1);
       g.add_stride = n;
@@ -286,7 +295,9 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
       auto kfn = raised_inner_kernel<W, 2, 1>;
       if constexpr (sizeof(W) == 8)
         if (split == 2) kfn = raised_inner_kernel<W, 2, 2>;
-      CERIUM_LAUNCH(kfn, dim3(128 * split, LK), dim3(64), 0, stream, g, tw, pcs);
+      TensorOf<W> t{};
+      if (tensor != nullptr) t = {static_cast<const W*>(tensor->a0), static_cast<const W*>(tensor->b0), static_cast<const W*>(tensor->b1)};
+      CERIUM_LAUNCH(kfn, dim3(128 * split, LK), dim3(64), 0, stream, g, t, tw, pcs);
     } else { auto kfn = inner_product_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, pcs); }
     CERIUM_LAUNCH_CHECK("inner_product");
     return CERIUM_OK;
@@ -1105,12 +1116,29 @@ int cerium_hmult(cerium_keyswitch* ks, void* out0, void* out1, const void* a0, c
   void* d1 = tmp + (size_t)ks->L * limb;
   void* d2 = tmp + (size_t)2 * ks->L * limb;
   if (do_rescale < 0 || do_rescale > 2) return fail(CERIUM_ERR_INVALID, "hmult: do_rescale is 0, 1 or 2");
-  if (int rc = cerium_tensor(ctx, d0, d1, d2, a0, a1, b0, b1, n, ks->q_idx.data(), ks->L, stream)) return rc;
-  if (!do_rescale) return keyswitch_impl(ks, out0, out1, d2, evk, d0, d1, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  // The tensor product inside the inverse transform and the inner product, which multiply as they read; a0 b0 and
+  // a0 b1 + a1 b0 are added before the ModDown, as [P] times themselves, whatever it divides by.  Not with two warps to a row:
+  // there are more rounds of CTAs then, and each would start with those products (24 limbs with as many digits 439 -> 447 us,
+  // where digits of five limbs give 334 -> 318 us for 34 limbs and 186 -> 173 for 20).
+  const bool fused = !ks->lifted && ks->dnum < kSplitDigits &&
+                     rows_with_inner(ks, reinterpret_cast<const void*>((uintptr_t)a0 | (uintptr_t)a1), evk, b0, b1);
+  if (!fused)
+    if (int rc = cerium_tensor(ctx, d0, d1, d2, a0, a1, b0, b1, n, ks->q_idx.data(), ks->L, stream)) return rc;
+  auto relinearise = [&](void* to0, void* to1, int r) -> int {
+    if (!fused) return keyswitch_impl(ks, to0, to1, d2, evk, d0, d1, st, 0, r);
+    const TensorInputs tensor{a0, b0, b1};
+    void* coef = static_cast<char*>(ks->ws) + ks->o_coef * wb;
+    if (int rc = keyswitch_begin(ks, coef, a1, st, 0, b1)) return rc;
+    if (int rc = keyswitch_raise(ks, coef, st, true)) return rc;
+    if (int rc = keyswitch_inner(ks, a1, evk, st, 0, false, nullptr, nullptr, true, &tensor)) return rc;
+    return keyswitch_moddown(ks, to0, to1, nullptr, nullptr, st, 0, 0, nullptr, r);
+  };
+  if (!do_rescale) return relinearise(out0, out1, 0);
   // one division by P * q_last: the last limb joins the extension limbs of the ModDown
-  if (do_rescale == 2) return keyswitch_impl(ks, out0, out1, d2, evk, d0, d1, (cudaStream_t)stream, 0, 1);
+  if (do_rescale == 2) return relinearise(out0, out1, 1);
   char* kso = static_cast<char*>(ks->ws) + ks->o_ksout * wb;  // [2][L][N], contiguous: two polynomials
-  if (int rc = keyswitch_impl(ks, kso, kso + (size_t)ks->L * limb, d2, evk, d0, d1, (cudaStream_t)stream)) return rc;
+  if (int rc = relinearise(kso, kso + (size_t)ks->L * limb, 0)) return rc;
   void* scratch = static_cast<char*>(ks->ws) + ks->o_scratch * wb;
   // out0 / out1 are separate buffers: the shared column pass works in the (now free) ModDown buffer
   void* outs[2] = {out0, out1};

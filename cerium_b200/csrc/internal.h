@@ -268,6 +268,8 @@ struct NttCall {
   bool lazy_in = false;
   // inverse transform only, not 0: the input limbs are read through the Galois automorphism of this element
   uint32_t in_galois = 0;
+  // inverse transform only: the input is the product with the limbs of this stack, which lie as those of `in` do
+  const void* factor = nullptr;
   // forward transform only: the column pass alone; raised_inner_kernel does the rows
   bool cols_only = false;
 };

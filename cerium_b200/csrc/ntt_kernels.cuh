@@ -61,6 +61,7 @@ constexpr int kMaxBatch = 512;     // limbs per launch
 // in_stride = 0 makes every entry read the same source limb (rescale broadcasts the last limb).
 template <typename W>
 struct StridedBatch {
+  static constexpr bool kProduct = false;
   const W* in;
   W* out;
   size_t in_stride;   // in words
@@ -89,10 +90,19 @@ struct GatherBatch : StridedBatch<W> {
   }
 };
 
+// StridedBatch whose input is the product of two stacks of words with one stride (inverse transform).
+template <typename W>
+struct ProductBatch : StridedBatch<W> {
+  static constexpr bool kProduct = true;
+  const W* factor;
+  __device__ __forceinline__ const W* factor_limb(int b) const { return factor + (size_t)this->pos[b] * this->in_stride; }
+};
+
 // Addressing through device-resident pointer tables, the layout the reference's launchers
 // take (args_outputs / args_inputs / bases, cerium/compiler/backend/kernels/function.cu:22-39).
 template <typename W>
 struct PointerBatch {
+  static constexpr bool kProduct = false;
   W* const* outs;
   const W* const* ins;
   const uint32_t* bases;
@@ -971,6 +981,21 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
       vec_unpack(in[k], t);
       GaloisGroup<RV::kWords>((uint32_t)(h * 256 + (u + 16 * k) * RV::kWords), elt).permute(t, w);
       in[k] = vec_pack(w);
+    }
+  }
+  if constexpr (Batch::kProduct) {
+    const Vec* factor = reinterpret_cast<const Vec*>(batch.factor_limb(b) + h * 256);
+    Vec f[RV::kPerThread];
+#pragma unroll
+    for (int k = 0; k < RV::kPerThread; k++) f[k] = factor[u + 16 * k];
+#pragma unroll
+    for (int k = 0; k < RV::kPerThread; k++) {
+      W x[RV::kWords], y[RV::kWords];
+      vec_unpack(in[k], x);
+      vec_unpack(f[k], y);
+#pragma unroll
+      for (int e = 0; e < RV::kWords; e++) x[e] = mul_mod<W>(x[e], y[e], pc);
+      in[k] = vec_pack(x);
     }
   }
 #pragma unroll

@@ -258,10 +258,20 @@ __device__ __forceinline__ void raised_row(W (&x)[8], W* ex, const RaisedRow<W>&
   }
 }
 
-// kSplit warps share a row: warp `part` takes digits part, part + kSplit, ..., and finishes polynomial `part` from the sums of
-// all of them (kSplit = 1: both).
+// The inputs of a multiplication (a0, a1) (b0, b1), a1 being `own` of the inner product: the switched polynomial is a1 b1, its
+// own limbs are multiplied as they are read, and a0 b0 and a0 b1 + a1 b0 join the sums, so that the three products of the
+// tensor are never stored.  b0 null: none of that.
+template <typename W>
+struct TensorOf {
+  const W* a0;
+  const W* b0;
+  const W* b1;
+};
+
+// kSplit warps share a row: warp `part` takes every kSplit-th digit, and finishes polynomial `part` from the sums of all of
+// them (kSplit = 1: both).
 template <typename W, int kMode, int kSplit>
-__device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, int b, int h, int part, const PrimeConst<W>& pc,
+__device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, const TensorOf<W>& tensor, int b, int h, int part, const PrimeConst<W>& pc,
                                                   RaisedRow<W>* rows, const typename WordTraits<W>::Pair* tw) {
   const Arith<W, kMode> ar(pc);
   using Sum = KeySum<W, kMode>;
@@ -278,51 +288,113 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
   uint64_t sum[2][8];
 #pragma unroll
   for (int j = 0; j < 8; j++) sum[0][j] = sum[1][j] = 0;  // 0.0 as well
-  auto fetch = [&](int d, int into) {
-    if (d < g.dnum && d != own_digit) {
+  // the digits without the limb's own one, whose transform the caller has
+  const int own = own_digit < 0 ? g.dnum : own_digit, digits = g.dnum - (own_digit < 0 ? 0 : 1);
+  auto digit = [&](int e) { return e < own ? e : e + 1; };
+  auto fetch = [&](int e, int into) {
+    if (e < digits) {
 #pragma unroll
       for (int j = 0; j < 8 / kWords; j++)
-        copy_async<16>(row.buf[into] + (j * 32 + lane) * kWords, rp + (size_t)d * g.raised_digit_stride + (j * 32 + lane) * kWords);
+        copy_async<16>(row.buf[into] + (j * 32 + lane) * kWords, rp + (size_t)digit(e) * g.raised_digit_stride + (j * 32 + lane) * kWords);
     }
   };
   fetch(part, 0);
-  int n = 0;  // terms so far
-#pragma unroll 1
-  for (int d = part; d < g.dnum; d += kSplit, n++) {
-    Quad<W> key[2][2];
+  auto fetch_key = [&](Quad<W> (&to)[2][2], int d) {
 #pragma unroll
     for (int p = 0; p < 2; p++)
 #pragma unroll
       for (int k = 0; k < 2; k++)
-        key[p][k] = quad_load_once(kp + (size_t)d * g.evk_digit_stride + (size_t)p * g.evk_poly_stride + k * 128);
-    W y[8];
-    row_twiddles_wait();             // this digit is here, and the first time the twiddles
-    fetch(d + kSplit, (n & 1) ^ 1);  // its buffer was the previous digit's
-    if (d != own_digit) {
-      W* ex = row.buf[n & 1];
-#pragma unroll
-      for (int j = 0; j < 8; j++) y[j] = ex[j * 32 + lane];
-      __syncwarp();
-      raised_row<W, kMode>(y, ex, row, tw, h, ar, pc);
-    } else {
-      const W* limb = g.own + (size_t)b * g.own_stride;
+        to[p][k] = quad_load_once(kp + (size_t)d * g.evk_digit_stride + (size_t)p * g.evk_poly_stride + k * 128);
+  };
+  // What is known without a transform comes first, while the first digit is on its way: the own digit's products (first warp)
+  // and what joins the sums (last warp).  In the middle of the loop the own digit cost registers (200 bytes spilled), and at the
+  // end every load is waited for: rotation of 35 limbs 302 -> 297 us, of 12 limbs 118.6 -> 116.7.
+  if (own_digit >= 0) {
+    Quad<W> own_key[2][2];
+    if (part == 0) fetch_key(own_key, own_digit);
+    const size_t limb = (size_t)b * g.own_stride + at;
+    if (tensor.b0 != nullptr) {
+      Quad<W> a0[2], a1[2], b0[2], b1[2];
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        if (g.own_elt != 0) {
-          // the automorphism maps aligned groups of words onto aligned groups
-          const GaloisGroup<4> gg((uint32_t)at + 128u * (uint32_t)k, g.own_elt);
-          const Quad<W> t = quad_load(limb + gg.at);
-          W w[4];
-          gg.permute(t.v, w);
+        a1[k] = quad_load(g.own + limb + 128 * k);
+        b1[k] = quad_load(tensor.b1 + limb + 128 * k);
+        if (part == kSplit - 1) {
+          a0[k] = quad_load(tensor.a0 + limb + 128 * k);
+          b0[k] = quad_load(tensor.b0 + limb + 128 * k);
+        }
+      }
 #pragma unroll
-          for (int e = 0; e < 4; e++) y[4 * k + e] = ar.enter(w[e]);
-        } else {
-          const Quad<W> t = quad_load_once(limb + at + 128 * k);
+      for (int j = 0; j < 8; j++) {
+        const W x1 = a1[j >> 2].v[j & 3], z1 = b1[j >> 2].v[j & 3];
+        if (part == 0) {
+          const W y = ar.enter(mul_mod<W>(x1, z1, pc));
+          ks.add(sum[0][j], y, own_key[0][j >> 2].v[j & 3]);
+          ks.add(sum[1][j], y, own_key[1][j >> 2].v[j & 3]);
+        }
+        if (part == kSplit - 1) {
+          const W x0 = a0[j >> 2].v[j & 3], z0 = b0[j >> 2].v[j & 3];
+          ks.add(sum[0][j], ar.enter(mul_mod<W>(x0, z0, pc)), g.add_factor[b]);
+          Acc2<W> acc;
+          acc.clear();
+          acc.mad(x0, z1);
+          acc.mad(x1, z0);
+          ks.add(sum[1][j], ar.enter(barrett2<W>(acc.hi(), acc.lo(), pc)), g.add_factor[b]);
+        }
+      }
+    } else {
+      if (part == 0) {
 #pragma unroll
-          for (int e = 0; e < 4; e++) y[4 * k + e] = ar.enter(t.v[e]);
+        for (int k = 0; k < 2; k++) {
+          Quad<W> t;
+          if (g.own_elt != 0) {
+            // the automorphism maps aligned groups of words onto aligned groups
+            const GaloisGroup<4> gg((uint32_t)at + 128u * (uint32_t)k, g.own_elt);
+            gg.permute(quad_load(g.own + (size_t)b * g.own_stride + gg.at).v, t.v);
+          } else {
+            t = quad_load_once(g.own + limb + 128 * k);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const W y = ar.enter(t.v[e]);
+            ks.add(sum[0][4 * k + e], y, own_key[0][k].v[e]);
+            ks.add(sum[1][4 * k + e], y, own_key[1][k].v[e]);
+          }
+        }
+      }
+      if (b < g.add_limbs && part == kSplit - 1) {
+        const W* adds[2] = {g.add0, g.add1};
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          if (adds[p] == nullptr) continue;
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const Quad<W> t = quad_load_once(adds[p] + (size_t)b * g.add_stride + at + 128 * k);
+#pragma unroll
+            for (int e = 0; e < 4; e++) ks.add(sum[p][4 * k + e], ar.enter(t.v[e]), g.add_factor[b]);
+          }
         }
       }
     }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      ks.reduce(sum[0][j]);
+      ks.reduce(sum[1][j]);
+    }
+  }
+  int n = 0;  // terms so far
+#pragma unroll 1
+  for (int e = part; e < digits; e += kSplit, n++) {
+    Quad<W> key[2][2];
+    fetch_key(key, digit(e));
+    W y[8];
+    row_twiddles_wait();             // this digit is here, and the first time the twiddles
+    fetch(e + kSplit, (n & 1) ^ 1);  // its buffer was the previous digit's
+    W* ex = row.buf[n & 1];
+#pragma unroll
+    for (int j = 0; j < 8; j++) y[j] = ex[j * 32 + lane];
+    __syncwarp();
+    raised_row<W, kMode>(y, ex, row, tw, h, ar, pc);
     if (n != 0 && n % Sum::kTerms == 0) {
 #pragma unroll
       for (int j = 0; j < 8; j++) {
@@ -335,18 +407,9 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
 #pragma unroll
       for (int j = 0; j < 8; j++) ks.add(sum[p][j], y[j], key[p][j >> 2].v[j & 3]);
   }
-  // adds what joins the sums, and stores
-  auto finish = [&](uint64_t (&s)[8], const W* add, W* out) {
+  auto finish = [&](uint64_t (&s)[8], W* out) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      if (b < g.add_limbs && add != nullptr) {
-        const Quad<W> t = quad_load_once(add + (size_t)b * g.add_stride + at + 128 * k);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          ks.reduce(s[4 * k + e]);
-          ks.add(s[4 * k + e], ar.enter(t.v[e]), g.add_factor[b]);
-        }
-      }
       Quad<W> o;
 #pragma unroll
       for (int e = 0; e < 4; e++) o.v[e] = ks.finish(s[4 * k + e], pc);
@@ -360,8 +423,8 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
     }
   };
   if constexpr (kSplit == 1) {
-    finish(sum[0], g.add0, g.out0.at(b, (int)at));
-    finish(sum[1], g.add1, g.out1.at(b, (int)at));
+    finish(sum[0], g.out0.at(b, (int)at));
+    finish(sum[1], g.out1.at(b, (int)at));
   } else {
     // the sums take the place of the digits and the twiddles; words of a lane 256 bytes apart
     static_assert(sizeof(RaisedRow<W>) >= 2 * 8 * 32 * 8, "room for the sums of a warp");
@@ -383,7 +446,7 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
 #pragma unroll
         for (int o = 0; o < kSplit; o++) ks.join(total[j], (reinterpret_cast<const uint64_t*>(rows + o) + lane)[(part * 8 + j) * 32]);
       }
-      finish(total, part == 0 ? g.add0 : g.add1, (part == 0 ? g.out0 : g.out1).at(b, (int)at));
+      finish(total, (part == 0 ? g.out0 : g.out1).at(b, (int)at));
     }
   }
 }
@@ -391,7 +454,7 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
 // A CTA has kWarps warps.  grid = (256 kSplit / kWarps, limbs), block = 32 kWarps.
 template <typename W, int kWarps, int kSplit>
 __global__ void __launch_bounds__(32 * kWarps, (sizeof(W) == 8 ? 16 : 20) / kWarps)
-    raised_inner_kernel(const InnerProductArgs<W> g, const typename WordTraits<W>::Pair* __restrict__ tw_all,
+    raised_inner_kernel(const InnerProductArgs<W> g, const TensorOf<W> tensor, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   static_assert(kSplit == 1 || kSplit == kWarps, "warps that share a row are the CTA");
   __shared__ RaisedRow<W> rows[kWarps];
@@ -403,7 +466,7 @@ __global__ void __launch_bounds__(32 * kWarps, (sizeof(W) == 8 ? 16 : 20) / kWar
   const uint32_t pi = g.prime[b];
   const PrimeConst<W> pc = pcs[pi];
   const auto* tw = tw_all + (size_t)pi * kN;
-  CERIUM_DISPATCH_ARITH(W, pc, raised_inner_body, kSplit, (g, b, h, part, pc, mine, tw));
+  CERIUM_DISPATCH_ARITH(W, pc, raised_inner_body, kSplit, (g, tensor, b, h, part, pc, mine, tw));
 }
 
 }  // namespace cerium

@@ -42,4 +42,9 @@ def test_key_switch(be, word_bits, L, K, dnum, offset):
     elt = be.lib.galois_elt_from_step(7, pc.LOGN)
     ks.hrot(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_evk) + offset, elt)
     assert np.array_equal(h.down(o), np.stack(h.orc.hrot(*modes, prm.q_idx, prm.p_idx, dnum, elt, c0, c1, evk)))
+    # a multiplication: the products of the tensor are taken where they are read
+    b0, b1 = (pc.rand_limbs(np.random.default_rng(8 + k), prm.moduli, prm.q_idx) for k in range(2))
+    d_b0, d_b1 = h.up(b0), h.up(b1)
+    ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_b0), h.p(d_b1), h.p(d_evk) + offset, 0)
+    assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, dnum, c0, c1, b0, b1, evk)))
     ks.close()
