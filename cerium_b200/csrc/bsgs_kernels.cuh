@@ -38,9 +38,9 @@ struct PtMacLanes {
 template <typename W>
 __device__ __forceinline__ void ptmac_load(const W* p, W (&v)[PtMacLanes<W>::kWords]) {
   if constexpr (sizeof(W) == 8) {
-    v[0] = __ldg(p);
+    v[0] = *p;
   } else {
-    const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
     v[0] = t.x;
     v[1] = t.y;
   }
@@ -93,17 +93,19 @@ struct PtMacSum<uint64_t, true> {
 };
 
 // out[i][p] = sum_j pt[i][j] * src_p[j] for the GI giant steps of a group.  Streams 2 + GI words per baby step and word
-// position: bound by memory.  The operands of the next baby step are fetched before this one's products, an absent
-// diagonal costs a predicate and no branch (a branch per diagonal kept the loads of a step apart: 423 us for 8 baby
-// and 4 giant steps at 35 limbs, 2.4 TB/s).
+// position: bound by memory.  A thread copies the operands of the next steps into shared memory of its own (cp.async, three
+// steps on their way), which keeps up to 110 KB of an SM in flight; with one step ahead in registers it was 25 KB and
+// XXX us for 8 baby and 4 giant steps at 35 limbs (1.0 GB), now XXX.  An absent diagonal costs a predicate and no branch.
 // grid = (N / (256 * kWords), limbs).
+constexpr int kPtMacStages = 4;
 template <typename W, int GI, bool kPieces>
-__global__ void __launch_bounds__(kEwThreads, 2) pt_mac_kernel(const PtMacArgs<W> a, const PrimeConst<W>* __restrict__ pcs) {
+__global__ void __launch_bounds__(kEwThreads, 3) pt_mac_kernel(const PtMacArgs<W> a, const PrimeConst<W>* __restrict__ pcs) {
   using Sum = PtMacSum<W, kPieces>;
+  constexpr int kWords = PtMacLanes<W>::kWords;
+  __shared__ __align__(16) W ring[kPtMacStages][2 + GI][kEwThreads * kWords];
   grid_dependency_launch();
   grid_dependency_wait();
-  constexpr int kWords = PtMacLanes<W>::kWords;
-  const int b = blockIdx.y;
+  const int b = blockIdx.y, mine = threadIdx.x * kWords;
   const PrimeConst<W> pc = pcs[a.prime[b]];
   const size_t off = (size_t)b * kN + (size_t)(blockIdx.x * kEwThreads + threadIdx.x) * kWords;
   Sum acc[GI][2][kWords];
@@ -114,30 +116,35 @@ __global__ void __launch_bounds__(kEwThreads, 2) pt_mac_kernel(const PtMacArgs<W
       acc[i][0][l].clear();
       acc[i][1][l].clear();
     }
-  W s[2][kWords], p[GI][kWords];
   auto fetch = [&](int j) {
-    ptmac_load<W>(a.src0[j] + off, s[0]);
-    ptmac_load<W>(a.src1[j] + off, s[1]);
+    if (j < a.g) {
+      auto* to = ring[j % kPtMacStages];
+      copy_async<8>(&to[0][mine], a.src0[j] + off);
+      copy_async<8>(&to[1][mine], a.src1[j] + off);
 #pragma unroll
-    for (int i = 0; i < GI; i++) {
-      const W* pp = a.pt[i][j];
-#pragma unroll
-      for (int l = 0; l < kWords; l++) p[i][l] = (W)0;
-      if (pp != nullptr) ptmac_load<W>(pp + off, p[i]);
+      for (int i = 0; i < GI; i++)
+        if (a.pt[i][j] != nullptr) copy_async<8>(&to[2 + i][mine], a.pt[i][j] + off);
     }
+    copy_async_commit();
   };
-  fetch(0);
+#pragma unroll
+  for (int j = 0; j < kPtMacStages - 1; j++) fetch(j);
 #pragma unroll 1
   for (int j = 0; j < a.g; j++) {
+    copy_async_wait<kPtMacStages - 2>();
+    const auto* from = ring[j % kPtMacStages];
     typename Sum::Operand so[2][kWords], po[GI][kWords];
 #pragma unroll
-    for (int l = 0; l < kWords; l++) {
-      so[0][l] = Sum::operand(s[0][l]);
-      so[1][l] = Sum::operand(s[1][l]);
+    for (int k = 0; k < 2 + GI; k++) {
+      W v[kWords];
+      ptmac_load<W>(&from[k][mine], v);
 #pragma unroll
-      for (int i = 0; i < GI; i++) po[i][l] = Sum::operand(p[i][l]);
+      for (int l = 0; l < kWords; l++) {
+        if (k < 2) so[k < 2 ? k : 0][l] = Sum::operand(v[l]);
+        else po[k < 2 ? 0 : k - 2][l] = Sum::operand(a.pt[k < 2 ? 0 : k - 2][j] != nullptr ? v[l] : (W)0);
+      }
     }
-    if (j + 1 < a.g) fetch(j + 1);
+    fetch(j + kPtMacStages - 1);  // into the step before this one
 #pragma unroll
     for (int i = 0; i < GI; i++)
 #pragma unroll

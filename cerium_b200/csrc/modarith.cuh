@@ -9,6 +9,7 @@
 // every value that leaves a kernel is canonical, i.e. in [0, q).
 #pragma once
 #include <cstdint>
+#include <cstring>
 
 #if defined(CERIUM_EMU)
 #include "emu_cuda.h"  // host stand-ins for the CUDA built-ins (kernel-logic tests on CPU)
@@ -39,6 +40,30 @@ __device__ __forceinline__ void grid_dependency_launch() {
 __device__ __forceinline__ void grid_dependency_wait() {
 #if !defined(CERIUM_EMU)
   asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+
+// Asynchronous copies to shared memory; a thread sees its own after copy_async_wait<n>: all but the last n groups it committed.
+template <int kBytes>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+#if defined(CERIUM_EMU)
+  std::memcpy(dst, src, kBytes);
+#else
+  if constexpr (kBytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "n"(kBytes) : "memory");
+#endif
+}
+__device__ __forceinline__ void copy_async_commit() {
+#if !defined(CERIUM_EMU)
+  asm volatile("cp.async.commit_group;" ::: "memory");
+#endif
+}
+template <int kPending>
+__device__ __forceinline__ void copy_async_wait() {
+#if !defined(CERIUM_EMU)
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 #endif
 }
 

@@ -490,17 +490,6 @@ struct alignas(16) RowsBuffer {
   RowTwiddles<W, kStage ? kRows : 1> tw;
 };
 
-template <int kBytes>
-__device__ __forceinline__ void copy_async(void* dst, const void* src) {
-#if defined(CERIUM_EMU)
-  std::memcpy(dst, src, kBytes);
-#else
-  if constexpr (kBytes == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "n"(kBytes) : "memory");
-#endif
-}
 // Starts the copies of this warp's two rows (h0: first row of the CTA); row_twiddles_wait() before they are used.
 template <typename W, int kRows>
 __device__ __forceinline__ void row_twiddles_start(RowTwiddles<W, kRows>& to, const typename WordTraits<W>::Pair* tw,
