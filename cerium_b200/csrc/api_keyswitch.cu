@@ -466,18 +466,38 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
   });
 }
 
-// Column sums of 28-bit pieces hold 16 products of residues below 2^56.
+// Sums that a plaintext multiply-accumulate over these primes takes (PtMacSum).  Column sums of 28-bit pieces hold 16
+// products of residues below 2^56.
 template <typename W>
-bool pt_mac_in_pieces(const cerium_context* ctx, const uint32_t* prime_idx, int count) {
-  bool fits = sizeof(W) == 8;
-  for (int i = 0; i < count; i++) fits = fits && ctx->moduli[prime_idx[i]] >> 56 == 0;
-  return fits;
+int pt_mac_kind(const cerium_context* ctx, const uint32_t* prime_idx, int count) {
+  if (sizeof(W) == 4) return kPtGeneral;
+  bool fp = true, pieces = true;
+  for (int i = 0; i < count; i++) {
+    fp = fp && ctx->fp_ok[prime_idx[i]] != 0;
+    pieces = pieces && ctx->moduli[prime_idx[i]] >> 56 == 0;
+  }
+  return fp ? kPtFp : pieces ? kPtPieces : kPtGeneral;
 }
+// Giant steps of a launch: sums of doubles leave room for eight, the others for four.
+int pt_mac_group(int kind) { return kind == kPtFp ? kBsgsGroup : kBsgsGroup / 2; }
 
-template <typename W, int GI>
-void launch_pt_mac(const PtMacArgs<W>& a, bool pieces, dim3 grid, cudaStream_t stream, const PrimeConst<W>* pcs) {
-  auto kfn = pieces ? pt_mac_kernel<W, GI, sizeof(W) == 8> : pt_mac_kernel<W, GI, false>;
-  CERIUM_LAUNCH(kfn, grid, dim3(kEwThreads), 0, stream, a, pcs);
+template <typename W, int GI, int kKind>
+void launch_pt_mac_of(const PtMacArgs<W>& a, int limbs, cudaStream_t stream, const PrimeConst<W>* pcs) {
+  auto kfn = pt_mac_kernel<W, GI, kKind>;
+  CERIUM_LAUNCH(kfn, dim3(kN / (ptmac_threads(GI) * PtMacLanes<W>::kWords), limbs), dim3(ptmac_threads(GI)), 0, stream, a, pcs);
+}
+template <typename W, int kKind, int GI = 1>
+void launch_pt_mac_kind(const PtMacArgs<W>& a, int count, int limbs, cudaStream_t stream, const PrimeConst<W>* pcs) {
+  if (count <= GI || GI == kBsgsGroup || (kKind != kPtFp && GI == kBsgsGroup / 2)) return launch_pt_mac_of<W, GI, kKind>(a, limbs, stream, pcs);
+  if constexpr (GI < (kKind == kPtFp ? kBsgsGroup : kBsgsGroup / 2)) launch_pt_mac_kind<W, kKind, GI + 1>(a, count, limbs, stream, pcs);
+}
+template <typename W>
+void launch_pt_mac(const PtMacArgs<W>& a, int kind, int count, int limbs, cudaStream_t stream, const PrimeConst<W>* pcs) {
+  if constexpr (sizeof(W) == 8) {
+    if (kind == kPtFp) return launch_pt_mac_kind<W, kPtFp>(a, count, limbs, stream, pcs);
+    if (kind == kPtPieces) return launch_pt_mac_kind<W, kPtPieces>(a, count, limbs, stream, pcs);
+  }
+  launch_pt_mac_kind<W, kPtGeneral>(a, count, limbs, stream, pcs);
 }
 
 // Steps 4-7.  Can be repeated with different keys on the same raised digits (hoisting).
@@ -1167,9 +1187,9 @@ int cerium_plaintext_mac(cerium_context* ctx, int n_out, int n_src, void* const*
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-    const bool pieces = pt_mac_in_pieces<W>(ctx, prime_idx, count);
-    for (int first = 0; first < n_out; first += kBsgsGroup) {
-      const int cnt = std::min(kBsgsGroup, n_out - first);
+    const int kind = pt_mac_kind<W>(ctx, prime_idx, count), group = pt_mac_group(kind);
+    for (int first = 0; first < n_out; first += group) {
+      const int cnt = std::min(group, n_out - first);
       PtMacArgs<W> a{};
       a.g = n_src;
       for (int j = 0; j < n_src; j++) {
@@ -1186,13 +1206,7 @@ int cerium_plaintext_mac(cerium_context* ctx, int n_out, int n_src, void* const*
         }
       }
       for (int b = 0; b < count; b++) a.prime[b] = (uint8_t)prime_idx[b];
-      const dim3 grid(kN / (kEwThreads * PtMacLanes<W>::kWords), count);
-      switch (cnt) {
-        case 1: launch_pt_mac<W, 1>(a, pieces, grid, st, pcs); break;
-        case 2: launch_pt_mac<W, 2>(a, pieces, grid, st, pcs); break;
-        case 3: launch_pt_mac<W, 3>(a, pieces, grid, st, pcs); break;
-        default: launch_pt_mac<W, 4>(a, pieces, grid, st, pcs); break;
-      }
+      launch_pt_mac<W>(a, kind, cnt, count, st, pcs);
     }
     CERIUM_LAUNCH_CHECK("plaintext_mac");
     return CERIUM_OK;
@@ -1252,15 +1266,15 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       if (int rc = cerium_hoisted_rotate(ks, bj, bj + poly, c0, c1, baby_keys_pre[j], baby_elts[j], stream)) return rc;
     }
   }
-  // 2. inner sums s_i = sum_j pt[i][j] * baby_j, kBsgsGroup giant steps per pass over the baby steps
+  // 2. inner sums s_i = sum_j pt[i][j] * baby_j, a group of giant steps per pass over the baby steps
   std::vector<char> have(n_giant, 0);
   int rc = dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     using V = Vec16<W>;
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-    const bool pieces = pt_mac_in_pieces<W>(ctx, ks->q_idx.data(), L);
-    for (int first = 0; first < n_giant; first += kBsgsGroup) {
-      const int cnt = std::min(kBsgsGroup, n_giant - first);
+    const int kind = pt_mac_kind<W>(ctx, ks->q_idx.data(), L), group = pt_mac_group(kind);
+    for (int first = 0; first < n_giant; first += group) {
+      const int cnt = std::min(group, n_giant - first);
       PtMacArgs<W> a{};
       a.g = g;
       for (int j = 0; j < g; j++) {
@@ -1268,25 +1282,19 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
         a.src0[j] = reinterpret_cast<const W*>(j == 0 ? static_cast<const char*>(c0) : b);
         a.src1[j] = reinterpret_cast<const W*>(j == 0 ? static_cast<const char*>(c1) : b + poly);
       }
-      for (int i = 0; i < kBsgsGroup; i++) {
-        const int gi = first + std::min(i, cnt - 1);   // unused slots of the last group repeat its last giant step
+      for (int i = 0; i < cnt; i++) {
+        const int gi = first + i;
         a.out0[i] = reinterpret_cast<W*>(inner + (size_t)gi * 2 * poly);
         a.out1[i] = reinterpret_cast<W*>(inner + (size_t)gi * 2 * poly + poly);
         for (int j = 0; j < g; j++) {
-          const void* p = i < cnt ? plaintexts[(size_t)(first + i) * g + j] : nullptr;
+          const void* p = plaintexts[(size_t)gi * g + j];
           if (p != nullptr && ((uintptr_t)p & 15u)) return fail(CERIUM_ERR_INVALID, "bsgs_apply: pointers must be 16-byte aligned");
           a.pt[i][j] = static_cast<const W*>(p);
-          if (p != nullptr) have[first + i] = 1;
+          if (p != nullptr) have[gi] = 1;
         }
       }
       for (int b = 0; b < L; b++) a.prime[b] = (uint8_t)ks->q_idx[b];
-      const dim3 grid(kN / (kEwThreads * PtMacLanes<W>::kWords), L);
-      switch (cnt) {
-        case 1: launch_pt_mac<W, 1>(a, pieces, grid, st, pcs); break;
-        case 2: launch_pt_mac<W, 2>(a, pieces, grid, st, pcs); break;
-        case 3: launch_pt_mac<W, 3>(a, pieces, grid, st, pcs); break;
-        default: launch_pt_mac<W, 4>(a, pieces, grid, st, pcs); break;
-      }
+      launch_pt_mac<W>(a, kind, cnt, L, st, pcs);
     }
     CERIUM_LAUNCH_CHECK("bsgs plaintext multiply-accumulate");
     // 3. sum0 = sum_i phi_i(s_i.c0) over every giant step, sum1 = sum of s_i.c1 over the un-rotated ones

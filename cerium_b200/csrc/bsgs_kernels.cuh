@@ -5,15 +5,16 @@
 // The reference lowers BsgsMultiplyAccumulate to one MuP and one Add instruction per diagonal and
 // polynomial inside a generated kernel group (cerium/compiler/backend/compiler.cc:2495-2522) and one
 // rotation + Add per giant step (:2562-2590).  Here a thread keeps the sums of up to kBsgsGroup giant
-// steps in two-word accumulators while it walks the baby steps, so the rotated copies of the input
+// steps in registers while it walks the baby steps, so the rotated copies of the input
 // are read once per group and every diagonal exactly once; one reduction per output.
 #pragma once
 #include "ewise_kernels.cuh"
+#include "ntt_kernels.cuh"
 
 namespace cerium {
 
 constexpr int kBsgsMaxBaby = 16;   // baby steps (rotated copies of the input)
-constexpr int kBsgsGroup = 4;      // giant steps whose inner sums one launch produces
+constexpr int kBsgsGroup = 8;      // giant steps whose inner sums one launch may produce
 constexpr int kBsgsMaxGiant = 32;  // giant steps of one multiply-accumulate
 
 template <typename W>
@@ -57,18 +58,42 @@ __device__ __forceinline__ void ptmac_store(W* p, const W (&v)[PtMacLanes<W>::kW
 // Sum of products of two residues for one word.  General: two words with carries.  Pieces (64-bit words, primes
 // below 2^56): the factors as 28-bit pieces, y = y0 + y1 2^28, so that a product is four wide multiply-adds into three
 // column sums and no carry anywhere (16 products: the middle column stays below 2^61): 16 cycles of the integer
-// multiply pipe against ~28 and twice the instructions.
-template <typename W, bool kPieces>
+// multiply pipe against ~28 and twice the instructions.  Fp (every prime of the launch below 2^50): reduced products of
+// doubles (Arith::product, below 7/8 q), eight of them on a reduced sum; one register pair a sum, so a launch serves eight giant
+// steps and the rotated inputs are read once where they were read for every four.
+enum : int { kPtGeneral = 0, kPtPieces = 1, kPtFp = 2 };
+template <typename W, int kKind>
 struct PtMacSum {
+  static constexpr int kTerms = 1 << 30;  // on a reduced sum
   using Operand = W;
+  struct Prime {
+    __device__ __forceinline__ explicit Prime(const PrimeConst<W>&) {}
+  };
   static __device__ __forceinline__ Operand operand(W x) { return x; }
   Acc2<W> acc;
   __device__ __forceinline__ void clear() { acc.clear(); }
-  __device__ __forceinline__ void mad(const Operand& a, const Operand& b) { acc.mad(a, b); }
-  __device__ __forceinline__ W finish(const PrimeConst<W>& pc) const { return barrett2<W>(acc.hi(), acc.lo(), pc); }
+  __device__ __forceinline__ void mad(const Operand& a, const Operand& b, const Prime&) { acc.mad(a, b); }
+  __device__ __forceinline__ void reduce(const Prime&) {}
+  __device__ __forceinline__ W finish(const Prime&, const PrimeConst<W>& pc) const { return barrett2<W>(acc.hi(), acc.lo(), pc); }
 };
 template <>
-struct PtMacSum<uint64_t, true> {
+struct PtMacSum<uint64_t, kPtFp> {
+  static constexpr int kTerms = 8;
+  using Operand = double;
+  using Prime = Arith<uint64_t, kArithFp>;
+  static __device__ __forceinline__ Operand operand(uint64_t x) { return fp_from_u64(x); }
+  double s;
+  __device__ __forceinline__ void clear() { s = 0.0; }
+  __device__ __forceinline__ void mad(double a, double b, const Prime& p) { s = __dadd_rn(s, p.product(a, b)); }
+  __device__ __forceinline__ void reduce(const Prime& p) { s = fp_reduce(s, p.qinv, p.nq); }
+  __device__ __forceinline__ uint64_t finish(const Prime& p, const PrimeConst<uint64_t>&) const {
+    return p.canonical(fp_reduce(s, p.qinv, p.nq));
+  }
+};
+template <>
+struct PtMacSum<uint64_t, kPtPieces> {
+  static constexpr int kTerms = 1 << 30;
+  using Prime = PtMacSum<uint64_t, kPtGeneral>::Prime;
   struct Operand {
     uint32_t lo, hi;
   };
@@ -77,14 +102,15 @@ struct PtMacSum<uint64_t, true> {
   }
   uint64_t c0, c1, c2;
   __device__ __forceinline__ void clear() { c0 = c1 = c2 = 0; }
-  __device__ __forceinline__ void mad(const Operand& a, const Operand& b) {
+  __device__ __forceinline__ void reduce(const Prime&) {}
+  __device__ __forceinline__ void mad(const Operand& a, const Operand& b, const Prime&) {
     c0 += (uint64_t)a.lo * b.lo;
     c1 += (uint64_t)a.lo * b.hi;
     c1 += (uint64_t)a.hi * b.lo;
     c2 += (uint64_t)a.hi * b.hi;
   }
   // c0 + c1 2^28 + c2 2^56
-  __device__ __forceinline__ uint64_t finish(const PrimeConst<uint64_t>& pc) const {
+  __device__ __forceinline__ uint64_t finish(const Prime&, const PrimeConst<uint64_t>& pc) const {
     const uint64_t m = c1 + (c0 >> 28);             // weight 2^28
     const uint64_t h = c2 + (m >> 28);              // weight 2^56
     const uint64_t lo = (c0 & 0xfffffffu) | (m & 0xfffffffu) << 28 | h << 56;
@@ -94,20 +120,22 @@ struct PtMacSum<uint64_t, true> {
 
 // out[i][p] = sum_j pt[i][j] * src_p[j] for the GI giant steps of a group.  Streams 2 + GI words per baby step and word
 // position: bound by memory.  A thread copies the operands of the next steps into shared memory of its own (cp.async, three
-// steps on their way), which keeps up to 110 KB of an SM in flight; with one step ahead in registers it was 25 KB and
-// XXX us for 8 baby and 4 giant steps at 35 limbs (1.0 GB), now XXX.  An absent diagonal costs a predicate and no branch.
-// grid = (N / (256 * kWords), limbs).
+// steps on their way): 60 to 110 KB of an SM in flight.  With one step ahead in registers it was 25 KB and 303 us for 8 baby and
+// 4 giant steps at 35 limbs (1.0 GB), now 228; 8 and 8 (64-bit primes below 2^50: 1.7 GB in one launch) 606 -> 262.  An absent diagonal costs a predicate and no branch.
+// grid = (N / (kThreads * kWords), limbs), block = kThreads = ptmac_threads(GI).
 constexpr int kPtMacStages = 4;
-template <typename W, int GI, bool kPieces>
-__global__ void __launch_bounds__(kEwThreads, 3) pt_mac_kernel(const PtMacArgs<W> a, const PrimeConst<W>* __restrict__ pcs) {
-  using Sum = PtMacSum<W, kPieces>;
-  constexpr int kWords = PtMacLanes<W>::kWords;
-  __shared__ __align__(16) W ring[kPtMacStages][2 + GI][kEwThreads * kWords];
+constexpr int ptmac_threads(int gi) { return gi > 4 ? 128 : 256; }
+template <typename W, int GI, int kKind>
+__global__ void __launch_bounds__(ptmac_threads(GI), GI > 4 ? 4 : 3) pt_mac_kernel(const PtMacArgs<W> a, const PrimeConst<W>* __restrict__ pcs) {
+  using Sum = PtMacSum<W, kKind>;
+  constexpr int kWords = PtMacLanes<W>::kWords, kThreads = ptmac_threads(GI);
+  __shared__ __align__(16) W ring[kPtMacStages][2 + GI][kThreads * kWords];
   grid_dependency_launch();
   grid_dependency_wait();
   const int b = blockIdx.y, mine = threadIdx.x * kWords;
   const PrimeConst<W> pc = pcs[a.prime[b]];
-  const size_t off = (size_t)b * kN + (size_t)(blockIdx.x * kEwThreads + threadIdx.x) * kWords;
+  const typename Sum::Prime prime(pc);
+  const size_t off = (size_t)b * kN + (size_t)(blockIdx.x * kThreads + threadIdx.x) * kWords;
   Sum acc[GI][2][kWords];
 #pragma unroll
   for (int i = 0; i < GI; i++)
@@ -145,21 +173,24 @@ __global__ void __launch_bounds__(kEwThreads, 3) pt_mac_kernel(const PtMacArgs<W
       }
     }
     fetch(j + kPtMacStages - 1);  // into the step before this one
+    const bool full = j != 0 && j % Sum::kTerms == 0;
 #pragma unroll
     for (int i = 0; i < GI; i++)
 #pragma unroll
-      for (int l = 0; l < kWords; l++) {
-        acc[i][0][l].mad(so[0][l], po[i][l]);
-        acc[i][1][l].mad(so[1][l], po[i][l]);
-      }
+      for (int l = 0; l < kWords; l++)
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          if (full) acc[i][p][l].reduce(prime);
+          acc[i][p][l].mad(so[p][l], po[i][l], prime);
+        }
   }
 #pragma unroll
   for (int i = 0; i < GI; i++) {
     W o0[kWords], o1[kWords];
 #pragma unroll
     for (int l = 0; l < kWords; l++) {
-      o0[l] = acc[i][0][l].finish(pc);
-      o1[l] = acc[i][1][l].finish(pc);
+      o0[l] = acc[i][0][l].finish(prime, pc);
+      o1[l] = acc[i][1][l].finish(prime, pc);
     }
     ptmac_store<W>(a.out0[i] + off, o0);
     ptmac_store<W>(a.out1[i] + off, o1);

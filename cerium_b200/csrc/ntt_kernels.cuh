@@ -182,6 +182,14 @@ struct Arith<uint64_t, kArithFp> {
   static __device__ __forceinline__ W u(double x) { return (W)__double_as_longlong(x); }
   __device__ __forceinline__ W enter(W x) const { return u(fp_from_u64(x)); }
   __device__ __forceinline__ W reduce(W x) const { return u(fp_reduce(d(x), qinv, nq)); }
+  // y k - c q with the quotient from the rounded product: |y| <= q, 0 <= k < q < 2^50 put RN(RN(y k) RN(1/q)) off by
+  // 3/2^53 * 2^50 = 3/8 at most before it is rounded, so the result is below 7/8 q (exact as in fp_mulmod)
+  __device__ __forceinline__ double product(double y, double k) const {
+    const double h = __dmul_rn(y, k);
+    const double l = __fma_rn(y, k, -h);
+    const double c = __dadd_rn(__fma_rn(h, qinv, kFpMagic), -kFpMagic);
+    return __dadd_rn(__fma_rn(c, nq, h), l);
+  }
   // quotient of a twiddle by q when the table holds the twiddle alone
   __device__ __forceinline__ W quotient(W w) const { return u(__dmul_rn(d(w), qinv)); }
   __device__ __forceinline__ void fwd(W& a, W& b, W w, W wq) const {

@@ -84,9 +84,7 @@ static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values mu
 //   hi(t * floor(2^(b + 62) / q)) is short by less than 1/2 + 1 + 1 + 2 (t, the factor, the product, mulhi_approx64), so the
 //   remainder is below 4.5 q, and a sum below 5q + 2^32 stays there when 5q leaves it where its high word says so (csub_high).
 //   Sums of two words take 64 registers and leave none for the key words that are on their way.
-//   Fp: every product comes back as y k - c q, c the rounded quotient.  With |y| <= q, 0 <= k < q < 2^50 the quotient
-//   RN(RN(y k) RN(1/q)) is off by 3/2^53 * 2^50 = 3/8 at most before it is rounded, so a product is below 7/8 q, and eight of
-//   them on a reduced sum stay below 8 q: exact (RN(y k) - c q is an integer below 2^53, as in fp_mulmod).
+//   Fp: every product is below 7/8 q (Arith::product), eight of them on a reduced sum stay below 8 q: exact.
 template <typename W, int kMode>
 struct KeySum {
   static constexpr int kTerms = 1 << 30;  // on a reduced sum
@@ -128,11 +126,7 @@ struct KeySum<uint64_t, kArithFp> {
   const A& ar;
   __device__ __forceinline__ KeySum(const A& a, const PrimeConst<uint64_t>&) : ar(a) {}
   __device__ __forceinline__ void add(uint64_t& s, uint64_t y, uint64_t k) const {
-    const double yd = A::d(y), kd = fp_from_u64(k);
-    const double h = __dmul_rn(yd, kd);
-    const double l = __fma_rn(yd, kd, -h);
-    const double c = __dadd_rn(__fma_rn(h, ar.qinv, kFpMagic), -kFpMagic);
-    s = A::u(__dadd_rn(A::d(s), __dadd_rn(__fma_rn(c, ar.nq, h), l)));
+    s = A::u(__dadd_rn(A::d(s), ar.product(A::d(y), fp_from_u64(k))));
   }
   __device__ __forceinline__ void reduce(uint64_t& s) const { s = ar.reduce(s); }
   __device__ __forceinline__ void join(uint64_t& s, uint64_t t) const { s = A::u(__dadd_rn(A::d(s), A::d(t))); }
