@@ -257,7 +257,9 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
         epi.factor[b] = (W)f;
         epi.factor_shoup[b] = (W)host::shoup(f, q, bits);
       }
-      if (c.reduce_src) {
+      if (c.cols_done) {
+        // the rows only
+      } else if (c.reduce_src) {
         ReduceLoader<W> ld{};
         ld.src_q = (W)c.src_q;
         ld.pre_add = (W)c.pre_add;

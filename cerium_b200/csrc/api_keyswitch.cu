@@ -239,6 +239,32 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
   });
 }
 
+// The raised digits, the polynomial that was raised, a key, and the plan's accumulators.
+template <typename W>
+InnerProductArgs<W> inner_args(const cerium_keyswitch* ks, const void* cpoly, const void* evk) {
+  const size_t n = kN;
+  const int LK = ks->LK;
+  W* acc = ws_at<W>(ks, ks->o_acc);
+  InnerProductArgs<W> g{};
+  g.raised = ws_at<W>(ks, ks->o_raised);
+  g.raised_digit_stride = (size_t)LK * n;
+  g.raised_limb_stride = n;
+  g.own = static_cast<const W*>(cpoly);
+  g.own_stride = n;
+  g.evk = static_cast<const W*>(evk);
+  g.evk_digit_stride = (size_t)2 * LK * n;
+  g.evk_poly_stride = (size_t)LK * n;
+  g.evk_limb_stride = n;
+  g.out0 = {acc, n};
+  g.out1 = {acc + (size_t)LK * n, n};
+  g.dnum = ks->dnum;
+  for (int b = 0; b < LK; b++) {
+    g.prime[b] = (uint8_t)ks->all_idx[b];
+    g.own_digit[b] = (int8_t)ks->own_digit[b];
+  }
+  return g;
+}
+
 // Of a multiplication (a0, a1) (b0, b1) whose a1 is the polynomial that the steps are given.
 struct TensorInputs {
   const void *a0, *b0, *b1;
@@ -260,32 +286,15 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
   return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     using V = Vec16<W>;
-    W* acc = ws_at<W>(ks, ks->o_acc);
-    InnerProductArgs<W> g{};
-    g.raised = ws_at<W>(ks, ks->o_raised);
-    g.raised_digit_stride = (size_t)LK * n;
-    g.raised_limb_stride = n;
-    g.own = static_cast<const W*>(cpoly);
-    g.own_stride = n;
+    InnerProductArgs<W> g = inner_args<W>(ks, cpoly, evk);
     g.own_elt = pre_elt;
     g.accumulate = accumulate ? 1 : 0;
-    g.evk = static_cast<const W*>(evk);
-    g.evk_digit_stride = (size_t)2 * LK * n;
-    g.evk_poly_stride = (size_t)LK * n;
-    g.evk_limb_stride = n;
-    g.out0 = {acc, n};
-    g.out1 = {acc + (size_t)LK * n, n};
-    g.dnum = dnum;
     if (add0 != nullptr || add1 != nullptr || tensor != nullptr) {
       g.add0 = static_cast<const W*>(add0);
       g.add1 = static_cast<const W*>(add1);
       g.add_stride = n;
       g.add_limbs = ks->L;
       for (int b = 0; b < ks->L; b++) g.add_factor[b] = (W)ks->pmod[b];
-    }
-    for (int b = 0; b < LK; b++) {
-      g.prime[b] = (uint8_t)ks->all_idx[b];
-      g.own_digit[b] = (int8_t)ks->own_digit[b];
     }
     const PrimeConst<W>* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
     // every local extended limb (Q and extension) in one launch
@@ -547,6 +556,96 @@ int keyswitch_impl(cerium_keyswitch* ks, void* out0, void* out1, const void* cpo
   return keyswitch_inner_moddown(ks, out0, out1, cpoly, evk, add0, add1, stream, pre_elt, 0, nullptr, r, fused);
 }
 
+// Whether two hoisted rotations may run together: the second one's accumulators and converted limbs lie where a rotation with
+// an output on an input, a multiplication and a rescale keep theirs (3L + 2L + 2 limbs).
+bool rotates_in_pairs(const cerium_keyswitch* ks) { return 2 * ks->LK + 2 * ks->L <= 5 * ks->L + 2; }
+
+// Two hoisted rotations of one ciphertext, each as cerium_hoisted_rotate has it: one pass over the raised digits, and a
+// ModDown whose small launches serve both (10 extension limbs take as long to transform back as 20).  The outputs are
+// aligned to 16 bytes and lie on none of the inputs.
+// Linear transforms one rotation at a time -> in pairs: 8 x 8 diagonals at 35 limbs 3270 -> 3210 us, 7 x 6 at 25 limbs
+// 1754 -> 1611, 5 x 3 at 20 limbs 820 -> 744, 8 x 4 at 12 limbs 854 -> 801.
+int hoisted_rotate_pair(cerium_keyswitch* ks, void* const (&out)[2][2], const void* c0, const void* c1, const void* const (&evk)[2],
+                        const uint32_t (&store_elt)[2], cudaStream_t stream) {
+  cerium_context* ctx = ks->ctx;
+  const size_t n = kN;
+  const int L = ks->L, K = ks->K, LK = ks->LK;
+  return dispatch_word(ctx->word_bits, [&](auto tag) -> int {
+    using W = decltype(tag);
+    using V = Vec16<W>;
+    W* acc[2] = {ws_at<W>(ks, ks->o_acc), ws_at<W>(ks, ks->o_tmp)};
+    W* conv[2] = {ws_at<W>(ks, ks->o_conv), acc[1] + (size_t)2 * LK * n};
+    const InnerProductArgs<W> g = inner_args<W>(ks, c1, evk[0]);
+    const InnerSecond<W> second{static_cast<const W*>(evk[1]), {acc[1], n}, {acc[1] + (size_t)LK * n, n}};
+    { auto kfn = inner_product_pair_kernel<W>; CERIUM_LAUNCH(kfn, dim3(kN / (kEwThreads * V::kLanes), LK), dim3(kEwThreads), 0, stream, g, second, static_cast<const PrimeConst<W>*>(ctx->d_pcs)); }
+    CERIUM_LAUNCH_CHECK("inner_product_pair");
+    // slots of the second rotation's limbs as the launches of both count them, from the first one's
+    const uint32_t acc_gap = (uint32_t)((ks->o_tmp - ks->o_acc) / n), conv_gap = (uint32_t)((conv[1] - conv[0]) / (ptrdiff_t)n);
+    {
+      std::vector<uint32_t> pos(ks->ext_pos), prime(ks->ext_prime);
+      for (int i = 0; i < 2 * K; i++) {
+        pos.push_back(ks->ext_pos[i] + acc_gap);
+        prime.push_back(ks->ext_prime[i]);
+      }
+      NttCall c{acc[0], acc[0], n, n, pos.data(), prime.data(), 4 * K};
+      if (int rc = launch_ntt_inverse(ctx, c, stream, ks->d_last_p, ks->d_add_p)) return rc;
+    }
+    {
+      BconvCall calls[4];
+      for (int i = 0; i < 4; i++) {
+        const size_t p = i & 1;
+        calls[i] = BconvCall{ks->down, conv[i >> 1] + p * L * n, n, acc[i >> 1] + (p * LK + L) * n, n};
+      }
+      if (int rc = launch_bconv(ctx, calls, 4, stream)) return rc;
+    }
+    std::vector<uint32_t> pos, prime;
+    for (int i = 0; i < 4 * L; i++) {
+      pos.push_back(i < 2 * L ? (uint32_t)i : (uint32_t)(i - 2 * L) + conv_gap);
+      prime.push_back(ks->q_idx[i % L]);
+    }
+    {
+      NttCall c{conv[0], conv[0], n, n, pos.data(), prime.data(), 4 * L};
+      c.lazy_in = true;
+      c.cols_only = true;
+      if (int rc = launch_ntt_forward(ctx, c, stream)) return rc;
+    }
+    std::vector<uint64_t> factor2(ks->pinv);
+    factor2.insert(factor2.end(), ks->pinv.begin(), ks->pinv.end());
+    const bool both = 2 * L <= kSudMaxBatch;
+    for (int i = 0; i < (both ? 2 : 4); i++) {
+      const int r = both ? i : i >> 1, p = both ? 0 : i & 1;
+      SudCall s{};
+      s.src = s.work = conv[r] + (size_t)p * L * n;
+      s.src_stride = s.work_stride = n;
+      s.cols_done = true;
+      s.dst = out[r][p];
+      s.dst_stride = n;
+      s.minuend = acc[r] + (size_t)p * LK * n;
+      s.minuend_stride = n;
+      s.addend = p == 0 ? c0 : nullptr;
+      s.addend_stride = n;
+      s.prime = prime.data();
+      s.factor = factor2.data();
+      s.count = both ? 2 * L : L;
+      if (both) {
+        s.split = L;
+        s.dst2 = out[r][1];
+        s.minuend2 = acc[r] + (size_t)LK * n;
+      }
+      s.store_galois = store_elt[r];
+      if (int rc = launch_sud(ctx, s, stream)) return rc;
+    }
+    return CERIUM_OK;
+  });
+}
+
+// Inverse of an odd element modulo 2N: Newton steps double the valid bits.
+uint32_t inverse_elt(uint32_t elt) {
+  uint32_t inv = elt;
+  for (int k = 0; k < 5; k++) inv *= 2u - elt * inv;
+  return inv & (2u * (uint32_t)kN - 1u);
+}
+
 }  // namespace
 
 extern "C" {
@@ -791,11 +890,11 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
     std::vector<uint64_t> all;
     if (exact) {
       for (int i = 0; i < L; i++) append_last(all, ks->q_idx[i], scale_q[i]);
-      for (int i = 0; i < 2 * Kl; i++) append_last(all, ks->p_idx[i % Kl], scale_p[i]);
+      for (int i = 0; i < 4 * Kl; i++) append_last(all, ks->p_idx[i % Kl], scale_p[i % Kl]);  // two rotations' accumulators
     }
     const size_t o_add = all.size() * wb;
     if (round_mode == CERIUM_ROUND_HALF)
-      for (int i = 0; i < 2 * Kl; i++) all.push_back(add_p[i % Kl]);
+      for (int i = 0; i < 4 * Kl; i++) all.push_back(add_p[i % Kl]);
     if (!all.empty()) {
       if (!upload(all, &ks->d_consts)) {
         cerium_keyswitch_destroy(ks);
@@ -1110,11 +1209,7 @@ int cerium_hoisted_rotate(cerium_keyswitch* ks, void* out0, void* out1, const vo
     const bool apart = !overlaps(out0, c0) && !overlaps(out1, c0) && !overlaps(out0, c1) && !overlaps(out1, c1);
     if (!apart && !aligned) return fail(CERIUM_ERR_INVALID, "hoisted_rotate: pointers must be 16-byte aligned");
     if (apart && aligned) {
-      // inverse of the element modulo 2N (odd, so it exists): Newton steps double the valid bits
-      uint32_t inv = galois_elt;
-      for (int k = 0; k < 5; k++) inv *= 2u - galois_elt * inv;
-      inv &= 2u * (uint32_t)kN - 1u;
-      return keyswitch_inner_moddown(ks, out0, out1, c1, evk_pre, c0, nullptr, (cudaStream_t)stream, 0, inv);
+      return keyswitch_inner_moddown(ks, out0, out1, c1, evk_pre, c0, nullptr, (cudaStream_t)stream, 0, inverse_elt(galois_elt));
     }
   }
   if (int rc = keyswitch_inner_moddown(ks, t0, t1, c1, evk_pre, c0, nullptr, (cudaStream_t)stream)) return rc;
@@ -1260,9 +1355,25 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
   // 1. baby steps: g - 1 hoisted rotations of the input (one ModUp)
   if (g > 1) {
     if (int rc = cerium_hoisted_begin(ks, c1, stream)) return rc;
+    // in pairs, unless the work buffer lies on the input
+    auto clear_of = [&](const void* in) {
+      const uintptr_t x = (uintptr_t)baby, y = (uintptr_t)in;
+      return x + (size_t)(g - 1) * 2 * poly <= y || y + poly <= x;
+    };
+    const bool pairs = rotates_in_pairs(ks) && clear_of(c0) && clear_of(c1);
     for (int j = 1; j < g; j++) {
       if (!baby_keys_pre[j]) return fail(CERIUM_ERR_INVALID, "bsgs_apply: a baby step has no key");
       char* bj = baby + (size_t)(j - 1) * 2 * poly;
+      if (pairs && j + 1 < g && baby_keys_pre[j + 1] != nullptr) {
+        for (int k = 0; k < 2; k++)
+          if (!(baby_elts[j + k] & 1) || baby_elts[j + k] >= 2u * kN) return fail(CERIUM_ERR_INVALID, "hoisted_rotate: Galois element is not valid");
+        void* const out[2][2] = {{bj, bj + poly}, {bj + 2 * poly, bj + 3 * poly}};
+        const void* const evk[2] = {baby_keys_pre[j], baby_keys_pre[j + 1]};
+        const uint32_t elt[2] = {inverse_elt(baby_elts[j]), inverse_elt(baby_elts[j + 1])};
+        if (int rc = hoisted_rotate_pair(ks, out, c0, c1, evk, elt, st)) return rc;
+        j++;
+        continue;
+      }
       if (int rc = cerium_hoisted_rotate(ks, bj, bj + poly, c0, c1, baby_keys_pre[j], baby_elts[j], stream)) return rc;
     }
   }

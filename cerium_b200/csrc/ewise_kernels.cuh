@@ -315,6 +315,56 @@ struct InnerProductArgs {
   int8_t own_digit[kEwMaxLimbs];  // digit that limb b belongs to (-1 for extension limbs)
 };
 
+// The inner products of two hoisted rotations with their keys in one pass over the raised digits (no rotation of the input, no
+// sums to add to, no additions).  80 registers, three CTAs: 128 MB of 2 x 482 are not read for 7 digits on 40 limbs.
+template <typename W>
+struct InnerSecond {
+  const W* evk;
+  Limbs<W> out0, out1;
+};
+
+template <typename W>
+__global__ void __launch_bounds__(kEwThreads, 3)
+    inner_product_pair_kernel(const InnerProductArgs<W> g, const InnerSecond<W> second, const PrimeConst<W>* __restrict__ pcs) {
+  grid_dependency_launch();
+  grid_dependency_wait();
+  using V = Vec16<W>;
+  const int b = blockIdx.y;
+  const PrimeConst<W> pc = pcs[g.prime[b]];
+  const int idx = (blockIdx.x * kEwThreads + threadIdx.x) * V::kLanes;
+  Acc2<W> acc[2][2][V::kLanes];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+#pragma unroll
+    for (int l = 0; l < V::kLanes; l++) acc[k >> 1][k & 1][l].clear();
+  const int own_digit = g.own_digit[b];
+#pragma unroll 1
+  for (int d = 0; d < g.dnum; d++) {
+    const W* ap = d == own_digit ? g.own + (size_t)b * g.own_stride + idx
+                                 : g.raised + (size_t)d * g.raised_digit_stride + (size_t)b * g.raised_limb_stride + idx;
+    const size_t at = (size_t)d * g.evk_digit_stride + (size_t)b * g.evk_limb_stride + idx;
+    const V a = V::load_once(ap);
+    V key[2][2];
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      key[0][p] = V::load_once(g.evk + at + p * g.evk_poly_stride);
+      key[1][p] = V::load_once(second.evk + at + p * g.evk_poly_stride);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int l = 0; l < V::kLanes; l++) acc[k >> 1][k & 1][l].mad(a.v[l], key[k >> 1][k & 1].v[l]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    V o;
+#pragma unroll
+    for (int l = 0; l < V::kLanes; l++) o.v[l] = barrett2<W>(acc[k >> 1][k & 1][l].hi(), acc[k >> 1][k & 1][l].lo(), pc);
+    const Limbs<W>& to = k == 0 ? g.out0 : k == 1 ? g.out1 : k == 2 ? second.out0 : second.out1;
+    o.store(to.at(b, idx));
+  }
+}
+
 template <typename W>
 __global__ void __launch_bounds__(kEwThreads, sizeof(W) == 8 ? 4 : 5)
     inner_product_kernel(const InnerProductArgs<W> g, const PrimeConst<W>* __restrict__ pcs) {

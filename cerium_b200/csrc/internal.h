@@ -304,6 +304,7 @@ struct SudCall {
   const void* minuend2 = nullptr;
   const void* addend2 = nullptr;
   bool lazy_src = false;  // the source words are below 4q instead of canonical
+  bool cols_done = false;  // `work` holds the column pass's results already
   // source re-reduction (only when reduce_src): residues of modulus src_q, optional rounding
   bool reduce_src = false;
   uint64_t src_q = 0;
