@@ -252,8 +252,11 @@ class HRotWorkload(Workload):
             self.streams = [torch.cuda.Stream() for _ in range(inflight)]
             self.outs = [torch.empty_like(self.cts[0]) for _ in range(max(self.n_cts, inflight))]
             k_loc = self.sks[0].k_local
-            # iNTT pair, [gather], BConv, NTT pair, inner product, iNTT pair, [gather], BConv, SuD pair
-            self.gpu_launches_per_step = 2 + 1 + 2 + 1 + (2 if k_loc else 0) + 1 + 2
+            # iNTT pair, [gather], BConv, NTT columns, rows with the inner product (one kernel where the rank's limbs
+            # have 1.8 rows for each of the 16 warps of an SM), iNTT pair, [gather], BConv, SuD pair
+            rows = 256 * (self.sks[0].n_local + k_loc)
+            one = rows >= 1.8 * 16 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+            self.gpu_launches_per_step = 2 + 1 + 1 + (1 if one else 2) + (2 if k_loc else 0) + 1 + 2
         else:
             gen = torch.Generator(device="cuda").manual_seed(0xCE210003 + rank)
             # exact conversion + rounding: the semantics that are low-noise with 50/60-bit primes.
@@ -268,9 +271,9 @@ class HRotWorkload(Workload):
             self.n_cts = self.inflight * -(-self.n_cts // self.inflight)   # a buffer is only ever used by one stream
             self.cts = [_rand_limbs_gpu(torch, prm.moduli, prm.q_idx, (2,), gen) for _ in range(self.n_cts)]
             self.outs = [torch.empty_like(self.cts[0]) for _ in range(self.n_cts)]
-            # iNTT pair, BConv, NTT pair, inner product, iNTT pair, BConv, SuD pair (the rotation itself is
-            # folded into the reads of the iNTT, the inner product and the SuD tail: no launch of its own)
-            self.gpu_launches_per_step = 2 + 1 + 2 + 1 + 2 + 1 + 2
+            # iNTT pair, BConv, NTT columns, rows with the inner product, iNTT pair, BConv, SuD pair (the rotation itself
+            # is folded into the reads of the iNTT, the inner product and the SuD tail: no launch of its own)
+            self.gpu_launches_per_step = 2 + 1 + 1 + 1 + 2 + 1 + 2
         self.elt = hrot_galois_elt()
         self.i = 0
         self.ct_bytes = self.cts[0].numel() * 8
@@ -452,9 +455,9 @@ class HMultWorkload(Workload):
         self.host_in[0].copy_(self.a.cpu())
         self.host_in[1].copy_(self.b.cpu())
         self.host_out = torch.empty(self.out.shape, dtype=torch.int64).pin_memory()
-        # tensor; key switch: iNTT pair, NTT pair x2 (576 limbs in two batches), inner product, iNTT pair,
+        # tensor; key switch: iNTT pair, NTT columns x2 (576 limbs in two batches), rows with the inner product, iNTT pair,
         # BConv, SuD pair; then the rescale of both polynomials (iNTT pair, SuD pair) unless it is folded into the ModDown
-        self.gpu_launches_per_step = 1 + (2 + 4 + 1 + 2 + 1 + 2) + (0 if self.rescale_mode == 2 else 4)
+        self.gpu_launches_per_step = 1 + (2 + 2 + 1 + 2 + 1 + 2) + (0 if self.rescale_mode == 2 else 4)
 
     def step(self):
         s = self.torch.cuda.current_stream().cuda_stream
@@ -671,9 +674,9 @@ class BsgsWorkload(HRotWorkload):
         limb = N * 8
         # ciphertext in and out, 14 keys, 64 plaintexts
         self.alg_bytes = (4 * prm.L + 2 * (G - 1) * prm.dnum * 2 * (prm.L + prm.K) + G * G * prm.L) * limb
-        # hoisted begin 5, baby rotation 6 each, 2 plaintext passes, 2 rotation sums, per giant step
-        # iNTT pair + BConv + NTT pair + inner product, final ModDown 5
-        self.gpu_launches_per_step = 5 + (G - 1) * 6 + 2 + 2 + (G - 1) * 6 + 5
+        # hoisted begin 5, baby rotations 7 a pair and 6 for one alone, a plaintext pass, 2 rotation sums, per giant step
+        # iNTT pair + BConv + NTT columns + rows with the inner product, final ModDown 5
+        self.gpu_launches_per_step = 5 + (G - 1) // 2 * 7 + (G - 1) % 2 * 6 + 1 + 2 + (G - 1) * 5 + 5
 
     def _run(self, ct, out, stream):
         self.op.run(out, ct, self.pts, self.baby_keys, self.giant_keys, self.baby_elts, self.giant_elts, stream)
@@ -763,10 +766,10 @@ class BootstrapWorkload(Workload):
         torch.cuda.synchronize()
         n = self.ev.count.n
         self.op_counts = dict(n)
-        # launches: ModRaise 21; a BSGS stage 5 + 7 * 6 + 2 + 2 + 8 * 6 + 5; an HMult 12; a conjugation 11;
+        # launches: ModRaise 20; a BSGS stage 5 + 3 * 7 + 6 + 1 + 2 + 8 * 5 + 5; an HMult 10; a conjugation 10;
         # a rescale 4; every other pass 1, and ModUps that convert their digits in two launches
-        self.gpu_launches_per_step = (21 * n["mod_raise"] + 104 * n["bsgs"] + 12 * n["hmult"] + 11 + 4 * n["rescale"]
-                                      + n["ewise"] + 2 * n["pt_mac"] + n["split_mod_up"])
+        self.gpu_launches_per_step = (20 * n["mod_raise"] + 80 * n["bsgs"] + 10 * n["hmult"] + 10 + 4 * n["rescale"]
+                                      + n["ewise"] + n["pt_mac"] + n["split_mod_up"])
         self.ev.count.n = {}
         self.alg_bytes = 0
 
