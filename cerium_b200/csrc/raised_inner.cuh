@@ -11,6 +11,8 @@
 // it would be 8.  The next digit's row is on its way (cp.async) while one is worked on, and the key rows are asked for before
 // the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against 301).
 // Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 117.3 us against 122.4).
+// Key words are the first to leave L2 by an explicit priority (with .cs alone rotation of 35 limbs 296.0 us, now 293.4; 24 limbs with
+// one-limb digits 431 -> 428).
 // Measured, row pass + inner product -> this kernel: rotation of 35 limbs 340.6 -> 301.3 us, multiplication of 24 limbs with
 // one-limb digits 540 -> 452, rotation of 51 32-bit limbs 197.2 -> 182.9.  When it is used: rows_with_inner
 // (api_keyswitch.cu).
@@ -51,7 +53,7 @@ __device__ __forceinline__ Quad<uint64_t> quad_load(const uint64_t* p) {
 }
 __device__ __forceinline__ Quad<uint64_t> quad_load_once(const uint64_t* p) {
   Quad<uint64_t> q;
-  asm volatile("ld.global.cs.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
   return q;
 }
 __device__ __forceinline__ void quad_store(uint64_t* p, const Quad<uint64_t>& q) {
