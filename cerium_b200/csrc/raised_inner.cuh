@@ -264,6 +264,15 @@ struct TensorOf {
   const W* b1;
 };
 
+// Gives up the 128 bytes at p, a whole line of a buffer that is written before it is read again.
+__device__ __forceinline__ void discard_line(const void* p) {
+#if !defined(CERIUM_EMU)
+  asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
+#else
+  (void)p;
+#endif
+}
+
 // kSplit warps share a row: warp `part` takes every kSplit-th digit, and finishes polynomial `part` from the sums of all of
 // them (kSplit = 1: both).
 template <typename W, int kMode, int kSplit>
@@ -386,6 +395,9 @@ __device__ __forceinline__ void raised_inner_body(const InnerProductArgs<W>& g, 
     W y[8];
     row_twiddles_wait();             // this digit is here, and the first time the twiddles
     fetch(e + kSplit, (n & 1) ^ 1);  // its buffer was the previous digit's
+    // The row was read for the last time: its lines, which the column pass left dirty in L2, need not go to memory (50 MB of a
+    // rotation of 35 limbs: 294.4 -> 289.0 us; 51 32-bit limbs 186.7 -> 182.0, 24 limbs with one-limb digits 428.3 / 429.5).
+    if (lane < 2 * (int)sizeof(W)) discard_line(rp + (size_t)digit(e) * g.raised_digit_stride + lane * (128 / (int)sizeof(W)));
     W* ex = row.buf[n & 1];
 #pragma unroll
     for (int j = 0; j < 8; j++) y[j] = ex[j * 32 + lane];
