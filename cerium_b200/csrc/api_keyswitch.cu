@@ -63,6 +63,7 @@ struct cerium_keyswitch {
   // lifted plan (ModRaise): one digit whose value arrives as an exact integer and is reduced modulo
   // every prime of the plan by the caller of keyswitch_inner_moddown; no converters, no own limbs
   bool lifted = false;
+  bool key_sums = true;  // KeySum takes every local prime
   std::vector<uint32_t> ext_pos, ext_prime;  // extension limbs of both accumulators
   // exact mode: per-limb scalars folded into the inverse transforms (device, one word per entry)
   void* d_consts = nullptr;  // what the next three point into
@@ -171,15 +172,15 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
 // with as many digits 467 -> 452 us, 15 limbs 257.5 -> 256.5); 7 digits on 40 limbs lose (301 -> 320 us).  32-bit words are never split:
 // rotations of 3 to 51 limbs lose 5 to 10 %.
 constexpr int kSplitDigits = 12;
-// Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where it can read the key
-// and the polynomials four words at a time, and 64-bit words have the rows that keep the resident warps (16 to an SM) busy.
+// Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where its sums take the plan's
+// primes, it can read the key and the polynomials four words at a time, and 64-bit words have the rows that keep the resident warps (16 to an SM) busy.
 // With fewer the serial walk over the digits shows: rotation of 10 limbs (15 with the extension) 102.9 us in two kernels and
 // 110.6 in one, 11 limbs 113.6 / 115.4, 12 limbs 118.0 / 117.3, 13 limbs 138.2 / 129.2; digits of one limb, 10 limbs
 // 180.1 / 183.6, 12 limbs 220.9 / 216.0.  32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 197.4 / 182.8).
 // Hoisted rotations transform the digits once for many keys and keep the two kernels.
 bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* evk, const void* add0, const void* add1) {
   const uintptr_t ptrs = (uintptr_t)cpoly | (uintptr_t)evk | (uintptr_t)add0 | (uintptr_t)add1;
-  if (ptrs % (4 * ks->ctx->word_bytes()) != 0) return false;
+  if (!ks->key_sums || ptrs % (4 * ks->ctx->word_bytes()) != 0) return false;
   if (ks->ctx->word_bits == 32) return true;
   const double rows_per_warp = 256.0 * ks->LK / (16.0 * ks->ctx->sm_count);
   return rows_per_warp >= (ks->dnum >= kSplitDigits ? 1.4 : 1.8);
@@ -707,6 +708,8 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
   ks->all_idx = ks->q_idx;
   ks->all_idx.insert(ks->all_idx.end(), ks->p_idx.begin(), ks->p_idx.end());
   const int LK = ks->LK;
+  for (uint32_t p : ks->all_idx)
+    if (ctx->word_bits == 64 && !ctx->fp_ok[p] && ctx->moduli[p] >> (kKeySumBits - 1) == 0) ks->key_sums = false;
   const int Kl = ks->K;  // local extension limbs
   ks->lifted = lifted;
   for (int e = 0; e < LK; e++) ks->own_digit.push_back((e < L && !lifted) ? ks->loc[e] % dnum : -1);

@@ -82,11 +82,14 @@ static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values mu
 // Sums of products of residues (integers: below 4q) with key words; 64 bits, so that partial sums of a row can be put
 // together.
 //   32-bit words: the products themselves, one reduction at the end.
-//   64-bit integers: every product x = y k < 4 q^2 is reduced: t = x / 2^(b - 2), q of b bits (52 to 60), is below 2^64, the quotient
-//   hi(t * floor(2^(b + 62) / q)) is short by less than 1/2 + 1 + 1 + 2 (t, the factor, the product, mulhi_approx64), so the
+//   64-bit integers: every product x = y k < 4 q^2 is reduced: t = x / 2^(b - 2), q of b bits (kKeySumBits to 60), is below 2^64, the
+//   quotient hi(t * floor(2^(b + 62) / q)) is short by less than 1/2 + 1 + 1 + 2 (t, the factor, the product, mulhi_approx64), so the
 //   remainder is below 4.5 q, and a sum below 5q + 2^32 stays there when 5q leaves it where its high word says so (csub_high).
+//   These are the primes from 2^50 on, and with integer butterflies everywhere smaller ones too: a plan with one that is too
+//   small for the shift, which passes over a whole word, keeps the two kernels (rows_with_inner).
 //   Sums of two words take 64 registers and leave none for the key words that are on their way.
 //   Fp: every product is below 7/8 q (Arith::product), eight of them on a reduced sum stay below 8 q: exact.
+constexpr int kKeySumBits = 34;
 template <typename W, int kMode>
 struct KeySum {
   static constexpr int kTerms = 1 << 30;  // on a reduced sum

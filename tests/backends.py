@@ -25,14 +25,16 @@ class EmuBackend:
         self._keep = []
 
     def to_dev(self, a: np.ndarray):
-        b = np.ascontiguousarray(a).copy()
-        assert b.ctypes.data % 16 == 0
+        b = self.empty(a.shape, a.dtype)
+        b[...] = a
         return b
 
     def empty(self, shape, dtype):
-        b = np.zeros(shape, dtype=dtype)
-        assert b.ctypes.data % 16 == 0
-        return b
+        # as aligned as an allocation on the device: numpy's own lie 16 bytes past a page
+        count = int(np.prod(shape))
+        raw = np.zeros(count * np.dtype(dtype).itemsize + 256, dtype=np.uint8)
+        at = -raw.ctypes.data % 256
+        return raw[at:at + count * np.dtype(dtype).itemsize].view(dtype).reshape(shape)
 
     def ptr(self, buf) -> int:
         return buf.ctypes.data

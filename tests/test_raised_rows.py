@@ -48,3 +48,24 @@ def test_key_switch(be, word_bits, L, K, dnum, offset):
     ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_b0), h.p(d_b1), h.p(d_evk) + offset, 0)
     assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, dnum, c0, c1, b0, b1, evk)))
     ks.close()
+
+
+@pytest.mark.parametrize("bits", [28, 32, 33, 34, 50])
+def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
+    """With integer butterflies asked for, 64-bit words of any prime; the sums of products want 34 bits."""
+    monkeypatch.setenv("CERIUM_B200_NTT_ARITH", "int")
+    L, K = (6, 3) if be.name == "emu" else (20, 7)   # rows for every warp of the device
+    mods = params.ntt_primes_below(bits, L + K, pc.LOGN)
+    prm = params.CkksParams(pc.LOGN, 64, mods, L, K, 3)
+    h = pc.Harness(be, 64, mods)
+    c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(bits), prm)
+    evk[..., ::2] = np.array(mods, dtype=np.uint64)[:, None] - 1
+    modes = (_capi.BCONV_EXACT, _capi.ROUND_HALF)
+    ks = _capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, 3, *modes)
+    d_evk, d_c0, d_c1, o = h.up(evk), h.up(c0), h.up(c1), h.new(2, L, pc.N)
+    second = h.p(o) + L * pc.N * 8
+    ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk))
+    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, prm.q_idx, prm.p_idx, 3, c1, evk)))
+    ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0)
+    assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, 3, c0, c1, c1, c0, evk)))
+    ks.close()
