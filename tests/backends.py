@@ -3,6 +3,7 @@ g++-compiled emulation build (tests/emu).  Both expose the same four calls so a 
 is written once and runs through the same C ABI on either."""
 from __future__ import annotations
 
+import ctypes as C
 import os
 import sys
 
@@ -45,6 +46,14 @@ class EmuBackend:
     def sync(self):
         pass
 
+    def launches(self, call) -> int:
+        """Kernels that call(stream) launches."""
+        count = self.lib.dll.cerium_emu_launches
+        count.restype = C.c_long
+        before = count()
+        call(0)
+        return count() - before
+
 
 class CudaBackend:
     """The shipped CUDA library on cuda:0."""
@@ -80,3 +89,19 @@ class CudaBackend:
 
     def sync(self):
         self.torch.cuda.synchronize()
+
+    def launches(self, call) -> int:
+        """Kernels that call(stream) launches: captured into a graph and counted, not run."""
+        from cuda.bindings import runtime as rt
+        stream = self.torch.cuda.Stream()
+        (err,) = rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)
+        assert err == rt.cudaError_t.cudaSuccess, err
+        try:
+            call(stream.cuda_stream)
+        finally:
+            err, graph = rt.cudaStreamEndCapture(stream.cuda_stream)
+        assert err == rt.cudaError_t.cudaSuccess, err
+        err, _, count = rt.cudaGraphGetNodes(graph)
+        assert err == rt.cudaError_t.cudaSuccess, err
+        rt.cudaGraphDestroy(graph)
+        return count

@@ -155,6 +155,7 @@ void launch(dim3 grid, dim3 block, size_t smem_bytes, const std::function<void()
 
 }  // namespace cerium_emu
 
+extern "C" long cerium_emu_launches() { return cerium_emu::launches(); }
 // how often a kernel's limit was lowered
 extern "C" long cerium_emu_lowered_smem_limits() { return cerium_emu::g_lowered; }
 // launches before the default stream's copies were waited for

@@ -1,6 +1,7 @@
 """Row pass of the raised digits inside the inner product of a key switch: every arithmetic (primes of 60, 51 and 50 bits),
-more digits than a sum of doubles holds before it is reduced, and keys that are aligned to 16 bytes only, which take the
-separate kernels."""
+more digits than a sum of doubles holds before it is reduced, for one warp to a row and for each of two, and keys that are
+aligned to 16 bytes only, which take the separate kernels with 64-bit words.  The launches are counted, so that a call that
+takes another path than the one it is here for fails."""
 import numpy as np
 import pytest
 
@@ -22,31 +23,51 @@ def _params(word_bits, L, K, dnum):
     return params.CkksParams(pc.LOGN, 64, q + p60[1:], L, K, dnum)
 
 
-@pytest.mark.parametrize("word_bits,L,K,dnum", [(64, 3, 1, 3), (64, 12, 1, 12), (64, 15, 2, 10), (32, 9, 2, 5)])
-@pytest.mark.parametrize("offset", [0, 16])
-def test_key_switch(be, word_bits, L, K, dnum, offset):
+# the last column: whether the plan has the rows for it on a GPU of 148 SMs (1.8 for each of 16 warps an SM, 1.4 from 12 digits
+# on); 12 digits in 13 limbs and 10 in 17 are just past the line, 19 and 25 limbs well
+SHAPES = [(64, 3, 1, 3, False), (64, 12, 1, 12, True), (64, 15, 2, 10, True), (32, 9, 2, 5, True), (64, 20, 5, 4, True)]
+
+
+@pytest.mark.parametrize("word_bits,L,K,dnum,rows,offset", [s + (o,) for o in (0, 16) for s in SHAPES] + [(64, 18, 1, 18, True, 0)])
+def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
     prm = _params(word_bits, L, K, dnum)
     h = pc.Harness(be, word_bits, prm.moduli)
     c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(dnum), prm)
     if offset == 0:  # the largest key words
         evk[..., ::2] = np.array([prm.moduli[p] - 1 for p in prm.q_idx + prm.p_idx], dtype=np.uint64)[:, None]
     modes = (_capi.BCONV_EXACT, _capi.ROUND_HALF) if word_bits == 64 else (_capi.BCONV_LAZY, _capi.ROUND_FLOOR)
-    ks = _capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, dnum, *modes)
+    shape = (prm.q_idx, prm.p_idx, dnum)
+    ks = _capi.KeySwitch(h.ctx, *shape[:2], dnum, *modes)
     words = offset * 8 // word_bits
-    d_evk = h.up(np.concatenate([np.zeros(words, dtype=np.uint64), evk.reshape(-1)]))
+    d_evk = h.up(np.concatenate([np.zeros(words, dtype=np.uint64), evk.reshape(-1), np.zeros(4, dtype=np.uint64)]))
+    key = h.p(d_evk) + offset
     d_c0, d_c1 = h.up(c0), h.up(c1)
     o = h.new(2, L, pc.N)
     second = h.p(o) + L * pc.N * word_bits // 8
-    ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk) + offset)
-    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, prm.q_idx, prm.p_idx, dnum, c1, evk)))
+    ks.apply(h.p(o), second, h.p(d_c1), key)
+    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, *shape, c1, evk)))
     elt = be.lib.galois_elt_from_step(7, pc.LOGN)
-    ks.hrot(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_evk) + offset, elt)
-    assert np.array_equal(h.down(o), np.stack(h.orc.hrot(*modes, prm.q_idx, prm.p_idx, dnum, elt, c0, c1, evk)))
+    ks.hrot(h.p(o), second, h.p(d_c0), h.p(d_c1), key, elt)
+    assert np.array_equal(h.down(o), np.stack(h.orc.hrot(*modes, *shape, elt, c0, c1, evk)))
     # a multiplication: the products of the tensor are taken where they are read
     b0, b1 = (pc.rand_limbs(np.random.default_rng(8 + k), prm.moduli, prm.q_idx) for k in range(2))
     d_b0, d_b1 = h.up(b0), h.up(b1)
-    ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_b0), h.p(d_b1), h.p(d_evk) + offset, 0)
-    assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, dnum, c0, c1, b0, b1, evk)))
+    inputs = [h.p(d_c0), h.p(d_c1), h.p(d_b0), h.p(d_b1)]
+    ks.hmult(h.p(o), second, *inputs, key, 0)
+    assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, *shape, c0, c1, b0, b1, evk)))
+    r = h.new(2, L - 1, pc.N)
+    # with a rescale, after the division and in it
+    for levels, want in ((1, lambda: h.orc.hmult_relin(*modes, True, *shape, c0, c1, b0, b1, evk)),
+                         (2, lambda: h.orc.hmult_relin_fused(*modes, *shape, c0, c1, b0, b1, evk)))[:2 if K > 1 else 0]:
+        ks.hmult(h.p(r), h.p(r) + (L - 1) * pc.N * word_bits // 8, *inputs, key, levels)
+        assert np.array_equal(h.down(r), np.stack(want())), levels
+    # which kernels these were: the row pass is one of its own, or not, and the tensor product likewise
+    one = (word_bits == 32 or offset == 0) and (rows or be.name == "emu")
+    tensor = one and dnum < 12
+    converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4  # ModUps in one launch or two
+    switch = 9 + converted + (not one)
+    assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), key, stream=st)) == switch
+    assert be.launches(lambda st: ks.hmult(h.p(o), second, *inputs, key, 0, st)) == switch + (not tensor)
     ks.close()
 
 
@@ -68,4 +89,6 @@ def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, prm.q_idx, prm.p_idx, 3, c1, evk)))
     ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0)
     assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, 3, c0, c1, c1, c0, evk)))
+    converted = be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4
+    assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == 9 + converted + (bits < 34)
     ks.close()
