@@ -64,6 +64,7 @@ struct cerium_keyswitch {
   // every prime of the plan by the caller of keyswitch_inner_moddown; no converters, no own limbs
   bool lifted = false;
   bool key_sums = true;  // KeySum takes every local prime
+  bool integer = false;  // most of the local limbs are 64-bit words with integer butterflies
   std::vector<uint32_t> ext_pos, ext_prime;  // extension limbs of both accumulators
   // exact mode: per-limb scalars folded into the inverse transforms (device, one word per entry)
   void* d_consts = nullptr;  // what the next three point into
@@ -168,22 +169,30 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
   return CERIUM_OK;
 }
 
-// Digits from which on two warps share a row of raised_inner_kernel<uint64_t>: whole rounds of CTAs are shorter (24 limbs
-// with as many digits 467 -> 452 us, 15 limbs 257.5 -> 256.5); 7 digits on 40 limbs lose (301 -> 320 us).  32-bit words are never split:
-// rotations of 3 to 51 limbs lose 5 to 10 %.
+// Digits from which on two warps share a row of raised_inner_kernel<uint64_t>: whole rounds of CTAs are shorter (13 limbs
+// with as many digits 202.4 -> 192.4 us, 24 limbs 424 / 426); 7 digits on 40 limbs lose (292 -> 313 us).  Not where the
+// butterflies are integers (60-bit primes, 16 limbs with as many digits 379.5 -> 381.8, 20 limbs 540.8 -> 553.0).  32-bit words are
+// never split: rotations of 3 to 51 limbs lose 5 to 10 %.
 constexpr int kSplitDigits = 12;
+bool splits_rows(const cerium_keyswitch* ks) { return ks->ctx->word_bits == 64 && ks->dnum >= kSplitDigits && !ks->integer; }
 // Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where its sums take the plan's
-// primes, it can read the key and the polynomials four words at a time, and 64-bit words have the rows that keep the resident warps (16 to an SM) busy.
-// With fewer the serial walk over the digits shows: rotation of 10 limbs (15 with the extension) 102.9 us in two kernels and
-// 110.6 in one, 11 limbs 113.6 / 115.4, 12 limbs 118.0 / 117.3, 13 limbs 138.2 / 129.2; digits of one limb, 10 limbs
-// 180.1 / 183.6, 12 limbs 220.9 / 216.0.  32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 197.4 / 182.8).
+// primes, it can read the key and the polynomials four words at a time, and 64-bit words have the rows that keep the resident
+// warps (16 to an SM) busy.  With fewer the serial walk over the digits shows; integer butterflies make it longer, and want more
+// rows where digits are many.  Rotations in two kernels / in one, us:
+//   50-bit primes, 5 extension limbs: 8 limbs 96.0 / 95.8, 10 limbs 103.6 / 104.5, 11 limbs 113.6 / 110.3, 12 limbs (17 with the
+//   extension) 118.5 / 110.7, 13 limbs 136.4 / 119.2; digits of one limb, 6 limbs 103.5 / 109.2, 8 limbs 136.8 / 129.6, 10 limbs
+//   173.0 / 158.0, 12 limbs 206.7 / 198.7.  The limits are those of the kernel's first form, which needed 12 limbs; smaller
+//   plans have come to gain since;
+//   60-bit primes, 5 extension limbs: 12 limbs 168.8 / 162.4, 24 limbs 300.3 / 289.7; digits of one limb, 16 limbs 370.3 / 379.5,
+//   20 limbs 529.6 / 540.8, 24 limbs 717.8 / 692.3; of two limbs, 24 limbs 456.6 / 452.6.
+// 32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 199.8 / 183.4).
 // Hoisted rotations transform the digits once for many keys and keep the two kernels.
 bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* evk, const void* add0, const void* add1) {
   const uintptr_t ptrs = (uintptr_t)cpoly | (uintptr_t)evk | (uintptr_t)add0 | (uintptr_t)add1;
   if (!ks->key_sums || ptrs % (4 * ks->ctx->word_bytes()) != 0) return false;
   if (ks->ctx->word_bits == 32) return true;
   const double rows_per_warp = 256.0 * ks->LK / (16.0 * ks->ctx->sm_count);
-  return rows_per_warp >= (ks->dnum >= kSplitDigits ? 1.4 : 1.8);
+  return rows_per_warp >= (ks->dnum < kSplitDigits ? 1.8 : ks->integer ? 2.5 : 1.4);
 }
 
 // Step 1: inverse transform of the local limbs of the switched polynomial into `dst`
@@ -301,7 +310,7 @@ int keyswitch_inner(cerium_keyswitch* ks, const void* cpoly, const void* evk, cu
     // every local extended limb (Q and extension) in one launch
     if (rows_left) {
       const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
-      const int split = sizeof(W) == 8 && dnum >= kSplitDigits ? 2 : 1;
+      const int split = splits_rows(ks) ? 2 : 1;
       auto kfn = raised_inner_kernel<W, 2, 1>;
       if constexpr (sizeof(W) == 8)
         if (split == 2) kfn = raised_inner_kernel<W, 2, 2>;
@@ -708,8 +717,13 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
   ks->all_idx = ks->q_idx;
   ks->all_idx.insert(ks->all_idx.end(), ks->p_idx.begin(), ks->p_idx.end());
   const int LK = ks->LK;
-  for (uint32_t p : ks->all_idx)
-    if (ctx->word_bits == 64 && !ctx->fp_ok[p] && ctx->moduli[p] >> (kKeySumBits - 1) == 0) ks->key_sums = false;
+  int with_integers = 0;
+  for (uint32_t p : ks->all_idx) {
+    if (ctx->word_bits == 32 || ctx->fp_ok[p]) continue;
+    with_integers++;
+    if (ctx->moduli[p] >> (kKeySumBits - 1) == 0) ks->key_sums = false;
+  }
+  ks->integer = 2 * with_integers > LK;
   const int Kl = ks->K;  // local extension limbs
   ks->lifted = lifted;
   for (int e = 0; e < LK; e++) ks->own_digit.push_back((e < L && !lifted) ? ks->loc[e] % dnum : -1);

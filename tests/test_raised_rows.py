@@ -92,3 +92,27 @@ def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     converted = be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4
     assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == 9 + converted + (bits < 34)
     ks.close()
+
+
+@pytest.mark.parametrize("L,K,dnum,rows", [(16, 1, 16, False)])
+def test_plans_of_60_bit_primes(be, L, K, dnum, rows):
+    """Integer butterflies: the kernels stay apart where many digits meet few limbs (2.5 rows for each of 16 warps an SM), and a
+    row keeps one warp."""
+    mods = params.ntt_primes_below(60, L + K, pc.LOGN)
+    h = pc.Harness(be, 64, mods)
+    shape = (list(range(L)), list(range(L, L + K)), dnum)
+    c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(L), params.CkksParams(pc.LOGN, 64, mods, L, K, dnum, q_idx=shape[0], p_idx=shape[1]))
+    evk[..., ::2] = np.array(mods, dtype=np.uint64)[:, None] - 1
+    modes = (_capi.BCONV_EXACT, _capi.ROUND_HALF)
+    ks = _capi.KeySwitch(h.ctx, *shape, *modes)
+    d_evk, d_c0, d_c1, o = h.up(evk), h.up(c0), h.up(c1), h.new(2, L, pc.N)
+    second = h.p(o) + L * pc.N * 8
+    ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk))
+    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, *shape, c1, evk)))
+    ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0)
+    assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, *shape, c0, c1, c1, c0, evk)))
+    converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4
+    switch = 9 + converted + (not rows and be.name != "emu")
+    assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == switch
+    assert be.launches(lambda st: ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0, st)) == switch + 1
+    ks.close()
