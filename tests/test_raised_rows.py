@@ -94,10 +94,10 @@ def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     ks.close()
 
 
-@pytest.mark.parametrize("L,K,dnum,rows", [(16, 1, 16, False)])
+@pytest.mark.parametrize("L,K,dnum,rows", [(16, 1, 16, False), (20, 5, 4, True)])
 def test_plans_of_60_bit_primes(be, L, K, dnum, rows):
-    """Integer butterflies: the kernels stay apart where many digits meet few limbs (2.5 rows for each of 16 warps an SM), and a
-    row keeps one warp."""
+    """Integer butterflies: the kernels stay apart where many digits meet few limbs (2.5 rows for each of 16 warps an SM), a row
+    keeps one warp, and the tensor product is a kernel of its own."""
     mods = params.ntt_primes_below(60, L + K, pc.LOGN)
     h = pc.Harness(be, 64, mods)
     shape = (list(range(L)), list(range(L, L + K)), dnum)
