@@ -63,7 +63,8 @@ def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
         assert np.array_equal(h.down(r), np.stack(want())), levels
     # which kernels these were: the row pass is one of its own, or not, and the tensor product likewise
     one = (word_bits == 32 or offset == 0) and (rows or be.name == "emu")
-    tensor = one and dnum < 12
+    integers = word_bits == 64 and 2 * sum(prm.moduli[p] >> 50 > 0 for p in prm.q_idx + prm.p_idx) > L + K
+    tensor = one and dnum < 12 and not integers
     converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4  # ModUps in one launch or two
     switch = 9 + converted + (not one)
     assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), key, stream=st)) == switch
