@@ -1251,11 +1251,12 @@ int cerium_hmult(cerium_keyswitch* ks, void* out0, void* out1, const void* a0, c
   cudaStream_t st = (cudaStream_t)stream;
   // The tensor product inside the inverse transform and the inner product, which multiply as they read; a0 b0 and
   // a0 b1 + a1 b0 are added before the ModDown, as [P] times themselves, whatever it divides by.  Separate -> inside: 35 limbs in
-  // digits of five 318.3 -> 315.9 us, 20 limbs 170.4 / 170.7, 14 limbs 137.8 -> 135.6.  Not with two warps to a row:
+  // digits of five 318.3 -> 315.9 us, 20 limbs 170.4 / 170.7, 14 limbs 137.8 -> 135.6;
+  // 32-bit words, 51 limbs in digits of four 323.2 -> 317.4, 24 limbs in digits of one 225.6 -> 219.7.  Not with two warps to a row:
   // there are more rounds of CTAs then, and each would start with those products (24 limbs with as many digits 433.4 -> 436.8).
   // Not with integer butterflies, whose sums leave the least room for them (60-bit primes, 24 limbs in digits of five 309.4 -> 323.3,
   // 20 limbs in digits of three 310.6 -> 330.3, where the separate kernels took 321.6 and 313.7).
-  const bool fused = !ks->lifted && !ks->integer && ks->dnum < kSplitDigits &&
+  const bool fused = !ks->lifted && !ks->integer && !splits_rows(ks) &&
                      rows_with_inner(ks, reinterpret_cast<const void*>((uintptr_t)a0 | (uintptr_t)a1), evk, b0, b1);
   if (!fused)
     if (int rc = cerium_tensor(ctx, d0, d1, d2, a0, a1, b0, b1, n, ks->q_idx.data(), ks->L, stream)) return rc;

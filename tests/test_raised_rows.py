@@ -28,7 +28,7 @@ def _params(word_bits, L, K, dnum):
 SHAPES = [(64, 3, 1, 3, False), (64, 12, 1, 12, True), (64, 15, 2, 10, True), (32, 9, 2, 5, True), (64, 20, 5, 4, True)]
 
 
-@pytest.mark.parametrize("word_bits,L,K,dnum,rows,offset", [s + (o,) for o in (0, 16) for s in SHAPES] + [(64, 18, 1, 18, True, 0)])
+@pytest.mark.parametrize("word_bits,L,K,dnum,rows,offset", [s + (o,) for o in (0, 16) for s in SHAPES] + [(64, 18, 1, 18, True, 0), (32, 12, 1, 12, True, 0)])
 def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
     prm = _params(word_bits, L, K, dnum)
     h = pc.Harness(be, word_bits, prm.moduli)
@@ -64,7 +64,7 @@ def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
     # which kernels these were: the row pass is one of its own, or not, and the tensor product likewise
     one = (word_bits == 32 or offset == 0) and (rows or be.name == "emu")
     integers = word_bits == 64 and 2 * sum(prm.moduli[p] >> 50 > 0 for p in prm.q_idx + prm.p_idx) > L + K
-    tensor = one and dnum < 12 and not integers
+    tensor = one and not integers and (word_bits == 32 or dnum < 12)
     converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4  # ModUps in one launch or two
     switch = 9 + converted + (not one)
     assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), key, stream=st)) == switch
