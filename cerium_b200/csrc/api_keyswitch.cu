@@ -621,27 +621,23 @@ int hoisted_rotate_pair(cerium_keyswitch* ks, void* const (&out)[2][2], const vo
     }
     std::vector<uint64_t> factor2(ks->pinv);
     factor2.insert(factor2.end(), ks->pinv.begin(), ks->pinv.end());
-    const bool both = 2 * L <= kSudMaxBatch;
-    for (int i = 0; i < (both ? 2 : 4); i++) {
-      const int r = both ? i : i >> 1, p = both ? 0 : i & 1;
+    for (int r = 0; r < 2; r++) {  // both polynomials together: a plan has at most 64 limbs
       SudCall s{};
-      s.src = s.work = conv[r] + (size_t)p * L * n;
+      s.src = s.work = conv[r];
       s.src_stride = s.work_stride = n;
       s.cols_done = true;
-      s.dst = out[r][p];
+      s.dst = out[r][0];
       s.dst_stride = n;
-      s.minuend = acc[r] + (size_t)p * LK * n;
+      s.minuend = acc[r];
       s.minuend_stride = n;
-      s.addend = p == 0 ? c0 : nullptr;
+      s.addend = c0;
       s.addend_stride = n;
       s.prime = prime.data();
       s.factor = factor2.data();
-      s.count = both ? 2 * L : L;
-      if (both) {
-        s.split = L;
-        s.dst2 = out[r][1];
-        s.minuend2 = acc[r] + (size_t)LK * n;
-      }
+      s.count = 2 * L;
+      s.split = L;
+      s.dst2 = out[r][1];
+      s.minuend2 = acc[r] + (size_t)LK * n;
       s.store_galois = store_elt[r];
       if (int rc = launch_sud(ctx, s, stream)) return rc;
     }

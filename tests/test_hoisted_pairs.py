@@ -16,3 +16,10 @@ def be(request):
 def test_linear_transform(be, word_bits, L, K, dnum, g):
     modes = (_capi.BCONV_EXACT, _capi.ROUND_HALF) if word_bits == 64 else (_capi.BCONV_LAZY, _capi.ROUND_FLOOR)
     pc.case_bsgs(be, word_bits, L, K, dnum, *modes, g=g, n_giant=2, r=0)
+
+
+@pytest.mark.gpu
+def test_the_largest_plan():
+    """64 limbs: both polynomials of a rotation fill the final transform's launch."""
+    from tests import backends
+    pc.case_bsgs(backends.CudaBackend(), 32, 64, 16, 4, _capi.BCONV_LAZY, _capi.ROUND_FLOOR, g=3, n_giant=2, r=0)
