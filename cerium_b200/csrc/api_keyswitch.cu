@@ -486,7 +486,7 @@ int keyswitch_moddown(cerium_keyswitch* ks, void* out0, void* out1, const void* 
 }
 
 // Sums that a plaintext multiply-accumulate over these primes takes (PtMacSum).  Column sums of 28-bit pieces hold 16
-// products of residues below 2^56.
+// products of residues below 2^56.  One kind for all limbs of a launch: the widest prime decides.
 template <typename W>
 int pt_mac_kind(const cerium_context* ctx, const uint32_t* prime_idx, int count) {
   if (sizeof(W) == 4) return kPtGeneral;
@@ -567,14 +567,17 @@ int keyswitch_impl(cerium_keyswitch* ks, void* out0, void* out1, const void* cpo
 }
 
 // Whether two hoisted rotations may run together: the second one's accumulators and converted limbs lie where a rotation with
-// an output on an input, a multiplication and a rescale keep theirs (3L + 2L + 2 limbs).
+// an output on an input, a multiplication and a rescale keep theirs (3L + 2L + 2 limbs).  A rule of room, not of speed: every plan
+// that was measured gains, and those with few limbs beside their extension (5 and fewer than 8, 13 and fewer than 24) rotate one at
+// a time.
 bool rotates_in_pairs(const cerium_keyswitch* ks) { return 2 * ks->LK + 2 * ks->L <= 5 * ks->L + 2; }
 
 // Two hoisted rotations of one ciphertext, each as cerium_hoisted_rotate has it: one pass over the raised digits, and a
 // ModDown whose small launches serve both (10 extension limbs take as long to transform back as 20).  The outputs are
 // aligned to 16 bytes and lie on none of the inputs.
-// Linear transforms one rotation at a time -> in pairs: 8 x 8 diagonals at 35 limbs 3270 -> 3210 us, 7 x 6 at 25 limbs
-// 1754 -> 1611, 5 x 3 at 20 limbs 820 -> 744, 8 x 4 at 12 limbs 854 -> 801.
+// Six baby rotations and the products with a row of diagonals, one at a time -> in pairs: 50-bit primes, 35 limbs 1282 -> 1173 us, 24
+// limbs 892 -> 756, 8 limbs 415 -> 349; 60-bit primes, 35 limbs 1561 -> 1417, 12 limbs 698 -> 573; 32-bit words with 13 extension
+// limbs, 35 limbs 552 -> 494, 24 limbs 409 -> 364, with 5, 12 limbs 278 -> 231.
 int hoisted_rotate_pair(cerium_keyswitch* ks, void* const (&out)[2][2], const void* c0, const void* c1, const void* const (&evk)[2],
                         const uint32_t (&store_elt)[2], cudaStream_t stream) {
   cerium_context* ctx = ks->ctx;

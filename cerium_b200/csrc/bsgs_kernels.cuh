@@ -119,9 +119,11 @@ struct PtMacSum<uint64_t, kPtPieces> {
 };
 
 // out[i][p] = sum_j pt[i][j] * src_p[j] for the GI giant steps of a group.  Streams 2 + GI words per baby step and word
-// position: bound by memory.  A thread copies the operands of the next steps into shared memory of its own (cp.async, three
-// steps on their way): 60 to 110 KB of an SM in flight.  With one step ahead in registers it was 25 KB and 303 us for 8 baby and
-// 4 giant steps at 35 limbs (1.0 GB), now 228; 8 and 8 (64-bit primes below 2^50: 1.7 GB in one launch) 606 -> 262.  An absent diagonal costs a predicate and no branch.
+// position: bound by memory (8 baby and 4 giant steps at 35 limbs are 1.0 GB, 8 and 8 in one launch 1.8).  A thread copies the operands of
+// the next steps into shared memory of its own (cp.async, three steps on their way): 60 to 110 KB of an SM in flight, where one step
+// ahead in registers was 25 KB.  8 and 4 steps, 8 and 8 steps at 35 limbs, that -> this: 50-bit primes 318 -> 166 us, 629 -> 282 (one
+// launch for two); pieces 312 -> 239, 627 -> 482; general 324 -> 243, 652 -> 490; 32-bit words 122 -> 85, 248 -> 170.  An absent
+// diagonal costs a predicate and no branch.
 // grid = (N / (kThreads * kWords), limbs), block = kThreads = ptmac_threads(GI).
 constexpr int kPtMacStages = 4;
 constexpr int ptmac_threads(int gi) { return gi > 4 ? 128 : 256; }

@@ -316,7 +316,8 @@ struct InnerProductArgs {
 };
 
 // The inner products of two hoisted rotations with their keys in one pass over the raised digits (no rotation of the input, no
-// sums to add to, no additions).  80 registers, three CTAs: 128 MB of 2 x 482 are not read for 7 digits on 40 limbs.
+// sums to add to, no additions).  80 registers, three CTAs: 128 MB of 2 x 482 are not read for 7 digits on 40 limbs
+// (152 us for a pair, 87 for one, in a profiler).
 template <typename W>
 struct InnerSecond {
   const W* evk;

@@ -5,17 +5,17 @@
 // sums that stay in its registers, so the raised digits are never written in transformed form (302 MB written and read again
 // for 24 digits of 24 limbs).
 //
-// Bound by memory: 482 MB for 7 digits on 40 limbs of 64-bit words, 945 MB for 24 digits on 25.  The twiddles of a row serve
-// every digit from shared memory (read through L1 for every digit they took the gain away: 147 us for the first shape, the
-// two kernels 143).  A lane keeps 8 words and 16 sums, so that 16 warps fit an SM at 128 registers; with 16 words to a lane
+// Bound by memory: 482 MB for 7 digits on 40 limbs of 64-bit words, 970 MB for 24 digits on 25 (451 MB through DRAM, and
+// 949 with the additions of a multiplication; 102 and 216 us in a profiler, half of the issue slots).  The twiddles of a row serve every digit
+// from shared memory (read through L1 for every digit they took the gain away: 147 us for the first shape, the two kernels 143).  A lane keeps 8 words and 16 sums, so that 16 warps fit an SM at 128 registers; with 16 words to a lane
 // it would be 8.  The next digit's row is on its way (cp.async) while one is worked on, and the key rows are asked for before
-// the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against 301).
-// Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 117.3 us against 122.4).
+// the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against the 301 of then).
+// Two rows to a CTA: whole rounds of CTAs are smaller than with four (12 limbs 117.3 us of then against 122.4).
 // Key words are the first to leave L2 by an explicit priority (with .cs alone rotation of 35 limbs 296.0 us, now 293.4; 24 limbs with
 // one-limb digits 431 -> 428).
-// Measured, row pass + inner product -> this kernel: rotation of 35 limbs 340.6 -> 301.3 us, multiplication of 24 limbs with
-// one-limb digits 540 -> 452, rotation of 51 32-bit limbs 197.2 -> 182.9.  When it is used: rows_with_inner
-// (api_keyswitch.cu).
+// Measured, row pass + inner product -> this kernel: rotation of 35 limbs 344 -> 291 us, multiplication of 24 limbs with
+// one-limb digits 542 -> 433, rotation of 51 32-bit limbs 200 -> 183; of 35 limbs of 60-bit primes 454 -> 446.  When it is used:
+// rows_with_inner (api_keyswitch.cu).
 #pragma once
 #include "ewise_kernels.cuh"
 #include "ntt_kernels.cuh"
