@@ -1362,7 +1362,15 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
       n_rot++;
     }
   }
-  if (n_rot == 0 && rescale_levels != 0) return fail(CERIUM_ERR_UNSUPPORTED, "bsgs_apply: rescale levels need at least one rotated giant step");
+  std::vector<char> have(n_giant, 0);  // giant steps with a diagonal
+  bool rotated = false;
+  for (int i = 0; i < n_giant; i++) {
+    for (int j = 0; j < g; j++)
+      if (plaintexts[(size_t)i * g + j] != nullptr) have[i] = 1;
+    rotated = rotated || (have[i] && giant_elts[i] != 1);
+  }
+  // the division is the ModDown's, and the outputs have no room for the sums themselves
+  if (!rotated && rescale_levels != 0) return fail(CERIUM_ERR_UNSUPPORTED, "bsgs_apply: rescale levels need at least one rotated giant step");
   DeviceGuard guard(ctx->device);
   cudaStream_t st = (cudaStream_t)stream;
   const size_t n = kN, wb = ctx->word_bytes(), poly = (size_t)L * n * wb;
@@ -1397,7 +1405,6 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
     }
   }
   // 2. inner sums s_i = sum_j pt[i][j] * baby_j, a group of giant steps per pass over the baby steps
-  std::vector<char> have(n_giant, 0);
   int rc = dispatch_word(ctx->word_bits, [&](auto tag) -> int {
     using W = decltype(tag);
     using V = Vec16<W>;
@@ -1420,7 +1427,6 @@ int cerium_bsgs_apply(cerium_keyswitch* ks, void* out0, void* out1, const void* 
           const void* p = plaintexts[(size_t)gi * g + j];
           if (p != nullptr && ((uintptr_t)p & 15u)) return fail(CERIUM_ERR_INVALID, "bsgs_apply: pointers must be 16-byte aligned");
           a.pt[i][j] = static_cast<const W*>(p);
-          if (p != nullptr) have[gi] = 1;
         }
       }
       for (int b = 0; b < L; b++) a.prime[b] = (uint8_t)ks->q_idx[b];

@@ -23,3 +23,22 @@ def test_the_largest_plan():
     """64 limbs: both polynomials of a rotation fill the final transform's launch."""
     from tests import backends
     pc.case_bsgs(backends.CudaBackend(), 32, 64, 16, 4, _capi.BCONV_LAZY, _capi.ROUND_FLOOR, g=3, n_giant=2, r=0)
+
+
+def test_a_rescale_without_a_rotated_diagonal_is_refused(be):
+    """The rotated giant step has a key and no diagonal: there is no ModDown that could divide, and the sums do not fit the outputs."""
+    prm = pc.small_params(64, 3, 1, 3)
+    h = pc.Harness(be, 64, prm.moduli)
+    ks = _capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, 3, _capi.BCONV_EXACT, _capi.ROUND_HALF)
+    limbs, key, work = h.new(5, 3, pc.N), h.new(3, 2, 4, pc.N), h.new(ks.bsgs_work_limbs(1, 2), pc.N)
+    poly = 3 * pc.N * 8
+    p = [h.p(limbs) + k * poly for k in range(5)]
+    call = lambda r, pts: ks.bsgs_apply(p[0], p[1], p[2], p[3], 1, 2, pts, [0], [1], [0, h.p(key)], [1, 5], r, h.p(work))  # noqa: E731
+    for r in (1, 2):
+        with pytest.raises(_capi.CeriumError) as e:
+            call(r, [p[4], 0])
+        assert e.value.code == _capi.ERR_UNSUPPORTED
+    call(0, [p[4], 0])
+    call(1, [0, p[4]])
+    be.sync()
+    ks.close()
