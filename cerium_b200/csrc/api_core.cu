@@ -51,13 +51,23 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
 template <typename W>
 static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
+// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen.  Columns: beyond these lines the second
+// barrier and the narrow tiles cost more than the shorter chain gives (column pass of 39 limbs in a rotation of 12 limbs 98.9 against
+// 100.7 us; 51 limbs of 32-bit words inverse 173.8 against 175.9).  Rows: fewer instructions decide where the GPU is full (384 limbs
+// forward 187.0 against 187.9 us under the power limit, inverse 163.7 / 167.2; 245 limbs 104.0 / 103.3 and 108.4 / 106.5).
+// Rows of 32-bit words: always inverse (245 limbs 73.6 / 71.1), and forward where the epilogue reads operands (rotation of
+// 51 limbs 176.9 -> 173.9; plain, 245 limbs 66.4 / 69.2).
+constexpr int kRadix8FwdCols = 32, kRadix8InvCols = 40, kRadix8Rows64 = 256;
 
 template <typename W, typename Batch, typename Loader>
 static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loader& loader, int limbs, cudaStream_t stream) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch<W>(ctx, limbs)) {
+  if (limbs <= kRadix8FwdCols) {
+    auto kfn = radix8_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
+    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
+  } else if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, loader, tw, pcs);
   } else {
@@ -70,7 +80,10 @@ static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvSc
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch<W>(ctx, limbs)) {
+  if (limbs <= kRadix8InvCols) {
+    auto kfn = radix8_inv_cols_kernel<W, kCols / 2, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, scale, tw, pcs);
+  } else if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_inv_cols_kernel<W, kCols / 2, Batch>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, scale, tw, pcs);
   } else {
@@ -84,12 +97,21 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch<W>(ctx, limbs)) {
-    auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, epi, tw, twr, pcs);
-  } else {
+  if (Epilogue::kHasOperands || (sizeof(W) == 8 && limbs <= kRadix8Rows64)) {
+    auto kfn = radix8_fwd_rows_kernel<W, Batch, Epilogue>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, epi, tw, twr, pcs);
+    return;
+  }
+  if constexpr (!Epilogue::kHasOperands) {
+    if constexpr (sizeof(W) == 4) {
+      if (small_batch<W>(ctx, limbs)) {
+        auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
+        CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
+        return;
+      }
+    }
     auto kfn = ntt_fwd_rows_kernel<W, kRowsPerCta, false, Batch, Epilogue>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, epi, tw, twr, pcs);
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
   }
 }
 template <typename W, typename Batch>
@@ -98,11 +120,13 @@ static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, 
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_inv);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (small_batch<W>(ctx, limbs)) {
-    auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
-  } else {
-    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
+  if (sizeof(W) == 4 || limbs <= kRadix8Rows64) {
+    auto kfn = radix8_inv_rows_kernel<W, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
+    return;
+  }
+  if constexpr (sizeof(W) == 8) {
+    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
   }
 }

@@ -22,6 +22,7 @@
 #include "ewise_kernels.cuh"
 #include "host_math.h"
 #include "ntt_kernels.cuh"
+#include "ntt_radix8.cuh"
 #include "raised_inner.cuh"
 
 namespace cerium {

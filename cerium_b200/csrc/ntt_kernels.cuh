@@ -42,13 +42,13 @@ struct NttCfg<uint32_t> {
 
 // Tiles of the two passes: `kCols` columns on 16 kCols threads, or rows of 256 coefficients on 16 threads each.  Batches
 // that do not fill the GPU take smaller tiles (the work is spread over all SMs: 160 tiles of 256 threads on 148 SMs
-// leave twelve with twice the work of the others) and copy a row's twiddles into shared memory before they wait
-// for the previous kernel, so that a warp's chain has one memory latency less.  On full launches both cost more than
+// leave twelve with twice the work of the others), and rows of 32-bit words then copy a row's twiddles into shared memory before
+// they wait for the previous kernel, so that a warp's chain has one memory latency less.  On full launches both cost more than
 // they give: the copies go through the same pipes as the data (71 -> 77 us for 245 limbs).
 constexpr int kRowsPerCta = 16;
 constexpr int kRowsSmall = 4;
 // ... up to this many usual tiles per SM (64 and 74 limbs on 148 SMs).  From there on the usual tiles are as fast or faster
-// (70 limbs of 64-bit words forward 36.9 against 37.7 us; 30 limbs inverse 20.4 against 17.9, 60 of 32-bit words 21.2 against 19.2)
+// (70 limbs of 64-bit words forward 36.9 against 37.7 us; 60 limbs of 32-bit words inverse 21.2 against 19.2)
 template <typename W>
 constexpr int kSmallBatchPerSm = sizeof(W) == 8 ? 7 : 8;
 // Lane-interleaved level-3 twiddles: [row h (256)][e = 2^t - 1 + g (15)][thread u (16)] pairs per
@@ -482,13 +482,12 @@ __device__ __forceinline__ void vec_unpack(const uint4& v, uint32_t* w) { w[0] =
 __device__ __forceinline__ ulonglong2 vec_pack(const uint64_t* w) { return make_ulonglong2(w[0], w[1]); }
 __device__ __forceinline__ uint4 vec_pack(const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); }
 
-// Twiddles of a row pass's rows in shared memory.  Tables of integer butterflies of 64-bit words are twice as long and
-// stay in global memory.
+// Twiddles of a row pass's rows in shared memory.
 template <typename W, int kRows>
 struct RowTwiddles {
   using Pair = typename WordTraits<W>::Pair;
-  static constexpr int kLane = sizeof(W) == 8 ? 8 * 16 : 15 * 16;  // entries of a row's lane table
-  static constexpr int kGroupPitch = 17;                           // rows of a warp in different banks
+  static constexpr int kLane = 15 * 16;   // entries of a row's lane table
+  static constexpr int kGroupPitch = 17;  // rows of a warp in different banks
   Pair lane[kRows][kLane];
   Pair group[kRows][kGroupPitch];
 };
@@ -496,6 +495,10 @@ template <typename W, int kRows, bool kStage>
 struct alignas(16) RowsBuffer {
   W tile[kRows * kRowPitch];
   RowTwiddles<W, kStage ? kRows : 1> tw;
+};
+template <typename W, int kRows>
+struct alignas(16) RowsBuffer<W, kRows, false> {
+  W tile[kRows * kRowPitch];
 };
 
 // Starts the copies of this warp's two rows (h0: first row of the CTA); row_twiddles_wait() before they are used.
@@ -665,14 +668,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 
 // What the row pass does with the finished NTT values, 16 bytes at a time.  kCanonicalInput says whether the
 // epilogue wants the values reduced to [0, q) first or takes them below 4q.  load() fetches what the epilogue reads
-// itself: the row pass calls it for half of a thread's vectors at a time before it finishes any of them (with one
-// vector at a time the SuD tail waited for memory in 7 of 12 warp cycles: 43 us for 70 limbs against 18 us of traffic).
+// itself: the row pass (radix8_fwd_rows_kernel) calls it for all of a thread's vectors before it finishes any of them.
 template <typename W>
 struct NoOperands {};
 template <typename W>
 struct StoreEpilogue {
   static constexpr bool kCanonicalInput = true;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
+  static constexpr bool kHasOperands = false;
   using Operands = NoOperands<W>;
   __device__ __forceinline__ Operands load(int, int) const { return {}; }
   template <int kWords>
@@ -686,6 +689,7 @@ template <typename W>
 struct LazyStoreEpilogue {
   static constexpr bool kCanonicalInput = false;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
+  static constexpr bool kHasOperands = false;
   using Operands = NoOperands<W>;
   __device__ __forceinline__ Operands load(int, int) const { return {}; }
   template <int kWords>
@@ -699,6 +703,7 @@ struct LazyStoreEpilogue {
 template <typename W>
 struct SudEpilogue {
   static constexpr bool kCanonicalInput = false;  // takes the transform below 4q
+  static constexpr bool kHasOperands = true;
   const W* minuend;
   const W* minuend2;
   size_t minuend_stride;
@@ -777,6 +782,7 @@ struct SudEpilogue {
 template <typename W>
 struct PtrSudEpilogue {
   static constexpr bool kCanonicalInput = false;
+  static constexpr bool kHasOperands = true;
   const W* const* ins;
   const W* factors;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
@@ -844,72 +850,49 @@ __device__ __forceinline__ void load16<uint32_t>(const uint32_t* src, uint32_t (
 }
 
 template <typename W, int kMode, int kRows, bool kStage, typename Batch, typename Epilogue>
-__device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epilogue& epi, int b, uint32_t pi,
-                                                  const PrimeConst<W>& pc, RowsBuffer<W, kRows, kStage>& buf,
+__device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc,
+                                                  RowsBuffer<W, kRows, kStage>& buf,
                                                   const typename WordTraits<W>::Pair* tw,
                                                   const typename WordTraits<W>::Pair* twr) {
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
-  constexpr bool kStaged = kStage && (sizeof(W) == 4 || kMode == kArithFp);
   W* tile = buf.tile;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
   const int h = blockIdx.x * kRows + r;
   const W* row = batch.in_limb(b) + (unsigned)(h * 256 + u);
-  W* limb_out = batch.out_limb(b);
-  W* drow = limb_out + (unsigned)(h * 256);
-  const int h_row = h * 256;
-  const uint32_t selt = epi.scatter_elt();
+  W* drow = batch.out_limb(b) + (unsigned)(h * 256);
   W* trow = tile + (unsigned)(r * kRowPitch);
   W* t_strided = trow + u;             // row_pos(j * 16 + u) = j * 17 + u
   W* t_own = trow + (unsigned)(u * 17);  // row_pos(u * 16 + j) = u * 17 + j
   W x[16];
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = row[j * 16];
-#pragma unroll
-  for (int k = 0; k < RV::kPerThread; k++) epi.prefetch(b, h * 256 + (u + 16 * k) * RV::kWords);
-  if (kStaged) row_twiddles_wait();
-  radix16_fwd<W, !kStaged, kMode, kStaged ? kTwGroup : kTwPlain, kFpFwdMid>(x, kStaged ? buf.tw.group[kStaged ? r : 0] : tw, 256u + (uint32_t)h, ar);
+  if constexpr (kStage) {
+    row_twiddles_wait();
+    radix16_fwd<W, false, kMode, kTwGroup, kFpFwdMid>(x, buf.tw.group[r], 0u, ar);
+  } else {
+    radix16_fwd<W, true, kMode, kTwPlain, kFpFwdMid>(x, tw, 256u + (uint32_t)h, ar);
+  }
 #pragma unroll
   for (int j = 0; j < 16; j++) t_strided[j * 17] = x[j];
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_own[j];
   // level 3: this thread's 15 twiddles from the lane-interleaved table of row h
-  radix16_fwd<W, !kStaged, kMode, kTwLane, kFpFwdL3>(
-      x, kStaged ? buf.tw.lane[kStaged ? r : 0] + u : twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  if constexpr (kStage) radix16_fwd<W, false, kMode, kTwLane, kFpFwdL3>(x, buf.tw.lane[r] + u, 0u, ar);
+  else radix16_fwd<W, true, kMode, kTwLane, kFpFwdL3>(x, twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.template finish_fwd<Epilogue::kCanonicalInput>(x[j], pc.one_shoup);
-  // own 16 words -> swizzled vectors -> coalesced vectors, then epilogue and store
+  // own 16 words -> swizzled vectors -> coalesced vectors
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
   Vec* vrow = reinterpret_cast<Vec*>(tile + r * kRowPitch);  // same private region as the exchange rows
 #pragma unroll
   for (int jj = 0; jj < RV::kPerThread; jj++)
     vrow[row_vec_slot<W>(u * RV::kPerThread + jj)] = vec_pack(&x[jj * RV::kWords]);
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
-  constexpr int kHalf = sizeof(W) == 8 ? RV::kPerThread / 2 : 1;
 #pragma unroll
-  for (int h = 0; h < RV::kPerThread; h += kHalf) {
-    typename Epilogue::Operands ops[kHalf];
-#pragma unroll
-    for (int k = 0; k < kHalf; k++) ops[k] = epi.load(b, h_row + (u + 16 * (h + k)) * RV::kWords);
-#pragma unroll
-    for (int k = 0; k < kHalf; k++) {
-      const int v = u + 16 * (h + k);
-      W w[RV::kWords];
-      vec_unpack(vrow[row_vec_slot<W>(v)], w);
-      epi.apply_vec(w, ops[k], b, h_row + v * RV::kWords, pi, pc);
-      if (selt != 0) {
-        // an aligned group of words lands on an aligned group of the output limb
-        const GaloisGroup<RV::kWords> gg((uint32_t)(h_row + v * RV::kWords), selt);
-        W t[RV::kWords];
-        gg.template permute<true>(w, t);
-        *reinterpret_cast<Vec*>(limb_out + gg.at) = vec_pack(t);
-      } else {
-        reinterpret_cast<Vec*>(drow)[v] = vec_pack(w);
-      }
-    }
-  }
+  for (int k = 0; k < RV::kPerThread; k++) reinterpret_cast<Vec*>(drow)[u + 16 * k] = vrow[row_vec_slot<W>(u + 16 * k)];
 }
 
 // Row pass (levels 2 and 3): reads the column pass's result from the batch's `in` stack and
@@ -920,8 +903,7 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, const Epil
 // The column pass gains nothing from it.
 template <typename W, int kRows, bool kStage, typename Batch, typename Epilogue>
 __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
-    ntt_fwd_rows_kernel(const Batch batch, const Epilogue epi,
-                        const typename WordTraits<W>::Pair* __restrict__ tw_all,
+    ntt_fwd_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const typename WordTraits<W>::Pair* __restrict__ twr_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
@@ -935,23 +917,22 @@ __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
   const PrimeConst<W> pc = pcs[pi];
   const Pair* tw = tw_all + (size_t)pi * kN;
   const Pair* twr = twr_all + (size_t)pi * kRowTwPerPrime;
-  if constexpr (kStage)
-    if (sizeof(W) == 4 || pc.fp_ok != 0) row_twiddles_start(buf.tw, tw, twr, blockIdx.x * kRows);
+  static_assert(!kStage || sizeof(W) == 4, "the lane tables of 64-bit words have other sizes");
+  if constexpr (kStage) row_twiddles_start(buf.tw, tw, twr, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_rows_body, CERIUM_TARGS(kRows, kStage, Batch, Epilogue), (batch, epi, b, pi, pc, buf, tw, twr));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_rows_body, CERIUM_TARGS(kRows, kStage, Batch, Epilogue), (batch, b, pc, buf, tw, twr));
 }
 
 // ---------------------------------------------------------------------------------------
 // inverse transform
 // ---------------------------------------------------------------------------------------
 
-template <typename W, int kMode, int kRows, bool kStage, typename Batch>
-__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, RowsBuffer<W, kRows, kStage>& buf,
+template <typename W, int kMode, int kRows, typename Batch>
+__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, RowsBuffer<W, kRows, false>& buf,
                                                   const typename WordTraits<W>::Pair* twi,
                                                   const typename WordTraits<W>::Pair* twri) {
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
-  constexpr bool kStaged = kStage && (sizeof(W) == 4 || kMode == kArithFp);
   W* tile = buf.tile;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
@@ -1004,9 +985,7 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
     vec_unpack(vrow[row_vec_slot<W>(u * RV::kPerThread + jj)], &x[jj * RV::kWords]);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.enter(x[j]);
-  if (kStaged) row_twiddles_wait();
-  radix16_inv<W, !kStaged, kMode, 0, kTwLane, kFpCanon>(
-      x, kStaged ? buf.tw.lane[kStaged ? r : 0] + u : twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  radix16_inv<W, true, kMode, 0, kTwLane, kFpCanon>(x, twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
   if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, kFpInvRowsExMask, ar);
   __syncwarp();
   W* t_own = trow + (unsigned)(u * 17);  // row_pos(u * 16 + j) = u * 17 + j
@@ -1016,30 +995,28 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_strided[j * 17];
-  radix16_inv<W, !kStaged, kMode, 4, kStaged ? kTwGroup : kTwPlain, kFpInvL3>(x, kStaged ? buf.tw.group[kStaged ? r : 0] : twi, 256u + (uint32_t)h, ar);
+  radix16_inv<W, true, kMode, 4, kTwPlain, kFpInvL3>(x, twi, 256u + (uint32_t)h, ar);
   W* dcol = dst + u;
 #pragma unroll
   for (int j = 0; j < 16; j++) dcol[j * 16] = x[j];
 }
 
 // Row pass (levels 3 and 2): in -> out; values leave below 2q (strict; 4q for 64-bit words) or below 2^10 q (lazy).
-template <typename W, int kRows, bool kStage, typename Batch>
+template <typename W, int kRows, typename Batch>
 __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
     ntt_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                         const typename WordTraits<W>::Pair* __restrict__ twri_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  __shared__ RowsBuffer<W, kRows, kStage> buf;
+  __shared__ RowsBuffer<W, kRows, false> buf;
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   const Pair* twi = twi_all + (size_t)pi * kN;
   const Pair* twri = twri_all + (size_t)pi * kRowTwPerPrime;
-  if constexpr (kStage)
-    if (sizeof(W) == 4 || pc.fp_ok != 0) row_twiddles_start(buf.tw, twi, twri, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, CERIUM_TARGS(kRows, kStage, Batch), (batch, b, pc, buf, twi, twri));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, CERIUM_TARGS(kRows, Batch), (batch, b, pc, buf, twi, twri));
 }
 
 // Optional per-limb scalar of the finished inverse transform (exact base conversion wants x * [Qhat^-1] mod q):

@@ -18,66 +18,9 @@
 // rows_with_inner (api_keyswitch.cu).
 #pragma once
 #include "ewise_kernels.cuh"
-#include "ntt_kernels.cuh"
+#include "ntt_radix8.cuh"
 
 namespace cerium {
-
-// Four consecutive words, one access of 32 bytes (64-bit words) or 16.
-template <typename W>
-struct Quad {
-  W v[4];
-};
-__device__ __forceinline__ Quad<uint32_t> quad_load(const uint32_t* p) {
-  const uint4 t = *reinterpret_cast<const uint4*>(p);
-  return {{t.x, t.y, t.z, t.w}};
-}
-// words that nothing reads again soon
-__device__ __forceinline__ Quad<uint32_t> quad_load_once(const uint32_t* p) {
-  const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p));
-  return {{t.x, t.y, t.z, t.w}};
-}
-__device__ __forceinline__ void quad_store(uint32_t* p, const Quad<uint32_t>& q) {
-  *reinterpret_cast<uint4*>(p) = make_uint4(q.v[0], q.v[1], q.v[2], q.v[3]);
-}
-#if defined(CERIUM_EMU)
-inline Quad<uint64_t> quad_load(const uint64_t* p) { return {{p[0], p[1], p[2], p[3]}}; }
-inline Quad<uint64_t> quad_load_once(const uint64_t* p) { return quad_load(p); }
-inline void quad_store(uint64_t* p, const Quad<uint64_t>& q) {
-  for (int e = 0; e < 4; e++) p[e] = q.v[e];
-}
-#else
-__device__ __forceinline__ Quad<uint64_t> quad_load(const uint64_t* p) {
-  Quad<uint64_t> q;
-  asm volatile("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
-  return q;
-}
-__device__ __forceinline__ Quad<uint64_t> quad_load_once(const uint64_t* p) {
-  Quad<uint64_t> q;
-  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(q.v[0]), "=l"(q.v[1]), "=l"(q.v[2]), "=l"(q.v[3]) : "l"(p) : "memory");
-  return q;
-}
-__device__ __forceinline__ void quad_store(uint64_t* p, const Quad<uint64_t>& q) {
-  asm volatile("st.global.v4.b64 [%0], {%1,%2,%3,%4};" ::"l"(p), "l"(q.v[0]), "l"(q.v[1]), "l"(q.v[2]), "l"(q.v[3]) : "memory");
-}
-#endif
-
-// Bounds of the Fp butterflies over the eight layers of a row, as fp_plan_fwd has them for four.
-struct FpRowPlan {
-  bool before[8];
-  int out;
-};
-__host__ __device__ constexpr FpRowPlan fp_plan_row(int bin) {
-  FpRowPlan p{};
-  int b = bin;
-  for (int t = 0; t < 8; t++) {
-    p.before[t] = b > kFpOperandMax;
-    if (p.before[t]) b = kFpReduced;
-    b += fp_product_bound(b, t < 6 ? 1 : kFpLaneK32);  // the last two layers compute their quotients
-  }
-  p.out = b;
-  return p;
-}
-static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values must stay exact integers");
 
 // Sums of products of residues (integers: below 4q) with key words; 64 bits, so that partial sums of a row can be put
 // together.
@@ -140,15 +83,6 @@ struct KeySum<uint64_t, kArithFp> {
   }
 };
 
-// Exchange buffer of a row: word i at i + 4 (i / 32), 64-bit words with bit 1 of i flipped where bit 4 is set.  The three
-// patterns (a run of 32; 8 runs of 4 at a distance of 32; 4 words of each of 32 neighbouring lanes, 16 bytes at a time) are
-// then free of bank conflicts.
-constexpr int kRaisedPitch = 256 + 8 * 4;
-template <typename W>
-__device__ __forceinline__ int raised_pos(int i) {
-  return (sizeof(W) == 8 ? i ^ ((i >> 3) & 2) : i) + (i >> 5) * 4;
-}
-
 // A row's shared memory: the digit that is worked on and the next one on its way, and the twiddles of the row, which serve
 // every digit.  Pair (1 << t) + g is entry ((256 + h) << t) + g of the table, layers t = 0..7.  64-bit words: layers 0..5
 // only; Fp has the last two without their quotients after them, word (1 << t) + g - 64 of `late`.  The integer butterflies of
@@ -177,34 +111,13 @@ __device__ __forceinline__ void raised_twiddles(RaisedRow<W>& row, const typenam
     prefetch_l2(lane < 8 ? tw + (S * 64u + 8u * (uint32_t)lane) : tw + (S * 128u + 8u * (uint32_t)(lane - 8)));
 }
 
-// Three layers on x[0..7]; layer t pairs (j, j + (4 >> t)) with twiddle (S << t) + (j >> (3 - t)).  kLayer: number of the
-// first one inside the row.
-template <typename W, int kMode, int kLayer>
-__device__ __forceinline__ void radix8_fwd(W (&x)[8], const typename WordTraits<W>::Pair* tw, int S, const Arith<W, kMode>& ar) {
-  constexpr FpRowPlan plan = fp_plan_row(kFpFwdMid);
-#pragma unroll
-  for (int t = 0; t < 3; t++) {
-    const int half = 4 >> t;
-    if (kMode == kArithFp && plan.before[kLayer + t]) {
-#pragma unroll
-      for (int j = 0; j < 8; j++) x[j] = ar.reduce(x[j]);
-    }
-#pragma unroll
-    for (int g = 0; g < (1 << t); g++) {
-      const auto w = tw[(S << t) + g];
-#pragma unroll
-      for (int k = 0; k < half; k++) ar.fwd(x[g * 2 * half + k], x[g * 2 * half + k + half], w.x, w.y);
-    }
-  }
-}
-
 // The eight layers of row h.  In: x[j] = word j * 32 + lane.  Out: x[r] = word (r / 4) * 128 + lane * 4 + r % 4, Fp:
 // |x| <= 0.51 q, integers: below 4q.
 template <typename W, int kMode>
 __device__ __forceinline__ void raised_row(W (&x)[8], W* ex, const RaisedRow<W>& row, const typename WordTraits<W>::Pair* tw, int h,
                                            const Arith<W, kMode>& ar, const PrimeConst<W>& pc) {
   using RV = RowVec<W>;
-  constexpr FpRowPlan plan = fp_plan_row(kFpFwdMid);
+  constexpr FpPassPlan plan = fp_plan_row(kFpFwdMid);
   const int lane = threadIdx.x & 31;
   radix8_fwd<W, kMode, 0>(x, row.tw, 1, ar);
 #pragma unroll

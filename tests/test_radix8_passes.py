@@ -1,0 +1,53 @@
+"""Transforms on both sides of the batch sizes where a pass changes from eight words a thread to sixteen (32 limbs forward and 40
+inverse of the column passes, 256 of the row passes of 64-bit words), for every arithmetic, and limbs of 64-bit words that are aligned to
+16 bytes only, whose rows move as pairs of words: exact against the oracle."""
+import numpy as np
+import pytest
+
+from cerium_b200 import _capi, params
+from tests import parity_cases as pc
+
+
+def gpu(*args):
+    return pytest.param(*args, marks=pytest.mark.gpu)
+
+
+def harness(name, word_bits):
+    from tests import backends
+    mods = pc.moduli_for(word_bits, 3, 1)
+    if word_bits == 64:
+        mods = mods + params.ntt_primes_below(51, 1, 16)
+    return pc.Harness(backends.EmuBackend() if name == "emu" else backends.CudaBackend(), word_bits, mods)
+
+
+@pytest.mark.parametrize("name,word_bits,count", [("emu", 64, 4), ("emu", 32, 3)] + [gpu("cuda", b, c) for b in (64, 32) for c in (1, 32, 33, 40, 41, 256, 257)])
+def test_batch_sizes(name, word_bits, count):
+    h = harness(name, word_bits)
+    idx = [(count + b) % len(h.moduli) for b in range(count)]
+    x = pc.rand_limbs(np.random.default_rng(count), h.moduli, idx)
+    x[0] = pc.edge_limbs(h.moduli, idx[:1])[0]
+    d = h.up(x)
+    h.ctx.ntt_forward(h.p(d), h.p(d), idx)
+    assert np.array_equal(h.down(d), h.orc.ntt_forward(x, idx))
+    h.ctx.ntt_inverse(h.p(d), h.p(d), idx)
+    assert np.array_equal(h.down(d), x)
+
+
+@pytest.mark.parametrize("name", ["emu", gpu("cuda")])
+def test_limbs_aligned_to_two_words(name):
+    h = harness(name, 64)
+    stride, idx = pc.N + 2, list(range(len(h.moduli)))
+    x = pc.rand_limbs(np.random.default_rng(3), h.moduli, idx)
+    flat = np.zeros((len(idx) + 1) * stride, dtype=np.uint64)
+    limbs = lambda a: np.lib.stride_tricks.as_strided(a[2:], (len(idx), pc.N), (8 * stride, 8))  # noqa: E731
+    limbs(flat)[...] = x
+    d, out = h.up(flat), h.new(flat.size)
+    h.ctx.ntt_forward(h.p(out) + 16, h.p(d) + 16, idx, stride, stride)
+    assert np.array_equal(limbs(h.down(out)), h.orc.ntt_forward(x, idx))
+    h.ctx.ntt_inverse(h.p(d) + 16, h.p(out) + 16, idx, stride, stride)
+    assert np.array_equal(limbs(h.down(d)), x)
+    # division by the last limb, whose row pass reads what it subtracts from as well
+    div, scratch, packed = h.new(flat.size), h.new(pc.N), h.up(np.concatenate([np.zeros(2, np.uint64), x.ravel()]))
+    h.ctx.rescale(h.p(div) + 16, h.p(packed) + 16, idx, 1, h.p(scratch), _capi.ROUND_HALF)
+    want = h.orc.rescale(_capi.ROUND_HALF, idx, x)
+    assert np.array_equal(h.down(div)[2:2 + want.size].reshape(want.shape), want)
