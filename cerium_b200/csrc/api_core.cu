@@ -278,8 +278,14 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
       for (int b = 0; b < cnt; b++) {
         const uint64_t q = ctx->moduli[c.prime[first + b]];
         const uint64_t f = c.factor[first + b] % q;
-        epi.factor[b] = (W)f;
-        epi.factor_shoup[b] = (W)host::shoup(f, q, bits);
+        if (ctx->fp_ok[c.prime[first + b]]) {
+          const double fd = host::centred(f, q), fq = fd / (double)q;
+          std::memcpy(&epi.factor[b], &fd, sizeof(W));
+          std::memcpy(&epi.factor_shoup[b], &fq, sizeof(W));
+        } else {
+          epi.factor[b] = (W)f;
+          epi.factor_shoup[b] = (W)host::shoup(f, q, bits);
+        }
       }
       if (c.cols_done) {
         // the rows only

@@ -666,20 +666,23 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 #endif
 }
 
-// What the row pass does with the finished NTT values, 16 bytes at a time.  kCanonicalInput says whether the
-// epilogue wants the values reduced to [0, q) first or takes them below 4q.  load() fetches what the epilogue reads
+// What the row pass does with its values, 16 bytes at a time, as the butterflies leave them.  kCanonical (epilogues without operands)
+// says whether they are stored reduced to [0, q) or below 4q.  load() fetches what the epilogue reads
 // itself: the row pass (radix8_fwd_rows_kernel) calls it for all of a thread's vectors before it finishes any of them.
 template <typename W>
 struct NoOperands {};
 template <typename W>
 struct StoreEpilogue {
-  static constexpr bool kCanonicalInput = true;
+  static constexpr bool kCanonical = true;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
   static constexpr bool kHasOperands = false;
   using Operands = NoOperands<W>;
   __device__ __forceinline__ Operands load(int, int) const { return {}; }
-  template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>&) const {}
+  template <int kMode, int kWords>
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>& pc, const Arith<W, kMode>& ar) const {
+#pragma unroll
+    for (int e = 0; e < kWords; e++) w[e] = ar.template finish_fwd<true>(w[e], pc.one_shoup);
+  }
   __device__ __forceinline__ void prefetch(int /*b*/, int /*idx*/) const {}
 };
 
@@ -687,22 +690,27 @@ struct StoreEpilogue {
 // wide accumulator (the raised digits of a key switch, read by the inner product).
 template <typename W>
 struct LazyStoreEpilogue {
-  static constexpr bool kCanonicalInput = false;
+  static constexpr bool kCanonical = false;
   __device__ __forceinline__ uint32_t scatter_elt() const { return 0u; }
   static constexpr bool kHasOperands = false;
   using Operands = NoOperands<W>;
   __device__ __forceinline__ Operands load(int, int) const { return {}; }
-  template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>&) const {}
+  template <int kMode, int kWords>
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands&, int, int, uint32_t, const PrimeConst<W>& pc, const Arith<W, kMode>& ar) const {
+#pragma unroll
+    for (int e = 0; e < kWords; e++) w[e] = ar.template finish_fwd<false>(w[e], pc.one_shoup);
+  }
   __device__ __forceinline__ void prefetch(int /*b*/, int /*idx*/) const {}
 };
 
 // SuD tail: out = (minuend - NTT(in)) * factor[b] [+ addend]   (all mod q).
 // minuend / addend are stacks of limbs: entry b at base + b * stride; entries b >= split belong
 // to a second polynomial and use minuend2 / addend2 at (b - split) * stride.
+// The row pass with it is bound by its reads (120 MB through DRAM for 70 limbs) and needs all 32 warps of an SM: operands copied to
+// shared memory leave 20 (rotation of 35 limbs 275.5 -> 281 us).  Doubles are finished as doubles (integer Shoup product: 35 limbs
+// 275.5 -> 274.0, 12 limbs 99.4 -> 98.6, plaintext product with rescale 32.0 -> 31.3).
 template <typename W>
 struct SudEpilogue {
-  static constexpr bool kCanonicalInput = false;  // takes the transform below 4q
   static constexpr bool kHasOperands = true;
   const W* minuend;
   const W* minuend2;
@@ -715,6 +723,7 @@ struct SudEpilogue {
   uint32_t store_elt;   // not 0: word i of the result is stored at pi(i), the index map of this element, so
                         // the output is the automorphism of the INVERSE element applied to the result
   __device__ __forceinline__ uint32_t scatter_elt() const { return store_elt; }
+  // the factor and its Shoup companion; Fp: the centred factor and its quotient by q, as bit patterns of doubles
   W factor[kSudMaxBatch];
   W factor_shoup[kSudMaxBatch];
   // starts the 16 bytes at word idx of the operands towards L2 (called before the transform, whose
@@ -747,9 +756,9 @@ struct SudEpilogue {
     }
     return o;
   }
-  template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int b, int idx0, uint32_t /*pi*/,
-                                            const PrimeConst<W>& pc) const {
+  template <int kMode, int kWords>
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int b, int idx0, uint32_t /*pi*/, const PrimeConst<W>& pc,
+                                            const Arith<W, kMode>& ar) const {
     const W* ap = b >= split ? addend2 : addend;
     W m[kWords], a[kWords];
     vec_unpack(o.m, m);
@@ -759,18 +768,33 @@ struct SudEpilogue {
       vec_unpack(o.a, t);
       GaloisGroup<kWords>((uint32_t)idx0, addend_elt).permute(t, a);
     }
+    const W f = factor[b], fs = factor_shoup[b];
 #pragma unroll
     for (int e = 0; e < kWords; e++) {
-      W d;
-      if (sizeof(W) == 4) {
-        // 32-bit words hold primes up to 2^30: m + 4q would pass 2^32, so the transform comes below 2q first
-        d = m[e] + pc.q2 - csub<W>(w[e], pc.q2);
+      if constexpr (kMode == kArithFp) {
+        // |x| <= 0.51 q after the reduction, the difference within (-0.51 q, 1.51 q), its product below 0.55 q, and with the
+        // addend within (-0.55 q, 1.55 q)
+        using A = Arith<W, kMode>;
+        const double d = __dadd_rn(fp_from_u64(m[e]), -A::d(ar.reduce(w[e])));
+        double r = fp_mulmod(d, A::d(f), A::d(fs), ar.nq);
+        if (ap != nullptr) {
+          r = __dadd_rn(r, fp_from_u64(a[e]));
+          if (r >= ar.q) r = __dadd_rn(r, ar.nq);
+        }
+        w[e] = ar.canonical(r);
       } else {
-        d = m[e] + (pc.q2 + pc.q2) - w[e];  // w < 4q: positive, and the Shoup product takes any word
+        const W x = ar.template finish_fwd<false>(w[e], pc.one_shoup);
+        W d;
+        if (sizeof(W) == 4) {
+          // 32-bit words hold primes up to 2^30: m + 4q would pass 2^32, so the transform comes below 2q first
+          d = m[e] + pc.q2 - csub<W>(x, pc.q2);
+        } else {
+          d = m[e] + (pc.q2 + pc.q2) - x;  // x < 4q: positive, and the Shoup product takes any word
+        }
+        d = csub<W>(mul_shoup_lazy<W>(d, f, fs, pc.q), pc.q);
+        if (ap != nullptr) d = add_mod<W>(d, a[e], pc.q);
+        w[e] = d;
       }
-      d = csub<W>(mul_shoup_lazy<W>(d, factor[b], factor_shoup[b], pc.q), pc.q);
-      if (ap != nullptr) d = add_mod<W>(d, a[e], pc.q);
-      w[e] = d;
     }
   }
 };
@@ -781,7 +805,6 @@ struct SudEpilogue {
 // residue per prime of the context, indexed by the entry's prime.
 template <typename W>
 struct PtrSudEpilogue {
-  static constexpr bool kCanonicalInput = false;
   static constexpr bool kHasOperands = true;
   const W* const* ins;
   const W* factors;
@@ -796,11 +819,11 @@ struct PtrSudEpilogue {
     for (int e = 0; e < RowVec<W>::kWords; e++) o.m[e] = ins[2 * b][idx0 + e];  // caller's limbs may be unaligned
     return o;
   }
-  template <int kWords>
-  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int /*b*/, int /*idx0*/, uint32_t pi,
-                                            const PrimeConst<W>& pc) const {
+  template <int kMode, int kWords>
+  __device__ __forceinline__ void apply_vec(W (&w)[kWords], const Operands& o, int /*b*/, int /*idx0*/, uint32_t pi, const PrimeConst<W>& pc,
+                                            const Arith<W, kMode>& ar) const {
 #pragma unroll
-    for (int e = 0; e < kWords; e++) w[e] = apply(w[e], o.m[e], pi, pc);
+    for (int e = 0; e < kWords; e++) w[e] = apply(ar.template finish_fwd<false>(w[e], pc.one_shoup), o.m[e], pi, pc);
   }
   __device__ __forceinline__ W apply(W x, W m, uint32_t pi, const PrimeConst<W>& pc) const {
     // x < 4q and m < q: bring the difference to [0, q) before the Barrett product
@@ -883,7 +906,7 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, con
   if constexpr (kStage) radix16_fwd<W, false, kMode, kTwLane, kFpFwdL3>(x, buf.tw.lane[r] + u, 0u, ar);
   else radix16_fwd<W, true, kMode, kTwLane, kFpFwdL3>(x, twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
 #pragma unroll
-  for (int j = 0; j < 16; j++) x[j] = ar.template finish_fwd<Epilogue::kCanonicalInput>(x[j], pc.one_shoup);
+  for (int j = 0; j < 16; j++) x[j] = ar.template finish_fwd<Epilogue::kCanonical>(x[j], pc.one_shoup);
   // own 16 words -> swizzled vectors -> coalesced vectors
   __syncwarp();  // a row's 16 threads share a warp; no other warp touches its staging rows
   Vec* vrow = reinterpret_cast<Vec*>(tile + r * kRowPitch);  // same private region as the exchange rows

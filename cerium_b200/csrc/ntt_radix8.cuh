@@ -371,8 +371,8 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
     for (int v = 0; v < kVecs; v++) {
       W w[RV::kWords];
 #pragma unroll
-      for (int e = 0; e < RV::kWords; e++) w[e] = ar.template finish_fwd<Epilogue::kCanonicalInput>(x[4 * k + v * RV::kWords + e], pc.one_shoup);
-      epi.apply_vec(w, ops[k][v], b, at + v * RV::kWords, pi, pc);
+      for (int e = 0; e < RV::kWords; e++) w[e] = x[4 * k + v * RV::kWords + e];
+      epi.apply_vec(w, ops[k][v], b, at + v * RV::kWords, pi, pc, ar);
 #pragma unroll
       for (int e = 0; e < RV::kWords; e++) o.v[v * RV::kWords + e] = w[e];
     }
