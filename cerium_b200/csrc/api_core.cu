@@ -477,29 +477,24 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
   return CERIUM_OK;
 }
 
-// Kernel of a batch: fragments in registers up to the number of steps they fit for, then the way outputs are finished.
+// Kernel of a batch: fragments in registers up to the number of steps they fit for, then the way outputs are finished.  half: the
+// inputs end in the first half of the last step.
 template <typename W, bool kPrepare>
-static auto bconv_mma_pick(int steps, int finish) -> decltype(&bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>) {
-  if constexpr (sizeof(W) == 8) {
-    if (finish == kMmaBig) return bconv_mma_kernel<W, 0, kMmaBig, kPrepare>;
-    if (finish <= kMmaLazyAdd && !kPrepare) {
-      const bool add = finish == kMmaLazyAdd;
-      if (steps == 1) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false> : bconv_mma_kernel<W, 1, kMmaLazy, false>;
-      if (steps == 2) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false> : bconv_mma_kernel<W, 2, kMmaLazy, false>;
-    }
-    if (steps == 1) return bconv_mma_kernel<W, 1, kMmaGeneral, kPrepare>;
-    if (steps == 2) return bconv_mma_kernel<W, 2, kMmaGeneral, kPrepare>;
-  } else {
-    if (finish <= kMmaLazyAdd && !kPrepare) {
-      const bool add = finish == kMmaLazyAdd;
-      if (steps == 1) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false> : bconv_mma_kernel<W, 1, kMmaLazy, false>;
-      if (steps == 2) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false> : bconv_mma_kernel<W, 2, kMmaLazy, false>;
+static auto bconv_mma_pick(int steps, int finish, bool half) -> decltype(&bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>) {
+  if (sizeof(W) == 8 && finish == kMmaBig) return bconv_mma_kernel<W, 0, sizeof(W) == 8 ? kMmaBig : kMmaGeneral, kPrepare>;
+  if (finish <= kMmaLazyAdd && !kPrepare) {
+    const bool add = finish == kMmaLazyAdd;
+    if (steps == 1 && half) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false, true> : bconv_mma_kernel<W, 1, kMmaLazy, false, true>;
+    if (steps == 1) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false> : bconv_mma_kernel<W, 1, kMmaLazy, false>;
+    if (steps == 2 && half) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false, true> : bconv_mma_kernel<W, 2, kMmaLazy, false, true>;
+    if (steps == 2) return add ? bconv_mma_kernel<W, 2, kMmaLazyAdd, false> : bconv_mma_kernel<W, 2, kMmaLazy, false>;
+    if constexpr (sizeof(W) == 4)
       if (steps == 4) return add ? bconv_mma_kernel<W, 4, kMmaLazyAdd, false> : bconv_mma_kernel<W, 4, kMmaLazy, false>;
-    }
-    if (steps == 1) return bconv_mma_kernel<W, 1, kMmaGeneral, kPrepare>;
-    if (steps == 2) return bconv_mma_kernel<W, 2, kMmaGeneral, kPrepare>;
-    if (steps == 4) return bconv_mma_kernel<W, 4, kMmaGeneral, kPrepare>;
   }
+  if (steps == 1) return bconv_mma_kernel<W, 1, kMmaGeneral, kPrepare>;
+  if (steps == 2) return bconv_mma_kernel<W, 2, kMmaGeneral, kPrepare>;
+  if constexpr (sizeof(W) == 4)
+    if (steps == 4) return bconv_mma_kernel<W, 4, kMmaGeneral, kPrepare>;
   return bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>;
 }
 
@@ -535,28 +530,13 @@ static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int c
       max_groups = std::max(max_groups, bconv_mma_groups<W>(bc->O));
     }
     const int finish = sizeof(W) == 8 && max_i > kMmaPairInputs ? kMmaBig : !lazy ? kMmaGeneral : add ? kMmaLazyAdd : kMmaLazy;
-    auto kfn = prepare ? bconv_mma_pick<W, true>(steps, finish) : bconv_mma_pick<W, false>(steps, finish);
-    // A warp per group of outputs, at most 8 to a CTA.  Stages of a CTA: a long walk spreads what a CTA does first
-    // (fragments, constants, filling the buffers: worth about two stages), whole rounds of CTAs keep the SMs
-    // busy to the end; an SM holds 24 warps of 80 registers a thread, 16 of the kernels that take 128.
+    const bool half = max_i * (int)sizeof(W) <= 32 * steps - 16;
+    auto kfn = prepare ? bconv_mma_pick<W, true>(steps, finish, half) : bconv_mma_pick<W, false>(steps, finish, half);
+    // a warp per group of outputs, at most 8 to a CTA
     const int slices = (max_groups + kMmaMaxWarps - 1) / kMmaMaxWarps, warps = (max_groups + slices - 1) / slices;
     const size_t smem = bconv_mma_smem_bytes<W>(max_i);
-    const bool wide_regs = prepare || (sizeof(W) == 4 && steps == 4);
-    const int resident = std::max(1, std::min((wide_regs ? 16 : 25) / warps, (int)(220 * 1024 / (smem + 1024))));
-    constexpr int kStages = kN / kMmaStage;
-    int stages = 1;
-    double best = 1e30;
-    for (int t = 1; t <= 32; t++) {
-      const double ctas = (double)((kStages + t - 1) / t) * slices * cnt;
-      const double cost = std::ceil(ctas / ((double)resident * ctx->sm_count)) * (t + 2);
-      if (cost < best) {
-        best = cost;
-        stages = t;
-      }
-    }
     if (smem > 48 * 1024) CERIUM_CUDA(allow_smem(kfn, bconv_mma_smem_bytes<W>(kMmaMaxInputs)));
-    CERIUM_LAUNCH(kfn, dim3((kStages + stages - 1) / stages, cnt, slices), 32 * warps, smem, stream, batch, stages,
-                  static_cast<const PrimeConst<W>*>(ctx->d_pcs));
+    CERIUM_LAUNCH(kfn, dim3(kN / kMmaStage, cnt, slices), 32 * warps, smem, stream, batch, static_cast<const PrimeConst<W>*>(ctx->d_pcs));
     first += cnt;
   }
   CERIUM_LAUNCH_CHECK("bconv");

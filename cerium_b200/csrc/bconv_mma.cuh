@@ -12,15 +12,20 @@
 // instructions an output before, 13 inputs of 32-bit words ~35); here an output costs ~13 instructions whatever
 // the number of inputs, beside 14 / 128 of an m16n8k32 product per step of 32 input bytes.
 //
-// Mapping: a CTA owns a run of coefficients of one conversion and stages their input words in shared memory, 128 at a
-// time through three buffers (cp.async: two in flight while one is worked on).  Each of its warps owns a group of
-// outputs and walks over tiles of 8 coefficients.  The 16 rows of a product are two byte planes of 8 outputs (64-bit
-// words) or one plane of 16 (32-bit words; two planes where at most 8 are left), so the accumulators of all planes give
-// a thread every byte of its own (output, coefficient) pairs and nothing is exchanged.  The table's fragments
+// Mapping: a CTA owns kMmaStage coefficients of one conversion and stages their input words in shared memory (cp.async).  Each of
+// its warps owns a group of outputs and walks over tiles of 8 coefficients.  The 16 rows of a product are two byte planes of 8
+// outputs (64-bit words) or one plane of 16 (32-bit words; two planes where at most 8 are left), so the accumulators of all
+// planes give a thread every byte of its own (output, coefficient) pairs and nothing is exchanged.  The table's fragments
 // stay in the warp's registers (kSteps <= 2 for 64-bit words, <= 4 for 32-bit ones, i.e. up to 8 and 32 inputs;
 // beyond that they are read again for every tile), and so do the constants of the thread's outputs.
-// Measured for 7 conversions 5 -> 35 of 64-bit words: warps that read the words from global memory themselves
-// waited for them half of the time (48 us), and 16 outputs to a warp took 152 registers (56 us).
+// Bound by the latencies of product and recombination (tensor pipe 43 % of its cycles, multiply pipe 39 %, issue slots 40 % for 7
+// conversions 5 -> 35 of 64-bit words), so many small CTAs that are in different phases do better than the walk over five to
+// ten stages through three buffers that was here before, whose warps met at a barrier for each stage and whose grid ended in a part of a
+// round: rotation of 35 limbs 275.1 -> 267.6 us, of 51 limbs of 32-bit words 173.3 -> 165.4, multiplication of 30 limbs 242.6 ->
+// 232.9, 12 limbs 99.0 / 98.4 (with the rule of few_ctas, which see).  64 coefficients: 35 limbs 272.0, 256: 268.8; 64 registers instead of 80: 267.5.
+// Where the inputs end in the first 16 bytes of a step the product is taken for those alone (35 limbs 278.7 -> 275.1).
+// Measured before: warps that read the words from global memory themselves waited for them half of the time, and 16 outputs to
+// a warp took 152 registers (56 us against 48).
 // The kernel was first built on tcgen05 (M = 128 coefficients, accumulators in TMEM): with K = 64 the product is over
 // in tens of cycles, and the round through barrier, commit, wait and TMEM load of every 8 outputs left the SM at 43 %
 // of its issue slots: 48 us for 7 conversions 5 -> 35 against 22 us of memory traffic.
@@ -35,8 +40,7 @@
 namespace cerium {
 
 constexpr int kMmaMaxWarps = 8;                   // groups of one CTA
-constexpr int kMmaStage = 128;                    // coefficients staged at a time
-constexpr int kMmaBuffers = 3;
+constexpr int kMmaStage = 128;                    // coefficients of a CTA
 template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
@@ -131,9 +135,10 @@ template <int kFinish>
 __device__ __forceinline__ uint64_t bconv_mma_finish(const uint32_t (&c)[8], const BconvMmaOut<uint64_t>& o) {
   using Sum = std::conditional_t<kFinish == kMmaBig, uint64_t, uint32_t>;
   const Sum a = c[0] + ((Sum)c[1] << 8), b = c[2] + ((Sum)c[3] << 8), cc = c[4] + ((Sum)c[5] << 8), d = c[6] + ((Sum)c[7] << 8);
-  const Sum u = cc + (b >> 16);
-  const uint64_t low = (uint64_t)a + ((uint64_t)(b & 0xffffu) << 16);
-  const uint64_t x = low + ((uint64_t)(u + (d << 16)) << 32);  // modulo 2^64
+  // x modulo 2^64 = low word of `low`, u + 2^16 d above it; pairs of up to kMmaPairInputs inputs leave u the room of the carry
+  const uint64_t low = (uint64_t)a + ((uint64_t)b << 16);
+  const Sum u = cc + (Sum)(low >> 32);
+  const uint64_t x = (uint64_t)(uint32_t)low | (uint64_t)(uint32_t)(u + (d << 16)) << 32;
   if (kFinish <= kMmaLazyAdd) {
     const uint32_t t = (uint32_t)(d + (u >> 16));
     const uint64_t r = x + (uint64_t)__umulhi(t, (uint32_t)o.mu) * o.nq;
@@ -147,7 +152,7 @@ __device__ __forceinline__ uint64_t bconv_mma_finish(const uint32_t (&c)[8], con
     // narrow, more than kMmaPairInputs inputs: x may pass 2^64 (below 2^65), so the bits above 2^32 come from the sums,
     // two fewer of them
     const uint32_t t = o.cls == kMmaWide     ? (uint32_t)(d + (u >> 16))
-                       : kFinish == kMmaBig ? (uint32_t)((u + (d << 16) + (low >> 32)) >> 2)
+                       : kFinish == kMmaBig ? (uint32_t)((u + (d << 16)) >> 2)
                                             : (uint32_t)(x >> 32);
     const int shift = kFinish == kMmaBig && o.cls == kMmaNarrow ? o.shift - 2 : o.shift;  // narrow: at least 7
     r = x + (uint64_t)(__umulhi(t, (uint32_t)o.mu) >> shift) * o.nq;
@@ -170,6 +175,17 @@ __device__ __forceinline__ void mma_u8(uint32_t (&c)[4], const uint4& a, uint32_
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
       : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
+// The first 16 of 32 input bytes alone, with the same fragments.
+__device__ __forceinline__ void mma_u8_half(uint32_t (&c)[4], const uint4& a, uint32_t b0) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a.x), "r"(a.y), "r"(b0));
+}
+__device__ __forceinline__ void mma_u8_half_first(uint32_t (&c)[4], const uint4& a, uint32_t b0) {
+  asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+      : "r"(a.x), "r"(a.y), "r"(b0), "r"(0));
+}
 __device__ __forceinline__ void mma_u8_first(uint32_t (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
       : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
@@ -177,16 +193,16 @@ __device__ __forceinline__ void mma_u8_first(uint32_t (&c)[4], const uint4& a, u
 }
 #endif
 
-// Bytes between the staged limbs of one buffer: a product's lanes read 8 coefficients of 2 limbs (64-bit words, both
+// Bytes between the staged limbs: a product's lanes read 8 coefficients of 2 limbs (64-bit words, both
 // halves) or 4 limbs (32-bit words), which the padding spreads over all 32 banks.
 template <typename W>
 constexpr int kMmaPitch = kMmaStage * (int)sizeof(W) + (sizeof(W) == 8 ? 64 : 32);
 template <typename W>
 __host__ __device__ inline size_t bconv_mma_smem_bytes(int inputs) {
-  return (size_t)kMmaBuffers * inputs * kMmaPitch<W>;
+  return (size_t)inputs * kMmaPitch<W>;
 }
 
-// Byte offset inside a buffer of the 32-bit piece that holds input bytes 4 piece .. 4 piece + 3 of coefficient 0.  A
+// Byte offset of the 32-bit piece that holds input bytes 4 piece .. 4 piece + 3 of coefficient 0.  A
 // piece past the last input is read from the last one: its table entries are zero.
 template <typename W>
 __device__ __forceinline__ int bconv_mma_piece(int piece, int inputs) {
@@ -195,7 +211,7 @@ __device__ __forceinline__ int bconv_mma_piece(int piece, int inputs) {
   return i * kMmaPitch<W> + piece % kPerWord * 4;
 }
 
-// Stages kMmaStage coefficients from `first` on of every input limb into a buffer.
+// Stages kMmaStage coefficients from `first` on of every input limb.
 template <typename W, bool kPrepare>
 __device__ __forceinline__ void bconv_mma_stage(const BconvMmaDesc<W>& d, const PrimeConst<W>* __restrict__ pcs,
                                                 unsigned char* buf, int first) {
@@ -220,9 +236,6 @@ __device__ __forceinline__ void bconv_mma_stage(const BconvMmaDesc<W>& d, const 
 #endif
     }
   }
-#if !defined(CERIUM_EMU)
-  asm volatile("cp.async.commit_group;" ::: "memory");
-#endif
 }
 
 #if defined(CERIUM_EMU)
@@ -241,12 +254,11 @@ inline uint32_t bconv_mma_emulate(const unsigned char* buf, const uint4* frag, i
 }
 #endif
 
-// The CTA's walk over `stages` stages from coefficient `first` on; this warp's group starts at output j0 (none: it only
-// helps to stage).  kPair: the group has at most 8 outputs, its fragments hold two planes.  kSteps = 0: any number of
-// steps, fragments read for every tile.
-template <typename W, int kSteps, int kFinish, bool kPrepare, bool kPair>
-__device__ __forceinline__ void bconv_mma_walk(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, int stages,
-                                               unsigned char* smem, const PrimeConst<W>* __restrict__ pcs) {
+// The CTA's coefficients from `first` on; this warp's group starts at output j0 (none: it only helps to stage).  kPair: the group
+// has at most 8 outputs, its fragments hold two planes.  kSteps = 0: any number of steps, fragments read for every tile.  kHalf: no
+// input has more than 16 bytes in the last step.
+template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf, bool kPair>
+__device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, unsigned char* buf, const PrimeConst<W>* __restrict__ pcs) {
   constexpr int kPlanes = sizeof(W);
   constexpr int kFrags = kPair ? kPlanes / 2 : kPlanes;
   constexpr int kRows = kPair ? 1 : 2;             // outputs of a thread
@@ -277,94 +289,88 @@ __device__ __forceinline__ void bconv_mma_walk(const BconvMmaDesc<W>& d, const u
   for (int s = 0; s < kRegSteps; s++)
 #pragma unroll
     for (int h = 0; h < 2; h++) piece[s][h] = bconv_mma_piece<W>(s * 8 + h * 4 + t, d.I) + g * (int)sizeof(W);
-  grid_dependency_wait();  // the tables above never change; the input limbs below come from the previous kernel
-  const size_t buf_bytes = (size_t)d.I * kMmaPitch<W>;
-  for (int k = 0; k < kMmaBuffers - 1 && k < stages; k++) bconv_mma_stage<W, kPrepare>(d, pcs, smem + k * buf_bytes, first + k * kMmaStage);
-  int in_use = 0;
-#pragma unroll 1
-  for (int k = 0; k < stages; k++) {
+  grid_dependency_wait();
+  if (!few_ctas()) grid_dependency_launch();  // the tables above never change; the input limbs below come from the previous kernel
+  bconv_mma_stage<W, kPrepare>(d, pcs, buf, first);
 #if !defined(CERIUM_EMU)
-    if (k + 1 < stages) asm volatile("cp.async.wait_group %0;" ::"n"(kMmaBuffers - 2) : "memory");
-    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
 #endif
-    __syncthreads();  // stage k is here for everybody, and everybody is done with the buffer that comes next
-    if (k + kMmaBuffers - 1 < stages) {
-      const int into = in_use + kMmaBuffers - 1 < kMmaBuffers ? in_use + kMmaBuffers - 1 : in_use - 1;
-      bconv_mma_stage<W, kPrepare>(d, pcs, smem + into * buf_bytes, first + (k + kMmaBuffers - 1) * kMmaStage);
-    }
-    const unsigned char* buf = smem + in_use * buf_bytes;
-    in_use = in_use + 1 < kMmaBuffers ? in_use + 1 : 0;
-    if (!busy) continue;
+  __syncthreads();
+  if (few_ctas()) grid_dependency_launch();
+  if (!busy) return;
 #if defined(CERIUM_EMU)
-    for (int base = 0; base < kMmaStage; base += kMmaTile)
-      for (int r = 0; r < kRows; r++)
-        for (int e = 0; e < 2; e++) {
-          uint32_t c[kPlanes];
-          for (int m = 0; m < kPlanes; m++)
-            c[m] = bconv_mma_emulate<W>(buf, frag + (size_t)(kPair ? m / 2 : m) * steps * 32, steps, d.I,
-                                        kPair ? g + 8 * (m & 1) : g + 8 * r, base + 2 * t + e);
-          if (live[r]) dst[r][k * kMmaStage + base + e] = bconv_mma_finish<kFinish>(c, o[r]);
-        }
+  for (int base = 0; base < kMmaStage; base += kMmaTile)
+    for (int r = 0; r < kRows; r++)
+      for (int e = 0; e < 2; e++) {
+        uint32_t c[kPlanes];
+        for (int m = 0; m < kPlanes; m++)
+          c[m] = bconv_mma_emulate<W>(buf, frag + (size_t)(kPair ? m / 2 : m) * steps * 32, steps, d.I,
+                                      kPair ? g + 8 * (m & 1) : g + 8 * r, base + 2 * t + e);
+        if (live[r]) dst[r][base + e] = bconv_mma_finish<kFinish>(c, o[r]);
+      }
 #else
 #pragma unroll 2
-    for (int base = 0; base < kMmaStage; base += kMmaTile) {
-      const unsigned char* tile = buf + base * (int)sizeof(W);
-      uint32_t c[kFrags][4];
-      if (kSteps > 0) {
+  for (int base = 0; base < kMmaStage; base += kMmaTile) {
+    const unsigned char* tile = buf + base * (int)sizeof(W);
+    uint32_t c[kFrags][4];
+    if (kSteps > 0) {
 #pragma unroll
-        for (int s = 0; s < kRegSteps; s++) {
-          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(tile + piece[s][0]);
-          const uint32_t b1 = *reinterpret_cast<const uint32_t*>(tile + piece[s][1]);
+      for (int s = 0; s < kRegSteps; s++) {
+        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(tile + piece[s][0]);
+        if (kHalf && s == kRegSteps - 1) {
 #pragma unroll
           for (int p = 0; p < kFrags; p++) {
-            if (s == 0) mma_u8_first(c[p], a[kSteps > 0 ? p : 0][s], b0, b1);
-            else mma_u8(c[p], a[kSteps > 0 ? p : 0][s], b0, b1);
+            if (s == 0) mma_u8_half_first(c[p], a[kSteps > 0 ? p : 0][s], b0);
+            else mma_u8_half(c[p], a[kSteps > 0 ? p : 0][s], b0);
           }
+          continue;
         }
-      } else {
+        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(tile + piece[s][1]);
 #pragma unroll
-        for (int p = 0; p < kFrags; p++) c[p][0] = c[p][1] = c[p][2] = c[p][3] = 0;
-        for (int s = 0; s < steps; s++) {
-          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(tile + bconv_mma_piece<W>(s * 8 + t, d.I) + g * (int)sizeof(W));
-          const uint32_t b1 = *reinterpret_cast<const uint32_t*>(tile + bconv_mma_piece<W>(s * 8 + 4 + t, d.I) + g * (int)sizeof(W));
-#pragma unroll
-          for (int p = 0; p < kFrags; p++) mma_u8(c[p], __ldg(frag + ((size_t)p * steps + s) * 32 + lane), b0, b1);
+        for (int p = 0; p < kFrags; p++) {
+          if (s == 0) mma_u8_first(c[p], a[kSteps > 0 ? p : 0][s], b0, b1);
+          else mma_u8(c[p], a[kSteps > 0 ? p : 0][s], b0, b1);
         }
       }
+    } else {
 #pragma unroll
-      for (int r = 0; r < kRows; r++) {
-        W v[2];
+      for (int p = 0; p < kFrags; p++) c[p][0] = c[p][1] = c[p][2] = c[p][3] = 0;
+      for (int s = 0; s < steps; s++) {
+        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(tile + bconv_mma_piece<W>(s * 8 + t, d.I) + g * (int)sizeof(W));
+        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(tile + bconv_mma_piece<W>(s * 8 + 4 + t, d.I) + g * (int)sizeof(W));
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-          uint32_t bytes[kPlanes];
-#pragma unroll
-          for (int m = 0; m < kPlanes; m++) bytes[m] = kPair ? c[m / 2][2 * (m & 1) + e] : c[kPair ? 0 : m][2 * r + e];
-          v[e] = bconv_mma_finish<kFinish>(bytes, o[r]);
-        }
-        if (live[r]) *reinterpret_cast<Two*>(dst[r] + base) = Two{v[0], v[1]};
+        for (int p = 0; p < kFrags; p++) mma_u8(c[p], __ldg(frag + ((size_t)p * steps + s) * 32 + lane), b0, b1);
       }
     }
 #pragma unroll
-    for (int r = 0; r < kRows; r++) dst[r] += kMmaStage;
-#endif
+    for (int r = 0; r < kRows; r++) {
+      W v[2];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        uint32_t bytes[kPlanes];
+#pragma unroll
+        for (int m = 0; m < kPlanes; m++) bytes[m] = kPair ? c[m / 2][2 * (m & 1) + e] : c[kPair ? 0 : m][2 * r + e];
+        v[e] = bconv_mma_finish<kFinish>(bytes, o[r]);
+      }
+      if (live[r]) *reinterpret_cast<Two*>(dst[r] + base) = Two{v[0], v[1]};
+    }
   }
+#endif
 }
 
-// grid = (ceil(N / (stages_per_cta * 128)), conversions, ceil(groups / warps)), block = 32 * warps, dynamic smem =
-// bconv_mma_smem_bytes of the largest number of inputs.
-template <typename W, int kSteps, int kFinish, bool kPrepare>
+// grid = (N / kMmaStage, conversions, ceil(groups / warps)), block = 32 * warps, dynamic smem = bconv_mma_smem_bytes of the largest
+// number of inputs.
+template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf = false>
 __global__ void __launch_bounds__(32 * kMmaMaxWarps, (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 2 : 3)
-    bconv_mma_kernel(const BconvMmaBatch<W> batch, const int stages_per_cta, const PrimeConst<W>* __restrict__ pcs) {
+    bconv_mma_kernel(const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs) {
   CERIUM_DYN_SMEM(smem);
-  grid_dependency_launch();
   const BconvMmaDesc<W>& d = batch.d[blockIdx.y];
   const int group = blockIdx.z * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const int j0 = group * kMmaRows<W>, stage0 = blockIdx.x * stages_per_cta, first = stage0 * kMmaStage;
-  const int stages = kN / kMmaStage - stage0 < stages_per_cta ? kN / kMmaStage - stage0 : stages_per_cta;
+  const int j0 = group * kMmaRows<W>, first = blockIdx.x * kMmaStage;
   if ((int)(blockIdx.z * (blockDim.x / 32)) * kMmaRows<W> >= d.O) return;
   const uint4* frag = d.table + bconv_mma_entry<W>(group, d.steps);
-  if (sizeof(W) == 8 || d.O - j0 <= 8) bconv_mma_walk<W, kSteps, kFinish, kPrepare, true>(d, frag, j0, first, stages, smem, pcs);
-  else bconv_mma_walk<W, kSteps, kFinish, kPrepare, sizeof(W) == 8>(d, frag, j0, first, stages, smem, pcs);
+  if (sizeof(W) == 8 || d.O - j0 <= 8) bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, true>(d, frag, j0, first, smem, pcs);
+  else bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, sizeof(W) == 8>(d, frag, j0, first, smem, pcs);
 }
 
 }  // namespace cerium

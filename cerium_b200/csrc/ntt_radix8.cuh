@@ -333,6 +333,7 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   LateTwiddles<W> late;
   late_row_load<W, kMode>(late, tw, twr, h);
   grid_dependency_wait();
+  if (!few_ctas()) grid_dependency_launch();
   const W* in = batch.in_limb(b) + (unsigned)(h * 256 + lane);
   W* limb_out = batch.out_limb(b);
   W x[8];
@@ -358,6 +359,7 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   for (int k = 0; k < 2; k++)
 #pragma unroll
     for (int v = 0; v < kVecs; v++) ops[k][v] = epi.load(b, h * 256 + k * 128 + lane * 4 + v * RV::kWords);
+  if (few_ctas()) grid_dependency_launch();
   row_get_quads<W>(row.ex, x);
   late_row_quotients<W, kMode>(late, ar);
   late_fwd<W, kMode, kFpFwdMid, kFpLaneK32>(x, late, ar);
@@ -394,7 +396,6 @@ __global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
     radix8_fwd_rows_kernel(const Batch batch, const Epilogue epi, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                            const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
@@ -412,6 +413,7 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
   LateTwiddles<W> late;
   late_row_load<W, kMode>(late, twi, twri, h);
   grid_dependency_wait();
+  if (!few_ctas()) grid_dependency_launch();
   const W* in = batch.in_limb(b);
   const uint32_t elt = batch.gather_elt();
   const bool wide = quad_aligned(in);
@@ -458,6 +460,7 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = row.ex[raised_pos<W>(j * 32 + lane)];
+  if (few_ctas()) grid_dependency_launch();
   radix8_inv<W, kMode, 0, kFpInvRow1.out>(x, row.tw, 1, ar);
   fp_reduce_masked<W, kMode>(x, kFpInvRow2.exchange, ar);
   W* out = batch.out_limb(b) + (unsigned)(h * 256 + lane);
@@ -470,7 +473,6 @@ __global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
     radix8_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                            const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  grid_dependency_launch();
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
@@ -542,6 +544,7 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
   radix8_quad_sync<kCols>();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(v * 8 + j, c)];
+  if (few_ctas()) grid_dependency_launch();
   LateTwiddles<W> late;
   late_column_load<W>(late, stw, v);
   late_fwd<W, kMode, Loader::kFpBound, 1>(x, late, ar);
@@ -556,12 +559,12 @@ __global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
-  grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(tw_all + (size_t)pi * kN + k);
   grid_dependency_wait();
+  if (!few_ctas()) grid_dependency_launch();
   CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw));
 }
 
@@ -605,6 +608,7 @@ __device__ __forceinline__ void radix8_inv_cols_body(const Batch& batch, const I
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(j * 32 + v, c)];
+  if (few_ctas()) grid_dependency_launch();
   radix8_inv_final<W, kMode, kFpInvCol1.out>(x, stw, last, ar);
   if (sc.add != nullptr) {
     const W a = __ldg(sc.add + b);
@@ -621,12 +625,12 @@ __global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
-  grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the row pass
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(twi_all + (size_t)pi * kN + k);
   grid_dependency_wait();
+  if (!few_ctas()) grid_dependency_launch();
   CERIUM_DISPATCH_ARITH(W, pc, radix8_inv_cols_body, CERIUM_TARGS(kCols, Batch), (batch, sc, b, pc, tile, stw));
 }
 
