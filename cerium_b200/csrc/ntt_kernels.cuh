@@ -54,7 +54,7 @@ constexpr int kSmallBatchPerSm = sizeof(W) == 8 ? 7 : 8;
 // Lane-interleaved level-3 twiddles: [row h (256)][e = 2^t - 1 + g (15)][thread u (16)] pairs per
 // prime; entry = bit-reversed table[((4096 + 16 h + u) << t) + g].
 constexpr int kRowTwPerPrime = 256 * 15 * 16;
-constexpr int kMaxBatch = 512;     // limbs per launch
+constexpr int kMaxBatch = 576;     // limbs per launch: 24 one-limb digits raised to 24 limbs more
 
 // Addressing of a batch of limbs: batch entry b lives at base + pos[b] * stride; its modulus
 // is prime[b] (index into the context's prime list).  Passed by value as a kernel parameter.
