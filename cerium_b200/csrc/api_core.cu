@@ -158,8 +158,10 @@ int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t strea
         for (int b = 0; b < cnt; b++)
           ml.small[b] = (c.src_prime != nullptr && ctx->moduli[c.src_prime[first + b]] < ((uint64_t)1 << 50)) ? 1 : 0;
         launch_fwd_cols<W>(ctx, gb, ml, cnt, stream);
-      } else if (c.lazy_in) {
-        launch_fwd_cols<W>(ctx, cols, LazyLoader<W>{}, cnt, stream);
+      } else if (c.raised_in) {
+        launch_fwd_cols<W>(ctx, cols, LazyLoader<W, kFpRaisedIn>{}, cnt, stream);
+      } else if (c.lowered_in) {
+        launch_fwd_cols<W>(ctx, cols, LazyLoader<W, kFpLoweredIn>{}, cnt, stream);
       } else {
         launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, stream);
       }
@@ -304,7 +306,7 @@ int launch_sud(cerium_context* ctx, const SudCall& c, cudaStream_t stream) {
           launch_fwd_cols<W>(ctx, cols, ld, cnt, stream);
         }
       } else if (c.lazy_src) {
-        launch_fwd_cols<W>(ctx, cols, LazyLoader<W>{}, cnt, stream);
+        launch_fwd_cols<W>(ctx, cols, LazyLoader<W, kFpLoweredIn>{}, cnt, stream);
       } else {
         launch_fwd_cols<W>(ctx, cols, PlainLoader<W>{}, cnt, stream);
       }
@@ -427,7 +429,7 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
     using W = decltype(tag);
     // table entry of (output j, byte plane m, input i, byte k): byte m of factor[j][i] * 2^(8k) mod p_j, laid out as
     // the fragments of an m16n8k32 product (bconv_mma.cuh)
-    bc->steps = (n_in * (int)sizeof(W) + 31) / 32;
+    bc->steps = (std::max(n_in, opt.inputs_together) * (int)sizeof(W) + 31) / 32;
     if (sizeof(W) == 4 && bc->steps == 3) bc->steps = 4;  // kernels with fragments in registers come for 1, 2 and 4 steps
     std::vector<uint4> table(bconv_mma_table_entries<W>(n_out, bc->steps), make_uint4(0, 0, 0, 0));
     unsigned char* bytes = reinterpret_cast<unsigned char*>(table.data());
@@ -501,7 +503,7 @@ static auto bconv_mma_pick(int steps, int finish, bool half) -> decltype(&bconv_
 template <typename W>
 static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int count, cudaStream_t stream) {
   for (int first = 0; first < count;) {
-    // conversions of one launch share the number of steps (which is how they come: the digits of a key switch)
+    // conversions of one launch share the number of steps (the digits of a key switch: BconvOptions::inputs_together)
     BconvMmaBatch<W> batch{};
     const int steps = calls[first].bc->steps;
     bool lazy = true, prepare = false, add = false;

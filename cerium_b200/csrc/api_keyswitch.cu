@@ -241,7 +241,7 @@ int keyswitch_raise(cerium_keyswitch* ks, const void* gathered, cudaStream_t str
     // 3. NTT of every converted limb
     {
       NttCall c{raised, raised, n, n, ks->ntt_pos.data(), ks->ntt_prime.data(), (int)ks->ntt_pos.size()};
-      c.lazy_in = true;  // the converters of step 2 are created with lazy_out
+      c.raised_in = true;  // the converters of step 2 are created with lazy_out
       c.cols_only = rows_left;
       if (int rc = launch_ntt_forward(ctx, c, stream, /*lazy_out=*/true)) return rc;
     }
@@ -618,7 +618,7 @@ int hoisted_rotate_pair(cerium_keyswitch* ks, void* const (&out)[2][2], const vo
     }
     {
       NttCall c{conv[0], conv[0], n, n, pos.data(), prime.data(), 4 * L};
-      c.lazy_in = true;
+      c.lowered_in = true;
       c.cols_only = true;
       if (int rc = launch_ntt_forward(ctx, c, stream)) return rc;
     }
@@ -752,6 +752,7 @@ static int keyswitch_create_impl(cerium_context* ctx, cerium_keyswitch** out, in
     opt.out_pos = out_pos;
     opt.in_pos = in_pos;
     opt.lazy_out = true;  // ModUp outputs go straight into the forward transform
+    opt.inputs_together = alpha;
     cerium_bconv* bc = nullptr;
     rc = create_bconv(ctx, &bc, bconv_mode, in_primes.data(), (int)in_primes.size(), out_primes.data(),
                       (int)out_primes.size(), opt);

@@ -236,6 +236,7 @@ struct BconvOptions {
   std::vector<uint32_t> out_pos;     // output limb slots (empty = 0..O-1)
   std::vector<uint32_t> in_pos;      // input limb slots (empty = 0..I-1)
   bool lazy_out = false;             // outputs feed the forward NTT directly: skip the final corrections
+  int inputs_together = 0;           // most inputs of the conversions that share a launch with this one (0: those of this one)
 };
 
 int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32_t* in_primes, int n_in,
@@ -265,8 +266,9 @@ struct NttCall {
   const uint32_t* src_pos = nullptr;
   // with src_pos: prime index of the modulus the words of entry b are residues of (null: unknown)
   const uint32_t* src_prime = nullptr;
-  // forward transform only: the input words are below 4q instead of canonical
-  bool lazy_in = false;
+  // forward transform only: the input words are what a base conversion with lazy_out left, without a rounding term or with one
+  // (kFpRaisedIn, kFpLoweredIn), instead of canonical
+  bool raised_in = false, lowered_in = false;
   // inverse transform only, not 0: the input limbs are read through the Galois automorphism of this element
   uint32_t in_galois = 0;
   // inverse transform only: the input is the product with the limbs of this stack, which lie as those of `in` do
@@ -304,7 +306,7 @@ struct SudCall {
   void* dst2 = nullptr;
   const void* minuend2 = nullptr;
   const void* addend2 = nullptr;
-  bool lazy_src = false;  // the source words are below 4q instead of canonical
+  bool lazy_src = false;  // the source words are what a base conversion with lazy_out left (kFpLoweredIn) instead of canonical
   bool cols_done = false;  // `work` holds the column pass's results already
   // source re-reduction (only when reduce_src): residues of modulus src_q, optional rounding
   bool reduce_src = false;

@@ -190,8 +190,12 @@ struct Arith<uint64_t, kArithFp> {
     const double c = __dadd_rn(__fma_rn(h, qinv, kFpMagic), -kFpMagic);
     return __dadd_rn(__fma_rn(c, nq, h), l);
   }
-  // quotient of a twiddle by q when the table holds the twiddle alone
+  // quotient of a twiddle by q when the table holds the twiddle alone, and one as good as a tabulated one (within 2^-55 and 2^-100)
   __device__ __forceinline__ W quotient(W w) const { return u(__dmul_rn(d(w), qinv)); }
+  __device__ __forceinline__ W close_quotient(W w) const {
+    const double c = __dmul_rn(d(w), qinv);
+    return u(__fma_rn(__fma_rn(c, nq, d(w)), qinv, c));
+  }
   __device__ __forceinline__ void fwd(W& a, W& b, W w, W wq) const {
     const double r = fp_mulmod(d(b), d(w), d(wq), nq);
     const double x = d(a);
@@ -310,11 +314,14 @@ __host__ __device__ constexpr FpExchange fp_plan_exchange(const FpInvPlan& p, in
 }
 constexpr int kFpInvExchangeMax = 2048;
 
-// bounds along the forward transform: the column pass starts from its loader's bound (canonical
-// words, or lazy ones below 4q) and stores at most kFpFwdMid, from which the row pass starts
-constexpr int kFpLazyIn = 4096;
-constexpr int kFpFwdMid = fp_plan_fwd(fp_plan_fwd(kFpLazyIn).out).out;
-static_assert(fp_plan_fwd(fp_plan_fwd(kFpCanon).out).out <= kFpFwdMid, "the lazy loader is the worst case");
+// bounds along the forward transform: the column pass starts from its loader's bound and stores at most kFpFwdMid, from which the
+// row pass starts, raised digits at most kFpRaisedMid: canonical words, and what a base conversion leaves (bconv_mma.cuh): below
+// 2.3 q, with a rounding term below 3.3 q.  (With 4 q for both the row of a raised digit is reduced twice on its way, so once.)
+constexpr int kFpRaisedIn = 2356, kFpLoweredIn = 3380;
+constexpr int fp_plan_cols(int bin) { return fp_plan_fwd(fp_plan_fwd(bin).out).out; }
+constexpr int fp_max(int a, int b) { return a > b ? a : b; }
+constexpr int kFpRaisedMid = fp_max(fp_plan_cols(kFpCanon), fp_plan_cols(kFpRaisedIn));
+constexpr int kFpFwdMid = fp_max(kFpRaisedMid, fp_plan_cols(kFpLoweredIn));
 constexpr int kFpFwdL3 = fp_plan_fwd(kFpFwdMid).out;
 constexpr int kFpLaneK32 = 3;  // level 3 (lane table) computes its quotients
 static_assert(fp_plan_fwd(kFpFwdL3, kFpLaneK32).out < 8192, "the transform's last values must stay exact integers");
@@ -569,11 +576,12 @@ struct ModLoader {
   }
 };
 
-// Words below 4q, as the ModUp base conversion leaves them for the transform.
-template <typename W>
+// Words as a base conversion leaves them for the transform, kBound / 1024 q at most for primes with double-precision butterflies and
+// below 4q for all.
+template <typename W, int kBound>
 struct LazyLoader {
   static constexpr bool kHasSmall = false;
-  static constexpr int kFpBound = kFpLazyIn;
+  static constexpr int kFpBound = kBound;
   __device__ __forceinline__ W apply(W x, int /*b*/, const PrimeConst<W>& /*pc*/) const { return x; }
 };
 

@@ -73,25 +73,29 @@ __device__ __forceinline__ void quad_store(uint64_t* p, const Quad<uint64_t>& q,
 // Bounds of the Fp butterflies, as fp_plan_fwd and fp_plan_inv have them for four layers.
 // ---------------------------------------------------------------------------------------
 
-// Eight forward layers; the last two compute their quotients when late_k32 is kFpLaneK32.
+// Eight forward layers; k6 and k7: how good the quotients of the last two are (k32 of fp_product_bound).
 struct FpPassPlan {
   bool before[8];
   int out;
 };
-__host__ __device__ constexpr FpPassPlan fp_plan_pass(int bin, int late_k32) {
+__host__ __device__ constexpr FpPassPlan fp_plan_pass(int bin, int k6, int k7) {
   FpPassPlan p{};
   int b = bin;
   for (int t = 0; t < 8; t++) {
     p.before[t] = b > kFpOperandMax;
     if (p.before[t]) b = kFpReduced;
-    b += fp_product_bound(b, t < 6 ? 1 : late_k32);
+    b += fp_product_bound(b, t < 6 ? 1 : t == 6 ? k6 : k7);
   }
   p.out = b;
   return p;
 }
-__host__ __device__ constexpr FpPassPlan fp_plan_row(int bin) { return fp_plan_pass(bin, kFpLaneK32); }
-static_assert(fp_plan_row(kFpFwdMid).out < 8192, "the transform's last values must stay exact integers");
-static_assert(fp_plan_pass(kFpLazyIn, 1).out <= kFpFwdMid && fp_plan_pass(kFpCanon, 1).out <= kFpFwdMid, "what the row pass starts from");
+// A row whose table has the twiddles of the last two layers alone.  kFpCloseK32: twice the error of a tabulated quotient, more than that of
+// Arith::close_quotient, which is enough for seven layers after a reduction (from 4 x 1024 on the last one would want another).
+constexpr int kFpCloseK32 = 2;
+__host__ __device__ constexpr FpPassPlan fp_plan_row(int bin, int k6) { return fp_plan_pass(bin, k6, kFpLaneK32); }
+static_assert(fp_plan_row(kFpFwdMid, kFpCloseK32).out < 8192 && fp_plan_row(kFpRaisedMid, kFpLaneK32).out < 8192, "the transform's last values must stay exact integers");
+static_assert(fp_plan_pass(kFpLoweredIn, 1, 1).out <= kFpFwdMid && fp_plan_pass(kFpRaisedIn, 1, 1).out <= kFpRaisedMid &&
+                  fp_plan_pass(kFpCanon, 1, 1).out <= kFpRaisedMid, "what the row pass starts from");
 
 // Inverse layers of `regs` (4 or 8) registers, each the distance after the one before: fp_plan_inv of that many.
 struct FpInvGroup {
@@ -153,9 +157,9 @@ __device__ __forceinline__ void fp_reduce_masked(W (&x)[8], unsigned mask, const
 
 // Three layers on x[0..7]; layer t pairs (j, j + (4 >> t)) with twiddle (S << t) + (j >> (3 - t)).  kLayer: number of the
 // first one inside the pass.
-template <typename W, int kMode, int kLayer, int kBin = kFpFwdMid>
+template <typename W, int kMode, int kLayer, int kBin>
 __device__ __forceinline__ void radix8_fwd(W (&x)[8], const typename WordTraits<W>::Pair* tw, int S, const Arith<W, kMode>& ar) {
-  constexpr FpPassPlan plan = fp_plan_pass(kBin, 1);  // the first six layers: whatever the last two are
+  constexpr FpPassPlan plan = fp_plan_pass(kBin, 1, 1);  // the first six layers: whatever the last two are
 #pragma unroll
   for (int t = 0; t < 3; t++) {
     const int half = 4 >> t;
@@ -211,10 +215,10 @@ template <typename W>
 struct LateTwiddles {
   W w6[2][2], w7[2][4];
 };
-// Layers 6 and 7 on two groups of four words; k32 = kFpLaneK32: the companions are computed quotients.
-template <typename W, int kMode, int kBin, int kK32>
+// Layers 6 and 7 on two groups of four words.
+template <typename W, int kMode, int kBin, int kK6, int kK7>
 __device__ __forceinline__ void late_fwd(W (&x)[8], const LateTwiddles<W>& l, const Arith<W, kMode>& ar) {
-  constexpr FpPassPlan plan = fp_plan_pass(kBin, kK32);
+  constexpr FpPassPlan plan = fp_plan_pass(kBin, kK6, kK7);
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     if (plan.before[6]) fp_reduce_masked<W, kMode>(x, 0xfu << 4 * k, ar);
@@ -310,7 +314,7 @@ __device__ __forceinline__ void late_row_quotients(LateTwiddles<W>& l, const Ari
   if constexpr (kMode == kArithFp) {
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      l.w6[k][1] = ar.quotient(l.w6[k][0]);
+      l.w6[k][1] = ar.close_quotient(l.w6[k][0]);
       l.w7[k][1] = ar.quotient(l.w7[k][0]), l.w7[k][3] = ar.quotient(l.w7[k][2]);
     }
   }
@@ -344,13 +348,13 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
 #pragma unroll
     for (int v = 0; v < kVecs; v++) epi.prefetch(b, h * 256 + k * 128 + lane * 4 + v * RV::kWords);
   row_twiddles_wait();
-  radix8_fwd<W, kMode, 0>(x, row.tw, 1, ar);
+  radix8_fwd<W, kMode, 0, kFpFwdMid>(x, row.tw, 1, ar);
 #pragma unroll
   for (int j = 0; j < 8; j++) row.ex[raised_pos<W>(j * 32 + lane)] = x[j];
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = row.ex[raised_pos<W>(own + 4 * j)];
-  radix8_fwd<W, kMode, 3>(x, row.tw, 8 + (lane >> 2), ar);
+  radix8_fwd<W, kMode, 3, kFpFwdMid>(x, row.tw, 8 + (lane >> 2), ar);
 #pragma unroll
   for (int j = 0; j < 8; j++) row.ex[raised_pos<W>(own + 4 * j)] = x[j];
   __syncwarp();
@@ -362,7 +366,7 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   if (few_ctas()) grid_dependency_launch();
   row_get_quads<W>(row.ex, x);
   late_row_quotients<W, kMode>(late, ar);
-  late_fwd<W, kMode, kFpFwdMid, kFpLaneK32>(x, late, ar);
+  late_fwd<W, kMode, kFpFwdMid, kFpCloseK32, kFpLaneK32>(x, late, ar);
   const uint32_t selt = epi.scatter_elt();
   const bool wide = quad_aligned(limb_out);
 #pragma unroll
@@ -547,7 +551,7 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
   if (few_ctas()) grid_dependency_launch();
   LateTwiddles<W> late;
   late_column_load<W>(late, stw, v);
-  late_fwd<W, kMode, Loader::kFpBound, 1>(x, late, ar);
+  late_fwd<W, kMode, Loader::kFpBound, 1, 1>(x, late, ar);
 #pragma unroll
   for (int j = 0; j < 8; j++) out[j * 256] = x[j];
 }

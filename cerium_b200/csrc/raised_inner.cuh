@@ -117,16 +117,16 @@ template <typename W, int kMode>
 __device__ __forceinline__ void raised_row(W (&x)[8], W* ex, const RaisedRow<W>& row, const typename WordTraits<W>::Pair* tw, int h,
                                            const Arith<W, kMode>& ar, const PrimeConst<W>& pc) {
   using RV = RowVec<W>;
-  constexpr FpPassPlan plan = fp_plan_row(kFpFwdMid);
+  constexpr FpPassPlan plan = fp_plan_row(kFpRaisedMid, kFpLaneK32);
   const int lane = threadIdx.x & 31;
-  radix8_fwd<W, kMode, 0>(x, row.tw, 1, ar);
+  radix8_fwd<W, kMode, 0, kFpRaisedMid>(x, row.tw, 1, ar);
 #pragma unroll
   for (int j = 0; j < 8; j++) ex[raised_pos<W>(j * 32 + lane)] = x[j];
   __syncwarp();
   const int own = (lane >> 2) * 32 + (lane & 3);
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = ex[raised_pos<W>(own + 4 * j)];
-  radix8_fwd<W, kMode, 3>(x, row.tw, 8 + (lane >> 2), ar);
+  radix8_fwd<W, kMode, 3, kFpRaisedMid>(x, row.tw, 8 + (lane >> 2), ar);
 #pragma unroll
   for (int j = 0; j < 8; j++) ex[raised_pos<W>(own + 4 * j)] = x[j];
   __syncwarp();
