@@ -58,6 +58,7 @@ SIGNATURES = {
                                             C.c_int, _vp]),
     "cerium_resolve2": (C.c_int, [_vp, _vp, _vp, _vp, _vp, _sz, C.c_uint32, C.c_uint32, C.c_int, _vp]),
     "cerium_mod2": (C.c_int, [_vp, _vp, _sz, _vp, _vp, _u32p, C.c_int, _vp]),
+    "cerium_pcg64_uniform": (C.c_int, [_u64p, _u32p, C.c_uint32, _vp, _sz]),
     "cerium_residues": (C.c_int, [_vp, _vp, _sz, _vp, _vp, _u32p, C.c_int, _vp]),
     "cerium_compose_create": (C.c_int, [_vp, C.POINTER(_vp), _u32p, C.c_int]),
     "cerium_compose_destroy": (C.c_int, [_vp]),
