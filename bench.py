@@ -455,9 +455,9 @@ class HMultWorkload(Workload):
         self.host_in[0].copy_(self.a.cpu())
         self.host_in[1].copy_(self.b.cpu())
         self.host_out = torch.empty(self.out.shape, dtype=torch.int64).pin_memory()
-        # tensor; key switch: iNTT pair, NTT columns x2 (576 limbs in two batches), rows with the inner product, iNTT pair,
-        # BConv, SuD pair; then the rescale of both polynomials (iNTT pair, SuD pair) unless it is folded into the ModDown
-        self.gpu_launches_per_step = 1 + (2 + 2 + 1 + 2 + 1 + 2) + (0 if self.rescale_mode == 2 else 4)
+        # tensor; key switch: iNTT pair, NTT columns (576 limbs), rows with the inner product, iNTT pair, BConv, SuD pair;
+        # then the rescale of both polynomials (iNTT pair, SuD pair) unless it is folded into the ModDown
+        self.gpu_launches_per_step = 1 + (2 + 1 + 1 + 2 + 1 + 2) + (0 if self.rescale_mode == 2 else 4)
 
     def step(self):
         s = self.torch.cuda.current_stream().cuda_stream
@@ -767,9 +767,9 @@ class BootstrapWorkload(Workload):
         n = self.ev.count.n
         self.op_counts = dict(n)
         # launches: ModRaise 20; a BSGS stage 5 + 3 * 7 + 6 + 1 + 2 + 8 * 5 + 5; an HMult 10; a conjugation 10;
-        # a rescale 4; every other pass 1, and ModUps that convert their digits in two launches
+        # a rescale 4; every other pass 1
         self.gpu_launches_per_step = (20 * n["mod_raise"] + 80 * n["bsgs"] + 10 * n["hmult"] + 10 + 4 * n["rescale"]
-                                      + n["ewise"] + n["pt_mac"] + n["split_mod_up"])
+                                      + n["ewise"] + n["pt_mac"])
         self.ev.count.n = {}
         self.alg_bytes = 0
 

@@ -158,12 +158,6 @@ class GpuEvaluator:
             self.plans[level] = ks
         return ks
 
-    def _splits(self, level: int) -> int:
-        """1 when a ModUp of this level takes a second conversion launch: digits of two sizes, one more step of 4 limbs
-        in the longer ones."""
-        dnum = self.m.dnum_at(level)
-        return int(level % dnum != 0 and level // dnum % 4 == 0)
-
     def _new(self, level: int) -> Ct:
         t = self.torch
         return Ct(t.empty((level, self.n), dtype=t.int64, device="cuda"), t.empty((level, self.n), dtype=t.int64, device="cuda"), level)
@@ -197,7 +191,6 @@ class GpuEvaluator:
         giants = sum(1 for e in st.giant_elts if e != 1)
         self.count.add("bsgs")
         self.count.add("keyswitch", (st.g - 1) + giants)
-        self.count.add("split_mod_up", (1 + giants) * self._splits(L))
         return out
 
     def conjugate(self, ct: Ct) -> Ct:
@@ -206,7 +199,6 @@ class GpuEvaluator:
         self.plan(L).hrot(out.c0.data_ptr(), out.c1.data_ptr(), ct.c0.data_ptr(), ct.c1.data_ptr(), self.m.conj_key(L).data_ptr(),
                           2 * self.n - 1, self.stream)
         self.count.add("keyswitch")
-        self.count.add("split_mod_up", self._splits(L))
         return out
 
     def hmult(self, a: Ct, b: Ct) -> Ct:
@@ -216,7 +208,6 @@ class GpuEvaluator:
                            self.m.relin_key(L).data_ptr(), 2, self.stream)
         self.count.add("hmult")
         self.count.add("keyswitch")
-        self.count.add("split_mod_up", self._splits(L))
         return out
 
     def _ew(self, op, a: Ct, b: Optional[Ct], scalars=None, level=None) -> Ct:

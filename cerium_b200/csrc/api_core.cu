@@ -51,20 +51,29 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
 template <typename W>
 static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
-// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen.  Columns: beyond these lines the second
-// barrier and the narrow tiles cost more than the shorter chain gives (column pass of 39 limbs in a rotation of 12 limbs 98.9 against
-// 100.7 us; 51 limbs of 32-bit words inverse 173.8 against 175.9).  Rows: fewer instructions decide where the GPU is full (384 limbs
-// forward 187.0 against 187.9 us under the power limit, inverse 163.7 / 167.2; 245 limbs 104.0 / 103.3 and 108.4 / 106.5).
-// Rows of 32-bit words: always inverse (245 limbs 73.6 / 71.1), and forward where the epilogue reads operands (rotation of
-// 51 limbs 176.9 -> 173.9; plain, 245 limbs 66.4 / 69.2).
-constexpr int kRadix8FwdCols = 32, kRadix8InvCols = 40, kRadix8Rows64 = 256;
+// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen, on either side of each line in us.
+//   Columns: beyond the lines the second barrier and the narrow tiles cost more than the shorter chain gives (column pass of 39 limbs
+//   in a rotation of 12 limbs 98.9 with sixteen words, 100.7 with eight).  Of 32-bit words inverse up to the 26 limbs of two
+//   polynomials' 13 extension primes (40 limbs alone 14.1 / 16.3), forward where the words come from a conversion
+//   or a division (rotation of 6 limbs 44.4 / 42.4; alone, 3 limbs 4.7 / 6.9, 20 limbs 9.3 / 9.9).
+//   Rows: fewer instructions decide where the GPU is full (384 limbs forward 187.0 / 187.9 under the power limit, inverse 161.7 / 163;
+//   240 limbs 101.5 / 98.3 and 105.2 / 108.3, 128 limbs inverse 61.0 / 60.3, 32-bit words 240 limbs inverse 67.6 / 67.6, 384 limbs
+//   104.6 / 106.9).  Rows of 32-bit words forward: where the epilogue reads operands (rotation of 51 limbs 176.9 / 173.9; plain, 245
+//   limbs 66.4 / 69.2).
+//   Inverse transforms of 64-bit words in a call of their own find their twiddles in L2, and from 25 to 64 limbs sixteen words are
+//   faster (30 limbs 17.8 / 18.2, 64 limbs 31.7 / 33.2); after a key has gone through L2 they are not (rotation of 35 limbs 286.6 / 282.8).
+template <typename W>
+constexpr int kRadix8InvCols = sizeof(W) == 8 ? 40 : 28;
+constexpr int kRadix8FwdCols = 32, kRadix8FwdRows64 = 256, kRadix8Alone64 = 24;
+template <typename W>
+constexpr int kRadix8InvRows = sizeof(W) == 8 ? 128 : 280;
 
 template <typename W, typename Batch, typename Loader>
 static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loader& loader, int limbs, cudaStream_t stream) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (limbs <= kRadix8FwdCols) {
+  if (limbs <= kRadix8FwdCols && (sizeof(W) == 8 || !Loader::kPlain)) {
     auto kfn = radix8_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
   } else if (small_batch<W>(ctx, limbs)) {
@@ -76,11 +85,11 @@ static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loade
   }
 }
 template <typename W, typename Batch>
-static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvScale<W>& scale, int limbs, cudaStream_t stream) {
+static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvScale<W>& scale, int limbs, cudaStream_t stream, bool alone = false) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (limbs <= kRadix8InvCols) {
+  if (limbs <= (alone && sizeof(W) == 8 ? kRadix8Alone64 : kRadix8InvCols<W>)) {
     auto kfn = radix8_inv_cols_kernel<W, kCols / 2, Batch>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, scale, tw, pcs);
   } else if (small_batch<W>(ctx, limbs)) {
@@ -97,7 +106,7 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (Epilogue::kHasOperands || (sizeof(W) == 8 && limbs <= kRadix8Rows64)) {
+  if (Epilogue::kHasOperands || (sizeof(W) == 8 && limbs <= kRadix8FwdRows64)) {
     auto kfn = radix8_fwd_rows_kernel<W, Batch, Epilogue>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, epi, tw, twr, pcs);
     return;
@@ -115,18 +124,19 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   }
 }
 template <typename W, typename Batch>
-static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, cudaStream_t stream) {
+static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, cudaStream_t stream, bool alone = false) {
   using Pair = typename WordTraits<W>::Pair;
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_inv);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (sizeof(W) == 4 || limbs <= kRadix8Rows64) {
+  if (sizeof(W) == 8 && alone && limbs > kRadix8Alone64 && small_batch<W>(ctx, limbs)) {
+    auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
+  } else if (limbs <= kRadix8InvRows<W>) {
     auto kfn = radix8_inv_rows_kernel<W, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
-    return;
-  }
-  if constexpr (sizeof(W) == 8) {
-    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, Batch>;
+  } else {
+    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
   }
 }
@@ -224,9 +234,9 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t strea
         pb.factor = static_cast<const W*>(c.factor);
         launch_inv_rows<W>(ctx, pb, cnt, stream);
       } else {
-        launch_inv_rows<W>(ctx, sb, cnt, stream);
+        launch_inv_rows<W>(ctx, sb, cnt, stream, c.alone);
       }
-      launch_inv_cols<W>(ctx, sb, sc, cnt, stream);
+      launch_inv_cols<W>(ctx, sb, sc, cnt, stream, c.alone);
     }
     CERIUM_LAUNCH_CHECK("ntt_inverse");
     return CERIUM_OK;
@@ -750,6 +760,7 @@ static int ntt_common(cerium_context* ctx, bool forward, void* out, size_t out_s
   if (int rc = check_stack(in, in_stride, ctx->word_bytes(), "ntt: in")) return rc;
   DeviceGuard guard(ctx->device);
   NttCall c{in, out, in_stride, out_stride, nullptr, prime_idx, count};
+  c.alone = true;
   return forward ? launch_ntt_forward(ctx, c, (cudaStream_t)stream)
                  : launch_ntt_inverse(ctx, c, (cudaStream_t)stream);
 }

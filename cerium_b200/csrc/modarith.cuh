@@ -45,11 +45,12 @@ __device__ __forceinline__ void grid_dependency_wait() {
 
 // Where a kernel lets the next one be placed.  CTAs of the next kernel take the room that they find, so that with a grid that is
 // resident at once they end up where this kernel's CTAs are not, several to an SM, and stay there for their own run: such a grid
-// lets them come only when its work is nearly done.  A larger one, which goes on round after round, lets them come once it has
-// started.  The kernels of a transform with eight words a thread and of the base conversion, at the start -> so: rotations of 8
+// lets them come only when its work is nearly done.  A larger one, which goes on round after round, lets them come at its start.
+// The kernels of a transform with eight words a thread and of the base conversion, always at the start -> so: rotations of 8
 // limbs 74.9 -> 73.3 us, 12 limbs 101.0 -> 94.0, 6 limbs of 32-bit words 44.9 -> 42.8, multiplication of 8 limbs with one-limb digits 108.2 ->
-// 105.3; 35 limbs 268.1 / 267.2 (never early 275.9; late for every grid 268.5), 51 limbs of 32-bit words 165.6 / 165.0 (late 166.8).
-// 1184 CTAs: eight to each of 148 SMs.  Late in the column passes of sixteen words loses (35 limbs 274.1).
+// 105.3; 35 limbs 268.1 / 267.7 (never early 275.9; late for every grid 268.5), 51 limbs of 32-bit words 165.6 / 165.0 (late 166.8).
+// 1184 CTAs: eight to each of 148 SMs.  Late in the column passes of sixteen words loses (35 limbs 274.1); large grids after their wait:
+// equal in a rotation, 3 % lost on 30 to 64 limbs of 64-bit words transformed alone.
 __device__ __forceinline__ bool few_ctas() { return gridDim.x * gridDim.y * gridDim.z <= 1184u; }
 
 // Asynchronous copies to shared memory; a thread sees its own after copy_async_wait<n>: all but the last n groups it committed.

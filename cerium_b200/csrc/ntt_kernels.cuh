@@ -42,13 +42,13 @@ struct NttCfg<uint32_t> {
 
 // Tiles of the two passes: `kCols` columns on 16 kCols threads, or rows of 256 coefficients on 16 threads each.  Batches
 // that do not fill the GPU take smaller tiles (the work is spread over all SMs: 160 tiles of 256 threads on 148 SMs
-// leave twelve with twice the work of the others), and rows of 32-bit words then copy a row's twiddles into shared memory before
+// leave twelve with twice the work of the others), and rows then copy their twiddles into shared memory before
 // they wait for the previous kernel, so that a warp's chain has one memory latency less.  On full launches both cost more than
 // they give: the copies go through the same pipes as the data (71 -> 77 us for 245 limbs).
 constexpr int kRowsPerCta = 16;
 constexpr int kRowsSmall = 4;
 // ... up to this many usual tiles per SM (64 and 74 limbs on 148 SMs).  From there on the usual tiles are as fast or faster
-// (70 limbs of 64-bit words forward 36.9 against 37.7 us; 60 limbs of 32-bit words inverse 21.2 against 19.2)
+// (70 limbs of 64-bit words forward 36.9 against 37.7 us; 30 limbs inverse 20.4 against 17.9, 60 of 32-bit words 21.2 against 19.2)
 template <typename W>
 constexpr int kSmallBatchPerSm = sizeof(W) == 8 ? 7 : 8;
 // Lane-interleaved level-3 twiddles: [row h (256)][e = 2^t - 1 + g (15)][thread u (16)] pairs per
@@ -489,12 +489,13 @@ __device__ __forceinline__ void vec_unpack(const uint4& v, uint32_t* w) { w[0] =
 __device__ __forceinline__ ulonglong2 vec_pack(const uint64_t* w) { return make_ulonglong2(w[0], w[1]); }
 __device__ __forceinline__ uint4 vec_pack(const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); }
 
-// Twiddles of a row pass's rows in shared memory.
+// Twiddles of a row pass's rows in shared memory.  Tables of integer butterflies of 64-bit words are twice as long and
+// stay in global memory.
 template <typename W, int kRows>
 struct RowTwiddles {
   using Pair = typename WordTraits<W>::Pair;
-  static constexpr int kLane = 15 * 16;   // entries of a row's lane table
-  static constexpr int kGroupPitch = 17;  // rows of a warp in different banks
+  static constexpr int kLane = sizeof(W) == 8 ? 8 * 16 : 15 * 16;  // entries of a row's lane table
+  static constexpr int kGroupPitch = 17;                           // rows of a warp in different banks
   Pair lane[kRows][kLane];
   Pair group[kRows][kGroupPitch];
 };
@@ -502,10 +503,6 @@ template <typename W, int kRows, bool kStage>
 struct alignas(16) RowsBuffer {
   W tile[kRows * kRowPitch];
   RowTwiddles<W, kStage ? kRows : 1> tw;
-};
-template <typename W, int kRows>
-struct alignas(16) RowsBuffer<W, kRows, false> {
-  W tile[kRows * kRowPitch];
 };
 
 // Starts the copies of this warp's two rows (h0: first row of the CTA); row_twiddles_wait() before they are used.
@@ -556,6 +553,7 @@ __device__ __forceinline__ void row_twiddles_wait() {
 // What the column pass does with a word it has just read.
 template <typename W>
 struct PlainLoader {
+  static constexpr bool kPlain = true;  // words of the caller, as they are
   static constexpr bool kHasSmall = false;
   static constexpr int kFpBound = kFpCanon;
   __device__ __forceinline__ W apply(W x, int /*b*/, const PrimeConst<W>& /*pc*/) const { return x; }
@@ -565,6 +563,7 @@ struct PlainLoader {
 // the whole base conversion of a one-limb digit (Qhat = 1), fused into the transform's first read.
 template <typename W>
 struct ModLoader {
+  static constexpr bool kPlain = false;
   static constexpr int kFpBound = kFpCanon;
   static constexpr bool kHasSmall = true;
   // small[b] != 0: the words of entry b are below 2^50 (their source prime is), so a prime with
@@ -580,6 +579,7 @@ struct ModLoader {
 // below 4q for all.
 template <typename W, int kBound>
 struct LazyLoader {
+  static constexpr bool kPlain = false;
   static constexpr bool kHasSmall = false;
   static constexpr int kFpBound = kBound;
   __device__ __forceinline__ W apply(W x, int /*b*/, const PrimeConst<W>& /*pc*/) const { return x; }
@@ -596,6 +596,7 @@ constexpr int kSudMaxBatch = 128;
 // (rescale, cerium/compiler/backend/compiler_rescale.cc:262-284).
 template <typename W>
 struct ReduceLoader {
+  static constexpr bool kPlain = false;
   static constexpr bool kHasSmall = false;
   static constexpr int kFpBound = kFpCanon;
   W src_q;
@@ -958,12 +959,13 @@ __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
 // inverse transform
 // ---------------------------------------------------------------------------------------
 
-template <typename W, int kMode, int kRows, typename Batch>
-__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, RowsBuffer<W, kRows, false>& buf,
+template <typename W, int kMode, int kRows, bool kStage, typename Batch>
+__device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, RowsBuffer<W, kRows, kStage>& buf,
                                                   const typename WordTraits<W>::Pair* twi,
                                                   const typename WordTraits<W>::Pair* twri) {
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
+  constexpr bool kStaged = kStage && (sizeof(W) == 4 || kMode == kArithFp);
   W* tile = buf.tile;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
@@ -1016,7 +1018,9 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
     vec_unpack(vrow[row_vec_slot<W>(u * RV::kPerThread + jj)], &x[jj * RV::kWords]);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.enter(x[j]);
-  radix16_inv<W, true, kMode, 0, kTwLane, kFpCanon>(x, twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  if (kStaged) row_twiddles_wait();
+  radix16_inv<W, !kStaged, kMode, 0, kTwLane, kFpCanon>(
+      x, kStaged ? buf.tw.lane[kStaged ? r : 0] + u : twri + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
   if (kMode == kArithFp) fp_reduce_masked<W, kMode>(x, kFpInvRowsExMask, ar);
   __syncwarp();
   W* t_own = trow + (unsigned)(u * 17);  // row_pos(u * 16 + j) = u * 17 + j
@@ -1026,28 +1030,30 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_strided[j * 17];
-  radix16_inv<W, true, kMode, 4, kTwPlain, kFpInvL3>(x, twi, 256u + (uint32_t)h, ar);
+  radix16_inv<W, !kStaged, kMode, 4, kStaged ? kTwGroup : kTwPlain, kFpInvL3>(x, kStaged ? buf.tw.group[kStaged ? r : 0] : twi, 256u + (uint32_t)h, ar);
   W* dcol = dst + u;
 #pragma unroll
   for (int j = 0; j < 16; j++) dcol[j * 16] = x[j];
 }
 
 // Row pass (levels 3 and 2): in -> out; values leave below 2q (strict; 4q for 64-bit words) or below 2^10 q (lazy).
-template <typename W, int kRows, typename Batch>
+template <typename W, int kRows, bool kStage, typename Batch>
 __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
     ntt_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                         const typename WordTraits<W>::Pair* __restrict__ twri_all,
                         const PrimeConst<W>* __restrict__ pcs) {
   using Pair = typename WordTraits<W>::Pair;
-  __shared__ RowsBuffer<W, kRows, false> buf;
+  __shared__ RowsBuffer<W, kRows, kStage> buf;
   grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   const Pair* twi = twi_all + (size_t)pi * kN;
   const Pair* twri = twri_all + (size_t)pi * kRowTwPerPrime;
+  if constexpr (kStage)
+    if (sizeof(W) == 4 || pc.fp_ok != 0) row_twiddles_start(buf.tw, twi, twri, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, CERIUM_TARGS(kRows, Batch), (batch, b, pc, buf, twi, twri));
+  CERIUM_DISPATCH_ARITH(W, pc, ntt_inv_rows_body, CERIUM_TARGS(kRows, kStage, Batch), (batch, b, pc, buf, twi, twri));
 }
 
 // Optional per-limb scalar of the finished inverse transform (exact base conversion wants x * [Qhat^-1] mod q):

@@ -337,7 +337,6 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   LateTwiddles<W> late;
   late_row_load<W, kMode>(late, tw, twr, h);
   grid_dependency_wait();
-  if (!few_ctas()) grid_dependency_launch();
   const W* in = batch.in_limb(b) + (unsigned)(h * 256 + lane);
   W* limb_out = batch.out_limb(b);
   W x[8];
@@ -400,6 +399,7 @@ __global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
     radix8_fwd_rows_kernel(const Batch batch, const Epilogue epi, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                            const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
+  if (!few_ctas()) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
@@ -417,7 +417,6 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
   LateTwiddles<W> late;
   late_row_load<W, kMode>(late, twi, twri, h);
   grid_dependency_wait();
-  if (!few_ctas()) grid_dependency_launch();
   const W* in = batch.in_limb(b);
   const uint32_t elt = batch.gather_elt();
   const bool wide = quad_aligned(in);
@@ -477,6 +476,7 @@ __global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
     radix8_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                            const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
+  if (!few_ctas()) grid_dependency_launch();
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
@@ -563,12 +563,12 @@ __global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
+  if (!few_ctas()) grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(tw_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  if (!few_ctas()) grid_dependency_launch();
   CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw));
 }
 
@@ -629,12 +629,12 @@ __global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
+  if (!few_ctas()) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the row pass
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(twi_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  if (!few_ctas()) grid_dependency_launch();
   CERIUM_DISPATCH_ARITH(W, pc, radix8_inv_cols_body, CERIUM_TARGS(kCols, Batch), (batch, sc, b, pc, tile, stw));
 }
 

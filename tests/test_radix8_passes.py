@@ -1,6 +1,6 @@
-"""Transforms on both sides of the batch sizes where a pass changes from eight words a thread to sixteen (32 limbs forward and 40
-inverse of the column passes, 256 of the row passes of 64-bit words), for every arithmetic, and limbs of 64-bit words that are aligned to
-16 bytes only, whose rows move as pairs of words: exact against the oracle."""
+"""Transforms on both sides of the batch sizes where a pass changes between eight words a thread and sixteen, for every arithmetic (64-bit
+words: 32 limbs and 256 forward, 24, 64 and 128 inverse; 32-bit words: 28 and 280 inverse), and limbs of 64-bit words that are aligned
+to 16 bytes only, whose rows move as pairs of words: exact against the oracle."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,8 @@ def harness(name, word_bits):
     return pc.Harness(backends.EmuBackend() if name == "emu" else backends.CudaBackend(), word_bits, mods)
 
 
-@pytest.mark.parametrize("name,word_bits,count", [("emu", 64, 4), ("emu", 32, 3)] + [gpu("cuda", b, c) for b in (64, 32) for c in (1, 32, 33, 40, 41, 256, 257)])
+@pytest.mark.parametrize("name,word_bits,count", [("emu", 64, 4), ("emu", 32, 3)] + [
+    gpu("cuda", 64, c) for c in (1, 24, 25, 32, 33, 64, 65, 128, 129, 256, 257)] + [gpu("cuda", 32, c) for c in (1, 28, 29, 33, 280, 281)])
 def test_batch_sizes(name, word_bits, count):
     h = harness(name, word_bits)
     idx = [(count + b) % len(h.moduli) for b in range(count)]
