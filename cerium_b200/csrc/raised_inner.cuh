@@ -6,7 +6,7 @@
 // for 24 digits of 24 limbs).
 //
 // Bound by memory: 482 MB for 7 digits on 40 limbs of 64-bit words, 970 MB for 24 digits on 25 (451 MB through DRAM, and
-// 949 with the additions of a multiplication; 102 and 216 us in a profiler, half of the issue slots).  The twiddles of a row serve every digit
+// 950 with the additions of a multiplication; 101 and 204 us in a profiler, half of the issue slots).  The twiddles of a row serve every digit
 // from shared memory (read through L1 for every digit they took the gain away: 147 us for the first shape, the two kernels 143).  A lane keeps 8 words and 16 sums, so that 16 warps fit an SM at 128 registers; with 16 words to a lane
 // it would be 8.  The next digit's row is on its way (cp.async) while one is worked on, and the key rows are asked for before
 // the butterflies that come first.  20 warps at 96 registers spill and are slower (rotation of 35 limbs 315 us against the 301 of then).
