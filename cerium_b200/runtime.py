@@ -23,7 +23,6 @@ equivalent, not byte-identical.  One process drives one GPU; a function compiled
 """
 from __future__ import annotations
 
-import contextlib
 import contextvars
 import ctypes
 import os
@@ -254,16 +253,13 @@ class CKKSEncryptor:
         return torch.empty((rows, self.context.n), dtype=torch.int32, pin_memory=self.context.device.type == "cuda")
 
     # -- sampling ---------------------------------------------------------------------------------------
-    @contextlib.contextmanager
-    def _draws(self):
-        """draw(below, out): fills a contiguous uint32 array with uniform words below `below`, the ones that
-        self.rng.integers would give.  The library draws them where the generator is numpy's default one; other threads that
-        use the generator wait until the draws of this block are done."""
+    def _draw(self, below, out):
+        """Fills a contiguous uint32 array with uniform words below `below`, the ones that self.rng.integers would give.  The
+        library draws them where the generator is numpy's default one.  Its lock is held for the draws alone, as numpy holds it:
+        threads may share the generator, and the copies of one limb do not keep the others waiting."""
         source = self.rng.bit_generator
         if type(source) is not np.random.PCG64:
-            def draw(below, out):
-                out[...] = self.rng.integers(0, below, size=out.shape, dtype=np.uint32)
-            yield draw
+            out[...] = self.rng.integers(0, below, size=out.shape, dtype=np.uint32)
             return
         lib, word = self.context.handle.lib, (1 << 64) - 1
         with source.lock:
@@ -271,21 +267,15 @@ class CKKSEncryptor:
             at, inc = now["state"]["state"], now["state"]["inc"]
             state = (ctypes.c_uint64 * 4)(at >> 64, at & word, inc >> 64, inc & word)
             buffered = (ctypes.c_uint32 * 2)(now["has_uint32"], now["uinteger"])
-
-            def draw(below, out):
-                lib.check(lib.dll.cerium_pcg64_uniform(state, buffered, int(below), out.ctypes.data, out.size))
-            try:
-                yield draw
-            finally:
-                now["state"]["state"] = state[0] << 64 | state[1]
-                now["has_uint32"], now["uinteger"] = buffered[0], buffered[1]
-                source.state = now
+            lib.check(lib.dll.cerium_pcg64_uniform(state, buffered, int(below), out.ctypes.data, out.size))
+            now["state"]["state"] = state[0] << 64 | state[1]
+            now["has_uint32"], now["uinteger"] = buffered[0], buffered[1]
+            source.state = now
 
     def _noise(self) -> np.ndarray:
         """Centred binomial error, 21 coin pairs per coefficient (standard deviation 3.24)."""
         bits = np.empty((2, self.context.n), dtype=np.uint32)
-        with self._draws() as draw:
-            draw(1 << 21, bits)
+        self._draw(1 << 21, bits)
         pop = _bit_count(bits).astype(np.int32)
         return pop[0] - pop[1]
 
@@ -295,11 +285,10 @@ class CKKSEncryptor:
         stage = self._staging(len(idx))
         host = np.empty((len(idx), ctx.n), dtype=np.uint32)
         dev = ctx.torch.empty((len(idx), ctx.n), dtype=ctx.torch.int32, device=ctx.device)
-        with self._draws() as draw:
-            for k, p in enumerate(idx):
-                draw(ctx.moduli[p], host[k])
-                stage[k].numpy().view(np.uint32)[:] = host[k]
-                dev[k].copy_(stage[k], non_blocking=True)
+        for k, p in enumerate(idx):
+            self._draw(ctx.moduli[p], host[k])
+            stage[k].numpy().view(np.uint32)[:] = host[k]
+            dev[k].copy_(stage[k], non_blocking=True)
         return host, dev
 
     def _encrypt(self, key_words, idx, message=None):

@@ -221,6 +221,30 @@ def test_residues_of_integer_valued_doubles(client):
         context.words_ntt(idx, v[:100])
 
 
+def test_the_generator_is_free_while_limbs_are_staged(emu, monkeypatch):
+    """Threads that share an encryptor wait for each other's draws and not for the copies between them."""
+    context, ectx, _enc = emu
+    enc, numpys = runtime.CKKSEncryptor(ectx, 3), np.random.default_rng([3])
+    plain, held = enc._staging, []
+
+    class Stage:
+        def __init__(self, rows):
+            self.rows = plain(rows)
+
+        def __getitem__(self, k):
+            free = enc.rng.bit_generator.lock.acquire(blocking=False)
+            held.append(not free)
+            if free:
+                enc.rng.bit_generator.lock.release()
+            return self.rows[k]
+
+    monkeypatch.setattr(enc, "_staging", Stage)
+    host, _dev = enc._uniform(Q_IDX[:3])
+    assert held and not any(held)
+    assert np.array_equal(host, [numpys.integers(0, PRIMES[p], size=context.n, dtype=np.uint32) for p in Q_IDX[:3]])
+    assert enc.rng.bit_generator.state == numpys.bit_generator.state
+
+
 def test_noise_without_the_bit_count_of_numpy_2(emu, monkeypatch):
     _context, _ectx, enc = emu
     monkeypatch.setattr(enc, "rng", np.random.default_rng(9))
