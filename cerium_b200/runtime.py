@@ -257,8 +257,8 @@ class CKKSEncryptor:
         """Fills a contiguous uint32 array with uniform words below `below`, the ones that self.rng.integers would give.  The
         library draws them where the generator is numpy's default one.  Its lock is held for the draws alone, as numpy holds it:
         threads may share the generator, and the copies of one limb do not keep the others waiting."""
-        source = self.rng.bit_generator
-        if type(source) is not np.random.PCG64:
+        source = self.rng.bit_generator if type(self.rng) is np.random.Generator else None
+        if type(source) is not np.random.PCG64:     # another generator, or one whose draws are its own
             out[...] = self.rng.integers(0, below, size=out.shape, dtype=np.uint32)
             return
         lib, word = self.context.handle.lib, (1 << 64) - 1

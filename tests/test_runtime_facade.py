@@ -245,6 +245,24 @@ def test_the_generator_is_free_while_limbs_are_staged(emu, monkeypatch):
     assert enc.rng.bit_generator.state == numpys.bit_generator.state
 
 
+def test_generators_with_draws_of_their_own(emu):
+    """An encryptor's generator may be anything with numpy's integers()."""
+    context, ectx, _enc = emu
+    enc = runtime.CKKSEncryptor(ectx, 3)
+
+    class Largest:
+        def integers(self, low, high, size, dtype):
+            return np.full(size, high - 1, dtype=dtype)
+
+    class LargestOfNumpy(np.random.Generator):
+        integers = Largest.integers
+
+    for enc.rng in (Largest(), LargestOfNumpy(np.random.PCG64(5))):
+        host, _dev = enc._uniform(Q_IDX[:2])
+        assert np.array_equal(host, np.array([[PRIMES[p] - 1] * context.n for p in Q_IDX[:2]]))
+        assert not enc._noise().any()
+
+
 def test_noise_without_the_bit_count_of_numpy_2(emu, monkeypatch):
     _context, _ectx, enc = emu
     monkeypatch.setattr(enc, "rng", np.random.default_rng(9))
