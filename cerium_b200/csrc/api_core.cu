@@ -439,8 +439,15 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
     using W = decltype(tag);
     // table entry of (output j, byte plane m, input i, byte k): byte m of factor[j][i] * 2^(8k) mod p_j, laid out as
     // the fragments of an m16n8k32 product (bconv_mma.cuh)
-    bc->steps = (std::max(n_in, opt.inputs_together) * (int)sizeof(W) + 31) / 32;
-    if (sizeof(W) == 4 && bc->steps == 3) bc->steps = 4;  // kernels with fragments in registers come for 1, 2 and 4 steps
+    const auto steps_of = [](int inputs) {
+      const int steps = (inputs * (int)sizeof(W) + 31) / 32;
+      return sizeof(W) == 4 && steps == 3 ? 4 : steps;  // kernels with fragments in registers come for 1, 2 and 4 steps
+    };
+    // A step more shares the launch of a longer conversion as long as the fragments stay in registers: digits of 5 and 4 64-bit
+    // limbs (9 limbs in a rotation) 79.8 us apart, 78.5 together; 9 and 8 (33 limbs) 254 apart, 291 together; 32-bit words, 9 and
+    // 8 limbs (25) 87.3 / 85.6, 17 and 16 (33) 110.5 / 107.5.
+    const int together = steps_of(std::max(n_in, opt.inputs_together));
+    bc->steps = together <= kMmaRegSteps<W> ? together : steps_of(n_in);
     std::vector<uint4> table(bconv_mma_table_entries<W>(n_out, bc->steps), make_uint4(0, 0, 0, 0));
     unsigned char* bytes = reinterpret_cast<unsigned char*>(table.data());
     std::vector<BconvMmaOut<W>> outc(n_out);
@@ -513,7 +520,7 @@ static auto bconv_mma_pick(int steps, int finish, bool half) -> decltype(&bconv_
 template <typename W>
 static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int count, cudaStream_t stream) {
   for (int first = 0; first < count;) {
-    // conversions of one launch share the number of steps (the digits of a key switch: BconvOptions::inputs_together)
+    // conversions of one launch share the number of steps (BconvOptions::inputs_together)
     BconvMmaBatch<W> batch{};
     const int steps = calls[first].bc->steps;
     bool lazy = true, prepare = false, add = false;

@@ -44,6 +44,8 @@ constexpr int kMmaStage = 128;                    // coefficients of a CTA
 template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
+template <typename W>
+constexpr int kMmaRegSteps = sizeof(W) == 8 ? 2 : 4;  // most steps whose fragments a warp keeps in registers
 constexpr int kMmaMaxBatch = 24;                  // conversions per launch (descriptors travel as parameters)
 constexpr int kMmaMaxInputs = 64;                 // of a conversion
 constexpr int kMmaPairInputs = 32;                // 64-bit inputs whose plane pairs c + 2^8 c' stay below 2^32:

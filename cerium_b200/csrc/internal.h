@@ -236,7 +236,7 @@ struct BconvOptions {
   std::vector<uint32_t> out_pos;     // output limb slots (empty = 0..O-1)
   std::vector<uint32_t> in_pos;      // input limb slots (empty = 0..I-1)
   bool lazy_out = false;             // outputs feed the forward NTT directly: skip the final corrections
-  int inputs_together = 0;           // most inputs of the conversions that share a launch with this one (0: those of this one)
+  int inputs_together = 0;           // most inputs of the conversions that may share a launch with this one (0: those of this one)
 };
 
 int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32_t* in_primes, int n_in,

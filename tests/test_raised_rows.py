@@ -74,6 +74,22 @@ def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
     ks.close()
 
 
+@pytest.mark.parametrize("word_bits,L,K,dnum,conversions", [(64, 9, 5, 2, 1), (64, 17, 9, 2, 2), (32, 17, 9, 2, 1)])
+def test_digits_of_two_sizes(be, word_bits, L, K, dnum, conversions):
+    """A digit takes a step more to share the launch of a longer one, but not where the longer one's fragments leave the registers
+    (9 limbs of 64-bit words)."""
+    prm = _params(word_bits, L, K, dnum)
+    h = pc.Harness(be, word_bits, prm.moduli)
+    _c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(L), prm)
+    modes = (_capi.BCONV_EXACT, _capi.ROUND_HALF) if word_bits == 64 else (_capi.BCONV_LAZY, _capi.ROUND_FLOOR)
+    ks = _capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, dnum, *modes)
+    d_c1, d_evk, o = h.up(c1), h.up(evk), h.new(2, L, pc.N)
+    ks.apply(h.p(o), h.p(o) + L * pc.N * word_bits // 8, h.p(d_c1), h.p(d_evk))
+    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, prm.q_idx, prm.p_idx, dnum, c1, evk)))
+    assert be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) == 4 + conversions   # two passes each way
+    ks.close()
+
+
 @pytest.mark.parametrize("bits", [28, 32, 33, 34, 50])
 def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     """With integer butterflies asked for, 64-bit words of any prime; the sums of products want 34 bits."""
