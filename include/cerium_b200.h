@@ -124,8 +124,8 @@ CERIUM_API int cerium_ntt_inverse_ptrs(cerium_context *ctx, void *const *outs, c
  * all arrays are DEVICE resident.  Entry b has two inputs: ins[2b] is the minuend (NTT form),
  * ins[2b+1] the coefficient-form limb; outs[b] = (ins[2b] - NTT(ins[2b+1])) * factors[bases[b]] mod q.
  * `factors` has one word per prime of the context (compute_sud_factors layout,
- * cerium/runtime/execution/function.cpp:685-732).  outs[b] may alias either input.  Results are
- * canonical.
+ * cerium/runtime/execution/function.cpp:685-732).  outs[b] may alias ins[2b+1], but not the
+ * minuend, which is read after outs[b] is written.  Results are canonical.
  */
 CERIUM_API int cerium_sud_ptrs(cerium_context *ctx, void *const *outs, const void *const *ins,
                                const uint32_t *bases, size_t num_bases, const void *factors, void *stream);
@@ -220,6 +220,15 @@ CERIUM_API int cerium_mod2(cerium_context *ctx, void *out, size_t out_stride, co
                 const uint32_t *prime_idx, int count, void *stream);
 
 /*
+ * Uniform words of the encryptor's sampling, in HOST memory: `count` words in [0, below) from the PCG64 generator (128-bit
+ * linear congruence, XSL-RR output; O'Neill 2014) whose state and increment are state[0..1] and state[2..3], high words
+ * first.  A 64-bit output serves two 32-bit draws, low half first; buffered[0] != 0 says that buffered[1] is a half still to be
+ * served.  A draw is scaled by multiplication and rejected where that would favour a value (Lemire 2019).  State and
+ * buffer are left where the next draw goes on: the stream of numpy's Generator(PCG64).integers for 32-bit words.
+ */
+CERIUM_API int cerium_pcg64_uniform(uint64_t state[4], uint32_t buffered[2], uint32_t below, uint32_t *out, size_t count);
+
+/*
  * Residues of integer-valued doubles: out[l] = (values + small) mod q_{prime_idx[l]}, coefficient form,
  * canonical.  values is a DEVICE array of N integer-valued doubles of any magnitude, small (may be NULL) a
  * DEVICE array of N integers added to them (encryption noise): the step of the reference's encoder from
@@ -230,15 +239,6 @@ CERIUM_API int cerium_mod2(cerium_context *ctx, void *out, size_t out_stride, co
  * rounded once to the nearest double (infinite past the range of a double).  32-bit contexts; out is a
  * DEVICE array of N doubles.  The handle holds the CRT tables of one prime list.
  */
-/*
- * Uniform words of the encryptor's sampling, in HOST memory: `count` words in [0, below) from the PCG64 generator (128-bit
- * linear congruence, XSL-RR output; O'Neill 2014) whose state and increment are state[0..1] and state[2..3], high words
- * first.  A 64-bit output serves two 32-bit draws, low half first; buffered[0] != 0 says that buffered[1] is a half still to be
- * served.  A draw is scaled by multiplication and rejected where that would favour a value (Lemire 2019).  State and
- * buffer are left where the next draw goes on: the stream of numpy's Generator(PCG64).integers for 32-bit words.
- */
-CERIUM_API int cerium_pcg64_uniform(uint64_t state[4], uint32_t buffered[2], uint32_t below, uint32_t *out, size_t count);
-
 CERIUM_API int cerium_residues(cerium_context *ctx, void *out, size_t out_stride, const double *values,
                                const int32_t *small, const uint32_t *prime_idx, int count, void *stream);
 CERIUM_API int cerium_compose_create(cerium_context *ctx, cerium_compose **out, const uint32_t *prime_idx, int count);
