@@ -22,7 +22,7 @@
 // conversions 5 -> 35 of 64-bit words), so many small CTAs that are in different phases do better than the walk over five to
 // ten stages through three buffers that was here before, whose warps met at a barrier for each stage and whose grid ended in a part of a
 // round: rotation of 35 limbs 275.1 -> 267.6 us, of 51 limbs of 32-bit words 173.3 -> 165.4, multiplication of 30 limbs 242.6 ->
-// 232.9, 12 limbs 99.0 / 98.4 (with the rule of few_ctas, which see).  64 coefficients: 35 limbs 272.0, 256: 268.8; 64 registers instead of 80: 267.5.
+// 232.9, 12 limbs 99.0 / 98.4 (with the next kernel let in late, see grid_dependency_launch).  64 coefficients: 35 limbs 272.0, 256: 268.8; 64 registers instead of 80: 267.5.
 // Where the inputs end in the first 16 bytes of a step the product is taken for those alone (35 limbs 278.7 -> 275.1).
 // Measured before: warps that read the words from global memory themselves waited for them half of the time, and 16 outputs to
 // a warp took 152 registers (56 us against 48).
@@ -44,6 +44,7 @@ constexpr int kMmaStage = 128;                    // coefficients of a CTA
 template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
+constexpr size_t kMmaSmemPerSm = 220 * 1024;      // shared memory for the CTAs of an SM, 1 KB of each the system's
 template <typename W>
 constexpr int kMmaRegSteps = sizeof(W) == 8 ? 2 : 4;  // most steps whose fragments a warp keeps in registers
 constexpr int kMmaMaxBatch = 24;                  // conversions per launch (descriptors travel as parameters)
@@ -260,7 +261,7 @@ inline uint32_t bconv_mma_emulate(const unsigned char* buf, const uint4* frag, i
 // has at most 8 outputs, its fragments hold two planes.  kSteps = 0: any number of steps, fragments read for every tile.  kHalf: no
 // input has more than 16 bytes in the last step.
 template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf, bool kPair>
-__device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, unsigned char* buf, const PrimeConst<W>* __restrict__ pcs) {
+__device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, unsigned char* buf, const PrimeConst<W>* __restrict__ pcs, bool late_next) {
   constexpr int kPlanes = sizeof(W);
   constexpr int kFrags = kPair ? kPlanes / 2 : kPlanes;
   constexpr int kRows = kPair ? 1 : 2;             // outputs of a thread
@@ -291,14 +292,14 @@ __device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const 
   for (int s = 0; s < kRegSteps; s++)
 #pragma unroll
     for (int h = 0; h < 2; h++) piece[s][h] = bconv_mma_piece<W>(s * 8 + h * 4 + t, d.I) + g * (int)sizeof(W);
-  grid_dependency_wait();
-  if (!few_ctas()) grid_dependency_launch();  // the tables above never change; the input limbs below come from the previous kernel
+  grid_dependency_wait();  // the tables above never change; the input limbs below come from the previous kernel
+  if (!late_next) grid_dependency_launch();
   bconv_mma_stage<W, kPrepare>(d, pcs, buf, first);
 #if !defined(CERIUM_EMU)
   asm volatile("cp.async.wait_all;" ::: "memory");
 #endif
   __syncthreads();
-  if (few_ctas()) grid_dependency_launch();
+  if (late_next) grid_dependency_launch();
   if (!busy) return;
 #if defined(CERIUM_EMU)
   for (int base = 0; base < kMmaStage; base += kMmaTile)
@@ -360,19 +361,23 @@ __device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const 
 #endif
 }
 
+// Warps that an SM holds: of 128 registers a thread or of 80.
+template <typename W, int kSteps, bool kPrepare>
+constexpr int kMmaWarpsPerSm = (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 16 : 24;
+
 // grid = (N / kMmaStage, conversions, ceil(groups / warps)), block = 32 * warps, dynamic smem = bconv_mma_smem_bytes of the largest
 // number of inputs.
 template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf = false>
-__global__ void __launch_bounds__(32 * kMmaMaxWarps, (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 2 : 3)
-    bconv_mma_kernel(const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs) {
+__global__ void __launch_bounds__(32 * kMmaMaxWarps, kMmaWarpsPerSm<W, kSteps, kPrepare> / kMmaMaxWarps)
+    bconv_mma_kernel(const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
   CERIUM_DYN_SMEM(smem);
   const BconvMmaDesc<W>& d = batch.d[blockIdx.y];
   const int group = blockIdx.z * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int j0 = group * kMmaRows<W>, first = blockIdx.x * kMmaStage;
   if ((int)(blockIdx.z * (blockDim.x / 32)) * kMmaRows<W> >= d.O) return;
   const uint4* frag = d.table + bconv_mma_entry<W>(group, d.steps);
-  if (sizeof(W) == 8 || d.O - j0 <= 8) bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, true>(d, frag, j0, first, smem, pcs);
-  else bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, sizeof(W) == 8>(d, frag, j0, first, smem, pcs);
+  if (sizeof(W) == 8 || d.O - j0 <= 8) bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, true>(d, frag, j0, first, smem, pcs, late_next);
+  else bconv_mma_group<W, kSteps, kFinish, kPrepare, kHalf, sizeof(W) == 8>(d, frag, j0, first, smem, pcs, late_next);
 }
 
 }  // namespace cerium

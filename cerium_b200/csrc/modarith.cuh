@@ -32,6 +32,18 @@ namespace cerium {
 // being placed; grid_dependency_wait() returns once every earlier kernel of the stream has
 // completed and its writes are visible.  EVERY kernel must call the wait before it touches a
 // buffer another kernel may have written or may still read.
+//
+// When to let the next kernel in: its CTAs take the room that they find, so let in by a grid that leaves some SMs empty, or while a
+// grid's last CTAs run, they end up several to an SM and stay there for their own run.  Grids that are resident at once, and kernels
+// before small CTAs, let them in when their own work is nearly done; a grid that goes on round after round at its start.
+//   Rows with eight words: late where all CTAs are resident.  At the start, 32-bit words: 5 limbs inverse 4.9 -> 6.2 us, division of
+//   10 limbs 6.8 -> 9.0; late for every grid: 22 limbs inverse 14.36 -> 14.73, rotation of 27 limbs of 32-bit words 95.9 -> 97.3.
+//   Forward columns with eight words: the same line.  Late up to 37 limbs, whatever an SM holds, lost 3 to 5 % from 19 limbs on (32 limbs
+//   alone 19.0 -> 18.3, a division 22.7 -> 21.8, rotation of 10 limbs 86.0 -> 84.5).
+//   Base conversion: the same line.  After its wait: rotation of 9 limbs of 32-bit words 47.1 -> 47.5, of 4 limbs with 4 extension limbs
+//   28.8 -> 32.4; late for every grid: 30 limbs 211.9 -> 213.5, 35 limbs 265.5 -> 266.7.
+//   Inverse columns with eight words: late for every grid, small CTAs of a conversion come after them (at the start: rotation of 9
+//   limbs of 32-bit words 47.3 -> 52.7; late where they are resident: 51.5).
 __device__ __forceinline__ void grid_dependency_launch() {
 #if !defined(CERIUM_EMU)
   asm volatile("griddepcontrol.launch_dependents;");
@@ -42,16 +54,6 @@ __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 #endif
 }
-
-// Where a kernel lets the next one be placed.  CTAs of the next kernel take the room that they find, so that with a grid that is
-// resident at once they end up where this kernel's CTAs are not, several to an SM, and stay there for their own run: such a grid
-// lets them come only when its work is nearly done.  A larger one, which goes on round after round, lets them come at its start.
-// The kernels of a transform with eight words a thread and of the base conversion, always at the start -> so: rotations of 8
-// limbs 74.9 -> 73.3 us, 12 limbs 101.0 -> 94.0, 6 limbs of 32-bit words 44.9 -> 42.8, multiplication of 8 limbs with one-limb digits 108.2 ->
-// 105.3; 35 limbs 268.1 / 267.7 (never early 275.9; late for every grid 268.5), 51 limbs of 32-bit words 165.6 / 165.0 (late 166.8).
-// 1184 CTAs: eight to each of 148 SMs.  Late in the column passes of sixteen words loses (35 limbs 274.1); large grids after their wait:
-// equal in a rotation, 3 % lost on 30 to 64 limbs of 64-bit words transformed alone.
-__device__ __forceinline__ bool few_ctas() { return gridDim.x * gridDim.y * gridDim.z <= 1184u; }
 
 // Asynchronous copies to shared memory; a thread sees its own after copy_async_wait<n>: all but the last n groups it committed.
 template <int kBytes>

@@ -323,12 +323,13 @@ __device__ __forceinline__ void late_row_quotients(LateTwiddles<W>& l, const Ari
 // ---------------------------------------------------------------------------------------
 // row passes: a warp has one row
 // ---------------------------------------------------------------------------------------
-constexpr int kRadix8Rows = 4;  // of a CTA
+constexpr int kRadix8Rows = 4;                      // of a CTA
+constexpr int kRadix8RowsPerSm = 32 / kRadix8Rows;  // CTAs that an SM holds: 32 warps of 64 registers a thread
 
 template <typename W, int kMode, typename Batch, typename Epilogue>
 __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const Epilogue& epi, int b, uint32_t pi, const PrimeConst<W>& pc,
                                                      Radix8Row<W>& row, const typename WordTraits<W>::Pair* tw,
-                                                     const typename WordTraits<W>::Pair* twr, int h) {
+                                                     const typename WordTraits<W>::Pair* twr, int h, bool late_next) {
   using RV = RowVec<W>;
   constexpr int kVecs = 4 / RV::kWords;  // 16-byte vectors of a group of four words
   const Arith<W, kMode> ar(pc);
@@ -362,7 +363,7 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   for (int k = 0; k < 2; k++)
 #pragma unroll
     for (int v = 0; v < kVecs; v++) ops[k][v] = epi.load(b, h * 256 + k * 128 + lane * 4 + v * RV::kWords);
-  if (few_ctas()) grid_dependency_launch();
+  if (late_next) grid_dependency_launch();
   row_get_quads<W>(row.ex, x);
   late_row_quotients<W, kMode>(late, ar);
   late_fwd<W, kMode, kFpFwdMid, kFpCloseK32, kFpLaneK32>(x, late, ar);
@@ -393,24 +394,24 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   }
 }
 
-// grid = (256 / kRadix8Rows, limbs), block = 32 kRadix8Rows.
+// grid = (256 / kRadix8Rows, limbs), block = 32 kRadix8Rows.  late_next (here and below): see grid_dependency_launch.
 template <typename W, typename Batch, typename Epilogue>
-__global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
+__global__ void __launch_bounds__(32 * kRadix8Rows, kRadix8RowsPerSm)
     radix8_fwd_rows_kernel(const Batch batch, const Epilogue epi, const typename WordTraits<W>::Pair* __restrict__ tw_all,
-                           const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs) {
+                           const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  if (!few_ctas()) grid_dependency_launch();
+  if (!late_next) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_rows_body, CERIUM_TARGS(Batch, Epilogue),
-                        (batch, epi, b, pi, pc, rows[warp], tw_all + (size_t)pi * kN, twr_all + (size_t)pi * kRowTwPerPrime, h));
+                        (batch, epi, b, pi, pc, rows[warp], tw_all + (size_t)pi * kN, twr_all + (size_t)pi * kRowTwPerPrime, h, late_next));
 }
 
 template <typename W, int kMode, typename Batch>
 __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, Radix8Row<W>& row,
-                                                     const typename WordTraits<W>::Pair* twi, const typename WordTraits<W>::Pair* twri, int h) {
+                                                     const typename WordTraits<W>::Pair* twi, const typename WordTraits<W>::Pair* twri, int h, bool late_next) {
   const Arith<W, kMode> ar(pc);
   const int lane = threadIdx.x & 31, own = (lane >> 2) * 32 + (lane & 3);
   radix8_row_twiddles<W>(row, twi, h);
@@ -463,7 +464,7 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = row.ex[raised_pos<W>(j * 32 + lane)];
-  if (few_ctas()) grid_dependency_launch();
+  if (late_next) grid_dependency_launch();
   radix8_inv<W, kMode, 0, kFpInvRow1.out>(x, row.tw, 1, ar);
   fp_reduce_masked<W, kMode>(x, kFpInvRow2.exchange, ar);
   W* out = batch.out_limb(b) + (unsigned)(h * 256 + lane);
@@ -472,22 +473,28 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
 }
 
 template <typename W, typename Batch>
-__global__ void __launch_bounds__(32 * kRadix8Rows, 32 / kRadix8Rows)
+__global__ void __launch_bounds__(32 * kRadix8Rows, kRadix8RowsPerSm)
     radix8_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
-                           const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs) {
+                           const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  if (!few_ctas()) grid_dependency_launch();
+  if (!late_next) grid_dependency_launch();
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   CERIUM_DISPATCH_ARITH(W, pc, radix8_inv_rows_body, CERIUM_TARGS(Batch),
-                        (batch, b, pc, rows[warp], twi_all + (size_t)pi * kN, twri_all + (size_t)pi * kRowTwPerPrime, h));
+                        (batch, b, pc, rows[warp], twi_all + (size_t)pi * kN, twri_all + (size_t)pi * kRowTwPerPrime, h, late_next));
 }
 
 // ---------------------------------------------------------------------------------------
 // column passes: 32 threads have a column, a CTA kCols adjacent ones
 // ---------------------------------------------------------------------------------------
+
+// CTAs that an SM holds: 256 threads of 64 registers, 512 of 40 (32-bit words forward) or 64
+template <typename W>
+constexpr int kRadix8FwdColsPerSm = sizeof(W) == 8 ? 4 : 3;
+template <typename W>
+constexpr int kRadix8InvColsPerSm = sizeof(W) == 8 ? 4 : 2;
 
 // Rows of the tile whose words share a bank lie eight apart in one of the three patterns (rows v * 8 + j of neighbouring
 // threads v): bits 3 and 4 of the row's number go into the lowest ones.
@@ -514,7 +521,7 @@ __device__ __forceinline__ void late_column_load(LateTwiddles<W>& l, const typen
 
 template <typename W, int kMode, int kCols, typename Batch, typename Loader>
 __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const Loader& loader, int b, const PrimeConst<W>& pc, W* tile,
-                                                     const typename WordTraits<W>::Pair* stw) {
+                                                     const typename WordTraits<W>::Pair* stw, bool late_next) {
   const Arith<W, kMode> ar(pc);
   const int c = threadIdx.x % kCols, v = threadIdx.x / kCols;
   const int col = blockIdx.x * kCols + c, own = (v >> 2) * 32 + (v & 3);
@@ -548,7 +555,7 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
   radix8_quad_sync<kCols>();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(v * 8 + j, c)];
-  if (few_ctas()) grid_dependency_launch();
+  if (late_next) grid_dependency_launch();
   LateTwiddles<W> late;
   late_column_load<W>(late, stw, v);
   late_fwd<W, kMode, Loader::kFpBound, 1, 1>(x, late, ar);
@@ -558,18 +565,18 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
 
 // grid = (256 / kCols, limbs), block = 32 kCols.
 template <typename W, int kCols, typename Batch, typename Loader>
-__global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
+__global__ void __launch_bounds__(kCols * 32, kRadix8FwdColsPerSm<W>)
     radix8_fwd_cols_kernel(const Batch batch, const Loader loader, const typename WordTraits<W>::Pair* __restrict__ tw_all,
-                           const PrimeConst<W>* __restrict__ pcs) {
+                           const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
-  if (!few_ctas()) grid_dependency_launch();
+  if (!late_next) grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(tw_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw));
+  CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw, late_next));
 }
 
 template <typename W, int kMode, int kCols, typename Batch>
@@ -612,7 +619,7 @@ __device__ __forceinline__ void radix8_inv_cols_body(const Batch& batch, const I
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(j * 32 + v, c)];
-  if (few_ctas()) grid_dependency_launch();
+  grid_dependency_launch();
   radix8_inv_final<W, kMode, kFpInvCol1.out>(x, stw, last, ar);
   if (sc.add != nullptr) {
     const W a = __ldg(sc.add + b);
@@ -624,12 +631,11 @@ __device__ __forceinline__ void radix8_inv_cols_body(const Batch& batch, const I
 }
 
 template <typename W, int kCols, typename Batch>
-__global__ void __launch_bounds__(kCols * 32, 1024 / (kCols * 32))
+__global__ void __launch_bounds__(kCols * 32, kRadix8InvColsPerSm<W>)
     radix8_inv_cols_kernel(const Batch batch, const InvScale<W> sc, const typename WordTraits<W>::Pair* __restrict__ twi_all,
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
-  if (!few_ctas()) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the row pass
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
