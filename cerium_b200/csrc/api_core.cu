@@ -51,8 +51,6 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
 template <typename W>
 static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
-// Whether a grid is resident at once: `limbs` times `ctas` CTAs, of which an SM holds `per_sm`.
-static bool resident(const cerium_context* ctx, int limbs, int ctas, int per_sm) { return limbs * ctas <= per_sm * ctx->sm_count; }
 // Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen, on either side of each line in us.
 //   Columns: beyond the lines the second barrier and the narrow tiles cost more than the shorter chain gives (column pass of 39 limbs
 //   in a rotation of 12 limbs 98.9 with sixteen words, 100.7 with eight).  Of 32-bit words inverse up to the 26 limbs of two
@@ -77,7 +75,7 @@ static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loade
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
   if (limbs <= kRadix8FwdCols && (sizeof(W) == 8 || !Loader::kPlain)) {
     auto kfn = radix8_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
-    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs, resident(ctx, limbs, 512 / kCols, kRadix8FwdColsPerSm<W>));
+    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
   } else if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, loader, tw, pcs);
@@ -110,7 +108,7 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
   if (Epilogue::kHasOperands || (sizeof(W) == 8 && limbs <= kRadix8FwdRows64)) {
     auto kfn = radix8_fwd_rows_kernel<W, Batch, Epilogue>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, epi, tw, twr, pcs, resident(ctx, limbs, 256 / kRadix8Rows, kRadix8RowsPerSm));
+    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, epi, tw, twr, pcs);
     return;
   }
   if constexpr (!Epilogue::kHasOperands) {
@@ -136,7 +134,7 @@ static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, 
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
   } else if (limbs <= kRadix8InvRows<W>) {
     auto kfn = radix8_inv_rows_kernel<W, Batch>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs, resident(ctx, limbs, 256 / kRadix8Rows, kRadix8RowsPerSm));
+    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
   } else {
     auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
@@ -557,10 +555,11 @@ static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int c
     const int slices = (max_groups + kMmaMaxWarps - 1) / kMmaMaxWarps, warps = (max_groups + slices - 1) / slices;
     const size_t smem = bconv_mma_smem_bytes<W>(max_i);
     if (smem > 48 * 1024) CERIUM_CUDA(allow_smem(kfn, bconv_mma_smem_bytes<W>(kMmaMaxInputs)));
-    const int warps_per_sm = sizeof(W) == 4 && steps == kMmaRegSteps<W> ? kMmaWarpsPerSm<W, kMmaRegSteps<W>, true> : prepare ? kMmaWarpsPerSm<W, 0, true> : kMmaWarpsPerSm<W, 0, false>;
+    const int warps_per_sm = prepare || (sizeof(W) == 4 && steps == kMmaRegSteps<W>) ? kMmaWarpsPerSm<W, 0, true> : kMmaWarpsPerSm<W, 0, false>;
     const int per_sm = std::min(warps_per_sm / warps, (int)(kMmaSmemPerSm / (smem + 1024)));
-    CERIUM_LAUNCH(kfn, dim3(kN / kMmaStage, cnt, slices), 32 * warps, smem, stream, batch, static_cast<const PrimeConst<W>*>(ctx->d_pcs),
-                  resident(ctx, cnt * slices, kN / kMmaStage, per_sm));
+    const bool late = kN / kMmaStage * cnt * slices <= per_sm * ctx->sm_count;  // all CTAs are resident
+    CERIUM_LAUNCH(kfn, dim3(kN / kMmaStage, cnt, slices), 32 * warps, smem, stream, late, batch,
+                  static_cast<const PrimeConst<W>*>(ctx->d_pcs));
     first += cnt;
   }
   CERIUM_LAUNCH_CHECK("bconv");

@@ -257,6 +257,10 @@ inline uint32_t bconv_mma_emulate(const unsigned char* buf, const uint4* frag, i
 }
 #endif
 
+// Warps that an SM holds: of 128 registers a thread or of 80.
+template <typename W, int kSteps, bool kPrepare>
+constexpr int kMmaWarpsPerSm = (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 16 : 24;
+
 // The CTA's coefficients from `first` on; this warp's group starts at output j0 (none: it only helps to stage).  kPair: the group
 // has at most 8 outputs, its fragments hold two planes.  kSteps = 0: any number of steps, fragments read for every tile.  kHalf: no
 // input has more than 16 bytes in the last step.
@@ -361,15 +365,11 @@ __device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const 
 #endif
 }
 
-// Warps that an SM holds: of 128 registers a thread or of 80.
-template <typename W, int kSteps, bool kPrepare>
-constexpr int kMmaWarpsPerSm = (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 16 : 24;
-
 // grid = (N / kMmaStage, conversions, ceil(groups / warps)), block = 32 * warps, dynamic smem = bconv_mma_smem_bytes of the largest
-// number of inputs.
+// number of inputs.  late_next: see grid_dependency_launch.
 template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf = false>
 __global__ void __launch_bounds__(32 * kMmaMaxWarps, kMmaWarpsPerSm<W, kSteps, kPrepare> / kMmaMaxWarps)
-    bconv_mma_kernel(const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
+    bconv_mma_kernel(const bool late_next, const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs) {
   CERIUM_DYN_SMEM(smem);
   const BconvMmaDesc<W>& d = batch.d[blockIdx.y];
   const int group = blockIdx.z * (blockDim.x / 32) + (threadIdx.x >> 5);

@@ -42,11 +42,21 @@ namespace cerium {
 //   alone 19.0 -> 18.3, a division 22.7 -> 21.8, rotation of 10 limbs 86.0 -> 84.5).
 //   Base conversion: the same line.  After its wait: rotation of 9 limbs of 32-bit words 47.1 -> 47.5, of 4 limbs with 4 extension limbs
 //   28.8 -> 32.4; late for every grid: 30 limbs 211.9 -> 213.5, 35 limbs 265.5 -> 266.7.
-//   Inverse columns with eight words: late for every grid, small CTAs of a conversion come after them (at the start: rotation of 9
-//   limbs of 32-bit words 47.3 -> 52.7; late where they are resident: 51.5).
+//   Inverse columns with eight words: late in grids of up to two rounds, small CTAs of a conversion come after them (at the start:
+//   rotation of 9 limbs of 32-bit words 47.3 -> 52.7; late only where they are resident: 51.5).
 __device__ __forceinline__ void grid_dependency_launch() {
 #if !defined(CERIUM_EMU)
   asm volatile("griddepcontrol.launch_dependents;");
+#endif
+}
+// Whether the CTAs of this grid are on the GPU at once, an SM holding per_sm of them.
+__device__ __forceinline__ bool grid_resident(unsigned per_sm) {
+#if defined(CERIUM_EMU)
+  return per_sm != 0;
+#else
+  unsigned sms;
+  asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+  return gridDim.x * gridDim.y * gridDim.z <= per_sm * sms;
 #endif
 }
 __device__ __forceinline__ void grid_dependency_wait() {

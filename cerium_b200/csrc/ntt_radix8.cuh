@@ -329,7 +329,7 @@ constexpr int kRadix8RowsPerSm = 32 / kRadix8Rows;  // CTAs that an SM holds: 32
 template <typename W, int kMode, typename Batch, typename Epilogue>
 __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const Epilogue& epi, int b, uint32_t pi, const PrimeConst<W>& pc,
                                                      Radix8Row<W>& row, const typename WordTraits<W>::Pair* tw,
-                                                     const typename WordTraits<W>::Pair* twr, int h, bool late_next) {
+                                                     const typename WordTraits<W>::Pair* twr, int h) {
   using RV = RowVec<W>;
   constexpr int kVecs = 4 / RV::kWords;  // 16-byte vectors of a group of four words
   const Arith<W, kMode> ar(pc);
@@ -363,7 +363,7 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   for (int k = 0; k < 2; k++)
 #pragma unroll
     for (int v = 0; v < kVecs; v++) ops[k][v] = epi.load(b, h * 256 + k * 128 + lane * 4 + v * RV::kWords);
-  if (late_next) grid_dependency_launch();
+  if (grid_resident(kRadix8RowsPerSm)) grid_dependency_launch();
   row_get_quads<W>(row.ex, x);
   late_row_quotients<W, kMode>(late, ar);
   late_fwd<W, kMode, kFpFwdMid, kFpCloseK32, kFpLaneK32>(x, late, ar);
@@ -394,24 +394,24 @@ __device__ __forceinline__ void radix8_fwd_rows_body(const Batch& batch, const E
   }
 }
 
-// grid = (256 / kRadix8Rows, limbs), block = 32 kRadix8Rows.  late_next (here and below): see grid_dependency_launch.
+// grid = (256 / kRadix8Rows, limbs), block = 32 kRadix8Rows.
 template <typename W, typename Batch, typename Epilogue>
 __global__ void __launch_bounds__(32 * kRadix8Rows, kRadix8RowsPerSm)
     radix8_fwd_rows_kernel(const Batch batch, const Epilogue epi, const typename WordTraits<W>::Pair* __restrict__ tw_all,
-                           const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
+                           const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  if (!late_next) grid_dependency_launch();
+  if (!grid_resident(kRadix8RowsPerSm)) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_rows_body, CERIUM_TARGS(Batch, Epilogue),
-                        (batch, epi, b, pi, pc, rows[warp], tw_all + (size_t)pi * kN, twr_all + (size_t)pi * kRowTwPerPrime, h, late_next));
+                        (batch, epi, b, pi, pc, rows[warp], tw_all + (size_t)pi * kN, twr_all + (size_t)pi * kRowTwPerPrime, h));
 }
 
 template <typename W, int kMode, typename Batch>
 __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc, Radix8Row<W>& row,
-                                                     const typename WordTraits<W>::Pair* twi, const typename WordTraits<W>::Pair* twri, int h, bool late_next) {
+                                                     const typename WordTraits<W>::Pair* twi, const typename WordTraits<W>::Pair* twri, int h) {
   const Arith<W, kMode> ar(pc);
   const int lane = threadIdx.x & 31, own = (lane >> 2) * 32 + (lane & 3);
   radix8_row_twiddles<W>(row, twi, h);
@@ -464,7 +464,7 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = row.ex[raised_pos<W>(j * 32 + lane)];
-  if (late_next) grid_dependency_launch();
+  if (grid_resident(kRadix8RowsPerSm)) grid_dependency_launch();
   radix8_inv<W, kMode, 0, kFpInvRow1.out>(x, row.tw, 1, ar);
   fp_reduce_masked<W, kMode>(x, kFpInvRow2.exchange, ar);
   W* out = batch.out_limb(b) + (unsigned)(h * 256 + lane);
@@ -475,15 +475,15 @@ __device__ __forceinline__ void radix8_inv_rows_body(const Batch& batch, int b, 
 template <typename W, typename Batch>
 __global__ void __launch_bounds__(32 * kRadix8Rows, kRadix8RowsPerSm)
     radix8_inv_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ twi_all,
-                           const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
+                           const typename WordTraits<W>::Pair* __restrict__ twri_all, const PrimeConst<W>* __restrict__ pcs) {
   __shared__ Radix8Row<W> rows[kRadix8Rows];
-  if (!late_next) grid_dependency_launch();
+  if (!grid_resident(kRadix8RowsPerSm)) grid_dependency_launch();
   const int b = blockIdx.y;
   const int warp = threadIdx.x >> 5, h = blockIdx.x * kRadix8Rows + warp;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   CERIUM_DISPATCH_ARITH(W, pc, radix8_inv_rows_body, CERIUM_TARGS(Batch),
-                        (batch, b, pc, rows[warp], twi_all + (size_t)pi * kN, twri_all + (size_t)pi * kRowTwPerPrime, h, late_next));
+                        (batch, b, pc, rows[warp], twi_all + (size_t)pi * kN, twri_all + (size_t)pi * kRowTwPerPrime, h));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -495,6 +495,10 @@ template <typename W>
 constexpr int kRadix8FwdColsPerSm = sizeof(W) == 8 ? 4 : 3;
 template <typename W>
 constexpr int kRadix8InvColsPerSm = sizeof(W) == 8 ? 4 : 2;
+// Inverse columns let the next kernel in late in grids of up to two rounds, which the lines of launch_inv_cols keep them to.  Without
+// the branch the compiler orders the last layers otherwise: 10 limbs of 64-bit words 8.57 -> 8.82 us.
+template <typename W>
+constexpr int kRadix8InvColsLate = 2 * kRadix8InvColsPerSm<W>;
 
 // Rows of the tile whose words share a bank lie eight apart in one of the three patterns (rows v * 8 + j of neighbouring
 // threads v): bits 3 and 4 of the row's number go into the lowest ones.
@@ -521,7 +525,7 @@ __device__ __forceinline__ void late_column_load(LateTwiddles<W>& l, const typen
 
 template <typename W, int kMode, int kCols, typename Batch, typename Loader>
 __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const Loader& loader, int b, const PrimeConst<W>& pc, W* tile,
-                                                     const typename WordTraits<W>::Pair* stw, bool late_next) {
+                                                     const typename WordTraits<W>::Pair* stw) {
   const Arith<W, kMode> ar(pc);
   const int c = threadIdx.x % kCols, v = threadIdx.x / kCols;
   const int col = blockIdx.x * kCols + c, own = (v >> 2) * 32 + (v & 3);
@@ -555,7 +559,7 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
   radix8_quad_sync<kCols>();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(v * 8 + j, c)];
-  if (late_next) grid_dependency_launch();
+  if (grid_resident(kRadix8FwdColsPerSm<W>)) grid_dependency_launch();
   LateTwiddles<W> late;
   late_column_load<W>(late, stw, v);
   late_fwd<W, kMode, Loader::kFpBound, 1, 1>(x, late, ar);
@@ -567,16 +571,16 @@ __device__ __forceinline__ void radix8_fwd_cols_body(const Batch& batch, const L
 template <typename W, int kCols, typename Batch, typename Loader>
 __global__ void __launch_bounds__(kCols * 32, kRadix8FwdColsPerSm<W>)
     radix8_fwd_cols_kernel(const Batch batch, const Loader loader, const typename WordTraits<W>::Pair* __restrict__ tw_all,
-                           const PrimeConst<W>* __restrict__ pcs, const bool late_next) {
+                           const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
-  if (!late_next) grid_dependency_launch();
+  if (!grid_resident(kRadix8FwdColsPerSm<W>)) grid_dependency_launch();
   const int b = blockIdx.y;
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
   for (int k = threadIdx.x; k < 256; k += kCols * 32) stw[k] = __ldg(tw_all + (size_t)pi * kN + k);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw, late_next));
+  CERIUM_DISPATCH_ARITH(W, pc, radix8_fwd_cols_body, CERIUM_TARGS(kCols, Batch, Loader), (batch, loader, b, pc, tile, stw));
 }
 
 template <typename W, int kMode, int kCols, typename Batch>
@@ -619,7 +623,7 @@ __device__ __forceinline__ void radix8_inv_cols_body(const Batch& batch, const I
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; j++) x[j] = tile[radix8_tile<W, kCols>(j * 32 + v, c)];
-  grid_dependency_launch();
+  if (grid_resident(kRadix8InvColsLate<W>)) grid_dependency_launch();
   radix8_inv_final<W, kMode, kFpInvCol1.out>(x, stw, last, ar);
   if (sc.add != nullptr) {
     const W a = __ldg(sc.add + b);
@@ -636,6 +640,7 @@ __global__ void __launch_bounds__(kCols * 32, kRadix8InvColsPerSm<W>)
                            const PrimeConst<W>* __restrict__ pcs) {
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
+  if (!grid_resident(kRadix8InvColsLate<W>)) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the row pass
   const uint32_t pi = batch.prime_of(b);
   const PrimeConst<W> pc = pcs[pi];
