@@ -51,32 +51,45 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
 template <typename W>
 static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
-// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen, on either side of each line in us.
-//   Columns: beyond the lines the second barrier and the narrow tiles cost more than the shorter chain gives (column pass of 39 limbs
-//   in a rotation of 12 limbs 98.9 with sixteen words, 100.7 with eight).  Of 32-bit words inverse up to the 26 limbs of two
-//   polynomials' 13 extension primes (40 limbs alone 14.1 / 16.3), forward where the words come from a conversion
-//   or a division (rotation of 6 limbs 44.4 / 42.4; alone, 3 limbs 4.7 / 6.9, 20 limbs 9.3 / 9.9).
-//   Rows: fewer instructions decide where the GPU is full (384 limbs forward 187.0 / 187.9 under the power limit, inverse 161.7 / 163;
-//   240 limbs 101.5 / 98.3 and 105.2 / 108.3, 128 limbs inverse 61.0 / 60.3, 32-bit words 240 limbs inverse 67.6 / 67.6, 384 limbs
-//   104.6 / 106.9).  Rows of 32-bit words forward: where the epilogue reads operands (rotation of 51 limbs 176.9 / 173.9; plain, 245
-//   limbs 66.4 / 69.2).
-//   Inverse transforms of 64-bit words in a call of their own find their twiddles in L2, and from 25 to 64 limbs sixteen words are
-//   faster (30 limbs 17.8 / 18.2, 64 limbs 31.7 / 33.2); after a key has gone through L2 they are not (rotation of 35 limbs 286.6 / 282.8).
+// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen; us with eight / sixteen.
+//   Columns: beyond the lines the second barrier and the narrow tiles cost more than the shorter chain gives.
+//     64-bit words inverse: 23 limbs alone 14.5 / 15.0, 24 limbs 15.9 / 15.5, 40 limbs 22.8 / 22.1, rotation of 24 limbs 167.9 / 167.4,
+//     of 35 limbs 271.6 / 270.7.  Integer butterflies alike: 23 limbs 21.9 / 23.0, 24 limbs 23.9 / 23.3.
+//     32-bit words inverse: 27 limbs 10.8 / 10.9, 28 limbs 11.9 / 11.3, rotation of 28 limbs with 14 extension limbs 88.2 / 86.0.
+//     Forward: 32 limbs 18.2 / 18.8; 32-bit words only where they come from a conversion or a division (rotation of 6
+//     limbs 42.4 / 44.4; alone, 3 limbs 6.9 / 4.7, 20 limbs 9.9 / 9.3).
+//   Forward rows: 64-bit words eight for every batch (257 limbs alone 115.5 / 117.8, in pointer tables 119.5 / 124.9, of integers
+//     176.3 / 183.9; 384 limbs under the power limit 185.3 / 185.7).  32-bit words only where the epilogue reads operands
+//     (rotation of 51 limbs 173.9 / 176.9; plain, 245 limbs 69.2 / 66.4).
+//   Inverse rows: eight, and sixteen without twiddles in shared memory from 129 limbs on where the GPU is at its power limit
+//     (128 limbs 59.2 / 62.6; 140 limbs 73.8 / 72.9, 384 limbs 197.8 / 193.3) and from 91 of 32-bit words (85 limbs 26.6 / 26.6, 100 limbs
+//     31.0 / 30.6, 256 limbs 72.6 / 70.8).  Stacks of limbs with their twiddles in shared memory, in small tiles, do better between:
+//     32-bit words from 56 limbs on (46 limbs 15.3 / 15.4, 60 limbs 19.6 / 19.2, 74 limbs 23.1 / 22.0, rotation of 60 limbs 207.3 / 208.4),
+//     64-bit words on doubles from 36 (32 limbs 18.2 / 18.3, 40 limbs 22.2 / 21.8, 64 limbs 32.9 / 31.8, rotation of 35 limbs 275.4 /
+//     276.4, of 45 limbs 406.7 / 407.4).  Not of pointer tables (74 limbs of 32-bit words 22.4 / 23.1) and not of products
+//     (multiplication of 25 limbs 226.9 / 231.8).  Stacks of integers take eight whatever their number (28 limbs 27.1 / 31.2, 64 limbs
+//     51.0 / 59.5, 140 limbs under the power limit 109.7 / 117.1).
 template <typename W>
-constexpr int kRadix8InvCols = sizeof(W) == 8 ? 40 : 28;
-constexpr int kRadix8FwdCols = 32, kRadix8FwdRows64 = 256, kRadix8Alone64 = 24;
+constexpr int kRadix8InvCols = sizeof(W) == 8 ? 23 : 27;
+constexpr int kRadix8FwdCols = 32;
 template <typename W>
-constexpr int kRadix8InvRows = sizeof(W) == 8 ? 128 : 280;
+constexpr int kRadix8InvRows = sizeof(W) == 8 ? 128 : 90;
+template <typename W>
+constexpr int kRadix8InvRowsOfStacks = sizeof(W) == 8 ? 35 : 55;
 
 template <typename W, typename Batch, typename Loader>
 static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loader& loader, int limbs, cudaStream_t stream) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (limbs <= kRadix8FwdCols && (sizeof(W) == 8 || !Loader::kPlain)) {
-    auto kfn = radix8_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
-    CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
-  } else if (small_batch<W>(ctx, limbs)) {
+  if constexpr (sizeof(W) == 8 || !Loader::kPlain) {
+    if (limbs <= kRadix8FwdCols) {
+      auto kfn = radix8_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
+      CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, loader, tw, pcs);
+      return;
+    }
+  }
+  if (small_batch<W>(ctx, limbs)) {
     auto kfn = ntt_fwd_cols_kernel<W, kCols / 2, Batch, Loader>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 8, 0, stream, batch, loader, tw, pcs);
   } else {
@@ -85,11 +98,11 @@ static void launch_fwd_cols(cerium_context* ctx, const Batch& batch, const Loade
   }
 }
 template <typename W, typename Batch>
-static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvScale<W>& scale, int limbs, cudaStream_t stream, bool alone = false) {
+static void launch_inv_cols(cerium_context* ctx, const Batch& batch, const InvScale<W>& scale, int limbs, cudaStream_t stream) {
   constexpr int kCols = NttCfg<W>::kCols;
   const auto* tw = static_cast<const typename WordTraits<W>::Pair*>(ctx->d_tw_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (limbs <= (alone && sizeof(W) == 8 ? kRadix8Alone64 : kRadix8InvCols<W>)) {
+  if (limbs <= kRadix8InvCols<W>) {
     auto kfn = radix8_inv_cols_kernel<W, kCols / 2, Batch>;
     CERIUM_LAUNCH(kfn, dim3(512 / kCols, limbs), kCols * 16, 0, stream, batch, scale, tw, pcs);
   } else if (small_batch<W>(ctx, limbs)) {
@@ -106,33 +119,33 @@ static void launch_fwd_rows(cerium_context* ctx, const Batch& batch, const Epilo
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_fwd);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_fwd);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (Epilogue::kHasOperands || (sizeof(W) == 8 && limbs <= kRadix8FwdRows64)) {
+  if constexpr (sizeof(W) == 8 || Epilogue::kHasOperands) {
     auto kfn = radix8_fwd_rows_kernel<W, Batch, Epilogue>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, epi, tw, twr, pcs);
-    return;
-  }
-  if constexpr (!Epilogue::kHasOperands) {
-    if constexpr (sizeof(W) == 4) {
-      if (small_batch<W>(ctx, limbs)) {
-        auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
-        CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
-        return;
-      }
-    }
+  } else if (small_batch<W>(ctx, limbs)) {
+    auto kfn = ntt_fwd_rows_kernel<W, kRowsSmall, true, Batch, Epilogue>;
+    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
+  } else {
     auto kfn = ntt_fwd_rows_kernel<W, kRowsPerCta, false, Batch, Epilogue>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
   }
 }
+// doubles: most of the primes have butterflies on doubles (stacks of 64-bit words)
 template <typename W, typename Batch>
-static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, cudaStream_t stream, bool alone = false) {
+static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, cudaStream_t stream, bool doubles = false) {
   using Pair = typename WordTraits<W>::Pair;
   const auto* tw = static_cast<const Pair*>(ctx->d_tw_inv);
   const auto* twr = static_cast<const Pair*>(ctx->d_twr_inv);
   const auto* pcs = static_cast<const PrimeConst<W>*>(ctx->d_pcs);
-  if (sizeof(W) == 8 && alone && limbs > kRadix8Alone64 && small_batch<W>(ctx, limbs)) {
-    auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
-  } else if (limbs <= kRadix8InvRows<W>) {
+  constexpr bool kStack = std::is_same_v<Batch, StridedBatch<W>>;
+  if constexpr (kStack) {
+    if (limbs > kRadix8InvRowsOfStacks<W> && small_batch<W>(ctx, limbs) && (sizeof(W) == 4 || doubles)) {
+      auto kfn = ntt_inv_rows_kernel<W, kRowsSmall, true, Batch>;
+      CERIUM_LAUNCH(kfn, dim3(256 / kRowsSmall, limbs), kRowsSmall * 16, 0, stream, batch, tw, twr, pcs);
+      return;
+    }
+  }
+  if (limbs <= kRadix8InvRows<W> || (kStack && sizeof(W) == 8 && !doubles)) {
     auto kfn = radix8_inv_rows_kernel<W, Batch>;
     CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
   } else {
@@ -234,9 +247,11 @@ int launch_ntt_inverse(cerium_context* ctx, const NttCall& c, cudaStream_t strea
         pb.factor = static_cast<const W*>(c.factor);
         launch_inv_rows<W>(ctx, pb, cnt, stream);
       } else {
-        launch_inv_rows<W>(ctx, sb, cnt, stream, c.alone);
+        int doubles = 0;
+        for (int b = 0; b < cnt; b++) doubles += ctx->fp_ok[c.prime[first + b]] ? 1 : 0;
+        launch_inv_rows<W>(ctx, sb, cnt, stream, 2 * doubles > cnt);
       }
-      launch_inv_cols<W>(ctx, sb, sc, cnt, stream, c.alone);
+      launch_inv_cols<W>(ctx, sb, sc, cnt, stream);
     }
     CERIUM_LAUNCH_CHECK("ntt_inverse");
     return CERIUM_OK;
@@ -771,7 +786,6 @@ static int ntt_common(cerium_context* ctx, bool forward, void* out, size_t out_s
   if (int rc = check_stack(in, in_stride, ctx->word_bytes(), "ntt: in")) return rc;
   DeviceGuard guard(ctx->device);
   NttCall c{in, out, in_stride, out_stride, nullptr, prime_idx, count};
-  c.alone = true;
   return forward ? launch_ntt_forward(ctx, c, (cudaStream_t)stream)
                  : launch_ntt_inverse(ctx, c, (cudaStream_t)stream);
 }

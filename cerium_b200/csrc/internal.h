@@ -273,8 +273,6 @@ struct NttCall {
   uint32_t in_galois = 0;
   // inverse transform only: the input is the product with the limbs of this stack, which lie as those of `in` do
   const void* factor = nullptr;
-  // a call of its own and no step of an operation: nothing but transforms has gone through L2, and the twiddles are there
-  bool alone = false;
   // forward transform only: the column pass alone; raised_inner_kernel does the rows
   bool cols_only = false;
 };

@@ -322,9 +322,7 @@ constexpr int fp_plan_cols(int bin) { return fp_plan_fwd(fp_plan_fwd(bin).out).o
 constexpr int fp_max(int a, int b) { return a > b ? a : b; }
 constexpr int kFpRaisedMid = fp_max(fp_plan_cols(kFpCanon), fp_plan_cols(kFpRaisedIn));
 constexpr int kFpFwdMid = fp_max(kFpRaisedMid, fp_plan_cols(kFpLoweredIn));
-constexpr int kFpFwdL3 = fp_plan_fwd(kFpFwdMid).out;
 constexpr int kFpLaneK32 = 3;  // level 3 (lane table) computes its quotients
-static_assert(fp_plan_fwd(kFpFwdL3, kFpLaneK32).out < 8192, "the transform's last values must stay exact integers");
 // bounds along the inverse transform: row pass (levels 3, 2) stores kFpInvMid
 constexpr int kFpInvL3 = fp_plan_exchange(fp_plan_inv(kFpCanon, kFpLaneK32), kFpInvExchangeMax).out;
 constexpr int kFpInvMid = fp_plan_inv(kFpInvL3).max_out;
@@ -375,27 +373,19 @@ __device__ __forceinline__ W lane_tw_fp(const typename WordTraits<W>::Pair* tw, 
 template <typename W, bool kGlobalTw, int kMode, int kTw = kTwPlain, int kBin = 0>
 __device__ __forceinline__ void radix16_fwd(W (&x)[16], const typename WordTraits<W>::Pair* tw,
                                             uint32_t S, const Arith<W, kMode>& ar) {
-  constexpr bool kPacked = kTw == kTwLane && kMode == kArithFp;
-  constexpr FpFwdPlan plan = fp_plan_fwd(kBin, kPacked ? kFpLaneK32 : 1);
+  static_assert(kTw == kTwPlain || kMode != kArithFp, "the lane tables of Fp primes have no companions");
+  constexpr FpFwdPlan plan = fp_plan_fwd(kBin);
 #pragma unroll
   for (int t = 0; t < 4; t++) {
     const int half = 8 >> t;
     if (kMode == kArithFp && plan.before[t]) fp_reduce_masked<W, kMode>(x, 0xffffu, ar);
 #pragma unroll
     for (int g = 0; g < (1 << t); g++) {
-      W w0, w1;
-      if constexpr (kPacked) {
-        w0 = lane_tw_fp<W, kGlobalTw>(tw, t, g);
-        w1 = ar.quotient(w0);
-      } else {
-        const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kTw>(S, t, g));
-        w0 = w.x;
-        w1 = w.y;
-      }
+      const auto w = load_tw<W, kGlobalTw>(tw, tw_index<kTw>(S, t, g));
 #pragma unroll
       for (int k = 0; k < half; k++) {
         const int j = g * 2 * half + k;
-        ar.fwd(x[j], x[j + half], w0, w1);
+        ar.fwd(x[j], x[j + half], w.x, w.y);
       }
     }
   }
@@ -881,7 +871,7 @@ __device__ __forceinline__ void load16<uint32_t>(const uint32_t* src, uint32_t (
   }
 }
 
-template <typename W, int kMode, int kRows, bool kStage, typename Batch, typename Epilogue>
+template <typename W, int kRows, bool kStage, typename Batch, typename Epilogue>
 __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, const PrimeConst<W>& pc,
                                                   RowsBuffer<W, kRows, kStage>& buf,
                                                   const typename WordTraits<W>::Pair* tw,
@@ -889,6 +879,7 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, con
   using RV = RowVec<W>;
   using Vec = typename RV::Vec;
   W* tile = buf.tile;
+  constexpr int kMode = kArithStrict;
   const Arith<W, kMode> ar(pc);
   const int tid = threadIdx.x, r = tid >> 4, u = tid & 15;
   const int h = blockIdx.x * kRows + r;
@@ -902,9 +893,9 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, con
   for (int j = 0; j < 16; j++) x[j] = row[j * 16];
   if constexpr (kStage) {
     row_twiddles_wait();
-    radix16_fwd<W, false, kMode, kTwGroup, kFpFwdMid>(x, buf.tw.group[r], 0u, ar);
+    radix16_fwd<W, false, kMode, kTwGroup>(x, buf.tw.group[r], 0u, ar);
   } else {
-    radix16_fwd<W, true, kMode, kTwPlain, kFpFwdMid>(x, tw, 256u + (uint32_t)h, ar);
+    radix16_fwd<W, true, kMode, kTwPlain>(x, tw, 256u + (uint32_t)h, ar);
   }
 #pragma unroll
   for (int j = 0; j < 16; j++) t_strided[j * 17] = x[j];
@@ -912,8 +903,8 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, con
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = t_own[j];
   // level 3: this thread's 15 twiddles from the lane-interleaved table of row h
-  if constexpr (kStage) radix16_fwd<W, false, kMode, kTwLane, kFpFwdL3>(x, buf.tw.lane[r] + u, 0u, ar);
-  else radix16_fwd<W, true, kMode, kTwLane, kFpFwdL3>(x, twr + ((size_t)h * (kMode == kArithFp ? 8 : 15) * 16 + u), 0u, ar);
+  if constexpr (kStage) radix16_fwd<W, false, kMode, kTwLane>(x, buf.tw.lane[r] + u, 0u, ar);
+  else radix16_fwd<W, true, kMode, kTwLane>(x, twr + ((size_t)h * 15 * 16 + u), 0u, ar);
 #pragma unroll
   for (int j = 0; j < 16; j++) x[j] = ar.template finish_fwd<Epilogue::kCanonical>(x[j], pc.one_shoup);
   // own 16 words -> swizzled vectors -> coalesced vectors
@@ -927,17 +918,15 @@ __device__ __forceinline__ void ntt_fwd_rows_body(const Batch& batch, int b, con
   for (int k = 0; k < RV::kPerThread; k++) reinterpret_cast<Vec*>(drow)[u + 16 * k] = vrow[row_vec_slot<W>(u + 16 * k)];
 }
 
-// Row pass (levels 2 and 3): reads the column pass's result from the batch's `in` stack and
-// writes the finished transform to its `out` stack (the two may be the same buffer).
+// Row pass (levels 2 and 3) of 32-bit words whose epilogue reads nothing: reads the column pass's result from the batch's `in` stack
+// and writes the finished transform to its `out` stack (the two may be the same buffer).
 // grid = (256 / kRows, limbs), block = 16 * kRows; 16 threads own one row.
-// Waits for its twiddles (L2 and L1) more than for its data: four CTAs per SM at 64 registers, a few words of the integer
-// arithmetic spilled, against three at 80 (rotation of 35 limbs 352.9 -> 349.5 us, 8x8 linear transform 4030 -> 3980 us).
-// The column pass gains nothing from it.
 template <typename W, int kRows, bool kStage, typename Batch, typename Epilogue>
 __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
     ntt_fwd_rows_kernel(const Batch batch, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const typename WordTraits<W>::Pair* __restrict__ twr_all,
                         const PrimeConst<W>* __restrict__ pcs) {
+  static_assert(sizeof(W) == 4, "64-bit words have radix8_fwd_rows_kernel");
   using Pair = typename WordTraits<W>::Pair;
   __shared__ RowsBuffer<W, kRows, kStage> buf;
   grid_dependency_launch();
@@ -949,10 +938,9 @@ __global__ void __launch_bounds__(kRows * 16, 1024 / (kRows * 16))
   const PrimeConst<W> pc = pcs[pi];
   const Pair* tw = tw_all + (size_t)pi * kN;
   const Pair* twr = twr_all + (size_t)pi * kRowTwPerPrime;
-  static_assert(!kStage || sizeof(W) == 4, "the lane tables of 64-bit words have other sizes");
   if constexpr (kStage) row_twiddles_start(buf.tw, tw, twr, blockIdx.x * kRows);
   grid_dependency_wait();
-  CERIUM_DISPATCH_ARITH(W, pc, ntt_fwd_rows_body, CERIUM_TARGS(kRows, kStage, Batch, Epilogue), (batch, b, pc, buf, tw, twr));
+  ntt_fwd_rows_body<W, kRows, kStage, Batch, Epilogue>(batch, b, pc, buf, tw, twr);
 }
 
 // ---------------------------------------------------------------------------------------

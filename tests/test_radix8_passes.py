@@ -1,6 +1,6 @@
 """Transforms on both sides of the batch sizes where a pass changes between eight words a thread and sixteen, for every arithmetic (64-bit
-words: 32 limbs and 256 forward, 24, 64 and 128 inverse; 32-bit words: 28 and 280 inverse), and limbs of 64-bit words that are aligned
-to 16 bytes only, whose rows move as pairs of words: exact against the oracle."""
+words: 32 limbs forward, 23, 35, 64 and 128 inverse; 32-bit words: 27, 55, 74 and 90 inverse), as stacks and as pointer tables, and
+limbs of 64-bit words that are aligned to 16 bytes only, whose rows move as pairs of words: exact against the oracle."""
 import numpy as np
 import pytest
 
@@ -32,6 +32,28 @@ def test_batch_sizes(name, word_bits, count):
     assert np.array_equal(h.down(d), h.orc.ntt_forward(x, idx))
     h.ctx.ntt_inverse(h.p(d), h.p(d), idx)
     assert np.array_equal(h.down(d), x)
+
+
+@pytest.mark.parametrize("name,word_bits,integers,count", [("emu", 64, False, 3), ("emu", 32, False, 2)] + [
+    gpu("cuda", 64, i, c) for c in (23, 24, 35, 36, 64, 65, 129) for i in (False, True)] + [
+    gpu("cuda", 32, False, c) for c in (27, 28, 55, 56, 74, 75, 90, 91)])
+def test_lines_of_the_inverse_passes(name, word_bits, integers, count):
+    from tests import backends
+    mods = params.ntt_primes_below(60, 3, pc.LOGN) if integers else pc.moduli_for(word_bits, 3, 1)
+    be = backends.EmuBackend() if name == "emu" else backends.CudaBackend()
+    h = pc.Harness(be, word_bits, mods)
+    idx = [b % len(mods) for b in range(count)]
+    want = pc.rand_limbs(np.random.default_rng(count), mods, idx)
+    x = h.orc.ntt_forward(want, idx)
+    d, out = h.up(x), h.new(count, pc.N)
+    h.ctx.ntt_inverse(h.p(out), h.p(d), idx)
+    assert np.array_equal(h.down(out), want)
+    at = lambda b: be.to_dev(np.array([h.p(b) + k * pc.N * h.ctx.word_bytes for k in range(count)], dtype=np.uint64))  # noqa: E731
+    outs, ins, bases = at(out), at(d), be.to_dev(np.array(idx, dtype=np.uint32))
+    h.ctx.ntt_inverse_ptrs(be.ptr(outs), be.ptr(ins), be.ptr(bases), count)
+    assert np.array_equal(h.down(out), want)
+    h.ctx.ntt_forward_ptrs(be.ptr(outs), be.ptr(outs), be.ptr(bases), count)
+    assert np.array_equal(h.down(out), x)
 
 
 @pytest.mark.parametrize("name", ["emu", gpu("cuda")])
