@@ -501,11 +501,11 @@ template <typename W>
 constexpr int kRadix8InvColsLate = 2 * kRadix8InvColsPerSm<W>;
 
 // Rows of the tile whose words share a bank lie eight apart in one of the three patterns (rows v * 8 + j of neighbouring
-// threads v): bits 3 and 4 of the row's number go into the lowest ones.
+// threads v).  Two rows make a line of 128 bytes, of 8 words of 64 bits or 16 of 32: bit 3 of the row's number goes into the lowest one.
 template <typename W, int kCols>
 __device__ __forceinline__ int radix8_tile(int r, int c) {
-  constexpr int kRowsPerLine = kCols * (int)sizeof(W) < 128 ? 128 / (kCols * (int)sizeof(W)) : 1;
-  return (r ^ (r >> 3 & (kRowsPerLine - 1))) * kCols + c;
+  static_assert(2 * kCols * sizeof(W) == 128, "two rows to a line");
+  return (r ^ (r >> 3 & 1)) * kCols + c;
 }
 // Barrier of the four threads that exchange a column's rows of one block of 32.
 template <int kCols>
