@@ -145,13 +145,15 @@ static void launch_inv_rows(cerium_context* ctx, const Batch& batch, int limbs, 
       return;
     }
   }
-  if (limbs <= kRadix8InvRows<W> || (kStack && sizeof(W) == 8 && !doubles)) {
-    auto kfn = radix8_inv_rows_kernel<W, Batch>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
-  } else {
-    auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
-    CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
+  if constexpr (!Batch::kProduct) {  // products have the limbs of a plan, 64 at most
+    if (limbs > kRadix8InvRows<W> && (!kStack || sizeof(W) == 4 || doubles)) {
+      auto kfn = ntt_inv_rows_kernel<W, kRowsPerCta, false, Batch>;
+      CERIUM_LAUNCH(kfn, dim3(256 / kRowsPerCta, limbs), kRowsPerCta * 16, 0, stream, batch, tw, twr, pcs);
+      return;
+    }
   }
+  auto kfn = radix8_inv_rows_kernel<W, Batch>;
+  CERIUM_LAUNCH(kfn, dim3(256 / kRadix8Rows, limbs), kRadix8Rows * 32, 0, stream, batch, tw, twr, pcs);
 }
 
 int launch_ntt_forward(cerium_context* ctx, const NttCall& c, cudaStream_t stream, bool lazy_out) {

@@ -982,21 +982,6 @@ __device__ __forceinline__ void ntt_inv_rows_body(const Batch& batch, int b, con
       in[k] = vec_pack(w);
     }
   }
-  if constexpr (Batch::kProduct) {
-    const Vec* factor = reinterpret_cast<const Vec*>(batch.factor_limb(b) + h * 256);
-    Vec f[RV::kPerThread];
-#pragma unroll
-    for (int k = 0; k < RV::kPerThread; k++) f[k] = factor[u + 16 * k];
-#pragma unroll
-    for (int k = 0; k < RV::kPerThread; k++) {
-      W x[RV::kWords], y[RV::kWords];
-      vec_unpack(in[k], x);
-      vec_unpack(f[k], y);
-#pragma unroll
-      for (int e = 0; e < RV::kWords; e++) x[e] = mul_mod<W>(x[e], y[e], pc);
-      in[k] = vec_pack(x);
-    }
-  }
 #pragma unroll
   for (int k = 0; k < RV::kPerThread; k++) vrow[row_vec_slot<W>(u + 16 * k)] = in[k];
   __syncwarp();
