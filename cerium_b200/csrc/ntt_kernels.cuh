@@ -54,7 +54,11 @@ constexpr int kSmallBatchPerSm = sizeof(W) == 8 ? 7 : 8;
 // Lane-interleaved level-3 twiddles: [row h (256)][e = 2^t - 1 + g (15)][thread u (16)] pairs per
 // prime; entry = bit-reversed table[((4096 + 16 h + u) << t) + g].
 constexpr int kRowTwPerPrime = 256 * 15 * 16;
-constexpr int kMaxBatch = 576;     // limbs per launch: 24 one-limb digits raised to 24 limbs more
+// Limbs per launch: the largest multiple of 64 with which the parameters of every kernel stay within 4 KB (the asserts in the
+// forward passes, whose loaders and epilogues are the long ones).  A call of more goes on in launches of that many: 512 loses 3 to 4 % on 513 to 576 limbs (576 forward 262.9 us
+// against 255.2); shared out evenly, 577 limbs of 32-bit words 155.8 -> 159.7, 625 of 64-bit words inverse 291 -> 307.
+constexpr int kMaxBatch = 576;
+constexpr size_t kMaxParameters = 4096;
 
 // Addressing of a batch of limbs: batch entry b lives at base + pos[b] * stride; its modulus
 // is prime[b] (index into the context's prime list).  Passed by value as a kernel parameter.
@@ -645,6 +649,7 @@ __global__ void __launch_bounds__(kCols * 16, (sizeof(W) == 8 ? 768 : 1024) / (k
     ntt_fwd_cols_kernel(const Batch batch, const Loader loader,
                         const typename WordTraits<W>::Pair* __restrict__ tw_all,
                         const PrimeConst<W>* __restrict__ pcs) {
+  static_assert(sizeof(Batch) + sizeof(Loader) + 2 * sizeof(void*) <= kMaxParameters);
   using Pair = typename WordTraits<W>::Pair;
   __shared__ W tile[256 * kCols];
   __shared__ Pair stw[256];

@@ -399,6 +399,7 @@ template <typename W, typename Batch, typename Epilogue>
 __global__ void __launch_bounds__(32 * kRadix8Rows, kRadix8RowsPerSm)
     radix8_fwd_rows_kernel(const Batch batch, const Epilogue epi, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                            const typename WordTraits<W>::Pair* __restrict__ twr_all, const PrimeConst<W>* __restrict__ pcs) {
+  static_assert(sizeof(Batch) + sizeof(Epilogue) + 3 * sizeof(void*) <= kMaxParameters);
   __shared__ Radix8Row<W> rows[kRadix8Rows];
   if (!grid_resident(kRadix8RowsPerSm)) grid_dependency_launch();
   const int b = (int)(gridDim.y - 1 - blockIdx.y);  // against the direction of the column pass
@@ -572,6 +573,7 @@ template <typename W, int kCols, typename Batch, typename Loader>
 __global__ void __launch_bounds__(kCols * 32, kRadix8FwdColsPerSm<W>)
     radix8_fwd_cols_kernel(const Batch batch, const Loader loader, const typename WordTraits<W>::Pair* __restrict__ tw_all,
                            const PrimeConst<W>* __restrict__ pcs) {
+  static_assert(sizeof(Batch) + sizeof(Loader) + 2 * sizeof(void*) <= kMaxParameters);
   __shared__ W tile[256 * kCols];
   __shared__ typename WordTraits<W>::Pair stw[256];
   if (!grid_resident(kRadix8FwdColsPerSm<W>)) grid_dependency_launch();

@@ -1,9 +1,9 @@
 """Parity at the shapes bench.py times: the CUDA build through the C ABI against the CPU oracle,
 bit-exact, at HRot L=35 / K=5 / dnum=7 and HMult L=24 / K=1 / dnum=24 (64-bit words, exact base
-conversion, rounding division).  These shapes take code paths the small cases never reach: 245
-raised limbs, seven 5 -> 35 conversions with the output split chosen from the wave count, 576
-raised limbs split over two transform launches with the one-limb-digit loader, two-polynomial
-SuD launches of 70 limbs.  The sequence compared is the reference's key-switch lowering
+conversion, rounding division), and at HMult L=26 / K=1 / dnum=26.  These shapes take code paths the
+small cases never reach: 245 raised limbs, seven 5 -> 35 conversions in one launch, 576 raised limbs
+in the largest launch of the one-limb-digit loader and 676 in two, two-polynomial SuD launches of 70
+limbs.  The sequence compared is the reference's key-switch lowering
 (cerium/compiler/backend/compiler_keyswitch.cc:253-432); comparison style as
 examples/common.py:134-142, but on every integer limb instead of decrypted slots."""
 import numpy as np
@@ -90,6 +90,20 @@ def test_hmult_bench_shape(be):
     ks.hmult(h.p(o0), h.p(o1), h.p(da0), h.p(da1), h.p(db0), h.p(db1), h.p(dk), False)
     w0, w1 = h.orc.hmult_relin(BM, RM, False, prm.q_idx, prm.p_idx, prm.dnum, a0, a1, b0, b1, evk)
     assert np.array_equal(h.down(o0), w0) and np.array_equal(h.down(o1), w1), "HMult+relin differs at L=24"
+    ks.close()
+
+
+def test_one_limb_digits_in_two_launches(be):
+    """676 raised limbs: the second launch of the one-limb-digit loader starts at its own source limbs and primes."""
+    prm = params.config_hmult(pc.LOGN, 26)
+    assert prm.dnum * (prm.L + prm.K) - prm.L == 676
+    h = pc.Harness(be, 64, prm.moduli)
+    _c0, c1, evk = pc.make_keyswitch_inputs(np.random.default_rng(26), prm)
+    ks = _capi.KeySwitch(h.ctx, prm.q_idx, prm.p_idx, prm.dnum, BM, RM)
+    d1, dk, o = h.up(c1), h.up(evk), h.new(2, prm.L, pc.N)
+    ks.apply(h.p(o), h.p(o) + 8 * prm.L * pc.N, h.p(d1), h.p(dk))
+    assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(BM, RM, prm.q_idx, prm.p_idx, prm.dnum, c1, evk)))
+    assert be.launches(lambda st: ks.hoisted_begin(h.p(d1), st)) == 2 + 2 * 2
     ks.close()
 
 
