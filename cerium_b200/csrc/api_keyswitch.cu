@@ -169,30 +169,34 @@ int rescale_impl(cerium_context* ctx, int round_mode, void* const* outs, void* p
   return CERIUM_OK;
 }
 
-// Digits from which on two warps share a row of raised_inner_kernel<uint64_t>: whole rounds of CTAs are shorter (13 limbs
-// with as many digits 202.4 -> 192.4 us, 24 limbs 424 / 426); 7 digits on 40 limbs lose (292 -> 313 us).  Not where the
-// butterflies are integers (60-bit primes, 16 limbs with as many digits 379.5 -> 381.8, 20 limbs 540.8 -> 553.0).  32-bit words are
-// never split: rotations of 3 to 51 limbs lose 5 to 10 %.
+// Digits from which on two warps share a row of raised_inner_kernel<uint64_t>: the rounds of CTAs are shorter.  One warp / two, us,
+// rotations with one-limb digits: 12 limbs 145.0 / 146.5, 13 limbs 156.5 / 151.8, 18 limbs 238 / 244, 24 limbs 389 / 377, 28 limbs 497 /
+// 497; multiplications, whose tensor product the rows of one warp take with them: 13 limbs 171.0 / 163.5, 16 limbs 217.5 / 218.5, 20 limbs
+// 303 / 295, 28 limbs 524 / 512.  Rotations of 45 limbs in digits of three 546 / 560, of 16 limbs in digits of four 121.7 / 135.0.  Not where the
+// butterflies are integers (60-bit primes, 16 limbs with as many digits 331 / 339, 20 limbs 482 / 493).  32-bit words are never
+// split: rotations of 3 to 51 limbs lose 5 to 10 %.
 constexpr int kSplitDigits = 12;
 bool splits_rows(const cerium_keyswitch* ks) { return ks->ctx->word_bits == 64 && ks->dnum >= kSplitDigits && !ks->integer; }
 // Whether the row pass of the raised digits runs inside the inner product (raised_inner_kernel): where its sums take the plan's
 // primes, it can read the key and the polynomials four words at a time, and 64-bit words have the rows that keep the resident
-// warps (16 to an SM) busy.  With fewer the serial walk over the digits shows; integer butterflies make it longer, and want more
-// rows where digits are many.  Rotations in two kernels / in one, us:
-//   50-bit primes, 5 extension limbs: 8 limbs 96.0 / 95.8, 10 limbs 103.6 / 104.5, 11 limbs 113.6 / 110.3, 12 limbs (17 with the
-//   extension) 118.5 / 110.7, 13 limbs 136.4 / 119.2; digits of one limb, 6 limbs 103.5 / 109.2, 8 limbs 136.8 / 129.6, 10 limbs
-//   173.0 / 158.0, 12 limbs 206.7 / 198.7.  The limits are those of the kernel's first form, which needed 12 limbs; smaller
-//   plans have come to gain since;
-//   60-bit primes, 5 extension limbs: 12 limbs 168.8 / 162.4, 24 limbs 300.3 / 289.7; digits of one limb, 16 limbs 370.3 / 379.5,
-//   20 limbs 529.6 / 540.8, 24 limbs 717.8 / 692.3; of two limbs, 24 limbs 456.6 / 452.6.
-// 32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 199.8 / 183.4).
+// warps (16 to an SM) busy.  With fewer the serial walk over the digits shows; integer butterflies make it longer.  In two kernels / in
+// one, us, rotations and then multiplications with a rescale after them:
+//   doubles, 5 extension limbs: 5 limbs (10 with the extension) 57.5 / 57.6 and 79.8 / 76.6, 8 limbs 72.8 / 74.5 and 103.2 / 97.9, 9 limbs
+//   79.0 / 78.9 and 110.2 / 105.5, 11 limbs 96.9 / 93.9 and 130.0 / 120.8, 12 limbs 99.2 / 94.9 and 135.2 / 125.0; digits of two limbs, 10
+//   limbs 96.2 / 92.1 and 127.2 / 118.7; of one limb, 6 limbs 73.6 / 78.0, 9 limbs 113.8 / 109.6 and 145.0 / 146.3, 11 limbs
+//   143.6 / 133.4.  1.8 rows are 12 limbs and 5 extension limbs: from there on nothing loses;
+//   integers, 5 extension limbs: 12 limbs 124.8 / 130.7, 16 limbs 166.2 / 169.5, 20 limbs 192.5 / 195.5, 30 limbs 322.5 / 322.5, 40
+//   limbs 501.6 / 491.6; digits of one limb, 16 limbs 321 / 331, 20 limbs 472 / 482, 22 limbs 549.8 / 543.4, 24 limbs 643 / 636; of two
+//   limbs, 24 limbs 393 / 395, 28 limbs 511 / 499.
+// 32-bit words gain at every size (3 limbs 47.8 / 46.3, 51 limbs 199.8 / 183.4 when the row pass had sixteen words to a thread; 1 to 6
+// limbs are equal now).
 // Hoisted rotations transform the digits once for many keys and keep the two kernels.
 bool rows_with_inner(const cerium_keyswitch* ks, const void* cpoly, const void* evk, const void* add0, const void* add1) {
   const uintptr_t ptrs = (uintptr_t)cpoly | (uintptr_t)evk | (uintptr_t)add0 | (uintptr_t)add1;
   if (!ks->key_sums || ptrs % (4 * ks->ctx->word_bytes()) != 0) return false;
   if (ks->ctx->word_bits == 32) return true;
   const double rows_per_warp = 256.0 * ks->LK / (16.0 * ks->ctx->sm_count);
-  return rows_per_warp >= (ks->dnum < kSplitDigits ? 1.8 : ks->integer ? 2.5 : 1.4);
+  return rows_per_warp >= (ks->integer ? 2.5 : ks->dnum < kSplitDigits ? 1.8 : 1.4);
 }
 
 // Step 1: inverse transform of the local limbs of the switched polynomial into `dst`

@@ -113,10 +113,10 @@ def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     ks.close()
 
 
-@pytest.mark.parametrize("L,K,dnum,rows", [(16, 1, 16, False), (20, 5, 4, True)])
+@pytest.mark.parametrize("L,K,dnum,rows", [(16, 1, 16, False), (20, 5, 4, True), (16, 5, 4, False)])
 def test_plans_of_60_bit_primes(be, L, K, dnum, rows):
-    """Integer butterflies: the kernels stay apart where many digits meet few limbs (2.5 rows for each of 16 warps an SM), a row
-    keeps one warp, and the tensor product is a kernel of its own."""
+    """Integer butterflies: the kernels stay apart below 2.5 rows for each of 16 warps an SM, a row keeps one warp, and the tensor
+    product is a kernel of its own."""
     if be.name == "emu":
         L, K, dnum = (6, 1, 6) if dnum == L else (6, 2, 3)
     mods = params.ntt_primes_below(60, L + K, pc.LOGN)
