@@ -67,7 +67,8 @@ def test_key_switch(be, word_bits, L, K, dnum, rows, offset):
     one = (word_bits == 32 or offset == 0) and (rows or be.name == "emu")
     integers = word_bits == 64 and 2 * sum(prm.moduli[p] >> 50 > 0 for p in prm.q_idx + prm.p_idx) > L + K
     tensor = one and not integers and (word_bits == 32 or dnum < 12)
-    converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4  # ModUps in one launch or two
+    converted = int(dnum != L)     # every digit's conversion in one launch
+    assert be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) == 4 + converted
     switch = 9 + converted + (not one)
     assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), key, stream=st)) == switch
     assert be.launches(lambda st: ks.hmult(h.p(o), second, *inputs, key, 0, st)) == switch + (not tensor)
@@ -108,8 +109,8 @@ def test_integer_butterflies_of_small_primes(be, monkeypatch, bits):
     assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, prm.q_idx, prm.p_idx, 3, c1, evk)))
     ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0)
     assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, prm.q_idx, prm.p_idx, 3, c0, c1, c1, c0, evk)))
-    converted = be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4
-    assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == 9 + converted + (bits < 34)
+    assert be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) == 5
+    assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == 10 + (bits < 34)
     ks.close()
 
 
@@ -132,7 +133,8 @@ def test_plans_of_60_bit_primes(be, L, K, dnum, rows):
     assert np.array_equal(h.down(o), np.stack(h.orc.keyswitch(*modes, *shape, c1, evk)))
     ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0)
     assert np.array_equal(h.down(o), np.stack(h.orc.hmult_relin(*modes, False, *shape, c0, c1, c1, c0, evk)))
-    converted = 0 if dnum == L else be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) - 4
+    converted = int(dnum != L)
+    assert be.launches(lambda st: ks.hoisted_begin(h.p(d_c1), st)) == 4 + converted
     switch = 9 + converted + (not rows and be.name != "emu")
     assert be.launches(lambda st: ks.apply(h.p(o), second, h.p(d_c1), h.p(d_evk), stream=st)) == switch
     assert be.launches(lambda st: ks.hmult(h.p(o), second, h.p(d_c0), h.p(d_c1), h.p(d_c1), h.p(d_c0), h.p(d_evk), 0, st)) == switch + 1
