@@ -573,9 +573,19 @@ static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int c
     const size_t smem = bconv_mma_smem_bytes<W>(max_i);
     if (smem > 48 * 1024) CERIUM_CUDA(allow_smem(kfn, bconv_mma_smem_bytes<W>(kMmaMaxInputs)));
     const int warps_per_sm = prepare || (sizeof(W) == 4 && steps == kMmaRegSteps<W>) ? kMmaWarpsPerSm<W, 0, true> : kMmaWarpsPerSm<W, 0, false>;
-    const int per_sm = std::min(warps_per_sm / warps, (int)(kMmaSmemPerSm / (smem + 1024)));
-    const bool late = kN / kMmaStage * cnt * slices <= per_sm * ctx->sm_count;  // all CTAs are resident
-    CERIUM_LAUNCH(kfn, dim3(kN / kMmaStage, cnt, slices), 32 * warps, smem, stream, late, batch,
+    const int ctas = kN / kMmaStage * cnt * slices, per_sm = std::min(warps_per_sm / warps, (int)(kSplitSmem / (smem + 1024)));
+    const bool late = ctas <= per_sm * ctx->sm_count;  // all of them are resident
+    // Small CTAs that a kernel lets in at its start crowd on the SMs that have room first.  A grid that is resident at once asks for
+    // the shared memory that keeps an SM to its share of the CTAs, and leaves the rest to the next kernel.  After an addition, 32-bit
+    // words: 1 input to 17 outputs 9.9 -> 5.0 us, 16 to 24 10.7 -> 6.1; called alone, 20 to 35 8.0 -> 6.4, 64-bit words 12 to 24 20.2 -> 16.7;
+    // rotations of 9 limbs of 32-bit words 46.8 -> 45.6, of 24 limbs in digits of 12 with 15 extension limbs 210 -> 199.  Not one
+    // warp of 64-bit words, which gains nothing and takes room from the next kernel (inverse transform, 5 to 5, forward 25.2 -> 26.8).
+    size_t room = smem;
+    if (late && (sizeof(W) == 4 || warps > 1)) {
+      const size_t share = (size_t)((ctas + ctx->sm_count - 1) / ctx->sm_count);
+      room = std::max(smem, std::min(kSplitSmem / (share + 1), (size_t)48 * 1024));
+    }
+    CERIUM_LAUNCH(kfn, dim3(kN / kMmaStage, cnt, slices), 32 * warps, room, stream, late, batch,
                   static_cast<const PrimeConst<W>*>(ctx->d_pcs));
     first += cnt;
   }

@@ -44,7 +44,6 @@ constexpr int kMmaStage = 128;                    // coefficients of a CTA
 template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
-constexpr size_t kMmaSmemPerSm = 220 * 1024;      // shared memory for the CTAs of an SM, 1 KB of each the system's
 template <typename W>
 constexpr int kMmaRegSteps = sizeof(W) == 8 ? 2 : 4;  // most steps whose fragments a warp keeps in registers
 constexpr int kMmaMaxBatch = 24;                  // conversions per launch (descriptors travel as parameters)

@@ -81,6 +81,7 @@ inline cudaError_t allow_smem(Kernel kfn, size_t bytes) {
   });
 }
 
+constexpr size_t kSplitSmem = 164 * 1024;  // shared memory of an SM, as every kernel asks for it (kCarveoutPercent)
 // Kernel launch through a function pointer (template-ids with commas stay out of the macro).
 #if defined(CERIUM_EMU)
 #define CERIUM_LAUNCH(kfn, grid, block, smem, stream, ...) \
