@@ -514,10 +514,16 @@ int create_bconv(cerium_context* ctx, cerium_bconv** out, int mode, const uint32
 }
 
 // Kernel of a batch: fragments in registers up to the number of steps they fit for, then the way outputs are finished.  half: the
-// inputs end in the first half of the last step.
+// inputs end in the first half of the last step.  more: 24 warps to an SM and not 16, for words of 64 bits that the kernel
+// prepares itself and reads its fragments for: where 16 do not hold the grid at once (9 inputs to 35 outputs 34.0 -> 21.7 us, 24
+// to 35 56.9 -> 40.2); with fewer CTAs 128 registers are better (24 inputs to 13 outputs 27.3 / 29.7, 32 to 24 34.4 / 40.4).
 template <typename W, bool kPrepare>
-static auto bconv_mma_pick(int steps, int finish, bool half) -> decltype(&bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>) {
-  if (sizeof(W) == 8 && finish == kMmaBig) return bconv_mma_kernel<W, 0, sizeof(W) == 8 ? kMmaBig : kMmaGeneral, kPrepare>;
+static auto bconv_mma_pick(int steps, int finish, bool half, bool more) -> decltype(&bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare>) {
+  if constexpr (sizeof(W) == 8) {
+    if (kPrepare && more && steps > kMmaRegSteps<W>)
+      return finish == kMmaBig ? bconv_mma_kernel<W, 0, kMmaBig, kPrepare, false, 24> : bconv_mma_kernel<W, 0, kMmaGeneral, kPrepare, false, 24>;
+    if (finish == kMmaBig) return bconv_mma_kernel<W, 0, kMmaBig, kPrepare>;
+  }
   if (finish <= kMmaLazyAdd && !kPrepare) {
     const bool add = finish == kMmaLazyAdd;
     if (steps == 1 && half) return add ? bconv_mma_kernel<W, 1, kMmaLazyAdd, false, true> : bconv_mma_kernel<W, 1, kMmaLazy, false, true>;
@@ -567,14 +573,17 @@ static int launch_bconv_words(cerium_context* ctx, const BconvCall* calls, int c
     }
     const int finish = sizeof(W) == 8 && max_i > kMmaPairInputs ? kMmaBig : !lazy ? kMmaGeneral : add ? kMmaLazyAdd : kMmaLazy;
     const bool half = max_i * (int)sizeof(W) <= 32 * steps - 16;
-    auto kfn = prepare ? bconv_mma_pick<W, true>(steps, finish, half) : bconv_mma_pick<W, false>(steps, finish, half);
     // a warp per group of outputs, at most 8 to a CTA
     const int slices = (max_groups + kMmaMaxWarps - 1) / kMmaMaxWarps, warps = (max_groups + slices - 1) / slices;
     const size_t smem = bconv_mma_smem_bytes<W>(max_i);
+    const int ctas = kN / kMmaStage * cnt * slices;
+    const auto resident = [&](int warps_per_sm) {
+      return ctas <= std::min(warps_per_sm / warps, (int)(kSplitSmem / (smem + 1024))) * ctx->sm_count;
+    };
+    bool late = resident(prepare || (sizeof(W) == 4 && steps == kMmaRegSteps<W>) ? kMmaWarpsPerSm<W, 0, true> : kMmaWarpsPerSm<W, 0, false>);
+    auto kfn = prepare ? bconv_mma_pick<W, true>(steps, finish, half, !late) : bconv_mma_pick<W, false>(steps, finish, half, false);
+    if (prepare && sizeof(W) == 8 && steps > kMmaRegSteps<W>) late = resident(kMmaWarpsPerSm<W, 0, false>);
     if (smem > 48 * 1024) CERIUM_CUDA(allow_smem(kfn, bconv_mma_smem_bytes<W>(kMmaMaxInputs)));
-    const int warps_per_sm = prepare || (sizeof(W) == 4 && steps == kMmaRegSteps<W>) ? kMmaWarpsPerSm<W, 0, true> : kMmaWarpsPerSm<W, 0, false>;
-    const int ctas = kN / kMmaStage * cnt * slices, per_sm = std::min(warps_per_sm / warps, (int)(kSplitSmem / (smem + 1024)));
-    const bool late = ctas <= per_sm * ctx->sm_count;  // all of them are resident
     // Small CTAs that a kernel lets in at its start crowd on the SMs that have room first.  A grid that is resident at once asks for
     // the shared memory that keeps an SM to its share of the CTAs, and leaves the rest to the next kernel.  After an addition, 32-bit
     // words: 1 input to 17 outputs 9.9 -> 5.0 us, 16 to 24 10.7 -> 6.1; called alone, 20 to 35 8.0 -> 6.4, 64-bit words 12 to 24 20.2 -> 16.7;

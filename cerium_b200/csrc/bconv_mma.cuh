@@ -366,8 +366,8 @@ __device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const 
 
 // grid = (N / kMmaStage, conversions, ceil(groups / warps)), block = 32 * warps, dynamic smem = bconv_mma_smem_bytes of the largest
 // number of inputs.  late_next: see grid_dependency_launch.
-template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf = false>
-__global__ void __launch_bounds__(32 * kMmaMaxWarps, kMmaWarpsPerSm<W, kSteps, kPrepare> / kMmaMaxWarps)
+template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf = false, int kWarpsPerSm = kMmaWarpsPerSm<W, kSteps, kPrepare>>
+__global__ void __launch_bounds__(32 * kMmaMaxWarps, kWarpsPerSm / kMmaMaxWarps)
     bconv_mma_kernel(const bool late_next, const BconvMmaBatch<W> batch, const PrimeConst<W>* __restrict__ pcs) {
   CERIUM_DYN_SMEM(smem);
   const BconvMmaDesc<W>& d = batch.d[blockIdx.y];

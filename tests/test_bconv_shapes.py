@@ -18,6 +18,7 @@ def be(request):
 @pytest.mark.parametrize("word_bits,n_in,n_out,mode", [
     (64, 1, 1, _capi.BCONV_LAZY), (64, 4, 8, _capi.BCONV_EXACT), (64, 5, 9, _capi.BCONV_LAZY), (64, 9, 17, _capi.BCONV_EXACT),
     (64, 33, 3, _capi.BCONV_LAZY), (64, 64, 6, _capi.BCONV_LAZY), (64, 8, 16, _capi.BCONV_LAZY), (64, 32, 7, _capi.BCONV_EXACT),
+    (64, 9, 35, _capi.BCONV_EXACT), (64, 33, 33, _capi.BCONV_EXACT),       # more warps than an SM holds at 128 registers
     (32, 1, 1, _capi.BCONV_LAZY), (32, 8, 9, _capi.BCONV_EXACT), (32, 17, 16, _capi.BCONV_LAZY), (32, 21, 25, _capi.BCONV_EXACT),
     (32, 32, 17, _capi.BCONV_LAZY), (32, 33, 8, _capi.BCONV_EXACT),
 ])
