@@ -47,9 +47,9 @@ from cerium_b200 import params  # noqa: E402
 LOGN = 16
 N = 1 << LOGN
 # dram__bytes_read.sum + dram__bytes_write.sum of the forward-NTT launch pair by number of u64 limbs, repeated on the same
-# buffers with the caches left alone (profiles/key_switch_u64_traffic_and_pipes.md).  Measured, not scaled: the second
+# buffers with the caches left alone (the forward pairs under profiles/).  Measured, not scaled: the second
 # pass starts where the first ended, so the share that L2 serves depends on the size.
-NTT_PAIR_DRAM_BYTES = {245: 361.8e6, 384: 745.1e6, 576: 1015.7e6}
+NTT_PAIR_DRAM_BYTES = {245: 360.9e6, 384: 743.1e6, 576: 1011.8e6}
 # what the CPU figure is: the checker, not a tuned evaluator
 PORT_QUALITY = ("unoptimised checker: plain-C restatement with a 128-bit remainder in every modular product outside "
                 "the transforms; a Barrett/Shoup CPU evaluator would be several times faster")

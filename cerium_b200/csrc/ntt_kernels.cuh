@@ -710,7 +710,8 @@ struct LazyStoreEpilogue {
 // SuD tail: out = (minuend - NTT(in)) * factor[b] [+ addend]   (all mod q).
 // minuend / addend are stacks of limbs: entry b at base + b * stride; entries b >= split belong
 // to a second polynomial and use minuend2 / addend2 at (b - split) * stride.
-// The row pass with it is bound by its reads (120 MB through DRAM for 70 limbs) and needs all 32 warps of an SM: operands copied to
+// The row pass with it is bound by its reads (120 MB through DRAM for 70 limbs) and needs all 32 warps of an SM, at whose 64 registers
+// it spills 140 bytes a thread (64-bit words; both polynomials, addend and scatter are in one kernel): operands copied to
 // shared memory leave 20 (rotation of 35 limbs 275.5 -> 281 us).  Doubles are finished as doubles (integer Shoup product: 35 limbs
 // 275.5 -> 274.0, 12 limbs 99.4 -> 98.6, plaintext product with rescale 32.0 -> 31.3).
 template <typename W>
