@@ -51,7 +51,7 @@ static int check_stack(const void* p, size_t stride_words, size_t word_bytes, co
 // The passes of `limbs` limbs, in small tiles where those of the usual size would leave SMs without a full set of CTAs.
 template <typename W>
 static bool small_batch(const cerium_context* ctx, int limbs) { return limbs * (256 / kRowsPerCta) <= kSmallBatchPerSm<W> * ctx->sm_count; }
-// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen; us with eight / sixteen.
+// Limbs up to which a pass takes eight words to a thread (ntt_radix8.cuh) and not sixteen, on 148 SMs; us with eight / sixteen.
 //   Columns: beyond the lines the second barrier and the narrow tiles cost more than the shorter chain gives.
 //     64-bit words inverse: 23 limbs alone 14.5 / 15.0, 24 limbs 15.9 / 15.5, 40 limbs 22.8 / 22.1, rotation of 24 limbs 167.9 / 167.4,
 //     of 35 limbs 271.6 / 270.7.  Integer butterflies alike: 23 limbs 21.9 / 23.0, 24 limbs 23.9 / 23.3.

@@ -22,7 +22,8 @@
 // conversions 5 -> 35 of 64-bit words), so many small CTAs that are in different phases do better than the walk over five to
 // ten stages through three buffers that was here before, whose warps met at a barrier for each stage and whose grid ended in a part of a
 // round: rotation of 35 limbs 275.1 -> 267.6 us, of 51 limbs of 32-bit words 173.3 -> 165.4, multiplication of 30 limbs 242.6 ->
-// 232.9, 12 limbs 99.0 / 98.4 (with the next kernel let in late, see grid_dependency_launch).  64 coefficients: 35 limbs 272.0, 256: 268.8; 64 registers instead of 80: 267.5.
+// 232.9, 12 limbs 99.0 / 98.4 (with the next kernel let in late, see grid_dependency_launch).  64 coefficients: 35 limbs 272.0,
+// 256: 268.8; 64 registers instead of 80: 267.5.
 // Where the inputs end in the first 16 bytes of a step the product is taken for those alone (35 limbs 278.7 -> 275.1).
 // Measured before: warps that read the words from global memory themselves waited for them half of the time, and 16 outputs to
 // a warp took 152 registers (56 us against 48).
@@ -44,8 +45,9 @@ constexpr int kMmaStage = 128;                    // coefficients of a CTA
 template <typename W>
 constexpr int kMmaRows = sizeof(W) == 8 ? 8 : 16;  // outputs of a group
 constexpr int kMmaTile = 8;                       // coefficients of a tile
+// Most steps whose fragments a warp keeps in registers.
 template <typename W>
-constexpr int kMmaRegSteps = sizeof(W) == 8 ? 2 : 4;  // most steps whose fragments a warp keeps in registers
+constexpr int kMmaRegSteps = sizeof(W) == 8 ? 2 : 4;
 constexpr int kMmaMaxBatch = 24;                  // conversions per launch (descriptors travel as parameters)
 constexpr int kMmaMaxInputs = 64;                 // of a conversion
 constexpr int kMmaPairInputs = 32;                // 64-bit inputs whose plane pairs c + 2^8 c' stay below 2^32:
@@ -264,7 +266,8 @@ constexpr int kMmaWarpsPerSm = (sizeof(W) == 4 && kSteps == 4) || kPrepare ? 16 
 // has at most 8 outputs, its fragments hold two planes.  kSteps = 0: any number of steps, fragments read for every tile.  kHalf: no
 // input has more than 16 bytes in the last step.
 template <typename W, int kSteps, int kFinish, bool kPrepare, bool kHalf, bool kPair>
-__device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, unsigned char* buf, const PrimeConst<W>* __restrict__ pcs, bool late_next) {
+__device__ __forceinline__ void bconv_mma_group(const BconvMmaDesc<W>& d, const uint4* frag, int j0, int first, unsigned char* buf,
+                                                const PrimeConst<W>* __restrict__ pcs, bool late_next) {
   constexpr int kPlanes = sizeof(W);
   constexpr int kFrags = kPair ? kPlanes / 2 : kPlanes;
   constexpr int kRows = kPair ? 1 : 2;             // outputs of a thread

@@ -41,7 +41,8 @@ namespace cerium {
 //   Forward columns with eight words: the same line.  Late up to 37 limbs, whatever an SM holds, lost 3 to 5 % from 19 limbs on (32 limbs
 //   alone 19.0 -> 18.3, a division 22.7 -> 21.8, rotation of 10 limbs 86.0 -> 84.5).
 //   Base conversion: the same line.  After its wait: rotation of 9 limbs of 32-bit words 47.1 -> 47.5, of 4 limbs with 4 extension limbs
-//   28.8 -> 32.4; late for every grid: 30 limbs 211.9 -> 213.5, 35 limbs 265.5 -> 266.7.
+//   28.8 -> 32.4; late for every grid: 30 limbs 211.9 -> 213.5, 35 limbs 265.5 -> 266.7.  Its CTAs keep to their share of an SM besides
+//   (launch_bconv_words).
 //   Inverse columns with eight words: late in grids of up to two rounds, small CTAs of a conversion come after them (at the start:
 //   rotation of 9 limbs of 32-bit words 47.3 -> 52.7; late only where they are resident: 51.5).
 __device__ __forceinline__ void grid_dependency_launch() {

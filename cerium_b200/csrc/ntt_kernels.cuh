@@ -55,8 +55,9 @@ constexpr int kSmallBatchPerSm = sizeof(W) == 8 ? 7 : 8;
 // prime; entry = bit-reversed table[((4096 + 16 h + u) << t) + g].
 constexpr int kRowTwPerPrime = 256 * 15 * 16;
 // Limbs per launch: the largest multiple of 64 with which the parameters of every kernel stay within 4 KB (the asserts in the
-// forward passes, whose loaders and epilogues are the long ones).  A call of more goes on in launches of that many: 512 loses 3 to 4 % on 513 to 576 limbs (576 forward 262.9 us
-// against 255.2); shared out evenly, 577 limbs of 32-bit words 155.8 -> 159.7, 625 of 64-bit words inverse 291 -> 307.
+// forward passes, whose loaders and epilogues are the long ones).  A call of more goes on in launches of that many.  512 loses 3 to
+// 4 % on 513 to 576 limbs (576 forward 262.9 us against 255.2); shared out evenly, 577 limbs of 32-bit words 155.8 -> 159.7, 625 of
+// 64-bit words inverse 291 -> 307.
 constexpr int kMaxBatch = 576;
 constexpr size_t kMaxParameters = 4096;
 
